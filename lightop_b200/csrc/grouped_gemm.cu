@@ -16,37 +16,36 @@
 // time: weight tiles are loaded with an evict-first L2 policy unless the chunk table says that
 // another chunk of the expert follows.  Persistent CTAs take items round-robin.
 //
-// Warp roles in a CTA of 20 or 24 warps:
-//   warp 0      : two TMA producers on two lanes with their own control flow: lane 0 streams
-//                 the weight tiles (HBM) into ring w[], lane 16 the chunk's token rows (L2) into
-//                 ring a[].  Token rows are read from an expert-sorted copy of the activations,
-//                 so a chunk is a run of consecutive rows and one tiled TMA load fetches it.
-//   warps 1, 3  : MMA issuers, alternating K-block steps (warp 1 alone in the per-channel
-//                 mode).  Three lanes of an issuer each follow one barrier ring (weights,
-//                 activations, free partial buffer), poll in the same instruction and agree by
-//                 a vote; lane 0 then issues the four MMAs of the step and one commit to done[].
-//                 Warp 1 owns the tensor-memory allocation.
-//   warp 2      : scale producer: the token scales of the K block (fetched two steps ahead)
-//                 times the weight-block scale -> per-step table in shared memory
-//   warps 4..   : promotion / epilogue, four warps (one per lane quarter of tensor memory) per
-//                 column group; the chunk's tokens are dealt to the groups in pieces of 16.  A
-//                 thread keeps the fp32 running sums of its output column for its pieces in
-//                 registers: per K block it loads 16 int32 partials, converts and does one
-//                 fused multiply-add per value with the scale product.
-// Pipelines: the two shared-memory rings (full_w / full_a, refilled when done[] says the MMAs
-// that read a slot have completed) and NBUF tensor-memory partial buffers (done[] as "full",
-// tmem_empty as "free") between the issuers and the promotion warps.
+// Warp roles in a CTA of 16 warps (block-scaled modes):
+//   warp 0       : weight producer: streams the weight tiles (HBM) into ring w[] by TMA
+//   warp 1       : MMA issuer.  Two lanes follow the two barriers of a step (operands ready, partial buffer free), poll in
+//                  the same instruction and agree by a vote; one elected lane issues the four MMAs of the step and one
+//                  commit to done[].  Owns the tensor-memory allocation.
+//   warp 2       : scale producer: token scales times weight-block scale, tables of four steps at a time
+//   warp 3       : activation producer: the chunk's token rows (L2) into ring a[] by TMA.  Token rows are read from an
+//                  expert-sorted copy of the activations, so a chunk is a run of consecutive rows.
+//   warps 4..11  : promotion, four warps (one per lane quarter of tensor memory) per column group; the chunk's tokens are
+//                  dealt to the two groups in pieces of 16.  The warps keep the fp32 running sums of their columns in
+//                  registers: per K block they load the int32 partials, convert and do one fused multiply-add per value.
+//   warps 12..15 : output: carry the finished tile from shared memory to global memory while the promotion warps are
+//                  already on the next item
+// Pipelines: the two shared-memory rings, refilled when done[] says the MMAs that read a slot have completed; NBUF
+// tensor-memory partial buffers between the issuer and the promotion warps (done[] as "full", consumed[] as "free"); the ring
+// of scale tables; and the staging tile between the promotion and the output warps.
 //
-// Epilogues run out of the register sums through a staging tile in shared memory, so that the
-// global stores are whole rows: gate_up keeps bf16(gate) there during the up pass, then forms
-// SiLU(gate)*up, the 128-wide group maximum and the int8 row; down stages bf16 rows and applies
-// the routed weight on the way out.
+// Epilogues go through the staging tile in shared memory, so that the global stores are whole rows: gate_up keeps
+// bf16(gate) there during the up pass, then SiLU(gate)*up in its place; the output warps take the 128-wide group maximum and
+// write the int8 row.  down stages bf16 rows, and the output warps apply the routed weight on the way out.
 //
-// Per-channel mode (one scale per token and one per output channel instead of 128x128 blocks) uses
-// the same pipeline without the promotion: a tensor-memory buffer is the int32 accumulator of a whole
-// item, summed over every K block by the tensor core, and the promotion warps only run an epilogue
-// (int32 -> fp32, times token scale, times channel scale) while the MMAs of the next items fill the
-// other buffers.  The scale-producer warp idles in that mode.
+// What it measured (DeepSeek-V3 shape, one layer, sustained at the 1000 W power cap; before = a per-step hand-over of scales
+// through the issuer, a thread on one channel and 16 tokens, two issuer warps and the output in the promotion warps):
+// 64 tokens 1764 -> 1470 us, 777 tokens 2290 -> 1880 us, 4096 tokens 3850 -> 3340 us.  The board is at its power cap in all of
+// these (SM clock 1.35 to 1.5 GHz), so what a change saves in cycles comes back as time only in part.
+//
+// Per-channel mode (one scale per token and one per output channel instead of 128x128 blocks) uses the same feed without the
+// promotion: a tensor-memory buffer is the int32 accumulator of a whole item, summed over every K block by the tensor core, and
+// 16 or 20 warps run an epilogue (int32 -> fp32, times token scale, times channel scale) while the MMAs of the next items fill
+// the other buffers.  The scale producer idles and there are no output warps in that mode.
 //
 // Every wait is bounded: after about a second a waiter records a timeout in the
 // status word, raises a CTA-wide abort flag, and all roles fall through to the
@@ -57,42 +56,31 @@
 #include <mutex>
 #include <map>
 #include <tuple>
+#include <type_traits>
 
 namespace lo {
 namespace {
 
-// Build parameters (the defaults are the measured best; the others exist so that a variant can be built and compared).
-// Column groups of the instantiations for chunks above 64 rows: five keep a group at two pieces of 16 tokens.
-#ifndef LO_NCG_WIDE
-#define LO_NCG_WIDE 5
-#endif
-// Interval between two polls of a barrier, in nanoseconds, by role.  A polling warp competes for issue slots with the
-// promotion warps that share its scheduler; longer intervals for the waiters with slack measured no different.
-#ifndef LO_SLEEP_PRODUCER
-#define LO_SLEEP_PRODUCER 128u
-#endif
-#ifndef LO_SLEEP_SCALE
-#define LO_SLEEP_SCALE 128u
-#endif
-#ifndef LO_SLEEP_MMA
-#define LO_SLEEP_MMA 20u
-#endif
-#ifndef LO_SLEEP_PROMO
-#define LO_SLEEP_PROMO 32u
-#endif
-#ifndef LO_SLEEP_PROMO_SLACK
-#define LO_SLEEP_PROMO_SLACK 32u
-#endif
+// Interval between two polls of a barrier, in nanoseconds, by role.  (Intervals from none to 2 us measured no different, in time
+// or in power.)
+constexpr uint32_t LO_SLEEP_PRODUCER = 128u, LO_SLEEP_SCALE = 128u, LO_SLEEP_MMA = 20u, LO_SLEEP_PROMO = 32u, LO_SLEEP_OUT = 256u;
 
 constexpr int TILE_N = 128;      // weight rows per accumulator (MMA M)
 constexpr int TILE_K = 128;      // int8 elements (= bytes) per K block
 constexpr int T_MAX = 128;       // default bound of the rows of a chunk
 constexpr int T_WIDE = 160;      // widest block-scaled chunk: three partial buffers of 160 columns fill tensor memory
 constexpr int FIRST_EPI_WARP = 4;
-constexpr int MAX_NCG = 5;
+constexpr int OUT_WARPS = 4;     // block-scaled modes: warps that carry the finished tile to global memory
+// Register budgets of the wide block-scaled instantiations, by role (setmaxnreg): 16 warps start with 128 registers each;
+// the feeding and the output warps give up some, the promotion warps (80 sums and three sets of 16 partials a thread) take
+// them: 80 + 2 x 184 + 64 = 512, the 512 registers that a lane of the four warp groups has.  (168 for the promotion warps
+// spilled at 160 rows.)
+constexpr int REGS_FEED = 80, REGS_PROMO = 184, REGS_OUT = 64;
+static_assert(REGS_FEED + 2 * REGS_PROMO + REGS_OUT <= 4 * 128, "the register split must not exceed what the block is launched with");
 constexpr int W_TILE_BYTES = TILE_N * TILE_K;   // 16 KiB
-constexpr int OUT_ROW_BYTES = TILE_N * 2;       // one token's 128 outputs as bf16 in the staging tile
+constexpr int OUT_ROW_BYTES = TILE_N * 2 + 16;  // one token's 128 outputs as bf16 in the staging tile; 16 bytes of padding: 8 rows = 32 banks
 constexpr uint32_t TMEM_COLS = 512;
+constexpr int SC_STEPS = 4, SC_BATCHES = 3;     // scale-product tables: K-block steps per batch, batches in the ring
 constexpr int ND = 16;                          // completion ring, see Smem::done
 constexpr int SMEM_LIMIT = 227 * 1024;          // dynamic shared memory a CTA can be given on this part
 
@@ -102,32 +90,31 @@ constexpr int SMEM_LIMIT = 227 * 1024;          // dynamic shared memory a CTA c
 template <int MODE, int A_ROWS> struct Cfg {
   // gate_up: an item is two passes over K on the same chunk, first the gate tile, then the up tile
   static constexpr int PHASES = MODE == GEMM_GATE_UP ? 2 : 1;
-  // Column groups: the chunk's tokens are dealt, in pieces of 16, to this many sets of four promotion warps (one
-  // warp per lane quarter of tensor memory).  Five groups keep a group at two pieces for chunks of up to 160
-  // tokens (the group with the most pieces paces the K loop); the CTA then has 24 warps and 80 registers per
-  // thread.  Narrow chunks use four groups: more warps would only add idle ones that have to keep step.
-  static constexpr int NCG = A_ROWS > 64 ? LO_NCG_WIDE : 4;
+  // Column groups: the chunk's tokens are dealt, in pieces of 16, to this many sets of four warps (one warp per lane quarter
+  // of tensor memory).  Block-scaled: two groups of up to five pieces, so that what a step costs a warp besides its pieces
+  // (barriers, addresses: as much as two pieces) is paid by eight warps, not twenty.
+  static constexpr int NCG = MODE == GEMM_CHANNEL ? (A_ROWS > 64 ? 5 : 4) : 2;
   static constexpr int EPI_WARPS = 4 * NCG;
-  static constexpr int NUM_THREADS = (FIRST_EPI_WARP + EPI_WARPS) * 32;
+  static constexpr int NUM_THREADS = (FIRST_EPI_WARP + EPI_WARPS + (MODE == GEMM_CHANNEL ? 0 : OUT_WARPS)) * 32;
+  static constexpr bool SPLIT_REGS = MODE != GEMM_CHANNEL && A_ROWS > 64;
+  static_assert(!SPLIT_REGS || NUM_THREADS == 512, "the register split is made for four warp groups");
   static constexpr int A_TILE_BYTES = A_ROWS * TILE_K;
   // Two rings.  Activation tiles come from L2 (the chunk's rows are read by every output tile of the expert): a
   // slot is refilled only after the MMAs that read it have completed, so the ring has to cover the load latency
   // plus the MMA queue, four K blocks at least.  Weight tiles come from HBM and get the shared memory that is left.
   static constexpr int NA_FIT = (64 * 1024) / A_TILE_BYTES;
-  static constexpr int NA = NA_FIT < 4 ? 4 : (NA_FIT > 10 ? 10 : NA_FIT);
-  // staging tile of the epilogue: [A_ROWS][128] bf16 (gate_up keeps the gate values there during the up pass)
+  static constexpr int NA = NA_FIT < 4 ? 4 : (NA_FIT > 8 ? 8 : NA_FIT);
+  // staging tile of the epilogue: A_ROWS rows of 128 bf16 (gate_up keeps the gate values there during the up pass)
   static constexpr int STAGING_BYTES = MODE == GEMM_CHANNEL ? 0 : A_ROWS * OUT_ROW_BYTES;
-  static constexpr int FIXED_BYTES = 14 * 1024;   // scale tables, maxima, barriers, alignment slack (checked below)
+  static constexpr int FIXED_BYTES = 10 * 1024;   // scale tables, barriers, alignment slack (checked below)
   static constexpr int NW_FIT = (SMEM_LIMIT - FIXED_BYTES - STAGING_BYTES - NA * A_TILE_BYTES) / W_TILE_BYTES;
   static constexpr int NW = NW_FIT > 12 ? 12 : NW_FIT;
   // tensor memory is cut into partial buffers of A_ROWS columns, one int32 accumulator each (at most 8 are used):
   // the partial of one 128-wide K block in the block-scaled modes (the fp32 running sums live in the registers of
   // the promotion warps), the accumulator of a whole item in the per-channel mode
   static constexpr int NBUF = (int)TMEM_COLS / A_ROWS > 8 ? 8 : (int)TMEM_COLS / A_ROWS;
-  // Ring of scale-product tables.  A slot written for K-block step i was last read at step
-  // i - SC_SLOTS; the producer of step i has seen the MMAs of step i - NW complete, which were
-  // issued after the promotion of step i - NW - NBUF finished, so NW + NBUF slots suffice.
-  static constexpr int SC_SLOTS = MODE == GEMM_CHANNEL ? 1 : NW + NBUF;
+  // Ring of scale-product tables: SC_BATCHES batches of SC_STEPS K-block steps each
+  static constexpr int SC_SLOTS = MODE == GEMM_CHANNEL ? 1 : SC_BATCHES * SC_STEPS;
 };
 
 template <int MODE, int A_ROWS> struct Smem {
@@ -135,22 +122,23 @@ template <int MODE, int A_ROWS> struct Smem {
   // operand tiles first: each is a multiple of 1024 bytes, base is 1024-aligned
   uint8_t w[C::NW][W_TILE_BYTES];
   uint8_t a[C::NA][C::A_TILE_BYTES];
-  // epilogue staging, row = token (column of the chunk), 256 bytes per row
-  uint8_t staging[C::STAGING_BYTES > 0 ? C::STAGING_BYTES : 16];
-  float sc[C::SC_SLOTS][A_ROWS];           // token scale x weight-block scale, ring indexed by the K-block counter
-  // gate_up epilogue: |act| maxima per (item parity, lane quarter, token); a stub in the other modes
-  uint32_t amax[MODE == GEMM_GATE_UP ? 2 : 1][4][MODE == GEMM_GATE_UP ? A_ROWS : 1];
-  uint64_t full_w[C::NW];
-  uint64_t full_a[C::NA];
-  // done[u % ND]: the MMAs of K-block step u have completed.  One tcgen05.commit per step serves everybody who
-  // waits for that event: the producers (a weight slot is free NW steps later, an activation slot NA steps later),
-  // the scale warp, and in the block-scaled modes the promotion warps (the partial of step u is in its buffer).
-  // ND exceeds every ring depth, so a waiter cannot be overtaken by the barrier's next phase.
+  // epilogue staging, row = token (column of the chunk)
+  alignas(16) uint8_t staging[C::STAGING_BYTES > 0 ? C::STAGING_BYTES : 16];
+  alignas(16) float sc[C::SC_SLOTS][A_ROWS];   // token scale x weight-block scale, see scale_place()
+  // Barriers of K-block step u, each a ring of ND indexed by u % ND whatever the depths of the operand rings: position and
+  // phase follow from the step number alone.  ND exceeds every ring depth, so that a waiter cannot be overtaken by a
+  // barrier's next phase.
+  uint64_t ready[ND];                      // weights and activations of the step are in place
+  // The MMAs of the step have completed.  One tcgen05.commit per step serves everybody who waits for that event: the
+  // producers (a weight slot is free NW steps later, an activation slot NA steps later) and in the block-scaled modes the
+  // promotion warps (the partial of the step is in its buffer).
   uint64_t done[ND];
+  uint64_t consumed[ND];                   // block-scaled modes: the partial of the step has been read, its buffer is free
+  uint64_t scales[SC_BATCHES];             // block-scaled modes: the batch's scale products are in place
   uint64_t tmem_full[C::NBUF];             // per-channel mode: the accumulator of an item is complete
-  uint64_t tmem_empty[C::NBUF];
-  uint64_t esync[MAX_NCG];                 // rendezvous of the 128 epilogue threads of a column group
-  uint64_t isync;                          // rendezvous of all promotion warps, once per item
+  uint64_t tmem_empty[C::NBUF];            // per-channel mode: the accumulator has been read
+  uint64_t stg_full;                       // the item's tile is in the staging buffer (promotion warps -> output warps)
+  uint64_t stg_free;                       // its rows have been read (output warps -> promotion warps)
   uint32_t tmem_base;
   volatile int abort_flag;
 };
@@ -291,6 +279,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
+// One lane of a converged warp, always the same one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
+
 // Shared-memory matrix descriptor: K-major operand, rows of 128 bytes, 128-byte
 // swizzle, 8-row groups 1024 bytes apart (tile base 1024-aligned).
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
@@ -314,13 +309,18 @@ __device__ __forceinline__ uint32_t make_idesc(uint32_t n) {
   return d;
 }
 
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// The descriptors' upper halves are the same for every operand; the lower ones hold the start address.
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint32_t adesc_lo, uint32_t bdesc_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %4, p;\n\t}"
+      ::"r"(tmem_d), "r"(adesc_lo), "r"(bdesc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+__device__ __forceinline__ void umma_commit_addr(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -336,24 +336,70 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// One promotion step on N (8 or 16) tokens of this thread's output channel: acc = fma(float(raw), scale product, acc).
-// The 128-long int8 dot is below 2^21 in magnitude, so the conversion is exact; one rounding per K block.
-// `sc_addr` is the shared-memory address of the N scale products.
-// Plain fp32 multiply-adds: the packed f32x2 form needs its operands in aligned register pairs, and assembling the
-// pairs from the converted values cost more than the packed instruction saved (measured: -6 % on the gate_up launch).
-template <int N>
-__device__ __forceinline__ void promote(const uint32_t *raw, float *acc, uint32_t sc_addr) {
+// Wait for this thread's outstanding tensor-memory loads; the registers are operands so that nothing that uses
+// them can be scheduled ahead of the wait.
+__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :: "memory");
+}
+// Partial sums in the layout of an MMA accumulator fragment, 16 registers a thread at a time ("unit"):
+// two pieces (32 columns) of one half of the warp's channels (16 lanes, taddr points at the first of them): register 4c + r is
+// channel 8(r >> 1) + lane / 4, token 8c + 2(lane % 4) + (r & 1) ...
+__device__ __forceinline__ void tmem_ld_two(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
+}
+// ... or one piece (16 columns) of both halves: register 8h + 4c + r is channel 16h + 8(r >> 1) + lane / 4, token as above.
+__device__ __forceinline__ void tmem_ld_one(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr + (16u << 16)) : "memory");
+}
+// Place of token t of a piece in its 16-entry row of the scale table: the four scales a thread needs of a piece are one
+// 16-byte load.
+__device__ __forceinline__ int scale_place(int t) { return (t & ~15) | ((t >> 1) & 3) << 2 | ((t >> 3) & 1) << 1 | (t & 1); }
+
+// acc = fma(float(raw), scale product, acc) on eight values, one half of a piece: s = the scale products of tokens 2i, 2i + 1,
+// 8 + 2i, 9 + 2i, i = lane % 4.  The 128-long int8 dot is below 2^21 in magnitude, so the conversion is exact; one rounding per
+// K block.  Two tokens of one channel at a time: the packed multiply-add takes the registers in pairs as they come.
+__device__ __forceinline__ void promote8(float *acc, const uint32_t *raw, const float (&s)[4]) {
 #pragma unroll
-  for (int j4 = 0; j4 < N / 4; ++j4) {
-    float s0, s1, s2, s3;               // scale products of four tokens
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s0), "=f"(s1), "=f"(s2), "=f"(s3) : "r"(sc_addr + 16u * j4));
-    acc[j4 * 4 + 0] = __fmaf_rn(__int2float_rn((int32_t)raw[j4 * 4 + 0]), s0, acc[j4 * 4 + 0]);
-    acc[j4 * 4 + 1] = __fmaf_rn(__int2float_rn((int32_t)raw[j4 * 4 + 1]), s1, acc[j4 * 4 + 1]);
-    acc[j4 * 4 + 2] = __fmaf_rn(__int2float_rn((int32_t)raw[j4 * 4 + 2]), s2, acc[j4 * 4 + 2]);
-    acc[j4 * 4 + 3] = __fmaf_rn(__int2float_rn((int32_t)raw[j4 * 4 + 3]), s3, acc[j4 * 4 + 3]);
+  for (int j = 0; j < 8; j += 2) {
+    const float f0 = __int2float_rn((int32_t)raw[j]), f1 = __int2float_rn((int32_t)raw[j + 1]);
+    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%0, %1};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(acc[j]), "+f"(acc[j + 1]) : "f"(f0), "f"(f1), "f"(s[(j >> 1) & 2]), "f"(s[((j >> 1) & 2) + 1]));
   }
+}
+__device__ __forceinline__ void lds4(uint32_t addr, float (&s)[4]) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s[0]), "=f"(s[1]), "=f"(s[2]), "=f"(s[3]) : "r"(addr));
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
+// Four 8 x 8 blocks of bf16 fragments to / from shared memory, transposed: fragment column (token) = row there.
+__device__ __forceinline__ void stmatrix4_t(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_t(uint32_t addr, uint32_t (&v)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
+
+// Element i of a small register array (no dynamic indexing: a chain of selects).
+template <typename T, int N> __device__ __forceinline__ T pick(const T (&v)[N], int i) {
+  T r = v[0];
+#pragma unroll
+  for (int u = 1; u < N; ++u) r = i == u ? v[u] : r;
+  return r;
 }
 
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
@@ -366,6 +412,14 @@ __device__ __forceinline__ float rcp_refined(float b) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
   return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+}
+// a / b from the approximate reciprocal, corrected by the remainder once: within a unit in the last place or better of the
+// quotient, whose next use is a rounding to bf16.  The same operand ranges.
+__device__ __forceinline__ float div_fast(float a, float b) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  const float q = __fmul_rn(a, y);
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 __device__ __forceinline__ float div_by(float a, float b, float y) {
   const float q = __fmul_rn(a, y);
@@ -402,12 +456,36 @@ struct AMaps {
 
 __device__ __forceinline__ int a_map_index(int T) { return T <= 16 ? 0 : (T <= 32 ? 1 : (T <= 64 ? 2 : 3)); }
 
+// Walks this CTA's items (chunk, output tile): blockIdx.x, blockIdx.x + gridDim.x, ... in chunk-major order.  Every role has
+// its own; the descriptor of the item after the current one is already on its way while the current one is worked on
+// (a round trip to L2 and two divisions between two items were a tenth of a down-GEMM item).
+struct ItemCursor {
+  const Chunk *chunks;
+  int num_chunks, n_tiles, ci, nt, step_c, step_t;
+  int4 next;
+  __device__ __forceinline__ void fetch() {
+    if (ci < num_chunks) next = *reinterpret_cast<const int4 *>(chunks + ci);
+  }
+  __device__ __forceinline__ ItemCursor(const Chunk *c, int n_chunks, int tiles)
+      : chunks(c), num_chunks(n_chunks), n_tiles(tiles), ci((int)blockIdx.x / tiles), nt((int)blockIdx.x % tiles),
+        step_c((int)gridDim.x / tiles), step_t((int)gridDim.x % tiles), next(make_int4(-1, 0, 0, 0)) { fetch(); }
+  __device__ __forceinline__ bool take(Chunk &ch, int &tile) {
+    if (ci >= num_chunks) return false;
+    ch.expert = next.x; ch.row0 = next.y; ch.rows = next.z; ch.pad = next.w;
+    tile = nt;
+    ci += step_c;
+    nt += step_t;
+    if (nt >= n_tiles) { nt -= n_tiles; ++ci; }
+    fetch();
+    return true;
+  }
+};
+
 template <int MODE, int A_ROWS>
 __global__ void __launch_bounds__((Cfg<MODE, A_ROWS>::NUM_THREADS), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ AMaps a_maps, const KParams p) {
   using SM = Smem<MODE, A_ROWS>;
   using CF = Cfg<MODE, A_ROWS>;
-  constexpr int SC_SLOTS = CF::SC_SLOTS;
   constexpr int NW = CF::NW;
   constexpr int NA = CF::NA;
   constexpr int NBUF = CF::NBUF;
@@ -425,18 +503,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
 
   // ------------------------------ set-up -----------------------------------
   if (tid == 0) {
-    for (int s = 0; s < NW; ++s) {
-      // weight producer (arrive.expect_tx) + the scale warp (per-channel mode has no scale tables)
-      mbar_init(&sm.full_w[s], MODE == GEMM_CHANNEL ? 1 : 2);
+    for (int s = 0; s < ND; ++s) {
+      mbar_init(&sm.ready[s], 2);            // the two producers
+      mbar_init(&sm.done[s], 1);             // tcgen05.commit of the MMA thread
+      mbar_init(&sm.consumed[s], EPI_WARPS);
     }
-    for (int s = 0; s < NA; ++s) mbar_init(&sm.full_a[s], 1);
-    for (int s = 0; s < ND; ++s) mbar_init(&sm.done[s], 1);   // tcgen05.commit of the MMA thread
+    for (int b = 0; b < SC_BATCHES; ++b) mbar_init(&sm.scales[b], 1);
     for (int b = 0; b < NBUF; ++b) {
       mbar_init(&sm.tmem_full[b], 1);
       mbar_init(&sm.tmem_empty[b], EPI_WARPS);
     }
-    for (int b = 0; b < NCG; ++b) mbar_init(&sm.esync[b], 128);
-    mbar_init(&sm.isync, EPI_WARPS);
+    mbar_init(&sm.stg_full, EPI_WARPS);
+    mbar_init(&sm.stg_free, OUT_WARPS);
     sm.abort_flag = 0;
     fence_barrier_init();
   }
@@ -464,10 +542,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   dependency_release();
 
   const int num_chunks = *p.num_chunks;
-  const int64_t num_items = (int64_t)num_chunks * p.n_tiles;
   const int KB = p.KB;
+  Chunk ch;      // the item at hand: chunk and output tile
+  int nt = 0;
 
   if (warp < FIRST_EPI_WARP) {
+    if constexpr (CF::SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_FEED));
     if (warp == 0) {
       // ============ weight producer: one 128 x 128 tile per K block (gate_up: gate pass, then up pass) ============
       if (lane == 0) {
@@ -476,9 +556,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         uint32_t it = 0;
         int s = 0;
         bool ok = true;
-        for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-          const Chunk ch = p.chunks[item / p.n_tiles];
-          const int nt = (int)(item % p.n_tiles);
+        for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
           if (ch.expert < 0) continue;
           // weight tiles are streamed (evict-first) unless another chunk of the same expert is about to read
           // them again: those stay in L2 under the normal policy
@@ -488,22 +566,23 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             for (int kb = 0; kb < KB; ++kb, ++it) {
               // slot s was read by step it - NW
               if (it >= (uint32_t)NW && !mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 1, LO_SLEEP_PRODUCER)) { ok = false; break; }
-              mbar_arrive_expect_tx(&sm.full_w[s], W_TILE_BYTES);
-              tma_load_2d(sm.w[s], &w_map, kb * TILE_K, row_g, &sm.full_w[s], pol_w);
+              mbar_arrive_expect_tx(&sm.ready[it % ND], W_TILE_BYTES);
+              tma_load_2d(sm.w[s], &w_map, kb * TILE_K, row_g, &sm.ready[it % ND], pol_w);
               s = s + 1 == NW ? 0 : s + 1;
             }
           }
         }
-      } else if (lane == 16) {
-      // ============ activation producer (a second lane of the same warp, on its own path): the chunk's token
-      // rows of every K block.  Token rows are read from an expert-sorted copy of the activations, so a chunk is
-      // a run of consecutive rows and one tiled load fetches it (a second one for the rows beyond 128).
+      }
+    } else if (warp == 3) {
+      // ============ activation producer: the chunk's token rows of every K block.  Token rows are read from an
+      // expert-sorted copy of the activations, so a chunk is a run of consecutive rows and one tiled load fetches
+      // it (a second one for the rows beyond 128).
+      if (lane == 0) {
         const uint64_t pol_a = policy_evict_last();
         uint32_t it = 0;
         int s = 0;
         bool ok = true;
-        for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-          const Chunk ch = p.chunks[item / p.n_tiles];
+        for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
           if (ch.expert < 0) continue;
           const int T = (ch.rows + 15) & ~15;
           const int T0 = T > 128 ? 128 : T;                  // first box; the rest (if any) goes into a second one
@@ -512,151 +591,299 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           const uint32_t a_bytes = (16u << mi) * TILE_K + (mi2 >= 0 ? (16u << mi2) * TILE_K : 0u);
           for (int ph = 0; ph < PHASES && ok; ++ph) {
             for (int kb = 0; kb < KB; ++kb, ++it) {
+              // slot s was read by step it - NA
               if (it >= (uint32_t)NA && !mbar_wait(sm, &sm.done[(it - NA) % ND], ((it - NA) / ND) & 1u, p.status, 6, LO_SLEEP_PRODUCER)) { ok = false; break; }
-              mbar_arrive_expect_tx(&sm.full_a[s], a_bytes);
-              tma_load_2d(sm.a[s], &a_maps.m[mi], kb * TILE_K, ch.row0, &sm.full_a[s], pol_a);
+              uint64_t *bar = &sm.ready[it % ND];
+              mbar_arrive_expect_tx(bar, a_bytes);
+              tma_load_2d(sm.a[s], &a_maps.m[mi], kb * TILE_K, ch.row0, bar, pol_a);
               if constexpr (A_ROWS > 128) {
-                if (mi2 >= 0)
-                  tma_load_2d(sm.a[s] + 128 * TILE_K, &a_maps.m[mi2], kb * TILE_K, ch.row0 + 128, &sm.full_a[s], pol_a);
+                if (mi2 >= 0) tma_load_2d(sm.a[s] + 128 * TILE_K, &a_maps.m[mi2], kb * TILE_K, ch.row0 + 128, bar, pol_a);
               }
               s = s + 1 == NA ? 0 : s + 1;
             }
           }
         }
       }
-    } else if (warp == 1 || warp == 3) {
-      // ============================ MMA issuers ===============================
-      // A step of this role is a chain of dependent scalar instructions and barrier round trips (a barrier poll
-      // takes more than a hundred cycles even when the phase has long completed), which costs more time than the
-      // 16 KB of weights of a step take to arrive however little the tensor core has to do.  So: lane 0 issues,
-      // lanes 0, 1 and 2 each own one of the step's three barriers (weights landed, activations landed, partial
-      // buffer free) with its ring position and poll it in the same instruction; one commit per step; and in the
-      // block-scaled modes two warps share the steps (even ones here, odd ones there: the partials of different
-      // steps are independent, a commit tracks the MMAs of its own thread, and the ring positions of a warp simply
-      // advance by two).  Per-channel mode accumulates an item's steps into one buffer, in order: warp 1 issues
-      // them all and the buffer ring advances once per item.
-      constexpr uint32_t NISS = MODE == GEMM_CHANNEL ? 1u : 2u;
-      const uint32_t which = warp == 1 ? 0u : 1u;
-      if (which < NISS) {
-        const uint32_t my_n = lane == 0 ? (uint32_t)NW : (lane == 1 ? (uint32_t)NA : (uint32_t)NBUF);
-        const uint32_t my_base = lane == 0 ? smem_u32(&sm.full_w[0]) : (lane == 1 ? smem_u32(&sm.full_a[0]) : smem_u32(&sm.tmem_empty[0]));
-        // ring position and phase parity of this lane's barrier at this warp's next step (global step index `it`);
-        // a fresh "buffer free" barrier is waited for with the opposite parity
-        uint32_t my_slot = which % my_n;
-        uint32_t my_par = ((which / my_n) & 1u) ^ (lane == 2 ? 1u : 0u);
-        uint32_t it = which, it_base = 0;
-        const uint64_t desc_w0 = make_smem_desc(smem_u32(sm.w[0])), desc_a0 = make_smem_desc(smem_u32(sm.a[0]));
-        bool ok = true;
-        for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-          const Chunk ch = p.chunks[item / p.n_tiles];
-          if (ch.expert < 0) continue;
-          const uint32_t idesc = make_idesc((uint32_t)((ch.rows + 15) & ~15));
-          const uint32_t steps = (uint32_t)(PHASES * KB);
-          for (uint32_t u = it - it_base; u < steps; u += NISS, it += NISS) {
-            // per-channel mode: the accumulator buffer is waited for at the item's first step only
-            const bool poll = lane < 2 || (lane == 2 && (MODE != GEMM_CHANNEL || u == 0));
-            const bool mine = poll ? mbar_wait_addr(sm, my_base + 8u * my_slot, my_par, p.status, 3 + lane, LO_SLEEP_MMA) : true;
-            if (!__all_sync(0xffffffffu, mine)) { ok = false; break; }
-            const uint32_t sw = __shfl_sync(0xffffffffu, my_slot, 0);
-            const uint32_t sa = __shfl_sync(0xffffffffu, my_slot, 1);
-            const uint32_t b = __shfl_sync(0xffffffffu, my_slot, 2);
-            if (lane == 0) {
-              tc_fence_after();
-              // descriptor start addresses are in 16-byte units
-              const uint64_t adesc = desc_w0 + (uint64_t)(sw * (W_TILE_BYTES >> 4));
-              const uint64_t bdesc = desc_a0 + (uint64_t)(sa * (uint32_t)(CF::A_TILE_BYTES >> 4));
-              const uint32_t d = tmem_base + b * (uint32_t)A_ROWS;
-#pragma unroll
-              for (int k4 = 0; k4 < TILE_K / 32; ++k4)
-                umma_i8(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc,
-                        (MODE == GEMM_CHANNEL ? (u | (uint32_t)k4) : (uint32_t)k4) != 0u ? 1u : 0u);
-              umma_commit(&sm.done[it & (uint32_t)(ND - 1)]);
-              if (MODE == GEMM_CHANNEL && u == steps - 1) umma_commit(&sm.tmem_full[b]);
-            }
-            __syncwarp();
-            // per-channel mode: the buffer ring (lane 2) advances once per item
-            if (MODE != GEMM_CHANNEL || lane != 2 || u == steps - 1) {
-              my_slot += (MODE == GEMM_CHANNEL && lane == 2) ? 1u : NISS;
-              if (my_slot >= my_n) { my_slot -= my_n; my_par ^= 1u; }
-            }
+    } else if (warp == 2) {
+      // ============ scale producer (block-scaled modes) ============
+      // Lane g multiplies the token scales of tokens g, g + 32, ... with the weight-block scale.  The promotion warps wait
+      // for the tables by themselves, four K-block steps at a time: a hand-over per step through the MMA issuer made this
+      // warp's chain (wait, multiply, store, arrive: 900 cycles) the slowest of the kernel.  Scales come from L2 (the chunk's
+      // scale rows are read by every output tile of the expert), one batch ahead, across the ends of passes and items.  Rows
+      // of scales whose length is a multiple of four are read with 16-byte loads.
+      if constexpr (MODE != GEMM_CHANNEL) {
+        constexpr int NU = (A_ROWS + 31) / 32;
+        const int64_t nblk = (p.n_rows_per_expert + TILE_N - 1) / TILE_N;
+        const bool vec = (KB & 3) == 0;
+        ItemCursor items(p.chunks, num_chunks, p.n_tiles);
+        struct Batch { Chunk ch; int nt, ph, kb; bool valid; };     // K blocks kb .. kb + 3 of a pass over an item
+        float a_cur[NU][4], b_cur[4], a_nxt[NU][4], b_nxt[4];
+        auto next_item = [&](Batch &b) {
+          do { b.valid = items.take(b.ch, b.nt); } while (b.valid && b.ch.expert < 0);
+        };
+        auto advance = [&](Batch &b) {
+          b.kb += SC_STEPS;
+          if (b.kb >= KB) {
+            b.kb = 0;
+            if (++b.ph == PHASES) { b.ph = 0; next_item(b); }
           }
-          it_base += steps;
-        }
-      }
-    } else if (MODE != GEMM_CHANNEL) {
-      // ========================= scale producer (warp 2) ====================
-      // Thread g owns tokens g, g + 32, ... of the chunk.  The scales of a K block are fetched two steps before
-      // they are used (they come from L2: the chunk's scale rows are read by every output tile of the expert), one
-      // value per token and step, which keeps this role to a few registers per token.
-      const int g = lane;
-      constexpr int NU = (A_ROWS + 31) / 32;
-      uint32_t it = 0;
-      int s = 0, slot = 0;
-      bool ok = true;
-      const int64_t nblk = (p.n_rows_per_expert + TILE_N - 1) / TILE_N;
-      for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const Chunk ch = p.chunks[item / p.n_tiles];
-        const int nt = (int)(item % p.n_tiles);
-        if (ch.expert < 0) continue;
-        const int T = (ch.rows + 15) & ~15;
-        const float *as_base = p.a_scale + (int64_t)ch.row0 * KB;
-        uint32_t as_off[NU];          // offset of the token's scale row; a token beyond the chunk reads row 0
-#pragma unroll
-        for (int u = 0; u < NU; ++u) as_off[u] = (uint32_t)((g + u * 32 < ch.rows ? g + u * 32 : 0) * KB);
-        for (int ph = 0; ph < PHASES && ok; ++ph) {
-          const float *bs_ptr = p.b_scale + ((int64_t)ch.expert * nblk + nt + (int64_t)ph * p.n_tiles) * KB;
-          float a0[NU], a1[NU], b0, b1;     // scales of this step and of the next one
+        };
+        // a token beyond the chunk reads row 0; its products are zeroed below
+        auto fetch = [&](const Batch &bt, float (&a)[NU][4], float (&b)[4]) {
+          const float *as_base = p.a_scale + (int64_t)bt.ch.row0 * KB + bt.kb;
 #pragma unroll
           for (int u = 0; u < NU; ++u) {
-            a0[u] = __ldg(as_base + as_off[u]);
-            a1[u] = KB > 1 ? __ldg(as_base + as_off[u] + 1) : 0.f;
+            const int t = lane + u * 32;
+            const float *src = as_base + (int64_t)(t < bt.ch.rows ? t : 0) * KB;
+            if (vec) {
+              const float4 v = __ldg(reinterpret_cast<const float4 *>(src));
+              a[u][0] = v.x; a[u][1] = v.y; a[u][2] = v.z; a[u][3] = v.w;
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) a[u][i] = bt.kb + i < KB ? __ldg(src + i) : 0.f;
+            }
           }
-          b0 = __ldg(bs_ptr);
-          b1 = KB > 1 ? __ldg(bs_ptr + 1) : 0.f;
-          for (int kb = 0; kb < KB; ++kb, ++it) {
-            float as_now[NU];
-            const float bs_now = b0;
-            b0 = b1;
-            if (kb + 2 < KB) b1 = __ldg(bs_ptr + kb + 2);
+          const float *bs = p.b_scale + ((int64_t)bt.ch.expert * nblk + bt.nt + (int64_t)bt.ph * p.n_tiles) * KB + bt.kb;
 #pragma unroll
-            for (int u = 0; u < NU; ++u) {
-              as_now[u] = a0[u];
-              a0[u] = a1[u];
-              if (kb + 2 < KB) a1[u] = __ldg(as_base + as_off[u] + kb + 2);
-            }
-            // the slot of this step is free once the weight stage is (see SC_SLOTS)
-            if (it >= (uint32_t)NW &&
-                !__all_sync(0xffffffffu, mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 4, LO_SLEEP_SCALE))) { ok = false; break; }
+          for (int i = 0; i < 4; ++i) b[i] = bt.kb + i < KB ? __ldg(bs + i) : 0.f;
+        };
+        Batch cur{ch, 0, 0, 0, false};
+        next_item(cur);
+        if (cur.valid) fetch(cur, a_cur, b_cur);
+        Batch nxt = cur;
+        if (nxt.valid) advance(nxt);
+        uint32_t n_batch = 0, slot = 0, it = 0;      // batches written, ring position, K-block steps written
+        uint32_t end_of[SC_BATCHES];                 // last step of the batch SC_BATCHES - i before this one
 #pragma unroll
-            for (int u = 0; u < NU; ++u) {
-              const int t = g + u * 32;
-              if (t < T) sm.sc[slot][t] = t < ch.rows ? __fmul_rn(as_now[u], bs_now) : 0.f;
+        for (int i = 0; i < SC_BATCHES; ++i) end_of[i] = 0u;
+        while (cur.valid) {
+          if (nxt.valid) fetch(nxt, a_nxt, b_nxt);
+          // the slot's previous batch has been read when the partial of its last step has been consumed
+          if (n_batch >= (uint32_t)SC_BATCHES &&
+              !__all_sync(0xffffffffu, mbar_wait(sm, &sm.consumed[end_of[0] % ND], (end_of[0] / ND) & 1u, p.status, 4, LO_SLEEP_SCALE))) break;
+          const int T = (cur.ch.rows + 15) & ~15;
+          float *sc = &sm.sc[slot * SC_STEPS][0];
+#pragma unroll
+          for (int u = 0; u < NU; ++u) {
+            const int t = lane + u * 32;
+            if (t < T) {
+              const float live = t < cur.ch.rows ? 1.f : 0.f;
+#pragma unroll
+              for (int i = 0; i < SC_STEPS; ++i) sc[i * A_ROWS + scale_place(t)] = live != 0.f ? __fmul_rn(a_cur[u][i], b_cur[i]) : 0.f;
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.full_w[s]);
-            s = s + 1 == NW ? 0 : s + 1;
-            slot = slot + 1 == SC_SLOTS ? 0 : slot + 1;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.scales[slot]);
+          slot = slot + 1 == (uint32_t)SC_BATCHES ? 0u : slot + 1;
+          ++n_batch;
+          it += (uint32_t)(KB - cur.kb < SC_STEPS ? KB - cur.kb : SC_STEPS);
+#pragma unroll
+          for (int i = 0; i + 1 < SC_BATCHES; ++i) end_of[i] = end_of[i + 1];
+          end_of[SC_BATCHES - 1] = it - 1;
+#pragma unroll
+          for (int u = 0; u < NU; ++u)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a_cur[u][i] = a_nxt[u][i];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) b_cur[i] = b_nxt[i];
+          cur = nxt;
+          if (nxt.valid) advance(nxt);
+        }
+      }
+    } else {
+      // ============================ MMA issuer (warp 1) ================================
+      // A step of this role is a chain of dependent instructions and barrier round trips, which takes longer than the
+      // tensor core needs for the step's MMAs.  So: lanes 0 and 1 each own one of the step's two barriers (operands ready,
+      // partial buffer free) and look at it in the same instruction; the look at the next step's barriers is issued before
+      // this step's MMAs; everything the MMAs take (ring positions, descriptors) is computed from values all lanes share,
+      // which keeps it in uniform registers (-11 % on the per-channel layer at 20 rows per expert against operands shuffled
+      // from the polling lanes).  Per-channel mode accumulates an item's steps into one buffer: lane 1 waits for the
+      // accumulator once per item.
+      uint32_t it = 0;
+      // ring positions of the step's operands and partial buffer
+      uint32_t sw = 0, sa = 0, sb = 0;
+      const uint32_t desc_w0 = (uint32_t)make_smem_desc(smem_u32(sm.w[0])), desc_a0 = (uint32_t)make_smem_desc(smem_u32(sm.a[0]));
+      const uint32_t desc_hi = (uint32_t)(make_smem_desc(0u) >> 32);
+      const uint32_t tm0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint32_t done0 = smem_u32(&sm.done[0]);
+      // this lane's barrier of step u is number (u + my_off) % ND of its ring; a buffer is waited for with the step that
+      // used it before (the steps before the first one read as complete: parity 1 of a fresh barrier)
+      const uint32_t my_base = smem_u32(lane == 0 ? &sm.ready[0] : &sm.consumed[0]);
+      const uint32_t my_off = lane == 0 ? 0u : 0u - (uint32_t)NBUF;
+      uint32_t acc_par = 1;              // per-channel mode: phase of the accumulator ring
+      bool ok = true, seen = lane > 1;
+      for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
+        if (ch.expert < 0) continue;
+        const uint32_t idesc = make_idesc((uint32_t)((__shfl_sync(0xffffffffu, ch.rows, 0) + 15) & ~15));
+        const uint32_t steps = (uint32_t)(PHASES * KB);
+#pragma unroll 1
+        for (uint32_t u = 0; u < steps; ++u, ++it) {
+          if (!__all_sync(0xffffffffu, seen)) {
+            if (!seen) {
+              uint32_t bar = my_base + 8u * ((it + my_off) & (uint32_t)(ND - 1)), par = ((it + my_off) >> 4) & 1u;
+              if (MODE == GEMM_CHANNEL && lane == 1) { bar = smem_u32(&sm.tmem_empty[sb]); par = acc_par; }
+              seen = mbar_wait_addr(sm, bar, par, p.status, 3 + lane, LO_SLEEP_MMA);
+            }
+            if (!__all_sync(0xffffffffu, seen)) { ok = false; break; }
+          }
+          tc_fence_after();
+          const bool last = u == steps - 1;
+          // the early look at the next step
+          const uint32_t nx = it + 1u + my_off;
+          if (MODE == GEMM_CHANNEL) seen = lane > 1 || (lane == 1 && !last) || (lane == 0 && mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u));
+          else seen = lane > 1 || mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u);
+          // descriptor start addresses are in 16-byte units
+          const uint32_t adesc = desc_w0 + sw * (uint32_t)(W_TILE_BYTES >> 4);
+          const uint32_t bdesc = desc_a0 + sa * (uint32_t)(CF::A_TILE_BYTES >> 4);
+          const uint32_t d = tm0 + sb * (uint32_t)A_ROWS;
+          if (elect_one()) {
+#pragma unroll
+            for (int k4 = 0; k4 < TILE_K / 32; ++k4)
+              umma_i8(d, adesc + (uint32_t)(k4 * 2), bdesc + (uint32_t)(k4 * 2), desc_hi, idesc,
+                      (MODE == GEMM_CHANNEL ? (u | (uint32_t)k4) : (uint32_t)k4) != 0u ? 1u : 0u);
+            umma_commit_addr(done0 + 8u * (it & (uint32_t)(ND - 1)));
+            if (MODE == GEMM_CHANNEL && last) umma_commit(&sm.tmem_full[sb]);
+          }
+          __syncwarp();
+          sw = sw + 1 == (uint32_t)NW ? 0u : sw + 1;
+          sa = sa + 1 == (uint32_t)NA ? 0u : sa + 1;
+          if (MODE != GEMM_CHANNEL || last) {
+            if (++sb == (uint32_t)NBUF) { sb = 0; acc_par ^= 1u; }
           }
         }
       }
     }
+  } else if (MODE != GEMM_CHANNEL && warp >= FIRST_EPI_WARP + EPI_WARPS) {
+    // ====================== output warps (block-scaled modes) ======================
+    // They turn the finished tile in the staging buffer (bf16, row = token) into rows of global memory while the
+    // promotion warps are already on the next item.
+    if constexpr (CF::SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OUT));
+    const int ow = warp - (FIRST_EPI_WARP + EPI_WARPS);
+    uint32_t par = 0;
+    for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); items.take(ch, nt);) {
+      if (ch.expert < 0) {
+        // block of a non-local expert: its output rows are zero
+        if (MODE == GEMM_SINGLE && p.C != nullptr) {
+          for (int t = ow; t < ch.rows; t += OUT_WARPS) {
+            const int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
+            if (sid >= 0 && sid < p.numel_valid)
+              for (int64_t n = (int64_t)nt * TILE_N + lane; n < (int64_t)(nt + 1) * TILE_N && n < p.n_store; n += 32)
+                p.C[(int64_t)(p.out_by_position ? ch.row0 + t : sid) * p.n_store + n] = __float2bfloat16_rn(0.f);
+          }
+        }
+        continue;
+      }
+      if constexpr (MODE == GEMM_GATE_UP) {
+        // A row of the tile is one token's 128-channel quantisation group: |act| maximum over the warp (four channels
+        // per lane), scale = max / 127, q = trunc(clamp(act / scale)), one 4-byte store per lane.
+        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9, LO_SLEEP_OUT))) break;
+        const int64_t I = (int64_t)p.n_tiles * TILE_N;
+        int8_t *q_out = p.act_q + (int64_t)ch.row0 * I + (int64_t)nt * TILE_N + lane * 4;
+        float *s_out = p.act_s + (int64_t)ch.row0 * p.n_tiles + nt;
+        constexpr int UN = 4;          // tokens in flight per warp
+#pragma unroll 1
+        for (int t0 = ow * UN; t0 < ch.rows; t0 += OUT_WARPS * UN) {
+          float v[UN][4];
+          uint32_t m[UN];
+#pragma unroll
+          for (int e = 0; e < UN; ++e) {
+            // (rows of the tile beyond the chunk are inside the staging buffer: T is a multiple of 16)
+            const uint2 raw = *reinterpret_cast<const uint2 *>(&sm.staging[(t0 + e) * OUT_ROW_BYTES + lane * 8]);
+            v[e][0] = __uint_as_float(raw.x << 16);
+            v[e][1] = __uint_as_float(raw.x & 0xffff0000u);
+            v[e][2] = __uint_as_float(raw.y << 16);
+            v[e][3] = __uint_as_float(raw.y & 0xffff0000u);
+            m[e] = __float_as_uint(fmaxf(fmaxf(fabsf(v[e][0]), fabsf(v[e][1])), fmaxf(fabsf(v[e][2]), fabsf(v[e][3]))));
+          }
+#pragma unroll
+          for (int e = 0; e < UN; ++e) m[e] = __reduce_max_sync(0xffffffffu, m[e]);
+          // lane e forms the scale of token e, the others fetch it
+          uint32_t m_own = m[0];
+#pragma unroll
+          for (int e = 1; e < UN; ++e) m_own = lane == e ? m[e] : m_own;
+          const float scale_own = __fdiv_rn(fmaxf(__uint_as_float(m_own), p.act_eps), 127.0f);
+          if (lane < UN && t0 + lane < ch.rows) s_out[(int64_t)(t0 + lane) * p.n_tiles] = scale_own;
+          const float rcp_own = rcp_refined(scale_own);
+#pragma unroll
+          for (int e = 0; e < UN; ++e) {
+            const float scale = __shfl_sync(0xffffffffu, scale_own, e), rcp = __shfl_sync(0xffffffffu, rcp_own, e);
+            uint32_t packed = 0u;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float r = fminf(fmaxf(div_by(v[e][i], scale, rcp), -128.0f), 127.0f);
+              packed |= ((uint32_t)__float2int_rz(r) & 0xffu) << (8 * i);
+            }
+            if (t0 + e < ch.rows) *reinterpret_cast<uint32_t *>(q_out + (int64_t)(t0 + e) * I) = packed;
+          }
+        }
+      } else {
+        // Two token rows per step and warp, sixteen lanes x 16 bytes each.  The rows' ids, weights and addresses are
+        // fetched before the wait: lane l of set i / 16 holds those of row half l & 1 of step i with i % 16 == l / 2.
+        constexpr int NSET = (A_ROWS / (2 * OUT_WARPS) + 15) / 16;
+        unsigned long long rowp_r[NSET];      // address of the row's first output column, 0 = no row
+        float wgt_r[NSET];
+#pragma unroll
+        for (int u = 0; u < NSET; ++u) {
+          rowp_r[u] = 0ull;
+          wgt_r[u] = 0.f;
+          const int t = (u * 16 + (lane >> 1)) * (2 * OUT_WARPS) + ow * 2 + (lane & 1);
+          if (t < ch.rows) {
+            // without a sorted-id table the id of a row is its position
+            const int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
+            if (sid >= 0 && sid < p.numel_valid) {
+              if (p.weight_mode == LO_WEIGHT_BF16_PRODUCT) wgt_r[u] = p.topk_weights[sid];
+              rowp_r[u] = p.row_dst != nullptr ? (unsigned long long)p.row_dst[sid]
+                                               : (unsigned long long)(p.C + (int64_t)(p.out_by_position ? ch.row0 + t : sid) * p.n_store);
+            }
+          }
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9, LO_SLEEP_OUT))) break;
+        const bool vec_ok = (p.n_store & 7) == 0;
+        const int64_t n0 = (int64_t)nt * TILE_N + (lane & 15) * 8;
+        const int n_steps = (ch.rows + 2 * OUT_WARPS - 1) / (2 * OUT_WARPS);
+#pragma unroll 4
+        for (int i = 0; i < n_steps; ++i) {
+          const int src_lane = (i & 15) * 2 + (lane >> 4);
+          const unsigned long long rowp = __shfl_sync(0xffffffffu, pick(rowp_r, i >> 4), src_lane);
+          // bf16-product order: bf16(sum) * bf16(w), rounded once more: one packed multiply per two outputs
+          const __nv_bfloat162 w2 = __float2bfloat162_rn(__shfl_sync(0xffffffffu, pick(wgt_r, i >> 4), src_lane));
+          const int t = i * (2 * OUT_WARPS) + ow * 2 + (lane >> 4);
+          if (rowp != 0ull && n0 < p.n_store) {
+            __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(rowp) + n0;
+            uint4 v = *reinterpret_cast<const uint4 *>(&sm.staging[t * OUT_ROW_BYTES + (lane & 15) * 16]);
+            if (p.weight_mode == LO_WEIGHT_BF16_PRODUCT) {
+              __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&v);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) h[e] = __hmul2(h[e], w2);
+            }
+            if (vec_ok) {
+              *reinterpret_cast<uint4 *>(dst) = v;
+            } else {
+              for (int e = 0; e < 8 && n0 + e < p.n_store; ++e) dst[e] = reinterpret_cast<const __nv_bfloat16 *>(&v)[e];
+            }
+          }
+        }
+      }
+      par ^= 1u;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.stg_free);
+    }
   } else {
-    // ====================== promotion + epilogue (16 warps) ====================
-    const int pw = warp - FIRST_EPI_WARP;   // 0..15
+    // ====================== promotion (block-scaled modes) / epilogue (per-channel mode) ======================
+    if constexpr (CF::SPLIT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_PROMO));
+    const int pw = warp - FIRST_EPI_WARP;
     const int q = warp & 3;              // lane quarter of tensor memory this warp may access
     const int cg = pw >> 2;              // column group: which share of the chunk's tokens
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
     const int n_local = q * 32 + lane;
-    uint32_t ab = 0, eph = 0, iph = 0, item_par = 0;
-    uint32_t sc_slot = 0, buf = 0, step = 0;     // block-scaled modes: ring positions of the K loop, K-block step count
-    bool ready = false;                          // the coming step's barrier was already seen complete
+    uint32_t ab = 0, fph = 1;                    // per-channel accumulator count; parity of the staging buffer's "free"
+    uint32_t sc_slot = 0, sc_par = 0;            // ring of scale batches
+    uint32_t buf = 0, step = 0;                  // block-scaled modes: partial buffer and count of the K-block step
     bool ok = true;
-    for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-      const Chunk ch = p.chunks[item / p.n_tiles];
-      const int nt = (int)(item % p.n_tiles);
+    for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
       if (ch.expert < 0) {
-        // block of a non-local expert: its output rows are zero
-        if (MODE != GEMM_GATE_UP && p.C != nullptr) {
+        // block of a non-local expert: its output rows are zero (the block-scaled modes leave that to the output warps)
+        if (MODE == GEMM_CHANNEL && p.C != nullptr) {
           for (int t = cg; t < ch.rows; t += NCG) {
             const int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
             if (sid >= 0 && sid < p.numel_valid && (int64_t)nt * TILE_N + n_local < p.n_store)
@@ -667,53 +894,37 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         continue;
       }
       // The chunk's T columns (a multiple of 16) are dealt to the column groups in pieces of 16, as evenly as
-      // that allows; a group owns at most two pieces (32 tokens) of a chunk of up to 160 tokens, four of a chunk
-      // of up to 256.
+      // that allows.
       const int T = (ch.rows + 15) & ~15;
       const int n_pieces = T >> 4;
       const int my_p = n_pieces / NCG + (cg < n_pieces % NCG ? 1 : 0);
       const int col_begin = (cg * (n_pieces / NCG) + min(cg, n_pieces % NCG)) * 16;
 
-      // Row id and routed weight of token col_begin + 32 * u + lane, fetched now so that the latency is
-      // hidden behind the K loop; broadcast by shuffle in the epilogue: piece pc of the group is in
-      // register set pc / 2, lanes 16 * (pc & 1) .. + 15.
-      constexpr int NPF = ((A_ROWS / 16 + NCG - 1) / NCG + 1) / 2;   // sets of 32 tokens that cover a group's pieces
-      int32_t sid_r[NPF];
-      float wgt_r[NPF];
-      // single mode: address of the row's first output column (0 = no row), so that the epilogue's row stores
-      // serve a table of row addresses (rows in a peer's memory) and the plain matrix alike
-      unsigned long long rowp_r[MODE == GEMM_SINGLE ? NPF : 1];
-      rowp_r[0] = 0ull;
+      if constexpr (MODE == GEMM_CHANNEL) {
+        // ---------------- per-channel mode: one pass over the finished int32 accumulator ----------------
+        // Row id and routed weight of token col_begin + 32 * u + lane, fetched now so that the latency is
+        // hidden behind the K loop; broadcast by shuffle in the epilogue: piece pc of the group is in
+        // register set pc / 2, lanes 16 * (pc & 1) .. + 15.
+        constexpr int NPF = ((A_ROWS / 16 + NCG - 1) / NCG + 1) / 2;   // sets of 32 tokens that cover a group's pieces
+        int32_t sid_r[NPF];
+        float wgt_r[NPF];
+        // token scale of column col_begin + lane (broadcast by shuffle) and the scale of this thread's channel
+        float as_r[NPF];
 #pragma unroll
-      for (int u = 0; u < NPF; ++u) {
-        sid_r[u] = -1;
-        wgt_r[u] = 0.f;
-        if (MODE == GEMM_SINGLE) rowp_r[MODE == GEMM_SINGLE ? u : 0] = 0ull;
-        if (MODE != GEMM_GATE_UP || p.weight_mode != LO_WEIGHT_NONE) {
+        for (int u = 0; u < NPF; ++u) {
+          sid_r[u] = -1;
+          wgt_r[u] = 0.f;
+          as_r[u] = 0.f;
           const int t = col_begin + u * 32 + lane;
           if (u * 32 + lane < my_p * 16 && t < ch.rows) {
             // without a sorted-id table the id of a row is its position
             int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
             if (sid < 0 || sid >= p.numel_valid) sid = -1;
             if (sid >= 0 && p.weight_mode != LO_WEIGHT_NONE) wgt_r[u] = p.topk_weights[sid];
-            if (MODE == GEMM_SINGLE && sid >= 0 && p.row_dst != nullptr)
-              rowp_r[MODE == GEMM_SINGLE ? u : 0] = (unsigned long long)p.row_dst[sid];
             if (sid >= 0 && p.out_by_position) sid = ch.row0 + t;
-            if (MODE == GEMM_SINGLE && sid >= 0 && p.row_dst == nullptr)
-              rowp_r[MODE == GEMM_SINGLE ? u : 0] = (unsigned long long)(p.C + (int64_t)sid * p.n_store);
             sid_r[u] = sid;
+            as_r[u] = __ldg(p.a_scale + ch.row0 + t);
           }
-        }
-      }
-
-      if constexpr (MODE == GEMM_CHANNEL) {
-        // ---------------- per-channel mode: one pass over the finished int32 accumulator ----------------
-        // token scale of column col_begin + lane (broadcast by shuffle) and the scale of this thread's channel
-        float as_r[NPF];
-#pragma unroll
-        for (int u = 0; u < NPF; ++u) {
-          const int t = col_begin + u * 32 + lane;
-          as_r[u] = (u * 32 + lane < my_p * 16 && t < ch.rows) ? __ldg(p.a_scale + ch.row0 + t) : 0.f;
         }
         const int64_t n_glob = (int64_t)nt * TILE_N + n_local;
         const bool n_ok = n_glob < p.n_store;
@@ -728,7 +939,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         for (int pc = 0; pc < my_p; ++pc) {
           uint32_t raw[16];
           tmem_ld16(part + pc * 16, raw);
-          tmem_ld_wait();
+          tmem_ld_wait16(raw);
           if (pc == my_p - 1) {
             // every value this warp needs is in registers: hand the buffer back before the stores
             tc_fence_before();
@@ -736,10 +947,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (lane == 0) mbar_arrive(&sm.tmem_empty[b]);
           }
           // piece pc holds tokens 16 * pc .. 16 * pc + 15 of this group: register set pc / 2, lanes 16 * (pc & 1) ..
-          const int u = NPF > 1 ? (pc >> 1) : 0;
-          const int32_t sid_u = NPF > 1 && u ? sid_r[NPF - 1] : sid_r[0];
-          const float wgt_u = NPF > 1 && u ? wgt_r[NPF - 1] : wgt_r[0];
-          const float as_u = NPF > 1 && u ? as_r[NPF - 1] : as_r[0];
+          const int32_t sid_u = pick(sid_r, pc >> 1);
+          const float wgt_u = pick(wgt_r, pc >> 1);
+          const float as_u = pick(as_r, pc >> 1);
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int src = (pc & 1) * 16 + j;
@@ -762,223 +972,208 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       } else {
         // ---------------- block-scaled modes: promotion once per K block, sums in registers ----------------
         // This warp owns the columns [col_begin, col_begin + 16 * my_p) of its 32 lanes.  Their fp32 running sums
-        // stay in registers over the whole K loop (NP pieces of 16 columns at most; the piece loop is unrolled and
-        // a piece beyond the chunk's width is skipped), so tensor memory holds nothing but partial buffers and a
-        // K block costs one tensor-memory load per piece.
+        // stay in registers over the whole K loop, so tensor memory holds nothing but partial buffers and a
+        // K block costs one tensor-memory load per piece of 16 columns.
         constexpr int NP = (A_ROWS / 16 + NCG - 1) / NCG;
         float acc[NP][16];
         // Addresses of this item, formed once: the loops below only add constants to them.  Ring positions
         // (scale slot, partial buffer and its phase) are carried as counters instead of being divided out of
         // the step numbers.
         const uint32_t part0 = tmem_base + lane_off + (uint32_t)col_begin;
-        const uint32_t sc0 = smem_u32(&sm.sc[0][0]) + (uint32_t)col_begin * 4u;
-        const uint32_t done0 = smem_u32(&sm.done[0]), empty0 = smem_u32(&sm.tmem_empty[0]);
-        // a warp with fewer pieces than the busiest group of the item has that much slack per step and polls at a
-        // longer interval; a warp without columns only has to keep step
-        const int max_p = (n_pieces + NCG - 1) / NCG;
-        const uint32_t wait_ns = my_p == 0 ? 256u : (my_p < max_p ? LO_SLEEP_PROMO_SLACK : LO_SLEEP_PROMO);
-        // this thread's column of the staging tile: row = token, 2 bytes per output channel.  Plain loads and
-        // stores (no volatile asm), so that the compiler can overlap the sixteen tokens of a piece; the barrier
-        // operations between the phases are compiler barriers as well.
-        __nv_bfloat16 *const stg_mine = reinterpret_cast<__nv_bfloat16 *>(&sm.staging[0]) + col_begin * TILE_N + n_local;
+        const uint32_t sc0 = smem_u32(&sm.sc[0][0]) + (uint32_t)col_begin * 4u + (uint32_t)(lane & 3) * 16u;
+        const uint32_t done0 = smem_u32(&sm.done[0]), consumed0 = smem_u32(&sm.consumed[0]), scales0 = smem_u32(&sm.scales[0]);
+        // a warp without columns only has to keep step
+        const uint32_t wait_ns = my_p == 0 ? 256u : LO_SLEEP_PROMO;
+        // this lane's row of the staging tile for the matrix stores and loads of a piece: lanes 8m .. 8m + 7 address the
+        // token rows of block m, blocks 0 / 1 are channels 0..7 / 8..15 of tokens 0..7, blocks 2 / 3 of tokens 8..15
+        const uint32_t stg_mine = smem_u32(&sm.staging[0]) + (uint32_t)(col_begin + (lane >> 4) * 8 + (lane & 7)) * OUT_ROW_BYTES +
+                                  (uint32_t)(q * 32 + ((lane >> 3) & 1) * 8) * 2u;
+        // fp32 routed weight of token t of the chunk (0 where there is no row)
+        auto weight_of = [&](int t) {
+          const int32_t sid = t < ch.rows ? (p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t) : -1;
+          return sid >= 0 && sid < p.numel_valid ? __ldg(p.topk_weights + sid) : 0.f;
+        };
 #pragma unroll 1
         for (int ph = 0; ph < PHASES; ++ph) {
 #pragma unroll
           for (int pc = 0; pc < NP; ++pc)
 #pragma unroll
             for (int j = 0; j < 16; ++j) acc[pc][j] = 0.f;
-#pragma unroll 1
-          for (int kb = 0; kb < KB; ++kb) {
-            const uint32_t sc_step = sc0 + sc_slot * (uint32_t)(A_ROWS * 4);
-            sc_slot = sc_slot + 1 == (uint32_t)SC_SLOTS ? 0u : sc_slot + 1;
-            const uint32_t b = buf;
-            buf = buf + 1 == (uint32_t)NBUF ? 0u : buf + 1;
-            const uint32_t dn = step & (uint32_t)(ND - 1), dph = (step >> 4) & 1u;
-            ++step;
-            // The scale products of this step were written to shared memory before the weight stage's full
-            // barrier completed, which the MMA thread observed before it issued the MMAs whose
-            // completion this wait observes.  Warp-uniform outcome: the accesses below are warp-collective.
-            if (!ready && !__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; break; }
+          // The K loop, instantiated for the number of pieces this warp owns in the chunk (and not unrolled further: the two
+          // groups run different instantiations, and with four steps unrolled the pair missed the instruction cache, +35 %).
+          // What bounds it is neither a pipe nor the issue slots but the chain of one warp (barrier, tensor-memory load,
+          // conversion, multiply-add, hand-back: 890 to 1100 cycles a step in the plain order of these, 710 to 790 so).  Every
+          // tensor-memory load is issued one unit ahead of its use, the first one of the next step included, and a buffer goes
+          // back to the MMA warp as soon as its last unit is in registers, before that unit is promoted.
+          auto k_loop = [&](auto pcs) {
+            constexpr int PC = decltype(pcs)::value;
+            static_assert(PC <= NP, "more pieces than sums");
+            constexpr int U = PC;                     // units of a step: two per pair of pieces, one for an odd last piece
+            // Units alternate between two register sets.  The next step's first unit goes into set 0 while the last one is
+            // promoted: with an odd number of units the last one takes a third set (a single unit: two steps per turn).
+            constexpr int UNROLL = PC == 1 ? 2 : 1;
+            constexpr int SETS = PC > 1 && (PC & 1) ? 3 : 2;
+            uint32_t raw[SETS][16];
+            auto load_unit = [&](int u, uint32_t part, uint32_t (&r)[16]) {
+              if ((PC & 1) && u == U - 1) tmem_ld_one(part + 16u * (PC - 1), r);
+              else tmem_ld_two(part + 32u * (u >> 1) + ((u & 1) ? 16u << 16 : 0u), r);
+            };
+            uint32_t dn = step & (uint32_t)(ND - 1), dph = (step >> 4) & 1u;      // the step's place in the rings of ND
+            if (!__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; return; }
             tc_fence_after();
-            // an early look at the next step's barrier: the answer arrives while this step's columns are promoted
-            // (a barrier round trip takes more than a hundred cycles even when the phase has long completed)
-            const bool next_done = mbar_test_addr(done0 + 8u * (step & (uint32_t)(ND - 1)), (step >> 4) & 1u);
-            const uint32_t part = part0 + b * (uint32_t)A_ROWS;
+            if (PC > 0) load_unit(0, part0 + buf * (uint32_t)A_ROWS, raw[0]);
+            uint32_t sc_at = 0;
+#pragma unroll 1
+            for (int kb0 = 0; kb0 < KB; kb0 += UNROLL) {
+              if ((kb0 & (SC_STEPS - 1)) == 0) {
+                // the scale products of the coming four steps
+                if (PC > 0 && !__all_sync(0xffffffffu, mbar_wait_addr(sm, scales0 + 8u * sc_slot, sc_par, p.status, 7))) { ok = false; return; }
+                sc_at = sc0 + sc_slot * (uint32_t)(SC_STEPS * A_ROWS * 4);
+                if (++sc_slot == (uint32_t)SC_BATCHES) { sc_slot = 0; sc_par ^= 1u; }
+              }
 #pragma unroll
-            for (int pc = 0; pc < NP; ++pc) {
-              if (pc < my_p) {
-                uint32_t r16[16];
-                tmem_ld16(part + pc * 16, r16);
-                tmem_ld_wait();
-                promote<16>(r16, &acc[pc][0], sc_step + (uint32_t)(pc * 64));
+              for (int i = 0; i < UNROLL; ++i) {
+                if (i > 0 && kb0 + i >= KB) break;
+                const uint32_t part = part0 + buf * (uint32_t)A_ROWS;
+                const uint32_t used = consumed0 + 8u * dn;
+                buf = buf + 1 == (uint32_t)NBUF ? 0u : buf + 1;
+                ++step;
+                dn = step & (uint32_t)(ND - 1);
+                dph = (step >> 4) & 1u;
+                float s0[4], s1[4];      // scale products of the pieces at hand
+                bool next_done = false;
+#pragma unroll
+                for (int u = 0; u < (U > 0 ? U : 1); ++u) {
+                  const bool last = u == (U > 0 ? U - 1 : 0);
+                  const int set = PC == 1 ? i : (SETS == 3 && last ? 2 : u & 1);
+                  const int next_set = PC == 1 ? i ^ 1 : (last ? 0 : (SETS == 3 && u + 1 == U - 1 ? 2 : (u + 1) & 1));
+                  const bool single = (PC & 1) && u == U - 1;
+                  if (PC > 0 && (single || (u & 1) == 0)) {
+                    const int pc = single ? PC - 1 : u;
+                    lds4(sc_at + (uint32_t)(pc * 64), s0);
+                    if (!single) lds4(sc_at + (uint32_t)((pc + 1) * 64), s1);
+                  }
+                  if (last) next_done = mbar_test_addr(done0 + 8u * dn, dph);
+                  if (PC > 0) tmem_ld_wait16(raw[set]);
+                  if (!last) {
+                    load_unit(u + 1, part, raw[next_set]);
+                  } else {
+                    // every value of the partial is in registers: the buffer goes back, the next step's first unit is asked for
+                    tc_fence_before();
+                    if (lane == 0) mbar_arrive_addr(used);
+                    if (kb0 + i + 1 < KB) {
+                      // warp-uniform outcome: the accesses to tensor memory are warp-collective
+                      if (!__all_sync(0xffffffffu, next_done) &&
+                          !__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; return; }
+                      tc_fence_after();
+                      if (PC > 0) load_unit(0, part0 + buf * (uint32_t)A_ROWS, raw[next_set]);
+                    }
+                  }
+                  if (PC > 0) {
+                    if (single) {
+                      promote8(&acc[PC > 0 ? PC - 1 : 0][0], &raw[set][0], s0);
+                      promote8(&acc[PC > 0 ? PC - 1 : 0][8], &raw[set][8], s0);
+                    } else {
+                      promote8(&acc[u & ~1][8 * (u & 1)], &raw[set][0], s0);
+                      promote8(&acc[(u | 1) < NP ? (u | 1) : 0][8 * (u & 1)], &raw[set][8], s1);
+                    }
+                  }
+                }
+                sc_at += (uint32_t)(A_ROWS * 4);
               }
             }
-            ready = __all_sync(0xffffffffu, next_done);
-            // every load of the partial has completed: hand the buffer back to the MMA warp
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_addr(empty0 + 8u * b);
+          };
+          // (each count is instantiated once: a lambda called from two places is not inlined, and its sums would go to memory)
+          if (my_p == 0) k_loop(std::integral_constant<int, 0>{});
+          else if (NP == 1 || my_p == 1) k_loop(std::integral_constant<int, 1>{});
+          if constexpr (NP >= 2) {
+            if (NP == 2 ? my_p >= 2 : my_p == 2) k_loop(std::integral_constant<int, 2>{});
+          }
+          if constexpr (NP >= 3) {
+            if (NP == 3 ? my_p >= 3 : my_p == 3) k_loop(std::integral_constant<int, 3>{});
+          }
+          if constexpr (NP >= 4) {
+            if (NP == 4 ? my_p >= 4 : my_p == 4) k_loop(std::integral_constant<int, 4>{});
+          }
+          if constexpr (NP >= 5) {
+            if (my_p >= 5) k_loop(std::integral_constant<int, 5>{});
           }
           if (!ok) break;
-          if (MODE == GEMM_GATE_UP && ph == 0) {
-            // End of the gate pass: bf16(gate) goes to this thread's column of the staging tile and is read back by
-            // the same thread after the up pass.  The rows may still be in use by the row stores of the previous
-            // item's epilogue, by any warp (the split of the rows over the column groups follows the chunk's
-            // width): all promotion warps meet first.
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.isync);
-            if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.isync, iph, p.status, 8))) { ok = false; break; }
-            iph ^= 1u;
+          // routed weight on the fp32 sums (before their rounding), where the mode asks for it
+          if (p.weight_mode == LO_WEIGHT_FP32) {
+#pragma unroll
+            for (int pc = 0; pc < NP; ++pc) {
+              if (pc < my_p) {
+                float w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = weight_of(col_begin + pc * 16 + (i >> 1) * 8 + (lane & 3) * 2 + (i & 1));
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[pc][j] *= w[((j >> 1) & 2) + (j & 1)];
+              }
+            }
+          }
+          if (MODE == GEMM_SINGLE || ph == 0) {
+            // The sums (gate_up: those of the gate pass, read back by the same warp below) go to the staging tile as
+            // bf16, once the output warps are done with the previous item's tile.
+            if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_free, fph, p.status, 8))) { ok = false; break; }
+            fph ^= 1u;
 #pragma unroll
             for (int pc = 0; pc < NP; ++pc) {
               if (pc < my_p) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  float gte = acc[pc][j];
-                  if (p.weight_mode == LO_WEIGHT_FP32)
-                    gte *= __shfl_sync(0xffffffffu, NPF > 1 && (pc >> 1) ? wgt_r[NPF - 1] : wgt_r[0], (pc & 1) * 16 + j);
-                  stg_mine[(pc * 16 + j) * TILE_N] = __float2bfloat16_rn(gte);
+                for (int h = 0; h < 2; ++h) {
+                  const float *a = &acc[pc][8 * h];
+                  stmatrix4_t(stg_mine + (uint32_t)(pc * 16 * OUT_ROW_BYTES + h * 32), pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]),
+                              pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
                 }
               }
+            }
+          } else {
+            // act = bf16(bf16(silu(bf16(gate))) * bf16(up)) in place of the gate values.  One rolled loop over the pieces:
+            // the body always works on piece 0 of the sums (bf16 by then) and the others move down one place afterwards
+            // (registers cannot be indexed by a loop counter, and a body unrolled over the pieces would be fetched cold once
+            // per item).
+            uint32_t up[NP][8];
+#pragma unroll
+            for (int pc = 0; pc < NP; ++pc)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) up[pc][j] = pack_bf16(acc[pc][2 * j], acc[pc][2 * j + 1]);
+#pragma unroll 1
+            for (int pc = 0; pc < my_p; ++pc) {
+              const uint32_t addr = stg_mine + (uint32_t)(pc * 16 * OUT_ROW_BYTES);
+              uint32_t g2[2][4];
+              ldmatrix4_t(addr, g2[0]);
+              ldmatrix4_t(addr + 32u, g2[1]);
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  float a[2];
+#pragma unroll
+                  for (int e = 0; e < 2; ++e) {
+                    const float gte = __uint_as_float(e ? g2[h][j] & 0xffff0000u : g2[h][j] << 16);
+                    // 1 + exp(-gate) capped below the fp32 maximum: the quotient is then zero instead of an invalid
+                    // operation in the correction (the exact quotient would be -0 or a number below 1e-36)
+                    a[e] = div_fast(gte, fminf(1.0f + expf(-gte), 1e38f));
+                  }
+                  // bf16(silu) * bf16(up), rounded once: the packed bf16 product
+                  const uint32_t sl = pack_bf16(a[0], a[1]);
+                  const __nv_bfloat162 act = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&sl), *reinterpret_cast<const __nv_bfloat162 *>(&up[0][4 * h + j]));
+                  g2[h][j] = *reinterpret_cast<const uint32_t *>(&act);
+                }
+                stmatrix4_t(addr + 32u * h, g2[h][0], g2[h][1], g2[h][2], g2[h][3]);
+              }
+#pragma unroll
+              for (int pp = 0; pp + 1 < NP; ++pp)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) up[pp][j] = up[pp + 1][j];
             }
           }
         }
         if (!ok) break;
-
-        // ------------------------------ epilogue -------------------------------
-        // One rolled loop over the warp's pieces: the body always works on piece 0 of the register sums and the
-        // remaining pieces move down one place afterwards (registers cannot be indexed by a loop counter, and an
-        // epilogue unrolled over the pieces would be fetched cold once per item).  Outputs go through the staging
-        // tile so that global memory sees whole rows: a thread holds one output channel of 16 tokens, a row of the
-        // output is 128 channels of one token.
-        if constexpr (MODE == GEMM_GATE_UP) {
-          const int64_t I = (int64_t)p.n_tiles * TILE_N;
-          uint32_t(*amax_tab)[A_ROWS] = sm.amax[item_par];
-#pragma unroll 1
-          for (int pc = 0; pc < my_p; ++pc) {
-            float *av = &acc[0][0];
-            const __nv_bfloat16 *gs = stg_mine + pc * 16 * TILE_N;
-            // Pass A: act = bf16(bf16(silu(bf16(gate))) * bf16(up)) in place of the up sums; maximum of |act|
-            // over this warp's 32 output columns, lane j keeps the one of token j.
-            float gte[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) gte[j] = __bfloat162float(gs[j * TILE_N]);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              float up = av[j];
-              if (p.weight_mode == LO_WEIGHT_FP32)
-                up *= __shfl_sync(0xffffffffu, NPF > 1 && (pc >> 1) ? wgt_r[NPF - 1] : wgt_r[0], (pc & 1) * 16 + j);
-              up = bf16_round(up);
-              // 1 + exp(-gate) capped below the fp32 maximum: the quotient is then zero instead of an invalid
-              // operation in the refinement (the exact quotient would be -0 or a number below 1e-36)
-              const float den = fminf(1.0f + expf(-gte[j]), 1e38f);
-              const float sl = bf16_round(div_by(gte[j], den, rcp_refined(den)));
-              av[j] = bf16_round(sl * up);
-            }
-            uint32_t own = 0u;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(av[j]) & 0x7fffffffu);
-              if (j == lane) own = m;
-            }
-            if (lane < 16) amax_tab[q][col_begin + pc * 16 + lane] = own;
-            // the four warps of this column group exchange their maxima (the table alternates between two
-            // copies from item to item; the pieces of one item use different entries); every gate value of the
-            // piece has been read when they have met
-            mbar_arrive(&sm.esync[cg]);
-            if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.esync[cg], eph, p.status, 9))) { ok = false; break; }
-            eph ^= 1u;
-            // Pass B: lane j (< 16) forms the group scale of token j of the piece, amax / 127; every thread then
-            // quantises its column of the 16 tokens, q = trunc(clamp(act / scale)), into byte n of the token's
-            // staging row.
-            float scale_r = 1.f, rcp_r = 1.f;
-            const int t_own = col_begin + pc * 16 + (lane & 15);
-            {
-              const uint32_t m = max(max(amax_tab[0][t_own], amax_tab[1][t_own]), max(amax_tab[2][t_own], amax_tab[3][t_own]));
-              scale_r = __fdiv_rn(fmaxf(__uint_as_float(m), p.act_eps), 127.0f);
-              rcp_r = rcp_refined(scale_r);
-              if (q == 0 && lane < 16 && t_own < ch.rows) p.act_s[((int64_t)ch.row0 + t_own) * p.n_tiles + nt] = scale_r;
-            }
-            int8_t *qs = reinterpret_cast<int8_t *>(&sm.staging[0]) + (col_begin + pc * 16) * OUT_ROW_BYTES + n_local;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float scale = __shfl_sync(0xffffffffu, scale_r, j);
-              float r = div_by(av[j], scale, __shfl_sync(0xffffffffu, rcp_r, j));
-              r = fminf(fmaxf(r, -128.0f), 127.0f);
-              qs[j * OUT_ROW_BYTES] = (int8_t)__float2int_rz(r);
-            }
-            mbar_arrive(&sm.esync[cg]);
-            if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.esync[cg], eph, p.status, 10))) { ok = false; break; }
-            eph ^= 1u;
-            // rows out: this warp takes tokens 4q .. 4q+3 of the piece, eight lanes x 16 bytes per row
-            {
-              const int t = col_begin + pc * 16 + 4 * q + (lane >> 3);
-              if (t < ch.rows) {
-                const uint4 v = *reinterpret_cast<const uint4 *>(&sm.staging[t * OUT_ROW_BYTES + (lane & 7) * 16]);
-                *reinterpret_cast<uint4 *>(p.act_q + ((int64_t)ch.row0 + t) * I + (int64_t)nt * TILE_N + (lane & 7) * 16) = v;
-              }
-            }
-#pragma unroll
-            for (int pp = 0; pp + 1 < NP; ++pp)
-#pragma unroll
-              for (int j = 0; j < 16; ++j) acc[pp][j] = acc[pp + 1][j];
-          }
-          if (!ok) break;
-          item_par ^= 1u;
-        } else {
-          // the staging rows may still be read by the row stores of the previous item, by any warp (the split of
-          // the rows over the column groups follows the chunk's width): all promotion warps meet first
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.isync);
-          if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.isync, iph, p.status, 8))) { ok = false; break; }
-          iph ^= 1u;
-          const bool vec_ok = (p.n_store & 7) == 0;
-#pragma unroll 1
-          for (int pc = 0; pc < my_p; ++pc) {
-            const float *av = &acc[0][0];
-            __nv_bfloat16 *os = stg_mine + pc * 16 * TILE_N;
-            const unsigned long long rowp_u = NPF > 1 && (pc >> 1) ? rowp_r[NPF - 1] : rowp_r[0];
-            const float wgt_u = NPF > 1 && (pc >> 1) ? wgt_r[NPF - 1] : wgt_r[0];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              float v = av[j];
-              if (p.weight_mode == LO_WEIGHT_FP32) v *= __shfl_sync(0xffffffffu, wgt_u, (pc & 1) * 16 + j);
-              os[j * TILE_N] = __float2bfloat16_rn(v);
-            }
-            mbar_arrive(&sm.esync[cg]);
-            if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.esync[cg], eph, p.status, 9))) { ok = false; break; }
-            eph ^= 1u;
-            // rows out: this warp takes tokens 4q .. 4q+3 of the piece, two rows per step, sixteen lanes x 16 bytes per row
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int tp = 4 * q + 2 * i + (lane >> 4);                       // token of the piece
-              const unsigned long long rowp = __shfl_sync(0xffffffffu, rowp_u, (pc & 1) * 16 + tp);
-              // bf16-product order: bf16(sum) * bf16(w), rounded once more: one packed multiply per two outputs
-              const __nv_bfloat162 w2 = __float2bfloat162_rn(__shfl_sync(0xffffffffu, wgt_u, (pc & 1) * 16 + tp));
-              const int64_t n0 = (int64_t)nt * TILE_N + (lane & 15) * 8;
-              if (rowp != 0ull && n0 < p.n_store) {
-                const uint8_t *src = &sm.staging[(col_begin + pc * 16 + tp) * OUT_ROW_BYTES + (lane & 15) * 16];
-                __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(rowp) + n0;
-                uint4 v = *reinterpret_cast<const uint4 *>(src);
-                if (p.weight_mode == LO_WEIGHT_BF16_PRODUCT) {
-                  __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&v);
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) h[e] = __hmul2(h[e], w2);
-                }
-                if (vec_ok) {
-                  *reinterpret_cast<uint4 *>(dst) = v;
-                } else {
-                  for (int e = 0; e < 8 && n0 + e < p.n_store; ++e) dst[e] = reinterpret_cast<const __nv_bfloat16 *>(&v)[e];
-                }
-              }
-            }
-#pragma unroll
-            for (int pp = 0; pp + 1 < NP; ++pp)
-#pragma unroll
-              for (int j = 0; j < 16; ++j) acc[pp][j] = acc[pp + 1][j];
-          }
-          if (!ok) break;
-        }
+        // the finished tile is in the staging buffer: over to the output warps
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.stg_full);
       }
     }
   }
