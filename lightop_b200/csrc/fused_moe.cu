@@ -380,6 +380,19 @@ extern "C" int lo_fused_moe_block_int8_noalloc(const void *x, const int8_t *w1, 
 // ---------------------------------------------------------------------------
 namespace lo {
 namespace {
+// Chunk sizes of the per-channel layer, by the rows an expert gets on average.  A chunk is one pass over the expert's weights and
+// one MMA N extent (an N = 256 MMA costs about 1.3 x an N = 128 one); the GEMM is instantiated per chunk cap, and narrow caps leave
+// shared memory for more weight slots and tensor memory for more accumulators.  Layer times at the DeepSeek-V3 shape:
+//   <= 56 rows per expert : 64-row chunks, 12 weight slots and 8 accumulators (against 128 rows: 1680 / 1760 us at 4 rows per
+//                           expert, 1780 / 1890 at 16, 1860 / 2040 at 32, 2040 / 2240 at 56; from 64 rows on it loses, 10 to 25 %
+//                           at 93, where most experts need a second chunk)
+//   57 .. 104             : 128-row chunks (at 93: 2480 us, with 256 rows 2550)
+//   105 .. 136            : 160-row chunks (at 128: 2600 us, with 128 rows 3150, with 256 rows 2740)
+//   above                 : 256-row chunks (at 187: 3080 us, with 160 rows 4190)
+inline int channel_chunk_rows_for(int64_t rows, int experts) {
+  const int64_t avg = rows / experts;
+  return avg <= 56 ? CHUNK_ROWS_SMALL : (avg <= 104 ? CHUNK_ROWS : (avg <= 136 ? CHUNK_ROWS_WIDE : 256));
+}
 struct ChannelLayout {
   int32_t *header;      // [0] num_tokens_post_pad, [1] num_chunks
   int8_t *xq;           // [sorted_cap, H]
@@ -448,11 +461,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   LO_REQUIRE(workspace_bytes >= L.bytes, "channel moe: workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t numel = M * topk;
-  // Largest chunk of one expert's rows handed to a CTA.  A chunk of up to 256 rows is one MMA N extent, so an
-  // expert with 129..256 rows streams its weights once instead of once per 128-row chunk (the second pass
-  // was found to miss L2 often), and an N = 256 MMA costs about 1.3x an N = 128 one.  The 256-row kernel
-  // stages fewer K blocks ahead, so it is used only when experts are expected to receive that many rows.
-  const int chunk_max = numel / align_E >= 64 ? 256 : 128;
+  const int chunk_max = channel_chunk_rows_for(numel, align_E);
   // 1. expert-major stable order, chunk table, position of every (token, slot)
   prof_mark(0, st);
   int rc = launch_align(topk_ids, ids_dtype, numel, align_E, FUSED_ALIGN_BLOCK, expert_map, expert_map ? 1 : 0,

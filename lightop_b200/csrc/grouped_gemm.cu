@@ -1305,6 +1305,7 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
     if (cap <= 32) return launch_mode<GEMM_CHANNEL, 32>(a, stream);
     if (cap <= 64) return launch_mode<GEMM_CHANNEL, 64>(a, stream);
     if (cap <= 128) return launch_mode<GEMM_CHANNEL, 128>(a, stream);
+    if (cap <= T_WIDE) return launch_mode<GEMM_CHANNEL, T_WIDE>(a, stream);
     return launch_mode<GEMM_CHANNEL, 256>(a, stream);
   }
   LO_REQUIRE(cap <= T_WIDE, "grouped gemm: block-scaled chunks hold at most 160 rows");

@@ -220,3 +220,18 @@ def test_fused_channel_rejects_bad_arguments(lo):
         lo.moe.fused_experts_impl_int8(x.to(DEV), w1.to(DEV), w2.to(DEV), w.to(DEV), ids.to(DEV), None,
                                        use_int8_w8a8=True, per_channel_quant=False, block_shape=None,
                                        w1_scale=w1_s.to(DEV), w2_scale=w2_s.to(DEV))
+
+
+@pytest.mark.parametrize("counts", [(56, 56), (57, 57), (104, 105), (105, 105), (160, 80), (161, 79), (145, 128), (136, 137), (137, 137), (7, 105)])
+def test_fused_channel_chunk_rule(lo, counts):
+    # both sides of every line of the chunk-size rule (rows per expert), chunks up to and just beyond each cap, a short second box
+    H, I, M = 256, 128, sum(counts)
+    w1, w2, _, _ = synthetic.make_weights(2, H, I, seed=3)
+    w1_s, w2_s = synthetic.make_channel_scales(2, H, I, seed=4)
+    x, _ = synthetic.make_activations(M, H, 2, seed=5)
+    g = torch.Generator().manual_seed(M)
+    ids = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)])[torch.randperm(M, generator=g)].view(M, 1)
+    w = torch.rand(M, 1, generator=g)
+    y = _run_fused(lo, x, w1, w2, w1_s, w2_s, w, ids)
+    _, mean_rel = assert_out_close(y, OC.fused_moe_channel_int8(x, w1, w2, w1_s, w2_s, w, ids), f"per-channel {counts}")
+    assert mean_rel < 2e-3
