@@ -245,12 +245,27 @@ int lo_expert_rows_block_int8_packed_put(const uint8_t *packed, int64_t T, const
  *           (python/lightop/gemmopt.py:633-639, csrc/asm/asm_gemm_w8a8.cu:136-147).
  * A [M,K] int8, a_scale [M,K/128] f32 (row-major), B [N,K] int8, b_scale [ceil(N/128), K/128] f32, C [M,N] bf16.
  * K a multiple of 128; N arbitrary (weight rows past N read as zero and are not stored).
- * Same kernel as the grouped GEMM with one expert.  workspace: lo_block_int8_linear_workspace_bytes(M).
+ * Same kernel as the grouped GEMM with one expert.  workspace: lo_block_int8_linear_workspace_bytes(M); with
+ * lo_block_int8_linear_split_workspace_bytes(M, N, K) bytes or more the K extent is dealt to several CTAs where the
+ * output tiles alone would leave most of them idle (the fp32 sums of the parts go through the workspace and are
+ * added in the order of K).
  */
 size_t lo_block_int8_linear_workspace_bytes(int64_t M);
 int lo_block_int8_linear(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale,
                          int64_t M, int64_t N, int64_t K, void *C, void *workspace, size_t workspace_bytes,
                          int32_t *status, void *stream);
+size_t lo_block_int8_linear_split_workspace_bytes(int64_t M, int64_t N, int64_t K);
+
+/*
+ * The same linear on activations that are not quantised yet: x [M,K] of type x_dtype (LO_BF16 / LO_F16 / LO_F32,
+ * 16-byte aligned) goes through lo_group_quant_int8 (group 128, eps 1e-10) into the workspace first.
+ * Replaces: apply_w8a8_block_int8_linear (python/lightop/_lmslim_native/layers/gemm/int8_utils.py:406-429).
+ * workspace: lo_block_int8_linear_dynamic_workspace_bytes(M, N, K).
+ */
+size_t lo_block_int8_linear_dynamic_workspace_bytes(int64_t M, int64_t N, int64_t K);
+int lo_block_int8_linear_dynamic(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N,
+                                 int64_t K, void *C, void *workspace, size_t workspace_bytes, int32_t *status,
+                                 void *stream);
 
 /* ---------------------------------------------------------------------------
  * Routers upstream of the expert layer other than plain softmax top-k.

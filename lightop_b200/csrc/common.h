@@ -79,6 +79,10 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
 int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, const int32_t *inv_pos, float eps,
                                int8_t *q_sorted, float *s_sorted, cudaStream_t stream);
 
+// Group quantisation of rows of any supported type, for a dependent launch of the kernel that follows.  quant.cu
+int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group_size, float eps, int8_t *q, float *s,
+                       cudaStream_t stream);
+
 // Per-token (whole-row) quantisation; with inv_pos the result goes to the token's sorted positions
 // (q_out [positions, K], s_out [positions]), without it to row `token`.  quant.cu
 int launch_token_quant(const void *x, int x_dtype, int64_t M, int64_t K, int topk, const int32_t *inv_pos, int8_t *q,
@@ -143,6 +147,15 @@ struct GemmArgs {
   // single (block-scaled) only: address of output row `sorted id`, one entry per id, instead of C + id * N.  The rows
   // may lie in another GPU's memory (a peer mapping): the epilogue writes them with plain 16-byte stores.
   const int64_t *row_dst;
+  // Without a chunk table: fixed_chunks chunks of at most max_chunk_rows rows, of one expert with rows_a rows (single mode) or of
+  // E experts with masked_m[e] rows each in a layout of max_m rows an expert (per-channel mode).
+  int fixed_chunks;
+  const int32_t *masked_m;
+  int64_t max_m;
+  // Single mode without a chunk table: the K extent of a tile in parts of split_steps K blocks (a multiple of 4), the fp32 sums
+  // of part i to partial[i][row][n] (null: not split).
+  int split_steps;
+  float *partial;
 };
 
 int launch_grouped_gemm(GemmMode mode, const GemmArgs &args, cudaStream_t stream);

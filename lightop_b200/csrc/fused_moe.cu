@@ -642,63 +642,158 @@ extern "C" int lo_expert_rows_block_int8_packed_put(const uint8_t *packed, int64
 // ---------------------------------------------------------------------------
 namespace lo {
 namespace {
-__global__ void linear_plan_kernel(int64_t M, int32_t *__restrict__ sorted_ids, Chunk *__restrict__ chunks,
-                                   int32_t *__restrict__ num_chunks) {
-  const int64_t n_chunks = (M + 127) / 128;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (int64_t)gridDim.x * blockDim.x)
-    sorted_ids[i] = (int32_t)i;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n_chunks; c += (int64_t)gridDim.x * blockDim.x) {
-    Chunk ch;
-    ch.expert = 0;
-    ch.row0 = (int32_t)(c * 128);
-    ch.rows = (int32_t)(M - c * 128 < 128 ? M - c * 128 : 128);
-    ch.pad = 0;
-    chunks[c] = ch;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *num_chunks = (int32_t)n_chunks;
-}
-struct LinearWs {
-  int32_t *num_chunks;
-  int32_t *sorted_ids;
-  Chunk *chunks;
-  size_t bytes;
+// How a dense call is cut.  Chunks of at most 128 rows; equally many each where all items run at the same time (129 rows: 80 and
+// 49), else full ones with the short one last, where it shortens the last wave (300 x 7168 x 2048: 18.7 against 20.6 us).
+// Where the tiles would leave half of the SMs or more without work, the K extent of a tile is dealt to n_split items of split_steps
+// K blocks (a multiple of four: the unit of the scale tables).  That adds a pass over the output in fp32 and a launch that adds
+// the parts up, 2 to 3 us, and takes K blocks off a CTA at about 0.2 us each: worth it from SPLIT_MIN_K K blocks on.  One row,
+// N = 576, K = 7168: 16.1 -> 8.3 us, 4096 x 7168: 16.5 -> 10.6 us, 129 rows, N = 4096: 27.0 -> 20.8 us; at K = 1280 to 2048 it
+// changed nothing or cost 1 us.
+constexpr int64_t LINEAR_CHUNK = 128;
+constexpr int SPLIT_MIN_STEPS = 4, SPLIT_MIN_K = 32;
+struct LinearPlan {
+  int chunk_rows, n_chunks, n_tiles, split_steps, n_split;
+  size_t partial_bytes;
 };
-LinearWs carve_linear(void *ws, int64_t M) {
-  LinearWs W;
-  Carver c(ws);
-  W.num_chunks = c.take<int32_t>(64);
-  W.sorted_ids = c.take<int32_t>(M);
-  W.chunks = c.take<Chunk>((M + 127) / 128 + 1);
-  W.bytes = c.off;
-  return W;
+LinearPlan plan_linear(int64_t M, int64_t N, int64_t K) {
+  LinearPlan L;
+  const int64_t n0 = ceil_div(M, LINEAR_CHUNK);
+  L.n_tiles = (int)ceil_div(N, 128);
+  L.chunk_rows = (int)(n0 == 1 ? M : (n0 * L.n_tiles <= sm_count() ? round_up(ceil_div(M, n0), 16) : LINEAR_CHUNK));
+  L.n_chunks = (int)ceil_div(M, L.chunk_rows);
+  const int64_t KB = K / 128, items = (int64_t)L.n_chunks * L.n_tiles;
+  const int64_t want = sm_count() / items;       // parts that fill the SMs once
+  L.split_steps = 0; L.n_split = 1; L.partial_bytes = 0;
+  if (want >= 2 && KB >= SPLIT_MIN_K) {
+    const int64_t steps = round_up(ceil_div(KB, want), SPLIT_MIN_STEPS);
+    if (ceil_div(KB, steps) >= 2) {
+      L.split_steps = (int)steps;
+      L.n_split = (int)ceil_div(KB, steps);
+      L.partial_bytes = (size_t)round_up((int64_t)L.n_split * M * N * 4, ALIGN_BYTES);
+    }
+  }
+  return L;
+}
+
+// C = bf16 of the parts' sum, added in the order of K.  One thread per VEC columns of a row of C.
+template <int VEC>
+__global__ void __launch_bounds__(128) linear_reduce_kernel(const float *__restrict__ partial, int n_split, int64_t total,
+                                                            __nv_bfloat16 *__restrict__ C) {
+  dependency_wait();
+  const int64_t i = ((int64_t)blockIdx.x * 128 + threadIdx.x) * VEC;
+  if (i >= total) return;
+  float a[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) a[v] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < n_split; ++s) {
+    const float *src = partial + (int64_t)s * total + i;
+    if (VEC == 4) {
+      const float4 f = *reinterpret_cast<const float4 *>(src);
+      a[0] += f.x; a[VEC > 1 ? 1 : 0] += f.y; a[VEC > 2 ? 2 : 0] += f.z; a[VEC > 3 ? 3 : 0] += f.w;
+    } else {
+      a[0] += *src;
+    }
+  }
+  if (VEC == 4) {
+    const __nv_bfloat162 lo2 = __floats2bfloat162_rn(a[0], a[VEC > 1 ? 1 : 0]), hi2 = __floats2bfloat162_rn(a[VEC > 2 ? 2 : 0], a[VEC > 3 ? 3 : 0]);
+    *reinterpret_cast<uint2 *>(C + i) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo2), *reinterpret_cast<const uint32_t *>(&hi2));
+  } else {
+    C[i] = __float2bfloat16_rn(a[0]);
+  }
+}
+
+int check_linear(int64_t M, int64_t N, int64_t K) {
+  LO_REQUIRE(M >= 0 && N >= 1 && K >= 128 && K % 128 == 0, "block int8 linear: bad shape (K must be a multiple of 128)");
+  LO_REQUIRE(M < (1LL << 30), "block int8 linear: too many rows");
+  return LO_OK;
+}
+
+int run_linear(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K,
+               void *C, const LinearPlan &L, float *partial, int32_t *status, cudaStream_t st) {
+  GemmArgs g{};
+  g.A = A; g.a_scale = a_scale; g.rows_a = M; g.max_chunk_rows = L.chunk_rows;
+  g.B = B; g.b_scale = b_scale; g.E = 1;
+  g.n_rows_per_expert = N; g.n_store = N; g.K = K; g.n_tiles = L.n_tiles;
+  g.numel_valid = M; g.fixed_chunks = L.n_chunks;
+  g.C = static_cast<__nv_bfloat16 *>(C);
+  g.weight_mode = LO_WEIGHT_NONE; g.status = status;
+  if (L.n_split > 1 && partial != nullptr) { g.split_steps = L.split_steps; g.partial = partial; }
+  const int rc = launch_grouped_gemm(GEMM_SINGLE, g, st);
+  if (rc != LO_OK || g.partial == nullptr) return rc;
+  const int64_t total = M * N;
+  const bool vec = total % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0;
+  const int64_t threads = vec ? total / 4 : total;
+  LO_CUDA_OK(launch_dependent(vec ? linear_reduce_kernel<4> : linear_reduce_kernel<1>, dim3((unsigned)ceil_div(threads, 128)), dim3(128), 0, st,
+                              (const float *)partial, L.n_split, total, static_cast<__nv_bfloat16 *>(C)));
+  return LO_OK;
 }
 }  // namespace
 }  // namespace lo
 
-extern "C" size_t lo_block_int8_linear_workspace_bytes(int64_t M) { return M <= 0 ? 0 : lo::carve_linear(nullptr, M).bytes; }
+extern "C" size_t lo_block_int8_linear_workspace_bytes(int64_t M) { return M <= 0 ? 0 : (size_t)lo::ALIGN_BYTES; }
+
+extern "C" size_t lo_block_int8_linear_split_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K < 128) return 0;
+  const size_t parts = lo::plan_linear(M, N, K).partial_bytes;
+  return parts > 0 ? parts : (size_t)lo::ALIGN_BYTES;
+}
 
 extern "C" int lo_block_int8_linear(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale,
                                     int64_t M, int64_t N, int64_t K, void *C, void *workspace, size_t workspace_bytes,
                                     int32_t *status, void *stream) {
   using namespace lo;
-  LO_REQUIRE(M >= 0 && N >= 1 && K >= 128 && K % 128 == 0, "block int8 linear: bad shape (K must be a multiple of 128)");
-  if (M == 0) return LO_OK;
+  const int rc = check_linear(M, N, K);
+  if (rc != LO_OK || M == 0) return rc;
   LO_REQUIRE(A && a_scale && B && b_scale && C && workspace, "block int8 linear: null pointer");
-  LO_REQUIRE(M < (1LL << 30), "block int8 linear: too many rows");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "block int8 linear: workspace must be 256-byte aligned");
-  LinearWs W = carve_linear(workspace, M);
-  LO_REQUIRE(workspace_bytes >= W.bytes, "block int8 linear: workspace of %zu bytes, %zu needed", workspace_bytes, W.bytes);
+  const LinearPlan L = plan_linear(M, N, K);
+  const size_t need = lo_block_int8_linear_workspace_bytes(M);
+  LO_REQUIRE(workspace_bytes >= need, "block int8 linear: workspace of %zu bytes, %zu needed", workspace_bytes, need);
+  // the K extent is split where the workspace has room for the parts
+  float *partial = L.n_split > 1 && workspace_bytes >= L.partial_bytes ? static_cast<float *>(workspace) : nullptr;
+  return run_linear(A, a_scale, B, b_scale, M, N, K, C, L, partial, status, static_cast<cudaStream_t>(stream));
+}
+
+namespace lo {
+namespace {
+struct DynLinearLayout {
+  int8_t *xq;
+  float *xs;
+  float *partial;
+  size_t bytes;
+};
+DynLinearLayout carve_dyn_linear(void *ws, int64_t M, int64_t K, const LinearPlan &L) {
+  DynLinearLayout D;
+  Carver c(ws);
+  D.xq = c.take<int8_t>(M * K);
+  D.xs = c.take<float>(M * (K / 128));
+  D.partial = c.take<float>((int64_t)(L.partial_bytes / 4));
+  D.bytes = c.off;
+  return D;
+}
+}  // namespace
+}  // namespace lo
+
+extern "C" size_t lo_block_int8_linear_dynamic_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K < 128) return 0;
+  return lo::carve_dyn_linear(nullptr, M, K, lo::plan_linear(M, N, K)).bytes;
+}
+
+extern "C" int lo_block_int8_linear_dynamic(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M,
+                                            int64_t N, int64_t K, void *C, void *workspace, size_t workspace_bytes,
+                                            int32_t *status, void *stream) {
+  using namespace lo;
+  int rc = check_linear(M, N, K);
+  if (rc != LO_OK || M == 0) return rc;
+  LO_REQUIRE(x && B && b_scale && C && workspace, "block int8 linear: null pointer");
+  LO_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0, "group quant: x must be 16-byte and q 8-byte aligned");
+  LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "block int8 linear: workspace must be 256-byte aligned");
+  const LinearPlan L = plan_linear(M, N, K);
+  DynLinearLayout D = carve_dyn_linear(workspace, M, K, L);
+  LO_REQUIRE(workspace_bytes >= D.bytes, "block int8 linear: workspace of %zu bytes, %zu needed", workspace_bytes, D.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int blocks = (int)(ceil_div(M, 256) > 1024 ? 1024 : ceil_div(M, 256));
-  linear_plan_kernel<<<blocks, 256, 0, st>>>(M, W.sorted_ids, W.chunks, W.num_chunks);
-  LO_LAUNCH_OK("linear_plan_kernel");
-  GemmArgs g{};
-  g.A = A; g.a_scale = a_scale; g.rows_a = M; g.max_chunk_rows = (int)(M < 128 ? M : 128);
-  g.B = B; g.b_scale = b_scale; g.E = 1;
-  g.n_rows_per_expert = N; g.n_store = N; g.K = K; g.n_tiles = (int)ceil_div(N, 128);
-  g.sorted_ids = W.sorted_ids; g.numel_valid = M;
-  g.chunks = W.chunks; g.num_chunks = W.num_chunks;
-  g.C = static_cast<__nv_bfloat16 *>(C);
-  g.weight_mode = LO_WEIGHT_NONE; g.status = status;
-  return launch_grouped_gemm(GEMM_SINGLE, g, st);
+  rc = launch_group_quant(x, x_dtype, M * (K / 128), 128, 1e-10f, D.xq, D.xs, st);
+  if (rc != LO_OK) return rc;
+  return run_linear(D.xq, D.xs, B, b_scale, M, N, K, C, L, D.partial, status, st);
 }

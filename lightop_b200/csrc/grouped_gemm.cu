@@ -446,6 +446,17 @@ struct KParams {
   int32_t *status;
   int out_by_position;      // bf16 output row = sorted position instead of the sorted id
   const int64_t *row_dst;   // single mode: address of the output row of every sorted id (null: C + id * n_store)
+  // Without a chunk table (chunks == null) the chunks follow from arithmetic: fixed_chunks of them, of at most chunk_rows rows.
+  int fixed_chunks;
+  int chunk_rows;
+  const int32_t *masked_m;  // per-channel mode: rows of each expert, in a layout of max_m rows an expert
+  int64_t max_m;
+  int64_t dense_rows;       // single mode: rows of the one expert
+  // Single mode: K blocks per item when the K extent of a tile is dealt to several items (0: not split), a multiple of
+  // SC_STEPS; the fp32 sums of part i then go to partial[i][row][n] instead of C.
+  int split_steps;
+  int n_split;
+  float *partial;
 };
 
 // Four tensor maps of the sorted activation matrix, box heights 16 / 32 / 64 / 128 rows.  A chunk of
@@ -459,20 +470,47 @@ __device__ __forceinline__ int a_map_index(int T) { return T <= 16 ? 0 : (T <= 3
 // Walks this CTA's items (chunk, output tile): blockIdx.x, blockIdx.x + gridDim.x, ... in chunk-major order.  Every role has
 // its own; the descriptor of the item after the current one is already on its way while the current one is worked on
 // (a round trip to L2 and two divisions between two items were a tenth of a down-GEMM item).
-struct ItemCursor {
-  const Chunk *chunks;
+// Where the chunks come from is part of the instantiation (a branch for it in the common kernel cost the block-scaled loops
+// registers and 3 to 9 % at 4096 rows).
+enum Form { TABLE, DENSE, SPLIT };      // chunk table / one expert, from arithmetic / the same with the K extent of a tile split
+template <int MODE, int FORM> struct ItemCursor {
+  const KParams &p;
   int num_chunks, n_tiles, ci, nt, step_c, step_t;
+  int k0, kn;            // K blocks of the item taken last
   int4 next;
   __device__ __forceinline__ void fetch() {
-    if (ci < num_chunks) next = *reinterpret_cast<const int4 *>(chunks + ci);
+    if (ci >= num_chunks) return;
+    if (FORM != TABLE || (MODE == GEMM_CHANNEL && p.chunks == nullptr)) {
+      if (MODE == GEMM_CHANNEL) {
+        const int per = (int)((p.max_m + p.chunk_rows - 1) / p.chunk_rows), e = ci / per, first = (ci - e * per) * p.chunk_rows;
+        const int64_t left = min((int64_t)p.masked_m[e], p.max_m) - first;
+        const int rows = left <= 0 ? 0 : (int)min(left, (int64_t)p.chunk_rows);
+        next = make_int4(rows > 0 ? e : -1, (int)(e * p.max_m) + first, rows, left > p.chunk_rows ? 1 : 0);
+      } else {
+        const int64_t first = (int64_t)ci * p.chunk_rows;
+        next = make_int4(0, (int)first, (int)min((int64_t)p.chunk_rows, p.dense_rows - first), 0);
+      }
+      return;
+    }
+    next = *reinterpret_cast<const int4 *>(p.chunks + ci);
   }
-  __device__ __forceinline__ ItemCursor(const Chunk *c, int n_chunks, int tiles)
-      : chunks(c), num_chunks(n_chunks), n_tiles(tiles), ci((int)blockIdx.x / tiles), nt((int)blockIdx.x % tiles),
-        step_c((int)gridDim.x / tiles), step_t((int)gridDim.x % tiles), next(make_int4(-1, 0, 0, 0)) { fetch(); }
+  __device__ __forceinline__ ItemCursor(const KParams &params, int n_chunks)
+      : p(params), num_chunks(n_chunks), n_tiles(FORM == SPLIT ? params.n_tiles * params.n_split : params.n_tiles),
+        k0(0), kn(params.KB), next(make_int4(-1, 0, 0, 0)) {
+    ci = (int)blockIdx.x / n_tiles; nt = (int)blockIdx.x % n_tiles;
+    step_c = (int)gridDim.x / n_tiles; step_t = (int)gridDim.x % n_tiles;
+    fetch();
+  }
   __device__ __forceinline__ bool take(Chunk &ch, int &tile) {
     if (ci >= num_chunks) return false;
     ch.expert = next.x; ch.row0 = next.y; ch.rows = next.z; ch.pad = next.w;
     tile = nt;
+    if constexpr (FORM == SPLIT) {
+      const int part = nt / p.n_tiles;
+      tile = nt - part * p.n_tiles;
+      k0 = part * p.split_steps;
+      kn = min(p.split_steps, p.KB - k0);
+    }
     ci += step_c;
     nt += step_t;
     if (nt >= n_tiles) { nt -= n_tiles; ++ci; }
@@ -481,7 +519,7 @@ struct ItemCursor {
   }
 };
 
-template <int MODE, int A_ROWS>
+template <int MODE, int A_ROWS, int FORM>
 __global__ void __launch_bounds__((Cfg<MODE, A_ROWS>::NUM_THREADS), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ AMaps a_maps, const KParams p) {
   using SM = Smem<MODE, A_ROWS>;
@@ -541,7 +579,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   dependency_wait();
   dependency_release();
 
-  const int num_chunks = *p.num_chunks;
+  static_assert(FORM == TABLE || (MODE == GEMM_SINGLE && A_ROWS <= T_MAX), "dense calls come with at most T_MAX rows a chunk");
+  const int num_chunks = FORM != TABLE || (MODE == GEMM_CHANNEL && p.chunks == nullptr) ? p.fixed_chunks : *p.num_chunks;
   const int KB = p.KB;
   Chunk ch;      // the item at hand: chunk and output tile
   int nt = 0;
@@ -556,14 +595,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         uint32_t it = 0;
         int s = 0;
         bool ok = true;
-        for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
+        for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
           if (ch.expert < 0) continue;
           // weight tiles are streamed (evict-first) unless another chunk of the same expert is about to read
           // them again: those stay in L2 under the normal policy
           const uint64_t pol_w = ch.pad ? pol_keep : pol_stream;
           for (int ph = 0; ph < PHASES && ok; ++ph) {
             const int32_t row_g = (int32_t)(ch.expert * p.n_rows_per_expert + (int64_t)(ph * p.n_tiles + nt) * TILE_N);
-            for (int kb = 0; kb < KB; ++kb, ++it) {
+            for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NW
               if (it >= (uint32_t)NW && !mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 1, LO_SLEEP_PRODUCER)) { ok = false; break; }
               mbar_arrive_expect_tx(&sm.ready[it % ND], W_TILE_BYTES);
@@ -582,7 +621,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         uint32_t it = 0;
         int s = 0;
         bool ok = true;
-        for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
+        for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
           if (ch.expert < 0) continue;
           const int T = (ch.rows + 15) & ~15;
           const int T0 = T > 128 ? 128 : T;                  // first box; the rest (if any) goes into a second one
@@ -590,7 +629,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           const int mi2 = T > 128 ? a_map_index(T - 128) : -1;
           const uint32_t a_bytes = (16u << mi) * TILE_K + (mi2 >= 0 ? (16u << mi2) * TILE_K : 0u);
           for (int ph = 0; ph < PHASES && ok; ++ph) {
-            for (int kb = 0; kb < KB; ++kb, ++it) {
+            for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NA
               if (it >= (uint32_t)NA && !mbar_wait(sm, &sm.done[(it - NA) % ND], ((it - NA) / ND) & 1u, p.status, 6, LO_SLEEP_PRODUCER)) { ok = false; break; }
               uint64_t *bar = &sm.ready[it % ND];
@@ -615,15 +654,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         constexpr int NU = (A_ROWS + 31) / 32;
         const int64_t nblk = (p.n_rows_per_expert + TILE_N - 1) / TILE_N;
         const bool vec = (KB & 3) == 0;
-        ItemCursor items(p.chunks, num_chunks, p.n_tiles);
-        struct Batch { Chunk ch; int nt, ph, kb; bool valid; };     // K blocks kb .. kb + 3 of a pass over an item
+        ItemCursor<MODE, FORM> items(p, num_chunks);
+        struct Batch { Chunk ch; int nt, ph, kb, k_end; bool valid; };     // K blocks kb .. kb + 3 of a pass over an item
         float a_cur[NU][4], b_cur[4], a_nxt[NU][4], b_nxt[4];
         auto next_item = [&](Batch &b) {
           do { b.valid = items.take(b.ch, b.nt); } while (b.valid && b.ch.expert < 0);
+          b.kb = FORM == SPLIT ? items.k0 : 0;
+          b.k_end = FORM == SPLIT ? items.k0 + items.kn : KB;
         };
         auto advance = [&](Batch &b) {
           b.kb += SC_STEPS;
-          if (b.kb >= KB) {
+          if (b.kb >= (FORM == SPLIT ? b.k_end : KB)) {
             b.kb = 0;
             if (++b.ph == PHASES) { b.ph = 0; next_item(b); }
           }
@@ -647,7 +688,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 4; ++i) b[i] = bt.kb + i < KB ? __ldg(bs + i) : 0.f;
         };
-        Batch cur{ch, 0, 0, 0, false};
+        Batch cur{ch, 0, 0, 0, 0, false};
         next_item(cur);
         if (cur.valid) fetch(cur, a_cur, b_cur);
         Batch nxt = cur;
@@ -676,7 +717,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           if (lane == 0) mbar_arrive(&sm.scales[slot]);
           slot = slot + 1 == (uint32_t)SC_BATCHES ? 0u : slot + 1;
           ++n_batch;
-          it += (uint32_t)(KB - cur.kb < SC_STEPS ? KB - cur.kb : SC_STEPS);
+          const int k_left = (FORM == SPLIT ? cur.k_end : KB) - cur.kb;
+          it += (uint32_t)(k_left < SC_STEPS ? k_left : SC_STEPS);
 #pragma unroll
           for (int i = 0; i + 1 < SC_BATCHES; ++i) end_of[i] = end_of[i + 1];
           end_of[SC_BATCHES - 1] = it - 1;
@@ -712,10 +754,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       const uint32_t my_off = lane == 0 ? 0u : 0u - (uint32_t)NBUF;
       uint32_t acc_par = 1;              // per-channel mode: phase of the accumulator ring
       bool ok = true, seen = lane > 1;
-      for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
+      for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
         if (ch.expert < 0) continue;
         const uint32_t idesc = make_idesc((uint32_t)((__shfl_sync(0xffffffffu, ch.rows, 0) + 15) & ~15));
-        const uint32_t steps = (uint32_t)(PHASES * KB);
+        const uint32_t steps = (uint32_t)(FORM == SPLIT ? items.kn : PHASES * KB);
 #pragma unroll 1
         for (uint32_t u = 0; u < steps; ++u, ++it) {
           if (!__all_sync(0xffffffffu, seen)) {
@@ -760,12 +802,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     if constexpr (CF::SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OUT));
     const int ow = warp - (FIRST_EPI_WARP + EPI_WARPS);
     uint32_t par = 0;
-    for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); items.take(ch, nt);) {
+    // (the parts of a split K extent leave the kernel as fp32 sums, straight from the promotion warps)
+    for (ItemCursor<MODE, FORM> items(p, FORM == SPLIT ? 0 : num_chunks); items.take(ch, nt);) {
       if (ch.expert < 0) {
         // block of a non-local expert: its output rows are zero
         if (MODE == GEMM_SINGLE && p.C != nullptr) {
           for (int t = ow; t < ch.rows; t += OUT_WARPS) {
-            const int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
+            const int32_t sid = FORM == TABLE && p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
             if (sid >= 0 && sid < p.numel_valid)
               for (int64_t n = (int64_t)nt * TILE_N + lane; n < (int64_t)(nt + 1) * TILE_N && n < p.n_store; n += 32)
                 p.C[(int64_t)(p.out_by_position ? ch.row0 + t : sid) * p.n_store + n] = __float2bfloat16_rn(0.f);
@@ -829,10 +872,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           const int t = (u * 16 + (lane >> 1)) * (2 * OUT_WARPS) + ow * 2 + (lane & 1);
           if (t < ch.rows) {
             // without a sorted-id table the id of a row is its position
-            const int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
+            const int32_t sid = FORM == TABLE && p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
             if (sid >= 0 && sid < p.numel_valid) {
               if (p.weight_mode == LO_WEIGHT_BF16_PRODUCT) wgt_r[u] = p.topk_weights[sid];
-              rowp_r[u] = p.row_dst != nullptr ? (unsigned long long)p.row_dst[sid]
+              rowp_r[u] = FORM == TABLE && p.row_dst != nullptr ? (unsigned long long)p.row_dst[sid]
                                                : (unsigned long long)(p.C + (int64_t)(p.out_by_position ? ch.row0 + t : sid) * p.n_store);
             }
           }
@@ -880,12 +923,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     uint32_t sc_slot = 0, sc_par = 0;            // ring of scale batches
     uint32_t buf = 0, step = 0;                  // block-scaled modes: partial buffer and count of the K-block step
     bool ok = true;
-    for (ItemCursor items(p.chunks, num_chunks, p.n_tiles); ok && items.take(ch, nt);) {
+    for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
       if (ch.expert < 0) {
         // block of a non-local expert: its output rows are zero (the block-scaled modes leave that to the output warps)
         if (MODE == GEMM_CHANNEL && p.C != nullptr) {
           for (int t = cg; t < ch.rows; t += NCG) {
-            const int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
+            const int32_t sid = FORM == TABLE && p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
             if (sid >= 0 && sid < p.numel_valid && (int64_t)nt * TILE_N + n_local < p.n_store)
               p.C[(int64_t)(p.out_by_position ? ch.row0 + t : sid) * p.n_store + (int64_t)nt * TILE_N + n_local] =
                   __float2bfloat16_rn(0.f);
@@ -918,7 +961,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           const int t = col_begin + u * 32 + lane;
           if (u * 32 + lane < my_p * 16 && t < ch.rows) {
             // without a sorted-id table the id of a row is its position
-            int32_t sid = p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
+            int32_t sid = FORM == TABLE && p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t;
             if (sid < 0 || sid >= p.numel_valid) sid = -1;
             if (sid >= 0 && p.weight_mode != LO_WEIGHT_NONE) wgt_r[u] = p.topk_weights[sid];
             if (sid >= 0 && p.out_by_position) sid = ch.row0 + t;
@@ -975,6 +1018,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         // stay in registers over the whole K loop, so tensor memory holds nothing but partial buffers and a
         // K block costs one tensor-memory load per piece of 16 columns.
         constexpr int NP = (A_ROWS / 16 + NCG - 1) / NCG;
+        const int kn = FORM == SPLIT ? items.kn : KB;
         float acc[NP][16];
         // Addresses of this item, formed once: the loops below only add constants to them.  Ring positions
         // (scale slot, partial buffer and its phase) are carried as counters instead of being divided out of
@@ -990,7 +1034,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                                   (uint32_t)(q * 32 + ((lane >> 3) & 1) * 8) * 2u;
         // fp32 routed weight of token t of the chunk (0 where there is no row)
         auto weight_of = [&](int t) {
-          const int32_t sid = t < ch.rows ? (p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t) : -1;
+          const int32_t sid = t < ch.rows ? (FORM == TABLE && p.sorted_ids ? p.sorted_ids[ch.row0 + t] : ch.row0 + t) : -1;
           return sid >= 0 && sid < p.numel_valid ? __ldg(p.topk_weights + sid) : 0.f;
         };
 #pragma unroll 1
@@ -1024,7 +1068,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (PC > 0) load_unit(0, part0 + buf * (uint32_t)A_ROWS, raw[0]);
             uint32_t sc_at = 0;
 #pragma unroll 1
-            for (int kb0 = 0; kb0 < KB; kb0 += UNROLL) {
+            for (int kb0 = 0; kb0 < kn; kb0 += UNROLL) {
               if ((kb0 & (SC_STEPS - 1)) == 0) {
                 // the scale products of the coming four steps
                 if (PC > 0 && !__all_sync(0xffffffffu, mbar_wait_addr(sm, scales0 + 8u * sc_slot, sc_par, p.status, 7))) { ok = false; return; }
@@ -1033,7 +1077,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
               }
 #pragma unroll
               for (int i = 0; i < UNROLL; ++i) {
-                if (i > 0 && kb0 + i >= KB) break;
+                if (i > 0 && kb0 + i >= kn) break;
                 const uint32_t part = part0 + buf * (uint32_t)A_ROWS;
                 const uint32_t used = consumed0 + 8u * dn;
                 buf = buf + 1 == (uint32_t)NBUF ? 0u : buf + 1;
@@ -1061,7 +1105,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                     // every value of the partial is in registers: the buffer goes back, the next step's first unit is asked for
                     tc_fence_before();
                     if (lane == 0) mbar_arrive_addr(used);
-                    if (kb0 + i + 1 < KB) {
+                    if (kb0 + i + 1 < kn) {
                       // warp-uniform outcome: the accesses to tensor memory are warp-collective
                       if (!__all_sync(0xffffffffu, next_done) &&
                           !__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; return; }
@@ -1099,8 +1143,22 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (my_p >= 5) k_loop(std::integral_constant<int, 5>{});
           }
           if (!ok) break;
+          if constexpr (FORM == SPLIT) {
+            // a part of the K extent: the sums as they are (eight lanes side by side hold eight channels of one token)
+            float *dst = p.partial + ((int64_t)(items.k0 / p.split_steps) * p.dense_rows + ch.row0) * p.n_store;
+#pragma unroll
+            for (int pc = 0; pc < NP; ++pc) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int t = col_begin + pc * 16 + ((j >> 2) & 1) * 8 + (lane & 3) * 2 + (j & 1);
+                const int64_t n = (int64_t)nt * TILE_N + q * 32 + (j >> 3) * 16 + ((j >> 1) & 1) * 8 + (lane >> 2);
+                if (pc < my_p && t < ch.rows && n < p.n_store) dst[t * p.n_store + n] = acc[pc][j];
+              }
+            }
+            continue;
+          }
           // routed weight on the fp32 sums (before their rounding), where the mode asks for it
-          if (p.weight_mode == LO_WEIGHT_FP32) {
+          if (FORM == TABLE && p.weight_mode == LO_WEIGHT_FP32) {
 #pragma unroll
             for (int pc = 0; pc < NP; ++pc) {
               if (pc < my_p) {
@@ -1171,6 +1229,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           }
         }
         if (!ok) break;
+        if (FORM == SPLIT) continue;
         // the finished tile is in the staging buffer: over to the output warps
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.stg_full);
@@ -1235,7 +1294,7 @@ int make_tile_map(CUtensorMap *map, const int8_t *base, int64_t rows, int64_t K,
   return LO_OK;
 }
 
-template <int MODE, int A_ROWS>
+template <int MODE, int A_ROWS, int FORM = TABLE>
 int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   using SM = Smem<MODE, A_ROWS>;
   static_assert(sizeof(SM) + 1024 <= SMEM_LIMIT, "shared-memory layout exceeds what a CTA can be given");
@@ -1248,7 +1307,7 @@ int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   int dev = 0;
   LO_CUDA_OK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !((configured_devices >> dev) & 1u)) {
-    LO_CUDA_OK(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, A_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
+    LO_CUDA_OK(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, A_ROWS, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
     if (dev >= 0 && dev < 64) configured_devices |= (uint64_t)1 << dev;
   }
   CUtensorMap wmap;
@@ -1266,9 +1325,11 @@ int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   p.chunks = a.chunks; p.num_chunks = a.num_chunks; p.act_q = a.act_q; p.act_s = a.act_s; p.C = a.C; p.row_dst = a.row_dst;
   p.topk_weights = a.topk_weights; p.weight_mode = a.weight_mode; p.act_eps = a.act_eps; p.status = a.status;
   p.out_by_position = a.out_by_position;
+  p.fixed_chunks = a.fixed_chunks; p.chunk_rows = a.max_chunk_rows; p.masked_m = a.masked_m; p.max_m = a.max_m; p.dense_rows = a.rows_a;
+  p.n_split = a.partial != nullptr ? (int)ceil_div(p.KB, a.split_steps) : 1; p.split_steps = a.split_steps; p.partial = a.partial;
   const int grid = sm_count();
   if (grid <= 0) return fail(LO_ERR_CUDA, "no CUDA device");
-  LO_CUDA_OK(launch_dependent(grouped_gemm_kernel<MODE, A_ROWS>, dim3(grid), dim3(Cfg<MODE, A_ROWS>::NUM_THREADS), smem_bytes, stream, wmap,
+  LO_CUDA_OK(launch_dependent(grouped_gemm_kernel<MODE, A_ROWS, FORM>, dim3(grid), dim3(Cfg<MODE, A_ROWS>::NUM_THREADS), smem_bytes, stream, wmap,
                               amaps, p));
   return LO_OK;
 }
@@ -1288,6 +1349,11 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
   LO_REQUIRE(a.row_dst == nullptr || (mode == GEMM_SINGLE && a.n_rows_per_expert % 8 == 0 && a.out_by_position == 0),
              "grouped gemm: a table of row addresses serves the single block-scaled mode with N a multiple of 8");
   LO_REQUIRE(mode == GEMM_GATE_UP || a.C != nullptr || a.row_dst != nullptr, "grouped gemm: no output");
+  LO_REQUIRE(a.chunks != nullptr || (a.fixed_chunks >= 1 && a.max_chunk_rows >= 1 && ((mode == GEMM_SINGLE && a.max_chunk_rows <= T_MAX) || (mode == GEMM_CHANNEL && a.masked_m != nullptr))),
+             "grouped gemm: no chunk table");
+  LO_REQUIRE(a.partial == nullptr || (mode == GEMM_SINGLE && a.chunks == nullptr && a.max_chunk_rows <= T_MAX && a.split_steps >= SC_STEPS &&
+                                      a.split_steps % SC_STEPS == 0 && a.weight_mode == LO_WEIGHT_NONE),
+             "grouped gemm: the K extent is split for dense calls only");
   // no chunk can hold more rows than max_chunk_rows (a bound the caller derives from the token count)
   const int cap = a.max_chunk_rows <= 0 ? T_MAX : a.max_chunk_rows;
   if (mode == GEMM_GATE_UP) {
@@ -1309,6 +1375,16 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
     return launch_mode<GEMM_CHANNEL, 256>(a, stream);
   }
   LO_REQUIRE(cap <= T_WIDE, "grouped gemm: block-scaled chunks hold at most 160 rows");
+  if (a.partial != nullptr) {
+    if (cap <= 32) return launch_mode<GEMM_SINGLE, 32, SPLIT>(a, stream);
+    if (cap <= 64) return launch_mode<GEMM_SINGLE, 64, SPLIT>(a, stream);
+    return launch_mode<GEMM_SINGLE, 128, SPLIT>(a, stream);
+  }
+  if (a.chunks == nullptr) {
+    if (cap <= 32) return launch_mode<GEMM_SINGLE, 32, DENSE>(a, stream);
+    if (cap <= 64) return launch_mode<GEMM_SINGLE, 64, DENSE>(a, stream);
+    return launch_mode<GEMM_SINGLE, 128, DENSE>(a, stream);
+  }
   if (cap <= 32) return launch_mode<GEMM_SINGLE, 32>(a, stream);
   if (cap <= 64) return launch_mode<GEMM_SINGLE, 64>(a, stream);
   if (cap <= 128) return launch_mode<GEMM_SINGLE, 128>(a, stream);

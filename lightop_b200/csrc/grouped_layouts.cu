@@ -4,7 +4,8 @@
 //               consecutive and every 128-row block holds rows of one expert only (the alignment the producer
 //               pads to, a multiple of 128), padding rows at the end of the expert's range;
 //   masked:     A [E, max_m, K]; only the first masked_m[e] rows of expert e exist.
-// Both only need a chunk table for the grouped GEMM kernel: no permutation, output rows = input rows.
+// The first needs a chunk table for the grouped GEMM kernel, which forms that of the second from the row counts itself: no
+// permutation, output rows = input rows.
 #include "common.h"
 
 namespace lo {
@@ -62,26 +63,6 @@ __global__ void contig_plan_kernel(const int32_t *__restrict__ m_indices, int64_
   }
 }
 
-// One thread per (expert, 256-row block of its max_m rows).
-__global__ void masked_plan_kernel(const int32_t *__restrict__ masked_m, int E, int64_t max_m, int blocks_per_expert,
-                                   Chunk *__restrict__ chunks, int32_t *__restrict__ num_chunks) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)E * blocks_per_expert) return;
-  const int e = (int)(i / blocks_per_expert);
-  const int b = (int)(i % blocks_per_expert);
-  int64_t valid = masked_m[e];
-  valid = valid < 0 ? 0 : (valid > max_m ? max_m : valid);
-  int64_t rows = valid - (int64_t)b * 256;
-  rows = rows < 0 ? 0 : (rows > 256 ? 256 : rows);
-  Chunk c;
-  c.expert = rows > 0 ? e : -1;
-  c.row0 = (int32_t)(e * max_m + (int64_t)b * 256);
-  c.rows = (int32_t)rows;
-  c.pad = 0;
-  chunks[i] = c;
-  if (i == 0) *num_chunks = E * blocks_per_expert;
-}
-
 struct PlanWs {
   int32_t *num_chunks;
   Chunk *chunks;
@@ -99,17 +80,16 @@ PlanWs carve_plan(void *ws, int64_t max_chunks) {
   return W;
 }
 
-int run_channel_gemm(const int8_t *A, const float *a_scale, int64_t rows_a, const int8_t *B, const float *b_scale, int E,
-                     int64_t N, int64_t K, void *C, const PlanWs &W, int cap, int32_t *status, cudaStream_t st) {
+GemmArgs channel_args(const int8_t *A, const float *a_scale, int64_t rows_a, const int8_t *B, const float *b_scale, int E,
+                      int64_t N, int64_t K, void *C, int cap, int32_t *status) {
   GemmArgs g{};
   g.A = A; g.a_scale = a_scale; g.rows_a = rows_a; g.max_chunk_rows = cap;
   g.B = B; g.b_scale = b_scale; g.E = E;
   g.n_rows_per_expert = N; g.K = K; g.n_tiles = (int)(N / 128);
   g.sorted_ids = nullptr; g.numel_valid = rows_a;       // output row = input row
-  g.chunks = W.chunks; g.num_chunks = W.num_chunks;
   g.C = static_cast<__nv_bfloat16 *>(C);
   g.weight_mode = LO_WEIGHT_NONE; g.status = status;
-  return launch_grouped_gemm(GEMM_CHANNEL, g, st);
+  return g;
 }
 
 }  // namespace
@@ -139,7 +119,9 @@ extern "C" int lo_m_grouped_w8a8_gemm_nt_contig(const int8_t *A, const float *a_
   const int64_t threads = n_sb * 32;
   contig_plan_kernel<<<(unsigned)ceil_div(threads, 256), 256, 0, st>>>(m_indices, M, E, W.chunks, W.num_chunks, status);
   LO_LAUNCH_OK("contig_plan_kernel");
-  return run_channel_gemm(A, a_scale, M, B, b_scale, E, N, K, C, W, (int)(M < 256 ? M : 256), status, st);
+  GemmArgs g = channel_args(A, a_scale, M, B, b_scale, E, N, K, C, (int)(M < 256 ? M : 256), status);
+  g.chunks = W.chunks; g.num_chunks = W.num_chunks;
+  return launch_grouped_gemm(GEMM_CHANNEL, g, st);
 }
 
 extern "C" int lo_m_grouped_w8a8_gemm_nt_masked(const int8_t *A, const float *a_scale, const int8_t *B,
@@ -153,11 +135,12 @@ extern "C" int lo_m_grouped_w8a8_gemm_nt_masked(const int8_t *A, const float *a_
   LO_REQUIRE(K % 128 == 0 && N % 128 == 0, "grouped gemm (masked): N and K must be multiples of 128");
   LO_REQUIRE((int64_t)E * max_m < (1LL << 31), "grouped gemm (masked): too many rows");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "grouped gemm (masked): workspace must be 256-byte aligned");
-  const int bpe = (int)((max_m + 255) / 256);
-  PlanWs W = carve_plan(workspace, (int64_t)E * bpe);
+  PlanWs W = carve_plan(workspace, (int64_t)E * ((max_m + 255) / 256));
   LO_REQUIRE(workspace_bytes >= W.bytes, "grouped gemm (masked): workspace of %zu bytes, %zu needed", workspace_bytes, W.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  masked_plan_kernel<<<(unsigned)ceil_div((int64_t)E * bpe, 256), 256, 0, st>>>(masked_m, E, max_m, bpe, W.chunks, W.num_chunks);
-  LO_LAUNCH_OK("masked_plan_kernel");
-  return run_channel_gemm(A, a_scale, (int64_t)E * max_m, B, b_scale, E, N, K, C, W, (int)(max_m < 256 ? max_m : 256), status, st);
+  // the chunks follow from the row counts: the kernel forms them itself
+  const int cap = (int)(max_m < 256 ? max_m : 256);
+  GemmArgs g = channel_args(A, a_scale, (int64_t)E * max_m, B, b_scale, E, N, K, C, cap, status);
+  g.masked_m = masked_m; g.max_m = max_m; g.fixed_chunks = E * (int)ceil_div(max_m, cap);
+  return launch_grouped_gemm(GEMM_CHANNEL, g, st);
 }

@@ -50,6 +50,7 @@ template <typename T, int LANES>
 __global__ void __launch_bounds__(256) group_quant_kernel(const T *__restrict__ x, int8_t *__restrict__ q,
                                                           float *__restrict__ s, int64_t num_groups,
                                                           float eps_t) {
+  dependency_release();      // (a dependent kernel waits for the whole grid before it reads)
   const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t group = gthread / LANES;
   const int lane_in_group = (int)(gthread % LANES);
@@ -330,6 +331,17 @@ int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, co
   return LO_OK;
 }
 
+int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group_size, float eps, int8_t *q, float *s,
+                       cudaStream_t st) {
+  const float eps_t = round_eps_to_dtype(eps, x_dtype);
+  switch (x_dtype) {
+    case LO_BF16: return launch_typed<__nv_bfloat16>(x, num_groups, group_size, eps_t, q, s, st);
+    case LO_F16: return launch_typed<__half>(x, num_groups, group_size, eps_t, q, s, st);
+    case LO_F32: return launch_typed<float>(x, num_groups, group_size, eps_t, q, s, st);
+    default: return fail(LO_ERR_UNSUPPORTED, "group quant: unsupported input dtype code %d", x_dtype);
+  }
+}
+
 int launch_token_quant(const void *x, int x_dtype, int64_t M, int64_t K, int topk, const int32_t *inv_pos, int8_t *q,
                        float *s, cudaStream_t stream) {
   if (M == 0) return LO_OK;
@@ -410,12 +422,5 @@ extern "C" int lo_group_quant_int8(const void *x, int x_dtype, int64_t num_group
   LO_REQUIRE(x && q && s, "group quant: null pointer");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0,
              "group quant: x must be 16-byte and q 8-byte aligned");
-  const float eps_t = round_eps_to_dtype(eps, x_dtype);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (x_dtype) {
-    case LO_BF16: return launch_typed<__nv_bfloat16>(x, num_groups, group_size, eps_t, q, s, st);
-    case LO_F16: return launch_typed<__half>(x, num_groups, group_size, eps_t, q, s, st);
-    case LO_F32: return launch_typed<float>(x, num_groups, group_size, eps_t, q, s, st);
-    default: return fail(LO_ERR_UNSUPPORTED, "group quant: unsupported input dtype code %d", x_dtype);
-  }
+  return launch_group_quant(x, x_dtype, num_groups, group_size, eps, q, s, static_cast<cudaStream_t>(stream));
 }

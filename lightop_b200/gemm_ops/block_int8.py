@@ -38,7 +38,7 @@ def matmul_block_int8(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs: to
     C = torch.empty(M, N, dtype=torch.bfloat16, device=A.device)
     if M:
         lib = _lib.load()
-        nbytes = lib.lo_block_int8_linear_workspace_bytes(M)
+        nbytes = lib.lo_block_int8_linear_split_workspace_bytes(M, N, K)
         ws = torch.empty(nbytes, dtype=torch.uint8, device=A.device)
         with torch.cuda.device(A.device):
             st = lib.lo_block_int8_linear(_lib.ptr(a2), _lib.ptr(as2), _lib.ptr(B), _lib.ptr(bs2), M, N, K,
@@ -67,6 +67,30 @@ def gemm_w8a8_asm(a, b, scale_a, scale_b, block_size, out_dtype, layout="TN"):
     return matmul_block_int8(a, b, scale_a.contiguous(), scale_b, block_size, output_dtype=out_dtype)
 
 
+def _dynamic_linear(x: torch.Tensor, w: torch.Tensor, block_size: List[int], w_s: torch.Tensor) -> Optional[torch.Tensor]:
+    """Quantisation and GEMM in one native call; None for the forms that the two separate operators take or refuse."""
+    if list(block_size) != [128, 128] or w.dim() != 2 or x.dim() == 0 or x.dtype not in (torch.bfloat16, torch.float16, torch.float32):
+        return None
+    N, K = w.shape
+    if (x.shape[-1] != K or K == 0 or K % 128 != 0 or x.numel() == 0 or N == 0 or w.dtype != torch.int8 or not w.is_contiguous()
+            or not x.is_contiguous() or tuple(w_s.shape) != ((N + 127) // 128, K // 128)
+            or not (x.is_cuda and x.device == w.device == w_s.device)):
+        return None
+    M = x.numel() // K
+    bs = w_s if w_s.dtype is torch.float32 and w_s.is_contiguous() else w_s.to(torch.float32).contiguous()
+    lib = _lib.load()
+    dev = x.device
+    C = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=dev)
+    nbytes = lib.lo_block_int8_linear_dynamic_workspace_bytes(M, N, K)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    with torch.cuda.device(dev):
+        st = lib.lo_block_int8_linear_dynamic(_lib.ptr(x), _lib.dtype_code(x.dtype), _lib.ptr(w), _lib.ptr(bs), M, N, K,
+                                              _lib.ptr(C), _lib.ptr(ws), nbytes, _lib.ptr(device_status_word(dev)),
+                                              _lib.current_stream(dev))
+    _lib.check(st, "apply_w8a8_block_int8_linear")
+    return C if x.dtype == torch.bfloat16 else C.to(x.dtype)
+
+
 def apply_w8a8_block_int8_linear(input: torch.Tensor, weight: torch.Tensor, block_size: List[int],
                                  weight_scale: torch.Tensor, input_scale: Optional[torch.Tensor] = None,
                                  bias: Optional[torch.Tensor] = None, config: Optional[dict] = None) -> torch.Tensor:
@@ -75,6 +99,9 @@ def apply_w8a8_block_int8_linear(input: torch.Tensor, weight: torch.Tensor, bloc
     Reference: ``apply_w8a8_block_int8_linear`` (int8_utils.py:406-429).
     """
     assert input_scale is None
+    output = _dynamic_linear(input, weight, block_size, weight_scale)
+    if output is not None:
+        return output if bias is None else (output + bias).to(dtype=input.dtype)
     input_2d = input.reshape(-1, input.shape[-1])
     output_shape = [*input.shape[:-1], weight.shape[0]]
     q_input, x_scale = per_token_group_quant_int8(input_2d, block_size[1])

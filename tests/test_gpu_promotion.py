@@ -40,3 +40,60 @@ def test_linear_remainders(M, N, K):
     torch.cuda.synchronize()
     lo.check_device_status()
     assert_gemm_close(out, ref, f"linear {M}x{N}x{K}")
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 576, 7168), (3, 201, 4096), (33, 128, 4224), (64, 1000, 4096), (129, 136, 7168), (300, 576, 4224), (500, 520, 4096)])
+def test_linear_with_a_split_k_extent(M, N, K):
+    # 32, 33 and 56 K blocks in parts that end even and uneven, rows and columns that leave remainders (201 * 3 is odd: the scalar
+    # form of the reduction), one to four chunks; the same call without room for the parts takes the undivided form
+    import lightop_b200 as lo
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16)
+    aq, a_s = O.group_quant_int8(x, 128)
+    B = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8)
+    b_s = torch.rand((N + 127) // 128, K // 128, generator=g) * 9e-3 + 1e-3
+    ref = O.block_int8_matmul(aq, B, a_s, b_s, (128, 128), torch.bfloat16)
+    d_aq, d_as, d_B, d_bs = aq.to(DEV), a_s.to(DEV), B.to(DEV), b_s.to(DEV)
+    assert lib.lo_block_int8_linear_split_workspace_bytes(M, N, K) >= 4 * 2 * M * N      # at least two parts
+    out = lo.gemm_ops.matmul_block_int8(d_aq, d_B, d_as, d_bs, [128, 128], torch.bfloat16)
+    fused = lo.gemm_ops.apply_w8a8_block_int8_linear(x.to(DEV), d_B, [128, 128], d_bs)
+    whole = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ws = torch.empty(256, dtype=torch.uint8, device=DEV)
+    st = lib.lo_block_int8_linear(d_aq.data_ptr(), d_as.data_ptr(), d_B.data_ptr(), d_bs.data_ptr(), M, N, K, whole.data_ptr(),
+                                  ws.data_ptr(), 256, 0, torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    torch.cuda.synchronize()
+    lo.check_device_status()
+    assert_gemm_close(out, ref, f"split linear {M}x{N}x{K}")
+    assert_gemm_close(whole, ref, f"undivided linear {M}x{N}x{K}")
+    assert torch.equal(out, fused)
+    # the sum of the parts is no further from 64 bits than the undivided sum (before their rounding to bf16 both err by a few
+    # ulps of fp32, so the bf16 results may differ by one step where they straddle a rounding)
+    exact = sum((aq[:, i:i + 128].double() @ B[:, i:i + 128].double().T) * a_s[:, i // 128, None].double()
+                * b_s[:, i // 128].double().repeat_interleave(128)[:N] for i in range(0, K, 128))
+    err = [float((y.cpu().double() - exact).norm() / exact.norm()) for y in (out, whole)]
+    assert err[0] <= err[1] * 1.001
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(5, 256), (2, 3, 4096), (256,)])
+def test_linear_in_one_call_equals_its_two_operators(dtype, shape):
+    import lightop_b200 as lo
+    g = torch.Generator().manual_seed(len(shape))
+    x = torch.randn(*shape, generator=g).to(dtype).to(DEV)
+    K = shape[-1]
+    B = torch.randint(-127, 128, (200, K), generator=g, dtype=torch.int8).to(DEV)
+    b_s = (torch.rand(2, K // 128, generator=g) * 9e-3 + 1e-3).to(DEV)
+    bias = torch.randn(200, generator=g).to(dtype).to(DEV)
+    q, s = lo.quant.per_token_group_quant_int8(x.reshape(-1, K), 128)
+    ref = lo.gemm_ops.matmul_block_int8(q, B, s, b_s, [128, 128], output_dtype=dtype)
+    y = lo.gemm_ops.apply_w8a8_block_int8_linear(x, B, [128, 128], b_s)
+    assert y.dtype == dtype and y.shape == x.shape[:-1] + (200,) and torch.equal(y.reshape(ref.shape), ref)
+    yb = lo.gemm_ops.apply_w8a8_block_int8_linear(x, B, [128, 128], b_s, bias=bias)
+    assert torch.equal(yb.reshape(ref.shape), (ref + bias).to(dtype))
+    # a strided input takes the general path, with the same result
+    wide = torch.zeros(*shape[:-1], 2 * K, dtype=dtype, device=DEV)
+    wide[..., ::2] = x
+    assert torch.equal(lo.gemm_ops.apply_w8a8_block_int8_linear(wide[..., ::2], B, [128, 128], b_s), y)
