@@ -97,22 +97,20 @@ int launch_silu_mul_token_quant(const void *in, int64_t rows, int64_t d, const i
 
 // Copy int8 rows and their scales into sorted-position order: row(pos) = sorted_ids[pos] / top_k.
 // scales_per_row = 0 means K / 128 (block scales); 1 is the per-token format.  a_stride = 0 means K bytes between
-// source rows; with a_scale == nullptr the scales of a row follow it inside its a_stride-byte record.  reduce.cu
+// source rows; with a_scale == nullptr the scales of a row follow it inside its a_stride-byte record.  With `chunks` the same
+// kernel writes the chunk table of the caller's block table (expert_ids, one entry per block_size positions): blocks of more
+// than 128 positions become chunks of 128.  reduce.cu
 int launch_permute_rows(const int8_t *A, const float *a_scale, int64_t rows_a, int64_t K, const int32_t *sorted_ids,
                         int64_t sorted_capacity, const int32_t *num_tokens_post_pad, int64_t numel_valid, int top_k,
                         int8_t *A_sorted, float *a_scale_sorted, cudaStream_t stream, int64_t scales_per_row = 0,
-                        int64_t a_stride = 0);
+                        int64_t a_stride = 0, const int32_t *expert_ids = nullptr, int block_size = 0, Chunk *chunks = nullptr,
+                        int32_t *num_chunks = nullptr);
 
 // Expert id and routed weight of packed dispatch records (lo_ep_dispatch_pack) into contiguous arrays.  reduce.cu
 int launch_ep_unpack_meta(const uint8_t *packed, int64_t rows, int64_t stride, int64_t meta_off, int32_t *row_expert,
                           float *row_weight, cudaStream_t stream, const int32_t *seg_first = nullptr,
                           const int64_t *seg_ret = nullptr, int world = 0, int64_t ret_row_bytes = 0,
                           int64_t *row_dst = nullptr);
-
-// Chunk table from an existing (expert_ids, num_tokens_post_pad) pair, see routing.cu.
-int launch_chunks_from_blocks(const int32_t *expert_ids, const int32_t *num_tokens_post_pad,
-                              int block_size, int64_t max_blocks, Chunk *chunks, int32_t *num_chunks,
-                              cudaStream_t stream);
 
 // GEMM_GATE_UP / GEMM_SINGLE: 128x128 block scales (a_scale [rows, K/128], b_scale [E, N/128, K/128]).
 // GEMM_CHANNEL: one scale per token and per output channel (a_scale [rows], b_scale [E, N]); bf16 output

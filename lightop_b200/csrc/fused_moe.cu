@@ -265,11 +265,8 @@ int grouped_gemm_on_blocks(GemmMode mode, const int8_t *A, const float *a_scale,
   GemmWs W = carve_gemm(workspace, sorted_capacity, block_size, K);   // sized for block scales; per-token scales need less
   LO_REQUIRE(workspace_bytes >= W.bytes, "grouped gemm: workspace of %zu bytes, %zu needed", workspace_bytes, W.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t max_blocks = ceil_div(sorted_capacity, block_size);
-  int rc = launch_chunks_from_blocks(expert_ids, num_tokens_post_pad, block_size, max_blocks, W.chunks, W.num_chunks, st);
-  if (rc != LO_OK) return rc;
-  rc = launch_permute_rows(A, a_scale, rows_a, K, sorted_ids, sorted_capacity, num_tokens_post_pad, numel_valid, top_k,
-                           W.a_sorted, W.as_sorted, st, mode == GEMM_CHANNEL ? 1 : 0);
+  int rc = launch_permute_rows(A, a_scale, rows_a, K, sorted_ids, sorted_capacity, num_tokens_post_pad, numel_valid, top_k,
+                           W.a_sorted, W.as_sorted, st, mode == GEMM_CHANNEL ? 1 : 0, 0, expert_ids, block_size, W.chunks, W.num_chunks);
   if (rc != LO_OK) return rc;
   GemmArgs g{};
   g.A = W.a_sorted; g.a_scale = W.as_sorted; g.rows_a = sorted_capacity;

@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(GATE_WARPS * 32) fused_gate_kernel(
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int64_t row = (int64_t)blockIdx.x * GATE_WARPS + warp;
+  dependency_release();      // the alignment kernel may get its block resident; it waits for this grid before it reads
   if (row >= M) return;
   float *s_row = gate_smem + (size_t)warp * 2 * E;
   float *p_row = s_row + E;

@@ -166,6 +166,8 @@ __global__ void __launch_bounds__(TOKEN_QUANT_THREADS) token_quant_kernel(const 
                                                                           int8_t *__restrict__ q, float *__restrict__ s) {
   __shared__ float red[8];
   const int64_t row = blockIdx.x;
+  dependency_wait();
+  dependency_release();
   const T *xr = x + row * K;
   // rows of a length that is not a multiple of 8 are not 16-byte aligned: they take the scalar loops only
   const int64_t vecs = (K & 7) == 0 ? K / 8 : 0;
@@ -222,6 +224,8 @@ __global__ void __launch_bounds__(TOKEN_QUANT_THREADS) silu_mul_token_quant_kern
     int8_t *__restrict__ q, float *__restrict__ s) {
   __shared__ float red[8];
   const int64_t row = blockIdx.x;
+  dependency_wait();
+  dependency_release();
   if (num_rows_dev && row >= *num_rows_dev) return;
   // masked layout [groups, group_rows, 2d]: only the first group_counts[g] rows of a group exist
   if (group_counts && row % group_rows >= group_counts[row / group_rows]) return;
@@ -352,17 +356,16 @@ int launch_token_quant(const void *x, int x_dtype, int64_t M, int64_t K, int top
   const unsigned blocks = (unsigned)M;
   switch (x_dtype) {
     case LO_BF16:
-      token_quant_kernel<__nv_bfloat16><<<blocks, TOKEN_QUANT_THREADS, 0, stream>>>(static_cast<const __nv_bfloat16 *>(x), K, topk, inv_pos, q, s);
+      LO_CUDA_OK(launch_dependent(token_quant_kernel<__nv_bfloat16>, dim3(blocks), dim3(TOKEN_QUANT_THREADS), 0, stream, static_cast<const __nv_bfloat16 *>(x), K, topk, inv_pos, q, s));
       break;
     case LO_F16:
-      token_quant_kernel<__half><<<blocks, TOKEN_QUANT_THREADS, 0, stream>>>(static_cast<const __half *>(x), K, topk, inv_pos, q, s);
+      LO_CUDA_OK(launch_dependent(token_quant_kernel<__half>, dim3(blocks), dim3(TOKEN_QUANT_THREADS), 0, stream, static_cast<const __half *>(x), K, topk, inv_pos, q, s));
       break;
     case LO_F32:
-      token_quant_kernel<float><<<blocks, TOKEN_QUANT_THREADS, 0, stream>>>(static_cast<const float *>(x), K, topk, inv_pos, q, s);
+      LO_CUDA_OK(launch_dependent(token_quant_kernel<float>, dim3(blocks), dim3(TOKEN_QUANT_THREADS), 0, stream, static_cast<const float *>(x), K, topk, inv_pos, q, s));
       break;
     default: return fail(LO_ERR_UNSUPPORTED, "per-token quant: unsupported input dtype code %d", x_dtype);
   }
-  LO_LAUNCH_OK("token_quant_kernel");
   return LO_OK;
 }
 
@@ -372,10 +375,9 @@ int launch_silu_mul_token_quant(const void *in, int64_t rows, int64_t d, const i
   if (rows == 0) return LO_OK;
   LO_REQUIRE(d >= 8 && d % 8 == 0, "silu-mul quant: width %lld must be a multiple of 8", (long long)d);
   LO_REQUIRE(rows <= 0x7fffffffLL, "silu-mul quant: too many rows");
-  silu_mul_token_quant_kernel<<<(unsigned)rows, TOKEN_QUANT_THREADS, 0, stream>>>(
-      static_cast<const __nv_bfloat16 *>(in), d, row_ids, numel_valid, num_rows_dev, group_rows > 0 ? group_rows : 1,
-      group_counts, q, s);
-  LO_LAUNCH_OK("silu_mul_token_quant_kernel");
+  LO_CUDA_OK(launch_dependent(silu_mul_token_quant_kernel, dim3((unsigned)rows), dim3(TOKEN_QUANT_THREADS), 0, stream,
+                              static_cast<const __nv_bfloat16 *>(in), d, row_ids, numel_valid, num_rows_dev,
+                              group_rows > 0 ? group_rows : (int64_t)1, group_counts, q, s));
   return LO_OK;
 }
 

@@ -384,8 +384,28 @@ __global__ void __launch_bounds__(128) permute_rows_kernel(const int8_t *__restr
                                                            const int32_t *__restrict__ num_tokens_post_pad,
                                                            int64_t numel_valid, int top_k, int64_t kb,
                                                            int8_t *__restrict__ A_sorted,
-                                                           float *__restrict__ a_scale_sorted, int64_t a_stride) {
+                                                           float *__restrict__ a_scale_sorted, int64_t a_stride,
+                                                           const int32_t *__restrict__ expert_ids, int block_size,
+                                                           Chunk *__restrict__ chunks, int32_t *__restrict__ num_chunks) {
   const int64_t pos = blockIdx.x;
+  dependency_wait();
+  dependency_release();
+  if (chunks != nullptr && threadIdx.x == 0) {
+    const int rows = block_size <= 128 ? block_size : 128;
+    const int64_t total = (int64_t)(*num_tokens_post_pad / block_size) * block_size;      // positions of whole blocks
+    if (pos % rows == 0 && pos < total) {
+      Chunk ch;
+      ch.expert = expert_ids[pos / block_size];
+      ch.row0 = (int32_t)pos;
+      ch.rows = rows;
+      ch.pad = 0;
+      chunks[pos / rows] = ch;
+    }
+    if (pos == 0) {
+      const int64_t there = ((int64_t)gridDim.x + rows - 1) / rows;
+      *num_chunks = (int32_t)(total / rows < there ? total / rows : there);
+    }
+  }
   if (pos >= *num_tokens_post_pad) return;
   const int32_t sid = sorted_ids[pos];
   if (sid < 0 || sid >= numel_valid) return;
@@ -405,14 +425,12 @@ __global__ void __launch_bounds__(128) permute_rows_kernel(const int8_t *__restr
 int launch_permute_rows(const int8_t *A, const float *a_scale, int64_t rows_a, int64_t K, const int32_t *sorted_ids,
                         int64_t sorted_capacity, const int32_t *num_tokens_post_pad, int64_t numel_valid, int top_k,
                         int8_t *A_sorted, float *a_scale_sorted, cudaStream_t stream, int64_t scales_per_row,
-                        int64_t a_stride) {
+                        int64_t a_stride, const int32_t *expert_ids, int block_size, Chunk *chunks, int32_t *num_chunks) {
   if (sorted_capacity <= 0) return LO_OK;
   LO_REQUIRE(sorted_capacity <= 0x7fffffffLL, "permute rows: too many positions");
-  permute_rows_kernel<<<(unsigned)sorted_capacity, 128, 0, stream>>>(A, a_scale, rows_a, K, sorted_ids, num_tokens_post_pad,
-                                                                     numel_valid, top_k,
-                                                                     scales_per_row > 0 ? scales_per_row : K / 128, A_sorted,
-                                                                     a_scale_sorted, a_stride > 0 ? a_stride : K);
-  LO_LAUNCH_OK("permute_rows_kernel");
+  LO_CUDA_OK(launch_dependent(permute_rows_kernel, dim3((unsigned)sorted_capacity), dim3(128), 0, stream, A, a_scale, rows_a, K, sorted_ids,
+                              num_tokens_post_pad, numel_valid, top_k, scales_per_row > 0 ? scales_per_row : K / 128, A_sorted,
+                              a_scale_sorted, a_stride > 0 ? a_stride : K, expert_ids, block_size, chunks, num_chunks));
   return LO_OK;
 }
 

@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(256) topk_softmax_kernel(const T *__restrict__
                                                            IdT *__restrict__ ids, int32_t *__restrict__ src_rows) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  dependency_release();      // the alignment kernel may get its block resident; it waits for this grid before it reads
   if (row >= M) return;
   const T *g = gating + row * E;
   float v[VPL];
@@ -155,13 +156,15 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_kernel(
   int32_t *warp_tot = chunk_off + (E + 1);    // [2][32]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  dependency_release();      // the next kernel may get its blocks resident; it waits for this grid before reading
-
   // warps that get a segment: with few ids (decode) only the first ones, so that the histogram rows to
   // clear and to scan shrink with the input
   const int nw = (int)(numel >= (int64_t)ALIGN_WARPS * 32 ? ALIGN_WARPS : (numel + 31) / 32 > 0 ? (numel + 31) / 32 : 1);
-  for (int64_t i = tid; i < sorted_capacity; i += blockDim.x) sorted_ids[i] = (int32_t)numel;
   for (int i = tid; i < nw * E; i += blockDim.x) hist[i] = 0;
+  // Global memory from here on.  The release comes after the wait: a dependent kernel that reads its own inputs ahead of its wait
+  // must find everything before this grid complete.
+  dependency_wait();
+  dependency_release();
+  for (int64_t i = tid; i < sorted_capacity; i += blockDim.x) sorted_ids[i] = (int32_t)numel;
   __syncthreads();
 
   // segment of this warp, a multiple of 32 ids long
@@ -321,10 +324,11 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
   int32_t *before = cta_cnt + E;              // [E] ids per expert in lower-ranked CTAs
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < ALIGN_WARPS * E; i += blockDim.x) hist[i] = 0;
+  dependency_wait();         // (see align_kernel)
   dependency_release();
   // sentinel fill: every CTA fills its share
   for (int64_t i = (int64_t)r * blockDim.x + tid; i < sorted_capacity; i += (int64_t)C * blockDim.x) sorted_ids[i] = (int32_t)numel;
-  for (int i = tid; i < ALIGN_WARPS * E; i += blockDim.x) hist[i] = 0;
   __syncthreads();
 
   // slice of this CTA and segment of this warp, both multiples of 32 ids long
@@ -458,27 +462,6 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
   cluster.sync();      // no CTA leaves while another may still read its counts
 }
 
-__global__ void chunks_from_blocks_kernel(const int32_t *__restrict__ expert_ids,
-                                          const int32_t *__restrict__ num_tokens_post_pad, int block_size,
-                                          int64_t max_blocks, Chunk *__restrict__ chunks,
-                                          int32_t *__restrict__ num_chunks) {
-  const int64_t total_blocks = min((int64_t)(*num_tokens_post_pad / block_size), max_blocks);
-  const int per_block = block_size <= 128 ? 1 : block_size / 128;
-  const int rows = block_size <= 128 ? block_size : 128;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total_blocks * per_block;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = i / per_block;
-    Chunk ch;
-    ch.expert = expert_ids[b];
-    ch.row0 = (int32_t)(b * block_size + (i % per_block) * 128);
-    ch.rows = rows;
-    ch.pad = 0;
-    chunks[i] = ch;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *num_chunks = (int32_t)(total_blocks * per_block);
-}
-
-
 }  // namespace
 
 int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_experts, int block_size,
@@ -502,13 +485,15 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
     cfg.blockDim = dim3(ALIGN_WARPS * 32, 1, 1);
     cfg.dynamicSmemBytes = csmem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ALIGN_CLUSTER;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     if (ids_dtype == LO_I32) {
       if (csmem > 48 * 1024)
         LO_CUDA_OK(cudaFuncSetAttribute(align_cluster_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
@@ -534,32 +519,20 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
       e = cudaFuncSetAttribute(align_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return fail(LO_ERR_CUDA, "moe_align: smem opt-in failed: %s", cudaGetErrorString(e));
     }
-    align_kernel<int32_t><<<1, ALIGN_WARPS * 32, smem, stream>>>(
+    LO_CUDA_OK(launch_dependent(align_kernel<int32_t>, dim3(1), dim3(ALIGN_WARPS * 32), smem, stream,
         static_cast<const int32_t *>(topk_ids), numel, num_experts, block_size, expert_map, map_mode, sorted_ids,
-        sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos, chunk_max);
+        sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos, chunk_max));
   } else if (ids_dtype == LO_I64) {
     if (smem > 48 * 1024) {
       e = cudaFuncSetAttribute(align_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return fail(LO_ERR_CUDA, "moe_align: smem opt-in failed: %s", cudaGetErrorString(e));
     }
-    align_kernel<int64_t><<<1, ALIGN_WARPS * 32, smem, stream>>>(
+    LO_CUDA_OK(launch_dependent(align_kernel<int64_t>, dim3(1), dim3(ALIGN_WARPS * 32), smem, stream,
         static_cast<const int64_t *>(topk_ids), numel, num_experts, block_size, expert_map, map_mode, sorted_ids,
-        sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos, chunk_max);
+        sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos, chunk_max));
   } else {
     return fail(LO_ERR_UNSUPPORTED, "moe_align: unsupported id dtype code %d", ids_dtype);
   }
-  LO_LAUNCH_OK("align_kernel");
-  return LO_OK;
-}
-
-int launch_chunks_from_blocks(const int32_t *expert_ids, const int32_t *num_tokens_post_pad, int block_size,
-                              int64_t max_blocks, Chunk *chunks, int32_t *num_chunks, cudaStream_t stream) {
-  const int per_block = block_size <= 128 ? 1 : block_size / 128;
-  const int64_t n = max_blocks * per_block;
-  const int blocks = (int)(ceil_div(n, 256) < 1 ? 1 : (ceil_div(n, 256) > 1024 ? 1024 : ceil_div(n, 256)));
-  chunks_from_blocks_kernel<<<blocks, 256, 0, stream>>>(expert_ids, num_tokens_post_pad, block_size, max_blocks,
-                                                       chunks, num_chunks);
-  LO_LAUNCH_OK("chunks_from_blocks_kernel");
   return LO_OK;
 }
 
