@@ -21,8 +21,9 @@ _status_words = {}
 
 def device_status_word(device) -> torch.Tensor:
     """Per-device int32 word that kernels set when one of their bounded waits ran out."""
-    dev = torch.device(device)
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
+    idx = device.index if isinstance(device, torch.device) else torch.device(device).index
+    if idx is None:
+        idx = torch.cuda.current_device()
     w = _status_words.get(idx)
     if w is None:
         w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))

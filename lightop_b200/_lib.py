@@ -161,5 +161,32 @@ def require_cuda(*tensors) -> None:
             raise RuntimeError("lightop_b200 runs on CUDA tensors only (no CPU fallback)")
 
 
-def current_stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+class _NoSwitch:
+    __slots__ = ()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_SWITCH = _NoSwitch()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)``, free of charge when that device is current already (the context manager proper costs
+    several microseconds a call, more than the launch it encloses)."""
+    index = device.index
+    return _NO_SWITCH if index is None or index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def current_stream(device: torch.device) -> int:
+    """Handle of the device's current stream, without building a ``torch.cuda.Stream`` around it."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+def f32(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as a contiguous fp32 tensor, itself where it is one."""
+    return t if t.dtype is torch.float32 and t.is_contiguous() else t.to(torch.float32).contiguous()

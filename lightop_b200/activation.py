@@ -43,7 +43,7 @@ def fuse_silu_mul_quant(input: torch.Tensor, num_local_tokens_tensor: Optional[t
         raise RuntimeError("scales must be a contiguous float32 tensor with one value per row")
     if rows == 0:
         return output, scales
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         st = _lib.load().lo_silu_mul_quant_int8(_lib.ptr(input), rows, d, _lib.ptr(output), _lib.ptr(scales),
                                                 _lib.current_stream(input.device))
     _lib.check(st, "fuse_silu_mul_quant")
@@ -82,7 +82,7 @@ def fuse_silu_mul_quant_ep(input: torch.Tensor, tokens_per_expert: Optional[torc
         if tokens_per_expert.numel() != E:
             raise RuntimeError("tokens_per_expert must hold one count per expert")
         counts = tokens_per_expert.to(torch.int32).contiguous()
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         st = _lib.load().lo_silu_mul_quant_int8_masked(_lib.ptr(input), E, T, d, _lib.ptr(counts), _lib.ptr(output),
                                                        _lib.ptr(scales), _lib.current_stream(input.device))
     _lib.check(st, "fuse_silu_mul_quant_ep")

@@ -33,14 +33,14 @@ def matmul_block_int8(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs: to
     assert As.shape[-1] == K // 128 and As.numel() == M * (K // 128), "As must be [..., K/128]"
     assert tuple(Bs.shape) == ((N + 127) // 128, K // 128), "Bs must be [ceil(N/128), K/128]"
     a2 = A.reshape(M, K).contiguous()
-    as2 = As.reshape(M, K // 128).to(torch.float32).contiguous()
-    bs2 = Bs.to(torch.float32).contiguous()
+    as2 = _lib.f32(As.reshape(M, K // 128))
+    bs2 = _lib.f32(Bs)
     C = torch.empty(M, N, dtype=torch.bfloat16, device=A.device)
     if M:
         lib = _lib.load()
         nbytes = lib.lo_block_int8_linear_split_workspace_bytes(M, N, K)
         ws = torch.empty(nbytes, dtype=torch.uint8, device=A.device)
-        with torch.cuda.device(A.device):
+        with _lib.on_device(A.device):
             st = lib.lo_block_int8_linear(_lib.ptr(a2), _lib.ptr(as2), _lib.ptr(B), _lib.ptr(bs2), M, N, K,
                                           _lib.ptr(C), _lib.ptr(ws), nbytes, _lib.ptr(device_status_word(A.device)),
                                           _lib.current_stream(A.device))
@@ -77,13 +77,13 @@ def _dynamic_linear(x: torch.Tensor, w: torch.Tensor, block_size: List[int], w_s
             or not (x.is_cuda and x.device == w.device == w_s.device)):
         return None
     M = x.numel() // K
-    bs = w_s if w_s.dtype is torch.float32 and w_s.is_contiguous() else w_s.to(torch.float32).contiguous()
+    bs = _lib.f32(w_s)
     lib = _lib.load()
     dev = x.device
     C = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=dev)
     nbytes = lib.lo_block_int8_linear_dynamic_workspace_bytes(M, N, K)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         st = lib.lo_block_int8_linear_dynamic(_lib.ptr(x), _lib.dtype_code(x.dtype), _lib.ptr(w), _lib.ptr(bs), M, N, K,
                                               _lib.ptr(C), _lib.ptr(ws), nbytes, _lib.ptr(device_status_word(dev)),
                                               _lib.current_stream(dev))

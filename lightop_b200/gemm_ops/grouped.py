@@ -22,7 +22,7 @@ def _operands(a, b):
         raise RuntimeError("inner dimensions differ")
     if b_scale.numel() != E * N:
         raise RuntimeError("b_scale must hold one value per expert and output channel ([E, N])")
-    return inp, a_scale.to(torch.float32).contiguous(), w, b_scale.to(torch.float32).contiguous(), E, N, K
+    return inp, _lib.f32(a_scale), w, _lib.f32(b_scale), E, N, K
 
 
 def m_grouped_w8a8_gemm_nt_contig_asm(a: Tuple[torch.Tensor, torch.Tensor], b: Tuple[torch.Tensor, torch.Tensor],
@@ -51,7 +51,7 @@ def m_grouped_w8a8_gemm_nt_contig_asm(a: Tuple[torch.Tensor, torch.Tensor], b: T
     ws_bytes = lib.lo_m_grouped_gemm_workspace_bytes(M, E)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=inp.device)
     status = device_status_word(inp.device)
-    with torch.cuda.device(inp.device):
+    with _lib.on_device(inp.device):
         st = lib.lo_m_grouped_w8a8_gemm_nt_contig(_lib.ptr(inp), _lib.ptr(a_scale), _lib.ptr(w), _lib.ptr(b_scale),
                                                   _lib.ptr(output), _lib.ptr(m_indices.contiguous()), M, E, N, K,
                                                   _lib.ptr(ws), ws_bytes, _lib.ptr(status),
@@ -87,7 +87,7 @@ def m_grouped_w8a8_gemm_nt_masked(a: Tuple[torch.Tensor, torch.Tensor], b: Tuple
     ws_bytes = lib.lo_m_grouped_gemm_workspace_bytes(E * max_m, E)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=inp.device)
     status = device_status_word(inp.device)
-    with torch.cuda.device(inp.device):
+    with _lib.on_device(inp.device):
         st = lib.lo_m_grouped_w8a8_gemm_nt_masked(_lib.ptr(inp), _lib.ptr(a_scale), _lib.ptr(w), _lib.ptr(b_scale),
                                                   _lib.ptr(d), _lib.ptr(masked_m.contiguous()), E, max_m, N, K,
                                                   _lib.ptr(ws), ws_bytes, _lib.ptr(status),

@@ -19,7 +19,7 @@ def ep_build_m_indices(topk_ids: torch.Tensor, m_indices: torch.Tensor, local_nu
     if m_indices.dtype != torch.int32:
         raise RuntimeError("m_indices must be int32")
     ids = topk_ids.contiguous()
-    with torch.cuda.device(ids.device):
+    with _lib.on_device(ids.device):
         st = _lib.load().lo_ep_build_m_indices(_lib.ptr(ids), _lib.dtype_code(ids.dtype), ids.numel(),
                                                _lib.ptr(m_indices), m_indices.numel(), int(local_num_experts),
                                                int(alignment), _lib.current_stream(ids.device))
@@ -54,7 +54,7 @@ def ep_scatter(aq: torch.Tensor, aq_scale: torch.Tensor, topk_ids: torch.Tensor,
         expert_map = expert_map.to(torch.int32)
     counts = expert_num_tokens.to(torch.int32) if expert_num_tokens is not None else None
     ids = topk_ids.contiguous()
-    with torch.cuda.device(aq.device):
+    with _lib.on_device(aq.device):
         st = _lib.load().lo_ep_scatter(
             _lib.ptr(aq.contiguous()), _lib.ptr(aq_scale.contiguous()), S, _lib.ptr(ids), _lib.dtype_code(ids.dtype),
             _lib.ptr(expert_map), _lib.ptr(counts), _lib.ptr(aq_out), _lib.ptr(aq_scale_out), _lib.ptr(m_indices),
@@ -78,8 +78,8 @@ def ep_gather(a: torch.Tensor, topk_ids: torch.Tensor, topk_weights: torch.Tenso
     if expert_map is not None and expert_map.dtype != torch.int32:
         expert_map = expert_map.to(torch.int32)
     ids = topk_ids.contiguous()
-    w = topk_weights.to(torch.float32).contiguous()
-    with torch.cuda.device(a.device):
+    w = _lib.f32(topk_weights)
+    with _lib.on_device(a.device):
         st = _lib.load().lo_ep_gather(_lib.ptr(a.contiguous()), _lib.ptr(ids), _lib.dtype_code(ids.dtype), _lib.ptr(w),
                                       _lib.ptr(inv_perm.contiguous()), _lib.ptr(expert_map), _lib.ptr(output), T, k, H,
                                       _lib.current_stream(a.device))

@@ -51,7 +51,7 @@ def moe_gemm_w8a8(input: torch.Tensor, b_qweight: torch.Tensor, output: torch.Te
     ws_bytes = lib.lo_grouped_gemm_workspace_bytes(sorted_token_ids.numel(), int(block_size), K)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=input.device)
     w = topk_weights.reshape(-1).contiguous() if topk_weights is not None else None
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         entry = lib.lo_moe_grouped_gemm_i8_channel if channel else lib.lo_moe_grouped_gemm_i8_block
         st = entry(
             _lib.ptr(input), _lib.ptr(a_scale), input.shape[0], _lib.ptr(b_qweight), _lib.ptr(b_scale), E, N, K,

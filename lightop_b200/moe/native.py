@@ -103,8 +103,8 @@ def fused_experts_impl_int8(hidden_states: torch.Tensor,
             raise AssertionError("apply_router_weight_on_input is only implemented for topk=1")
     elif tuple(w1_scale.shape) != (E, N // 128, H // 128) or tuple(w2_scale.shape) != (E, H // 128, I // 128):
         raise RuntimeError("block scales must be [E, N/128, K/128]")
-    w1_scale = w1_scale.to(torch.float32).contiguous()
-    w2_scale = w2_scale.to(torch.float32).contiguous()
+    w1_scale = _lib.f32(w1_scale)
+    w2_scale = _lib.f32(w2_scale)
     if global_num_experts == -1:
         global_num_experts = E
     top_k = topk_ids.shape[1]
@@ -113,7 +113,7 @@ def fused_experts_impl_int8(hidden_states: torch.Tensor,
     if topk_ids.dtype not in (torch.int32, torch.int64):
         topk_ids = topk_ids.to(torch.int32)
     topk_ids = topk_ids.contiguous()
-    topk_weights = topk_weights.to(torch.float32).contiguous()
+    topk_weights = _lib.f32(topk_weights)
     if expert_map is not None and expert_map.dtype != torch.int32:
         expert_map = expert_map.to(torch.int32)
     if shared_output is not None:
@@ -139,28 +139,32 @@ def fused_experts_impl_int8(hidden_states: torch.Tensor,
     workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     status = device_status_word(dev)
     factor = 1.0 if routed_scaling_factor is None else float(routed_scaling_factor)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         for begin in range(0, num_tokens, CHUNK):
             end = min(begin + CHUNK, num_tokens)
             m = end - begin
-            x_c = hidden_states[begin:end]
+            # a slice costs about as much as a launch: the usual call is one chunk and takes the tensors as they are
+            x_c, w_c, ids_c, out_c, shared_c = hidden_states, topk_weights, topk_ids, out, shared_output
+            if m != num_tokens:
+                x_c, w_c, ids_c, out_c = x_c[begin:end], w_c[begin:end], ids_c[begin:end], out_c[begin:end]
+                shared_c = shared_c[begin:end] if shared_c is not None else None
             if channel:
                 st = lib.lo_fused_moe_channel_int8(
                     _lib.ptr(x_c), _lib.dtype_code(x_c.dtype), _lib.ptr(w1), _lib.ptr(w2), _lib.ptr(w1_scale),
-                    _lib.ptr(w2_scale), _lib.ptr(topk_weights[begin:end]), _lib.ptr(topk_ids[begin:end]),
+                    _lib.ptr(w2_scale), _lib.ptr(w_c), _lib.ptr(ids_c),
                     _lib.dtype_code(topk_ids.dtype), _lib.ptr(expert_map), int(global_num_experts), m, E, top_k, H, I,
                     _lib.ptr(cache13),
-                    _lib.ptr(shared_output[begin:end]) if shared_output is not None else 0, _lib.ptr(out[begin:end]),
+                    _lib.ptr(shared_c), _lib.ptr(out_c),
                     int(bool(apply_router_weight_on_input)), factor, _lib.ptr(workspace), ws_bytes, _lib.ptr(status),
                     stream)
                 _lib.check(st, "fused_experts_impl_int8")
                 continue
             st = lib.lo_fused_moe_block_int8(
                 _lib.ptr(x_c), _lib.ptr(w1), _lib.ptr(w2), _lib.ptr(w1_scale), _lib.ptr(w2_scale),
-                _lib.ptr(topk_weights[begin:end]), _lib.ptr(topk_ids[begin:end]), _lib.dtype_code(topk_ids.dtype),
+                _lib.ptr(w_c), _lib.ptr(ids_c), _lib.dtype_code(topk_ids.dtype),
                 _lib.ptr(expert_map), int(global_num_experts), m, E, top_k, H, I, _lib.ptr(cache13),
-                _lib.ptr(shared_output[begin:end]) if shared_output is not None else 0, _lib.ptr(out[begin:end]),
+                _lib.ptr(shared_c), _lib.ptr(out_c),
                 int(bool(apply_router_weight_on_input)), factor, _lib.ptr(workspace), ws_bytes, _lib.ptr(status),
                 stream)
             _lib.check(st, "fused_experts_impl_int8")

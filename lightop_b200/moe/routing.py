@@ -39,7 +39,7 @@ def topk_softmax(topk_weights: torch.Tensor, topk_indices: torch.Tensor,
         raise RuntimeError("token_expert_indices must be int32")
     if not (gating_output.is_contiguous() and topk_weights.is_contiguous() and topk_indices.is_contiguous()):
         raise RuntimeError("topk_softmax expects contiguous tensors")
-    with torch.cuda.device(gating_output.device):
+    with _lib.on_device(gating_output.device):
         st = _lib.load().lo_topk_softmax(_lib.ptr(gating_output), _lib.dtype_code(gating_output.dtype), M, E, k,
                                          int(bool(Is_renormalize)), _lib.ptr(topk_weights), _lib.ptr(topk_indices),
                                          _lib.dtype_code(topk_indices.dtype), _lib.ptr(token_expert_indices),
@@ -65,7 +65,7 @@ def moe_align_block_size_out(topk_ids, num_experts, block_size, sorted_ids, expe
     ids = topk_ids if topk_ids.is_contiguous() else topk_ids.contiguous()
     if expert_map is not None and expert_map.dtype != torch.int32:
         expert_map = expert_map.to(torch.int32)
-    with torch.cuda.device(ids.device):
+    with _lib.on_device(ids.device):
         st = _lib.load().lo_moe_align_block_size(
             _lib.ptr(ids), _lib.dtype_code(ids.dtype), ids.numel(), int(num_experts), int(block_size),
             _lib.ptr(expert_map), 1 if expert_map is not None else 0, _lib.ptr(sorted_ids), sorted_ids.numel(),
@@ -103,7 +103,7 @@ def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: i
         if expert_map.dtype != torch.int32:
             expert_map = expert_map.to(torch.int32)
         mode = 1 if ignore_invalid_experts else 2
-    with torch.cuda.device(ids.device):
+    with _lib.on_device(ids.device):
         st = _lib.load().lo_moe_align_block_size(
             _lib.ptr(ids), _lib.dtype_code(ids.dtype), numel, int(num_experts), int(block_size),
             _lib.ptr(expert_map), mode, _lib.ptr(sorted_ids), sorted_ids.numel(), _lib.ptr(expert_ids),
@@ -139,7 +139,7 @@ def moe_sum(input: torch.Tensor, output: torch.Tensor, bias: Optional[torch.Tens
         raise RuntimeError("moe_sum bias must be a contiguous [num_tokens, hidden] tensor of the input dtype")
     if expert_mask is not None:
         expert_mask = expert_mask.to(torch.bool).contiguous()
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         st = _lib.load().lo_moe_sum(_lib.ptr(input), _lib.ptr(output), _lib.ptr(bias), _lib.dtype_code(input.dtype),
                                     M, topk, H, float(factor), _lib.ptr(expert_mask), _lib.ptr(num_local_tokens),
                                     _lib.current_stream(input.device))
@@ -170,7 +170,7 @@ def moe_fused_gate(x: torch.Tensor, bias: torch.Tensor, num_expert_group: int, t
     M, E = x.shape
     weights = torch.empty(M, topk, dtype=torch.float32, device=x.device)
     ids = torch.empty(M, topk, dtype=torch.int64 if output_indices_int64 else torch.int32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         st = _lib.load().lo_moe_fused_gate(_lib.ptr(x), _lib.dtype_code(x.dtype), _lib.ptr(bias),
                                            _lib.dtype_code(bias.dtype), M, E, int(num_expert_group), int(topk_group),
                                            int(topk), int(n_share_experts_fusion), float(routed_scaling_factor),
@@ -198,7 +198,7 @@ def _gate_topk(x, bias, groups, topk_group, topk, n_shared, score_fn, renormaliz
         raise RuntimeError(f"{what}: input and bias must be contiguous")
     weights = torch.empty(M, topk, dtype=torch.float32, device=x.device)
     ids = torch.empty(M, topk, dtype=ids_dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         st = _lib.load().lo_moe_gate_topk(_lib.ptr(x), _lib.dtype_code(x.dtype), _lib.ptr(bias), _lib.dtype_code(bias.dtype),
                                           E if bias.dim() == 2 else 0, M, E, int(groups), int(topk_group), int(topk),
                                           int(n_shared), int(score_fn), int(bool(renormalize)), float(norm_eps),
@@ -308,7 +308,7 @@ def topk_ids_postprocess(topk_ids: torch.Tensor, logical_to_physical_map: Option
             raise RuntimeError(f"{name} expects int32 or int64 tensor")
     m = logical_to_physical_map
     n = num_token_non_padded
-    with torch.cuda.device(topk_ids.device):
+    with _lib.on_device(topk_ids.device):
         st = _lib.load().lo_topk_ids_postprocess(
             _lib.ptr(topk_ids), _lib.dtype_code(topk_ids.dtype), topk_ids.shape[0], topk_ids.shape[1],
             _lib.ptr(m.contiguous()) if m is not None else 0, _lib.dtype_code(m.dtype) if m is not None else 0,

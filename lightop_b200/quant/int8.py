@@ -27,7 +27,7 @@ def per_token_group_quant_int8(x: torch.Tensor, group_size: int, eps: float = 1e
         x = x.contiguous()
     x_q = torch.empty_like(x, dtype=torch.int8)
     x_s = torch.empty(x.shape[:-1] + (x.shape[-1] // group_size,), device=x.device, dtype=torch.float32)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         st = _lib.load().lo_group_quant_int8(_lib.ptr(x), _lib.dtype_code(x.dtype), x.numel() // group_size,
                                              int(group_size), float(eps), _lib.ptr(x_q), _lib.ptr(x_s),
                                              _lib.current_stream(x.device))
@@ -52,7 +52,7 @@ def per_token_quant_int8(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     scales = torch.empty(x.shape[:-1] + (1,), device=x.device, dtype=torch.float32)
     if M == 0:
         return x_q, scales
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         st = _lib.load().lo_per_token_quant_int8(_lib.ptr(x), _lib.dtype_code(x.dtype), M, K, _lib.ptr(x_q),
                                                  _lib.ptr(scales), _lib.current_stream(x.device))
     _lib.check(st, "per_token_quant_int8")
