@@ -403,7 +403,8 @@ template <typename T, int N> __device__ __forceinline__ T pick(const T (&v)[N], 
 }
 
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-// Reciprocal refined by one Newton step, and the quotient a / b from it with the remainder folded back in
+// Reciprocal refined by one Newton step, and the quotient a / b from it with the remainder folded back in (Markstein's method,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990)
 // (q = a*y, then q + (a - b*q)*y): the IEEE round-to-nearest quotient for operands whose quotient and reciprocal
 // are normal numbers, which holds for every division of the epilogues (denominators in [1, 1e38] or a group
 // scale of at least 1e-10 / 127).  Inline, so the sixteen divisions of a piece overlap; the library division is
