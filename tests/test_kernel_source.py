@@ -1,0 +1,37 @@
+"""CPU checks of rules that the kernels' source has to keep and that no run can show (a memory-model race that the hardware's
+in-order issue hides, a figure in a comment that a layout constant contradicts)."""
+import os
+import re
+
+import lightop_b200
+
+CSRC = os.path.join(os.path.dirname(lightop_b200.__file__), "csrc")
+
+
+def _statements(name):
+    """The file's statements in order, comments removed and white space folded."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = f.read()
+    text = re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+    return [re.sub(r"\s+", " ", s).strip() for s in re.split(r"[;{}]", text) if s.strip()]
+
+
+def test_an_arrive_orders_the_reads_of_the_whole_warp():
+    # what a barrier hands back was read by all lanes of a warp: either every lane arrives for itself, or lane 0 does behind a
+    # __syncwarp() (neither converged execution nor a vote orders memory)
+    st = _statements("grouped_gemm.cu")
+    one = [i for i, s in enumerate(st) if re.match(r"if \(lane == 0\) mbar_arrive(_addr)?\(", s)]
+    assert len(one) >= 5
+    bare = [f"{st[i - 1]}; {st[i]}" for i in one if st[i - 1] != "__syncwarp()"]
+    assert not bare, bare
+    # the partial buffers: the one barrier that every lane arrives at, and counted so
+    assert "mbar_arrive_addr(used)" in st and "mbar_init(&sm.consumed[s], EPI_WARPS * 32)" in st
+
+
+def test_what_one_lane_waited_for_is_ordered_before_the_mma():
+    # the MMA issuer's two polling lanes agree by a vote; the elected lane issues only after a __syncwarp() that follows it
+    st = _statements("grouped_gemm.cu")
+    wait = next(i for i, s in enumerate(st) if "LO_SLEEP_MMA)" in s and s.startswith("seen = "))
+    issue = next(i for i, s in enumerate(st) if i > wait and "elect_one()" in s)
+    vote = max(i for i in range(wait, issue) if "__all_sync" in st[i])
+    assert "__syncwarp()" in st[vote + 1:issue]
