@@ -446,6 +446,7 @@ struct KParams {
   float act_eps;
   int32_t *status;
   int out_by_position;      // bf16 output row = sorted position instead of the sorted id
+  int vec_store;            // block-scaled bf16 output: every group of 8 columns of every row begins on a 16-byte boundary
   const int64_t *row_dst;   // single mode: address of the output row of every sorted id (null: C + id * n_store)
   // Without a chunk table (chunks == null) the chunks follow from arithmetic: fixed_chunks of them, of at most chunk_rows rows.
   int fixed_chunks;
@@ -883,7 +884,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           }
         }
         if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9, LO_SLEEP_OUT))) break;
-        const bool vec_ok = (p.n_store & 7) == 0;
         const int64_t n0 = (int64_t)nt * TILE_N + (lane & 15) * 8;
         const int n_steps = (ch.rows + 2 * OUT_WARPS - 1) / (2 * OUT_WARPS);
 #pragma unroll 4
@@ -901,7 +901,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
 #pragma unroll
               for (int e = 0; e < 4; ++e) h[e] = __hmul2(h[e], w2);
             }
-            if (vec_ok) {
+            if (p.vec_store) {
               *reinterpret_cast<uint4 *>(dst) = v;
             } else {
               for (int e = 0; e < 8 && n0 + e < p.n_store; ++e) dst[e] = reinterpret_cast<const __nv_bfloat16 *>(&v)[e];
@@ -1330,6 +1330,8 @@ int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   p.chunks = a.chunks; p.num_chunks = a.num_chunks; p.act_q = a.act_q; p.act_s = a.act_s; p.C = a.C; p.row_dst = a.row_dst;
   p.topk_weights = a.topk_weights; p.weight_mode = a.weight_mode; p.act_eps = a.act_eps; p.status = a.status;
   p.out_by_position = a.out_by_position;
+  // (C is the caller's: a view may begin anywhere; a table of row addresses holds 16-byte aligned ones)
+  p.vec_store = (p.n_store & 7) == 0 && (a.row_dst != nullptr || (reinterpret_cast<uintptr_t>(a.C) & 15) == 0) ? 1 : 0;
   p.fixed_chunks = a.fixed_chunks; p.chunk_rows = a.max_chunk_rows; p.masked_m = a.masked_m; p.max_m = a.max_m; p.dense_rows = a.rows_a;
   p.n_split = a.partial != nullptr ? (int)ceil_div(p.KB, a.split_steps) : 1; p.split_steps = a.split_steps; p.partial = a.partial;
   const int grid = sm_count();
@@ -1354,6 +1356,7 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
   LO_REQUIRE(a.row_dst == nullptr || (mode == GEMM_SINGLE && a.n_rows_per_expert % 8 == 0 && a.out_by_position == 0),
              "grouped gemm: a table of row addresses serves the single block-scaled mode with N a multiple of 8");
   LO_REQUIRE(mode == GEMM_GATE_UP || a.C != nullptr || a.row_dst != nullptr, "grouped gemm: no output");
+  LO_REQUIRE((reinterpret_cast<uintptr_t>(a.C) & 1) == 0, "grouped gemm: the output must be aligned to its bf16 elements");
   LO_REQUIRE(a.chunks != nullptr || (a.fixed_chunks >= 1 && a.max_chunk_rows >= 1 && ((mode == GEMM_SINGLE && a.max_chunk_rows <= T_MAX) || (mode == GEMM_CHANNEL && a.masked_m != nullptr))),
              "grouped gemm: no chunk table");
   LO_REQUIRE(a.partial == nullptr || (mode == GEMM_SINGLE && a.chunks == nullptr && a.max_chunk_rows <= T_MAX && a.split_steps >= SC_STEPS &&

@@ -97,3 +97,50 @@ def test_linear_in_one_call_equals_its_two_operators(dtype, shape):
     wide = torch.zeros(*shape[:-1], 2 * K, dtype=dtype, device=DEV)
     wide[..., ::2] = x
     assert torch.equal(lo.gemm_ops.apply_w8a8_block_int8_linear(wide[..., ::2], B, [128, 128], b_s), y)
+
+
+@pytest.mark.parametrize("offset", [1, 4])      # elements of bf16: 2 and 8 bytes off a 16-byte boundary
+@pytest.mark.parametrize("M,N,K", [(5, 256, 384), (131, 136, 512), (1, 576, 7168)])
+def test_linear_output_off_a_16_byte_boundary(M, N, K, offset):
+    # a caller's C that begins anywhere in a buffer: the row stores take the scalar form, the elements around stay untouched
+    import lightop_b200 as lo
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    B = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8).to(DEV)
+    b_s = (torch.rand((N + 127) // 128, K // 128, generator=g) * 9e-3 + 1e-3).to(DEV)
+    q, s = lo.quant.per_token_group_quant_int8(x, 128)
+    ref = lo.gemm_ops.matmul_block_int8(q, B, s, b_s, [128, 128], torch.bfloat16)
+    stream = torch.cuda.current_stream().cuda_stream
+    for form in ("undivided", "split", "dynamic"):
+        buf = torch.full((M * N + 16,), 7.0, dtype=torch.bfloat16, device=DEV)
+        c = buf[offset:offset + M * N]
+        n = {"undivided": 256, "split": lib.lo_block_int8_linear_split_workspace_bytes(M, N, K),
+             "dynamic": lib.lo_block_int8_linear_dynamic_workspace_bytes(M, N, K)}[form]
+        ws = torch.empty(n, dtype=torch.uint8, device=DEV)
+        if form == "dynamic":
+            st = lib.lo_block_int8_linear_dynamic(x.data_ptr(), _lib.LO_BF16, B.data_ptr(), b_s.data_ptr(), M, N, K, c.data_ptr(), ws.data_ptr(), n, 0, stream)
+        else:
+            st = lib.lo_block_int8_linear(q.data_ptr(), s.data_ptr(), B.data_ptr(), b_s.data_ptr(), M, N, K, c.data_ptr(), ws.data_ptr(), n, 0, stream)
+        assert st == 0, form
+        assert_gemm_close(c.view(M, N), ref, f"{form} {M}x{N}x{K} at {offset}")
+        assert bool((buf[:offset] == 7.0).all()) and bool((buf[offset + M * N:] == 7.0).all()), form
+
+
+def test_moe_gemm_output_off_a_16_byte_boundary():
+    import lightop_b200 as lo
+    E, k, H, N, M, block = 8, 2, 256, 384, 33, 16
+    g = torch.Generator().manual_seed(9)
+    w = torch.randint(-127, 128, (E, N, H), generator=g, dtype=torch.int8).to(DEV)
+    w_s = (torch.rand(E, N // 128, H // 128, generator=g) * 9e-3 + 1e-3).to(DEV)
+    q, s = lo.quant.per_token_group_quant_int8(torch.randn(M, H, generator=g).to(torch.bfloat16).to(DEV), 128)
+    ids = torch.randint(0, E, (M, k), generator=g, dtype=torch.int32).to(DEV)
+    wgt = torch.rand(M, k, generator=g).to(DEV)
+    sorted_ids, expert_ids, num_post = lo.moe.moe_align_block_size(ids, block, E)
+    ref = torch.empty(M, k, N, dtype=torch.bfloat16, device=DEV)
+    lo.moe.moe_gemm_w8a8(q, w, ref, s, w_s, wgt, sorted_ids, expert_ids, num_post, k, {"BLOCK_SIZE_M": block})
+    buf = torch.full((M * k * N + 8,), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = buf[3:3 + M * k * N].view(M, k, N)
+    lo.moe.moe_gemm_w8a8(q, w, out, s, w_s, wgt, sorted_ids, expert_ids, num_post, k, {"BLOCK_SIZE_M": block})
+    assert torch.equal(out, ref) and bool((buf[:3] == 7.0).all()) and bool((buf[3 + M * k * N:] == 7.0).all())

@@ -35,3 +35,11 @@ def test_what_one_lane_waited_for_is_ordered_before_the_mma():
     issue = next(i for i, s in enumerate(st) if i > wait and "elect_one()" in s)
     vote = max(i for i in range(wait, issue) if "__all_sync" in st[i])
     assert "__syncwarp()" in st[vote + 1:issue]
+
+
+def test_vector_stores_to_the_callers_output_look_at_its_address():
+    # the 16-byte row stores are decided on the host from the row length and the address, not from the length alone
+    st = _statements("grouped_gemm.cu")
+    assert any(s.startswith("p.vec_store = ") and "& 7) == 0" in s and "a.C) & 15) == 0" in s for s in st)
+    i = next(i for i, s in enumerate(st) if "*reinterpret_cast<uint4 *>(dst) = v" in s)
+    assert st[i - 1] == "if (p.vec_store)"
