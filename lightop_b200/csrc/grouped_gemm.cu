@@ -839,7 +839,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             v[e][1] = __uint_as_float(raw.x & 0xffff0000u);
             v[e][2] = __uint_as_float(raw.y << 16);
             v[e][3] = __uint_as_float(raw.y & 0xffff0000u);
-            m[e] = __float_as_uint(fmaxf(fmaxf(fabsf(v[e][0]), fabsf(v[e][1])), fmaxf(fabsf(v[e][2]), fabsf(v[e][3]))));
+            // (as bit patterns, like the warp's maximum below: a NaN is above every number there, where fmaxf would drop it, so
+            // the group's scale does not depend on which of its channels holds one)
+            m[e] = max(max(__float_as_uint(v[e][0]) & 0x7fffffffu, __float_as_uint(v[e][1]) & 0x7fffffffu),
+                       max(__float_as_uint(v[e][2]) & 0x7fffffffu, __float_as_uint(v[e][3]) & 0x7fffffffu));
           }
 #pragma unroll
           for (int e = 0; e < UN; ++e) m[e] = __reduce_max_sync(0xffffffffu, m[e]);

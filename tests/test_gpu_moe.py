@@ -140,6 +140,27 @@ def _stage2_from_workspace(lo, M, E, k, H, I, x, w1, w2, w1_s, w2_s, w, ids):
     return out.cpu(), header, xq, xs, sorted_ids, act_q, act_s
 
 
+@pytest.mark.parametrize("channels", [(5,), (0,), (127,), (34,), (4, 5, 6, 7), (64, 67), tuple(range(128))])
+@pytest.mark.parametrize("M", [3, 70])
+def test_a_nan_in_a_quantisation_group(lo, M, channels):
+    # Gate sums of some channels overflow to infinity, whose SiLU here is a NaN (the quotient's correction).  Wherever in the
+    # 128-channel group the NaN sits, the group's scale is the one of the clamp's lower bound, the next group's is its own.
+    H, I = 128, 256
+    w1 = torch.zeros(1, 2 * I, H, dtype=torch.int8)
+    w1[0, :, 0] = 1
+    for c in channels:
+        w1[0, c, :] = 127                       # dot 2e6 x scale 1e35 / 127: beyond the range of fp32
+    w1_s = torch.tensor([[[1e35], [1.0], [1e-3], [1.0]]])
+    w2, w2_s = torch.zeros(1, H, I, dtype=torch.int8), torch.ones(1, 1, 2)
+    x = torch.ones(M, H, dtype=torch.bfloat16)
+    _, header, _, _, _, act_q, act_s = _stage2_from_workspace(lo, M, 1, 1, H, I, x, w1, w2, w1_s, w2_s, torch.ones(M, 1),
+                                                              torch.zeros(M, 1, dtype=torch.int32))
+    eps = torch.tensor(1e-10).to(torch.bfloat16).float() / 127.0
+    assert torch.equal(act_s[:M, 0], eps.expand(M))
+    assert bool((act_q[:M, list(channels)] == -128).all())
+    assert bool((act_q[:M, 128:] == 127).all()) and bool((act_s[:M, 1] > 1e-3).all())
+
+
 @pytest.mark.parametrize("name,shape", [("c0", (8, 2, 32, 256, 512)), ("ragged", (16, 4, 77, 512, 256)), ("big_chunk", (2, 1, 300, 256, 256)),
                                         ("wide_pair", (2, 1, 620, 256, 256)), ("wide_many", (8, 2, 580, 384, 256))])
 def test_fused_intermediates_bit_exact(lo, name, shape):
