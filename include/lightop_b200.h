@@ -5,6 +5,10 @@
  * Conventions
  *   - every pointer is a DEVICE pointer unless the comment says "host";
  *   - `stream` is a cudaStream_t passed as void* (NULL = legacy default stream);
+ *   - matrices that the kernels read or write 16 bytes at a time (int8 and bf16
+ *     operands, rows and results) begin on a 16-byte boundary; a call that does
+ *     not keep to that is refused (LO_ERR_INVALID_ARGUMENT).  The bf16 result C of
+ *     a GEMM entry may begin at any element;
  *   - every function only enqueues work on `stream`: no host synchronisation and
  *     no allocation (scratch memory is passed in by the caller);
  *   - the return value is a status code, 0 on success; lo_last_error() returns

@@ -53,6 +53,9 @@ inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
 
 int sm_count();
 
+// Do all of these (null ones included) begin on a 16-byte boundary?  The kernels' vector accesses to caller memory need it.
+template <typename... P> inline bool aligned16(const P *...p) { return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0; }
+
 // ---------------------------------------------------------------------------
 // Internal kernels shared between translation units
 // ---------------------------------------------------------------------------

@@ -154,6 +154,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   const int align_E = expert_map ? global_num_experts : E_local;
   LO_REQUIRE(align_E <= 1024, "fused moe: more than 1024 experts");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "fused moe: workspace must be 256-byte aligned");
+  LO_REQUIRE(aligned16(x, cache3, shared_output, out), "fused moe: activations, cache, shared output and result must be 16-byte aligned");
   FusedLayout L = carve_fused(workspace, M, align_E, topk, H, I);
   LO_REQUIRE(workspace_bytes >= L.bytes, "fused moe: workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -262,6 +263,7 @@ int grouped_gemm_on_blocks(GemmMode mode, const int8_t *A, const float *a_scale,
   LO_REQUIRE(top_k >= 1 && E >= 1 && rows_a >= 0 && sorted_capacity >= 1, "grouped gemm: bad shape");
   LO_REQUIRE(K % 128 == 0 && N % 128 == 0, "grouped gemm: N and K must be multiples of 128");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "grouped gemm: workspace must be 256-byte aligned");
+  LO_REQUIRE(aligned16(A), "grouped gemm: operands and scales must be 16-byte aligned");
   GemmWs W = carve_gemm(workspace, sorted_capacity, block_size, K);   // sized for block scales; per-token scales need less
   LO_REQUIRE(workspace_bytes >= W.bytes, "grouped gemm: workspace of %zu bytes, %zu needed", workspace_bytes, W.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -454,6 +456,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   const int align_E = expert_map ? global_num_experts : E_local;
   LO_REQUIRE(align_E <= 1024, "channel moe: more than 1024 experts");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "channel moe: workspace must be 256-byte aligned");
+  LO_REQUIRE(aligned16(x, cache3, shared_output, out), "channel moe: activations, cache, shared output and result must be 16-byte aligned");
   ChannelLayout L = carve_channel(workspace, M, align_E, topk, H, I);
   LO_REQUIRE(workspace_bytes >= L.bytes, "channel moe: workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -528,6 +531,7 @@ int expert_rows_impl(const int8_t *xq, const float *xs, int64_t x_stride, const 
   LO_REQUIRE(H % 128 == 0 && I % 128 == 0, "expert rows: hidden and intermediate sizes must be multiples of 128");
   LO_REQUIRE(T < (1LL << 30), "expert rows: too many rows");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "expert rows: workspace must be 256-byte aligned");
+  LO_REQUIRE(aligned16(xq), "expert rows: rows must be 16-byte aligned");
   FusedLayout L = carve_fused(workspace, T, E_local, 1, H, I);
   LO_REQUIRE(workspace_bytes >= L.bytes, "expert rows: workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -465,6 +465,7 @@ extern "C" int lo_moe_sum(const void *in, void *out, const void *bias, int dtype
   LO_REQUIRE(in && out, "moe_sum: null pointer");
   LO_REQUIRE(H % 8 == 0, "moe_sum: hidden size %lld is not a multiple of 8", (long long)H);
   LO_REQUIRE(M <= 0x7fffffffLL, "moe_sum: too many tokens");
+  LO_REQUIRE(aligned16(in, out, bias), "moe_sum: input, output and bias must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (dtype) {
     case LO_BF16: return launch_sum<__nv_bfloat16, int32_t>(in, out, bias, M, topk, H, factor, expert_mask, num_local_tokens, nullptr, nullptr, st);
@@ -497,6 +498,7 @@ extern "C" int lo_ep_scatter(const int8_t *aq, const float *aq_scale, int scale_
   LO_REQUIRE(H % 16 == 0, "ep_scatter: hidden size %lld is not a multiple of 16", (long long)H);
   LO_REQUIRE(aq && aq_scale && topk_ids && aq_out && aq_scale_out && m_indices && inv_perm, "ep_scatter: null pointer");
   LO_REQUIRE(T * k <= 0x7fffffffLL, "ep_scatter: too many (token, slot) pairs");
+  LO_REQUIRE(T * k == 0 || aligned16(aq, aq_out), "ep_scatter: rows must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc;
   if (ids_dtype == LO_I64)
@@ -525,6 +527,7 @@ extern "C" int lo_ep_dispatch_pack(const int8_t *aq, const float *aq_scale, cons
   LO_REQUIRE(aq && aq_scale && topk_ids && topk_weights && rank_of_expert && packed && dest_rank && inv_perm && counts,
              "ep_dispatch_pack: null pointer");
   LO_REQUIRE(T * k <= 0x7fffffffLL, "ep_dispatch_pack: too many (token, slot) pairs");
+  LO_REQUIRE(T == 0 || aligned16(aq, packed), "ep_dispatch_pack: rows and records must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t rows = T * k;
   int rc;
@@ -577,6 +580,7 @@ extern "C" int lo_ep_dispatch_put(const int8_t *aq, const float *aq_scale, const
   LO_REQUIRE(aq && aq_scale && topk_ids && topk_weights && rank_of_expert && inv_perm && seg_first && seg_dst,
              "ep_dispatch_put: null pointer");
   LO_REQUIRE(T * k <= 0x7fffffffLL, "ep_dispatch_put: too many (token, slot) pairs");
+  LO_REQUIRE(aligned16(aq), "ep_dispatch_put: rows must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t rows = T * k;
   if (rows == 0) return LO_OK;
@@ -602,6 +606,7 @@ extern "C" int lo_ep_gather(const void *a, const void *topk_ids, int ids_dtype, 
   LO_REQUIRE(T >= 0 && k >= 1 && H % 8 == 0, "ep_gather: bad shape");
   if (T == 0) return LO_OK;
   LO_REQUIRE(a && topk_ids && topk_weights && inv_perm && out, "ep_gather: null pointer");
+  LO_REQUIRE(aligned16(a, out), "ep_gather: rows and result must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t H8 = H / 8;
   dim3 grid((unsigned)(ceil_div(H8, 256)), (unsigned)T);

@@ -119,3 +119,44 @@ def test_noalloc_size_check_boundary_without_a_gpu():
     assert st == 1 and b"built-in array" in msg
     st, msg = call(402)           # passes the size check; what stops it afterwards is the missing device or the null pointers
     assert st != 0 and b"built-in array" not in msg
+
+
+def _entries_with_vector_access(lib):
+    """(entry, arguments with `None` at the pointer under test, positions of such pointers) of every entry whose kernels read or
+    write caller memory 16 bytes at a time.  The addresses are never used: each call has to be refused on the host."""
+    from lightop_b200 import _lib
+    P, E, M, k, H, I = 4096, 2, 4, 2, 128, 128
+    big = 1 << 30
+    fused = [P] * 7 + [_lib.LO_I32, 0, E, M, E, k, H, I, P, P, P, 0, 1.0, P, big, 0, 0]
+    channel = [P, _lib.LO_BF16] + [P] * 6 + [_lib.LO_I32, 0, E, M, E, k, H, I, P, P, P, 0, 1.0, P, big, 0, 0]
+    gemm = [P, P, M, P, P, E, 128, H, P, P, 0, P, 64, P, P, M * k, k, 16, P, big, 0]
+    return [(lib.lo_fused_moe_block_int8, fused, (0, 15, 16, 17)),
+            (lib.lo_fused_moe_channel_int8, channel, (0, 16, 17, 18)),
+            (lib.lo_moe_grouped_gemm_i8_block, gemm, (0,)),
+            (lib.lo_moe_grouped_gemm_i8_channel, gemm, (0,)),
+            (lib.lo_expert_rows_block_int8, [P] * 8 + [M, E, H, I, P, P, big, 0, 0], (0,)),
+            (lib.lo_moe_sum, [P, P, P, _lib.LO_BF16, M, k, H, 1.0, 0, 0, 0], (0, 1, 2)),
+            (lib.lo_ep_scatter, [P, P, 1, P, _lib.LO_I32, 0, 0, P, P, P, P, M, k, H, 64, E, 16, 0], (0, 7)),
+            (lib.lo_ep_dispatch_pack, [P, P, P, _lib.LO_I32, P, P, M, k, H, E, 2, P, P, P, P, 0], (0, 11)),
+            (lib.lo_ep_dispatch_put, [P, P, P, _lib.LO_I32, P, P, P, M, k, H, E, 2, P, P, 0], (0,)),
+            (lib.lo_ep_gather, [P, P, _lib.LO_I32, P, P, 0, P, M, k, H, 0], (0, 6))]
+
+
+def test_misaligned_caller_memory_is_refused_on_the_host():
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    for entry, args, positions in _entries_with_vector_access(lib):
+        for i in positions:
+            for off in (2, 8):
+                bad = list(args)
+                bad[i] += off
+                assert entry(*bad) == 1, (entry.__name__, i, off)
+                assert b"16-byte aligned" in lib.lo_last_error(), (entry.__name__, i, lib.lo_last_error())
+
+
+def test_alignment_does_not_matter_without_work():
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    assert lib.lo_moe_sum(18, 18, 0, _lib.LO_BF16, 0, 2, 128, 1.0, 0, 0, 0) == 0
+    assert lib.lo_ep_gather(18, 16, _lib.LO_I32, 16, 16, 0, 18, 0, 2, 128, 0) == 0
+    assert lib.lo_ep_dispatch_put(18, 16, 16, _lib.LO_I32, 16, 16, 16, 0, 2, 128, 2, 2, 16, 16, 0) == 0
