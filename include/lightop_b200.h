@@ -251,8 +251,8 @@ int lo_expert_rows_block_int8_packed_put(const uint8_t *packed, int64_t T, const
  * K a multiple of 128; N arbitrary (weight rows past N read as zero and are not stored).
  * Same kernel as the grouped GEMM with one expert.  workspace: lo_block_int8_linear_workspace_bytes(M); with
  * lo_block_int8_linear_split_workspace_bytes(M, N, K) bytes or more the K extent is dealt to several CTAs where the
- * output tiles alone would leave most of them idle (the fp32 sums of the parts go through the workspace and are
- * added in the order of K).
+ * output tiles alone would leave most of them idle and that is faster.  The result has the same bits either way: a
+ * row of C depends on its row of A and on B alone, whatever M is.
  */
 size_t lo_block_int8_linear_workspace_bytes(int64_t M);
 int lo_block_int8_linear(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale,

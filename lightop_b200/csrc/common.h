@@ -153,10 +153,10 @@ struct GemmArgs {
   int fixed_chunks;
   const int32_t *masked_m;
   int64_t max_m;
-  // Single mode without a chunk table: the K extent of a tile in parts of split_steps K blocks (a multiple of 4), the fp32 sums
-  // of part i to partial[i][row][n] (null: not split).
+  // Single mode without a chunk table: the K extent of a tile in parts of split_steps K blocks, the int32 sum of K block kb to
+  // partial[kb][row][n], without scales (null: not split).
   int split_steps;
-  float *partial;
+  int32_t *partial;
 };
 
 int launch_grouped_gemm(GemmMode mode, const GemmArgs &args, cudaStream_t stream);

@@ -645,13 +645,27 @@ namespace lo {
 namespace {
 // How a dense call is cut.  Chunks of at most 128 rows; equally many each where all items run at the same time (129 rows: 80 and
 // 49), else full ones with the short one last, where it shortens the last wave (300 x 7168 x 2048: 18.7 against 20.6 us).
-// Where the tiles would leave half of the SMs or more without work, the K extent of a tile is dealt to n_split items of split_steps
-// K blocks (a multiple of four: the unit of the scale tables).  That adds a pass over the output in fp32 and a launch that adds
-// the parts up, 2 to 3 us, and takes K blocks off a CTA at about 0.2 us each: worth it from SPLIT_MIN_K K blocks on.  One row,
-// N = 576, K = 7168: 16.1 -> 8.3 us, 4096 x 7168: 16.5 -> 10.6 us, 129 rows, N = 4096: 27.0 -> 20.8 us; at K = 1280 to 2048 it
-// changed nothing or cost 1 us.
+//
+// Where the tiles would leave half of the SMs or more without work, the K extent of a tile can be dealt to n_split items of
+// split_steps K blocks.  The items write the int32 sum of every K block and a second kernel carries the fp32 chain over them in
+// the order of K, so a row has the same bits whatever the form and whatever the other rows of the call are.  (fp32 sums of
+// the parts are a quarter of the traffic and less, but associate differently: one bf16 output in 5000 changed with the batch.)
+// split_gain_us() is the rule, in microseconds: a K block taken off a CTA's chain saves 0.17 us and 0.0015 us a row; the second
+// kernel costs 2.5 us and 0.08 us a K block of its chain, the sums 0.55 us a million (written and read through L2, up to 9
+// million of them).  Undivided and split, kernel time in us:
+//     1 x 576 x 7168: 13.6, 9.2     32 x 576 x 7168: 14.1, 11.0    128 x 576 x 7168: 22.7, 13.9    200 x 576 x 7168: 23.2, 16.5
+//     1 x 4096 x 7168: 14.6, 13.5    8 x 4096 x 7168: 14.6, 14.4   16 x 4096 x 7168: 14.8, 16.1     64 x 4096 x 7168: 16.9, 27.3
+//    16 x 2048 x 7168: 14.2, 12.3   64 x 2048 x 7168: 16.1, 16.0   96 x 2048 x 7168: 20.6, 22.8    128 x 2048 x 7168: 23.1, 26.2
+//     1 x 576 x 4096: 9.0, 6.9      300 x 576 x 4096: 15.9, 14.4   16 x 2048 x 4096: 9.5, 8.5       32 x 2048 x 4096: 9.6, 10.1
+// The rule errs by up to 0.8 us at 64 to 128 x 2048 x 4096 (15.4, 16.2) and by 2 us at 500 x 520 x 4096 (15.6, 17.6).
+// Below 32 K blocks it changes little or loses: 576 x 2048 from 5.9, 5.5 (1 row) to 9.7, 9.3 (128), 1024 x 3072 from 7.6, 7.1 to
+// 12.6, 11.9 with losses up to 1 us between, 1536 x 1536 5.3, 7.1.
 constexpr int64_t LINEAR_CHUNK = 128;
-constexpr int SPLIT_MIN_STEPS = 4, SPLIT_MIN_K = 32;
+constexpr int SPLIT_MIN_STEPS = 2, SPLIT_MIN_K = 32, SPLIT_MAX_K = 512;      // K blocks: of a part, of a split call
+constexpr int64_t SPLIT_MAX_SUMS = 9000000;
+inline double split_gain_us(int64_t KB, int64_t steps, int64_t chunk_rows, int64_t sums) {
+  return (double)(KB - steps) * (0.17 + 0.0015 * (double)chunk_rows) - (2.5 + 0.08 * (double)KB + 0.55e-6 * (double)sums);
+}
 struct LinearPlan {
   int chunk_rows, n_chunks, n_tiles, split_steps, n_split;
   size_t partial_bytes;
@@ -665,43 +679,37 @@ LinearPlan plan_linear(int64_t M, int64_t N, int64_t K) {
   const int64_t KB = K / 128, items = (int64_t)L.n_chunks * L.n_tiles;
   const int64_t want = sm_count() / items;       // parts that fill the SMs once
   L.split_steps = 0; L.n_split = 1; L.partial_bytes = 0;
-  if (want >= 2 && KB >= SPLIT_MIN_K) {
-    const int64_t steps = round_up(ceil_div(KB, want), SPLIT_MIN_STEPS);
-    if (ceil_div(KB, steps) >= 2) {
+  if (want >= 2 && KB >= SPLIT_MIN_K && KB <= SPLIT_MAX_K) {
+    int64_t steps = ceil_div(KB, want);
+    if (steps < SPLIT_MIN_STEPS) steps = SPLIT_MIN_STEPS;
+    const int64_t sums = KB * M * N;
+    if (ceil_div(KB, steps) >= 2 && sums <= SPLIT_MAX_SUMS && split_gain_us(KB, steps, L.chunk_rows, sums) > 0) {
       L.split_steps = (int)steps;
       L.n_split = (int)ceil_div(KB, steps);
-      L.partial_bytes = (size_t)round_up((int64_t)L.n_split * M * N * 4, ALIGN_BYTES);
+      L.partial_bytes = (size_t)round_up(sums * 4, ALIGN_BYTES);
     }
   }
   return L;
 }
 
-// C = bf16 of the parts' sum, added in the order of K.  One thread per VEC columns of a row of C.
-template <int VEC>
-__global__ void __launch_bounds__(128) linear_reduce_kernel(const float *__restrict__ partial, int n_split, int64_t total,
-                                                            __nv_bfloat16 *__restrict__ C) {
+// C from the int32 sums of the K blocks: acc = fma(float(dot), a_s * b_s, acc) over the K blocks in their order, the chain that the
+// promotion warps of the undivided form carry, so both forms give the same bits.  One block per row and 128 columns; bound by the
+// latency of its loads (sixteen in flight a thread): 3 us of the 9.2 at 1 x 576 x 7168.
+__global__ void __launch_bounds__(128) linear_promote_kernel(const int32_t *__restrict__ partial, const float *__restrict__ a_scale,
+                                                             const float *__restrict__ b_scale, int64_t M, int64_t N, int KB,
+                                                             __nv_bfloat16 *__restrict__ C) {
+  __shared__ float sc[SPLIT_MAX_K];
+  const int64_t row = blockIdx.y, n = (int64_t)blockIdx.x * 128 + threadIdx.x;
   dependency_wait();
-  const int64_t i = ((int64_t)blockIdx.x * 128 + threadIdx.x) * VEC;
-  if (i >= total) return;
-  float a[VEC];
-#pragma unroll
-  for (int v = 0; v < VEC; ++v) a[v] = 0.f;
-#pragma unroll 4
-  for (int s = 0; s < n_split; ++s) {
-    const float *src = partial + (int64_t)s * total + i;
-    if (VEC == 4) {
-      const float4 f = *reinterpret_cast<const float4 *>(src);
-      a[0] += f.x; a[VEC > 1 ? 1 : 0] += f.y; a[VEC > 2 ? 2 : 0] += f.z; a[VEC > 3 ? 3 : 0] += f.w;
-    } else {
-      a[0] += *src;
-    }
-  }
-  if (VEC == 4) {
-    const __nv_bfloat162 lo2 = __floats2bfloat162_rn(a[0], a[VEC > 1 ? 1 : 0]), hi2 = __floats2bfloat162_rn(a[VEC > 2 ? 2 : 0], a[VEC > 3 ? 3 : 0]);
-    *reinterpret_cast<uint2 *>(C + i) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo2), *reinterpret_cast<const uint32_t *>(&hi2));
-  } else {
-    C[i] = __float2bfloat16_rn(a[0]);
-  }
+  for (int kb = threadIdx.x; kb < KB; kb += 128) sc[kb] = __fmul_rn(a_scale[row * KB + kb], b_scale[(int64_t)blockIdx.x * KB + kb]);
+  __syncthreads();
+  if (n >= N) return;
+  const int64_t slab = M * N;
+  const int32_t *src = partial + row * N + n;
+  float acc = 0.f;
+#pragma unroll 16
+  for (int kb = 0; kb < KB; ++kb) acc = __fmaf_rn(__int2float_rn(__ldg(src + kb * slab)), sc[kb], acc);
+  C[row * N + n] = __float2bfloat16_rn(acc);
 }
 
 int check_linear(int64_t M, int64_t N, int64_t K) {
@@ -711,7 +719,7 @@ int check_linear(int64_t M, int64_t N, int64_t K) {
 }
 
 int run_linear(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K,
-               void *C, const LinearPlan &L, float *partial, int32_t *status, cudaStream_t st) {
+               void *C, const LinearPlan &L, int32_t *partial, int32_t *status, cudaStream_t st) {
   GemmArgs g{};
   g.A = A; g.a_scale = a_scale; g.rows_a = M; g.max_chunk_rows = L.chunk_rows;
   g.B = B; g.b_scale = b_scale; g.E = 1;
@@ -722,11 +730,8 @@ int run_linear(const int8_t *A, const float *a_scale, const int8_t *B, const flo
   if (L.n_split > 1 && partial != nullptr) { g.split_steps = L.split_steps; g.partial = partial; }
   const int rc = launch_grouped_gemm(GEMM_SINGLE, g, st);
   if (rc != LO_OK || g.partial == nullptr) return rc;
-  const int64_t total = M * N;
-  const bool vec = total % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0;
-  const int64_t threads = vec ? total / 4 : total;
-  LO_CUDA_OK(launch_dependent(vec ? linear_reduce_kernel<4> : linear_reduce_kernel<1>, dim3((unsigned)ceil_div(threads, 128)), dim3(128), 0, st,
-                              (const float *)partial, L.n_split, total, static_cast<__nv_bfloat16 *>(C)));
+  LO_CUDA_OK(launch_dependent(linear_promote_kernel, dim3((unsigned)L.n_tiles, (unsigned)M), dim3(128), 0, st, (const int32_t *)partial, a_scale,
+                              b_scale, M, N, (int)(K / 128), static_cast<__nv_bfloat16 *>(C)));
   return LO_OK;
 }
 }  // namespace
@@ -752,7 +757,7 @@ extern "C" int lo_block_int8_linear(const int8_t *A, const float *a_scale, const
   const size_t need = lo_block_int8_linear_workspace_bytes(M);
   LO_REQUIRE(workspace_bytes >= need, "block int8 linear: workspace of %zu bytes, %zu needed", workspace_bytes, need);
   // the K extent is split where the workspace has room for the parts
-  float *partial = L.n_split > 1 && workspace_bytes >= L.partial_bytes ? static_cast<float *>(workspace) : nullptr;
+  int32_t *partial = L.n_split > 1 && workspace_bytes >= L.partial_bytes ? static_cast<int32_t *>(workspace) : nullptr;
   return run_linear(A, a_scale, B, b_scale, M, N, K, C, L, partial, status, static_cast<cudaStream_t>(stream));
 }
 
@@ -761,7 +766,7 @@ namespace {
 struct DynLinearLayout {
   int8_t *xq;
   float *xs;
-  float *partial;
+  int32_t *partial;
   size_t bytes;
 };
 DynLinearLayout carve_dyn_linear(void *ws, int64_t M, int64_t K, const LinearPlan &L) {
@@ -769,7 +774,7 @@ DynLinearLayout carve_dyn_linear(void *ws, int64_t M, int64_t K, const LinearPla
   Carver c(ws);
   D.xq = c.take<int8_t>(M * K);
   D.xs = c.take<float>(M * (K / 128));
-  D.partial = c.take<float>((int64_t)(L.partial_bytes / 4));
+  D.partial = c.take<int32_t>((int64_t)(L.partial_bytes / 4));
   D.bytes = c.off;
   return D;
 }

@@ -454,11 +454,11 @@ struct KParams {
   const int32_t *masked_m;  // per-channel mode: rows of each expert, in a layout of max_m rows an expert
   int64_t max_m;
   int64_t dense_rows;       // single mode: rows of the one expert
-  // Single mode: K blocks per item when the K extent of a tile is dealt to several items (0: not split), a multiple of
-  // SC_STEPS; the fp32 sums of part i then go to partial[i][row][n] instead of C.
+  // Single mode: K blocks per item when the K extent of a tile is dealt to several items (0: not split); the int32 sum of every
+  // K block then goes to partial[kb][row][n] instead of C, without scales.
   int split_steps;
   int n_split;
-  float *partial;
+  int32_t *partial;
 };
 
 // Four tensor maps of the sorted activation matrix, box heights 16 / 32 / 64 / 128 rows.  A chunk of
@@ -532,6 +532,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   constexpr int PHASES = CF::PHASES;
   constexpr int NCG = CF::NCG;
   constexpr int EPI_WARPS = CF::EPI_WARPS;
+  constexpr bool RESPLIT = CF::SPLIT_REGS && FORM != SPLIT;      // (a split K extent has no running sums)
   extern __shared__ uint8_t smem_raw[];
   SM &sm = *reinterpret_cast<SM *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
@@ -588,7 +589,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   int nt = 0;
 
   if (warp < FIRST_EPI_WARP) {
-    if constexpr (CF::SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_FEED));
+    if constexpr (RESPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_FEED));
     if (warp == 0) {
       // ============ weight producer: one 128 x 128 tile per K block (gate_up: gate pass, then up pass) ============
       if (lane == 0) {
@@ -652,21 +653,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       // warp's chain (wait, multiply, store, arrive: 900 cycles) the slowest of the kernel.  Scales come from L2 (the chunk's
       // scale rows are read by every output tile of the expert), one batch ahead, across the ends of passes and items.  Rows
       // of scales whose length is a multiple of four are read with 16-byte loads.
-      if constexpr (MODE != GEMM_CHANNEL) {
+      if constexpr (MODE != GEMM_CHANNEL && FORM != SPLIT) {
         constexpr int NU = (A_ROWS + 31) / 32;
         const int64_t nblk = (p.n_rows_per_expert + TILE_N - 1) / TILE_N;
         const bool vec = (KB & 3) == 0;
         ItemCursor<MODE, FORM> items(p, num_chunks);
-        struct Batch { Chunk ch; int nt, ph, kb, k_end; bool valid; };     // K blocks kb .. kb + 3 of a pass over an item
+        struct Batch { Chunk ch; int nt, ph, kb; bool valid; };     // K blocks kb .. kb + 3 of a pass over an item
         float a_cur[NU][4], b_cur[4], a_nxt[NU][4], b_nxt[4];
         auto next_item = [&](Batch &b) {
           do { b.valid = items.take(b.ch, b.nt); } while (b.valid && b.ch.expert < 0);
-          b.kb = FORM == SPLIT ? items.k0 : 0;
-          b.k_end = FORM == SPLIT ? items.k0 + items.kn : KB;
         };
         auto advance = [&](Batch &b) {
           b.kb += SC_STEPS;
-          if (b.kb >= (FORM == SPLIT ? b.k_end : KB)) {
+          if (b.kb >= KB) {
             b.kb = 0;
             if (++b.ph == PHASES) { b.ph = 0; next_item(b); }
           }
@@ -690,7 +689,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 4; ++i) b[i] = bt.kb + i < KB ? __ldg(bs + i) : 0.f;
         };
-        Batch cur{ch, 0, 0, 0, 0, false};
+        Batch cur{ch, 0, 0, 0, false};
         next_item(cur);
         if (cur.valid) fetch(cur, a_cur, b_cur);
         Batch nxt = cur;
@@ -719,7 +718,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           if (lane == 0) mbar_arrive(&sm.scales[slot]);
           slot = slot + 1 == (uint32_t)SC_BATCHES ? 0u : slot + 1;
           ++n_batch;
-          const int k_left = (FORM == SPLIT ? cur.k_end : KB) - cur.kb;
+          const int k_left = KB - cur.kb;
           it += (uint32_t)(k_left < SC_STEPS ? k_left : SC_STEPS);
 #pragma unroll
           for (int i = 0; i + 1 < SC_BATCHES; ++i) end_of[i] = end_of[i + 1];
@@ -802,10 +801,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     // ====================== output warps (block-scaled modes) ======================
     // They turn the finished tile in the staging buffer (bf16, row = token) into rows of global memory while the
     // promotion warps are already on the next item.
-    if constexpr (CF::SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OUT));
+    if constexpr (RESPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OUT));
     const int ow = warp - (FIRST_EPI_WARP + EPI_WARPS);
     uint32_t par = 0;
-    // (the parts of a split K extent leave the kernel as fp32 sums, straight from the promotion warps)
+    // (the parts of a split K extent leave the kernel as int32 sums, straight from the promotion warps)
     for (ItemCursor<MODE, FORM> items(p, FORM == SPLIT ? 0 : num_chunks); items.take(ch, nt);) {
       if (ch.expert < 0) {
         // block of a non-local expert: its output rows are zero
@@ -918,7 +917,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     }
   } else {
     // ====================== promotion (block-scaled modes) / epilogue (per-channel mode) ======================
-    if constexpr (CF::SPLIT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_PROMO));
+    if constexpr (RESPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_PROMO));
     const int pw = warp - FIRST_EPI_WARP;
     const int q = warp & 3;              // lane quarter of tensor memory this warp may access
     const int cg = pw >> 2;              // column group: which share of the chunk's tokens
@@ -1017,13 +1016,42 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           __syncwarp();
           if (lane == 0) mbar_arrive(&sm.tmem_empty[b]);
         }
+      } else if constexpr (FORM == SPLIT) {
+        // ---------------- a part of the K extent: the int32 sum of every K block as it is ----------------
+        // What comes after them (scales, fp32 sum, rounding) is left to the kernel that follows, which takes the K blocks in
+        // their order: the result has the bits of the undivided form.  Lane = output channel, so a store of a warp is 128
+        // consecutive bytes of one token's row.
+        const int64_t n = (int64_t)nt * TILE_N + n_local;
+        const int64_t slab = p.dense_rows * p.n_store;
+        int32_t *dst = p.partial + items.k0 * slab + (int64_t)(ch.row0 + col_begin) * p.n_store + n;
+        const int my_rows = n < p.n_store ? min(ch.rows - col_begin, my_p * 16) : 0;
+        for (int kb = 0; kb < items.kn; ++kb, ++step, dst += slab) {
+          const uint32_t slot = step % ND;
+          if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.done[slot], (step / ND) & 1u, p.status, 5))) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t part = tmem_base + lane_off + buf * (uint32_t)A_ROWS + (uint32_t)col_begin;
+#pragma unroll 1
+          for (int pc = 0; pc < my_p; ++pc) {
+            uint32_t raw[16];
+            tmem_ld16(part + pc * 16, raw);
+            tmem_ld_wait16(raw);
+            if (pc == my_p - 1) {
+              tc_fence_before();
+              mbar_arrive(&sm.consumed[slot]);
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (pc * 16 + j < my_rows) dst[(int64_t)(pc * 16 + j) * p.n_store] = (int32_t)raw[j];
+          }
+          if (my_p == 0) mbar_arrive(&sm.consumed[slot]);
+          buf = buf + 1 == (uint32_t)NBUF ? 0u : buf + 1;
+        }
       } else {
         // ---------------- block-scaled modes: promotion once per K block, sums in registers ----------------
         // This warp owns the columns [col_begin, col_begin + 16 * my_p) of its 32 lanes.  Their fp32 running sums
         // stay in registers over the whole K loop, so tensor memory holds nothing but partial buffers and a
         // K block costs one tensor-memory load per piece of 16 columns.
         constexpr int NP = (A_ROWS / 16 + NCG - 1) / NCG;
-        const int kn = FORM == SPLIT ? items.kn : KB;
         float acc[NP][16];
         // Addresses of this item, formed once: the loops below only add constants to them.  Ring positions
         // (scale slot, partial buffer and its phase) are carried as counters instead of being divided out of
@@ -1073,7 +1101,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (PC > 0) load_unit(0, part0 + buf * (uint32_t)A_ROWS, raw[0]);
             uint32_t sc_at = 0;
 #pragma unroll 1
-            for (int kb0 = 0; kb0 < kn; kb0 += UNROLL) {
+            for (int kb0 = 0; kb0 < KB; kb0 += UNROLL) {
               if ((kb0 & (SC_STEPS - 1)) == 0) {
                 // the scale products of the coming four steps
                 if (PC > 0 && !__all_sync(0xffffffffu, mbar_wait_addr(sm, scales0 + 8u * sc_slot, sc_par, p.status, 7))) { ok = false; return; }
@@ -1082,7 +1110,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
               }
 #pragma unroll
               for (int i = 0; i < UNROLL; ++i) {
-                if (i > 0 && kb0 + i >= kn) break;
+                if (i > 0 && kb0 + i >= KB) break;
                 const uint32_t part = part0 + buf * (uint32_t)A_ROWS;
                 const uint32_t used = consumed0 + 8u * dn;
                 buf = buf + 1 == (uint32_t)NBUF ? 0u : buf + 1;
@@ -1113,7 +1141,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                     // 4096 tokens 2965 -> 3100 us, sharded 8192 788 -> 820 us; arriving with all lanes 2965 -> 2980 us.)
                     tc_fence_before();
                     mbar_arrive_addr(used);
-                    if (kb0 + i + 1 < kn) {
+                    if (kb0 + i + 1 < KB) {
                       // warp-uniform outcome: the accesses to tensor memory are warp-collective
                       if (!__all_sync(0xffffffffu, next_done) &&
                           !__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; return; }
@@ -1151,20 +1179,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (my_p >= 5) k_loop(std::integral_constant<int, 5>{});
           }
           if (!ok) break;
-          if constexpr (FORM == SPLIT) {
-            // a part of the K extent: the sums as they are (eight lanes side by side hold eight channels of one token)
-            float *dst = p.partial + ((int64_t)(items.k0 / p.split_steps) * p.dense_rows + ch.row0) * p.n_store;
-#pragma unroll
-            for (int pc = 0; pc < NP; ++pc) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int t = col_begin + pc * 16 + ((j >> 2) & 1) * 8 + (lane & 3) * 2 + (j & 1);
-                const int64_t n = (int64_t)nt * TILE_N + q * 32 + (j >> 3) * 16 + ((j >> 1) & 1) * 8 + (lane >> 2);
-                if (pc < my_p && t < ch.rows && n < p.n_store) dst[t * p.n_store + n] = acc[pc][j];
-              }
-            }
-            continue;
-          }
           // routed weight on the fp32 sums (before their rounding), where the mode asks for it
           if (FORM == TABLE && p.weight_mode == LO_WEIGHT_FP32) {
 #pragma unroll
@@ -1237,7 +1251,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           }
         }
         if (!ok) break;
-        if (FORM == SPLIT) continue;
         // the finished tile is in the staging buffer: over to the output warps
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.stg_full);
@@ -1362,8 +1375,8 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
   LO_REQUIRE((reinterpret_cast<uintptr_t>(a.C) & 1) == 0, "grouped gemm: the output must be aligned to its bf16 elements");
   LO_REQUIRE(a.chunks != nullptr || (a.fixed_chunks >= 1 && a.max_chunk_rows >= 1 && ((mode == GEMM_SINGLE && a.max_chunk_rows <= T_MAX) || (mode == GEMM_CHANNEL && a.masked_m != nullptr))),
              "grouped gemm: no chunk table");
-  LO_REQUIRE(a.partial == nullptr || (mode == GEMM_SINGLE && a.chunks == nullptr && a.max_chunk_rows <= T_MAX && a.split_steps >= SC_STEPS &&
-                                      a.split_steps % SC_STEPS == 0 && a.weight_mode == LO_WEIGHT_NONE),
+  LO_REQUIRE(a.partial == nullptr || (mode == GEMM_SINGLE && a.chunks == nullptr && a.max_chunk_rows <= T_MAX && a.split_steps >= 1 &&
+                                      a.weight_mode == LO_WEIGHT_NONE),
              "grouped gemm: the K extent is split for dense calls only");
   // no chunk can hold more rows than max_chunk_rows (a bound the caller derives from the token count)
   const int cap = a.max_chunk_rows <= 0 ? T_MAX : a.max_chunk_rows;

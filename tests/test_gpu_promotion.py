@@ -144,3 +144,43 @@ def test_moe_gemm_output_off_a_16_byte_boundary():
     out = buf[3:3 + M * k * N].view(M, k, N)
     lo.moe.moe_gemm_w8a8(q, w, out, s, w_s, wgt, sorted_ids, expert_ids, num_post, k, {"BLOCK_SIZE_M": block})
     assert torch.equal(out, ref) and bool((buf[:3] == 7.0).all()) and bool((buf[3 + M * k * N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("N,K", [(576, 7168), (201, 4096), (1024, 4224), (256, 640)])
+def test_linear_rows_do_not_depend_on_the_batch(N, K):
+    # the same row among 1 and among 700 others: chunks of other widths, the K extent split or not, the same bits
+    import lightop_b200 as lo
+    g = torch.Generator().manual_seed(N + K)
+    x = torch.randn(700, K, generator=g).to(torch.bfloat16).to(DEV)
+    B = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8).to(DEV)
+    b_s = (torch.rand((N + 127) // 128, K // 128, generator=g) * 9e-3 + 1e-3).to(DEV)
+    whole = lo.gemm_ops.apply_w8a8_block_int8_linear(x, B, [128, 128], b_s)
+    for M in (1, 3, 17, 64, 128, 129, 300):
+        part = lo.gemm_ops.apply_w8a8_block_int8_linear(x[:M].contiguous(), B, [128, 128], b_s)
+        assert torch.equal(part, whole[:M]), f"{M} rows: {int((part != whole[:M]).sum())} outputs differ"
+    torch.cuda.synchronize()
+    lo.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 576, 7168), (2, 129, 4096), (16, 2048, 7168), (65, 136, 4096), (128, 1024, 4096), (129, 576, 4224), (1, 1, 65536), (3, 256, 4352)])
+def test_split_linear_has_the_bits_of_the_undivided_form(M, N, K):
+    import lightop_b200 as lo
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(M + N + K)
+    A = torch.randint(-127, 128, (M, K), generator=g, dtype=torch.int8).to(DEV)
+    a_s = (torch.rand(M, K // 128, generator=g) * 1e-2).to(DEV)
+    B = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8).to(DEV)
+    b_s = (torch.rand((N + 127) // 128, K // 128, generator=g) * 1e-2).to(DEV)
+    out = []
+    n = lib.lo_block_int8_linear_split_workspace_bytes(M, N, K)
+    assert n >= 4 * (K // 128) * M * N          # the call is split
+    for nbytes in (n, 256):
+        c = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+        assert lib.lo_block_int8_linear(A.data_ptr(), a_s.data_ptr(), B.data_ptr(), b_s.data_ptr(), M, N, K, c.data_ptr(), ws.data_ptr(), nbytes, 0,
+                                        torch.cuda.current_stream().cuda_stream) == 0
+        out.append(c)
+    torch.cuda.synchronize()
+    lo.check_device_status()
+    assert torch.equal(out[0], out[1])
