@@ -402,6 +402,12 @@ template <typename T, int N> __device__ __forceinline__ T pick(const T (&v)[N], 
   return r;
 }
 
+// Maximum that is NaN when an operand is (fmaxf gives the other operand).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 // Reciprocal refined by one Newton step, and the quotient a / b from it with the remainder folded back in (Markstein's method,
 // "Computation of elementary functions on the IBM RISC System/6000 processor", 1990)
@@ -838,10 +844,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             v[e][1] = __uint_as_float(raw.x & 0xffff0000u);
             v[e][2] = __uint_as_float(raw.y << 16);
             v[e][3] = __uint_as_float(raw.y & 0xffff0000u);
-            // (as bit patterns, like the warp's maximum below: a NaN is above every number there, where fmaxf would drop it, so
-            // the group's scale does not depend on which of its channels holds one)
-            m[e] = max(max(__float_as_uint(v[e][0]) & 0x7fffffffu, __float_as_uint(v[e][1]) & 0x7fffffffu),
-                       max(__float_as_uint(v[e][2]) & 0x7fffffffu, __float_as_uint(v[e][3]) & 0x7fffffffu));
+            // (a NaN is kept, and as a bit pattern it is above every number in the warp's maximum below: the group's scale does not
+            // depend on which of its channels holds one)
+            m[e] = __float_as_uint(max_nan(max_nan(fabsf(v[e][0]), fabsf(v[e][1])), max_nan(fabsf(v[e][2]), fabsf(v[e][3]))));
           }
 #pragma unroll
           for (int e = 0; e < UN; ++e) m[e] = __reduce_max_sync(0xffffffffu, m[e]);
