@@ -249,8 +249,8 @@ int lo_expert_rows_block_int8_packed_put(const uint8_t *packed, int64_t T, const
  *           (python/lightop/gemmopt.py:633-639, csrc/asm/asm_gemm_w8a8.cu:136-147).
  * A [M,K] int8, a_scale [M,K/128] f32 (row-major), B [N,K] int8, b_scale [ceil(N/128), K/128] f32, C [M,N] bf16.
  * K a multiple of 128; N arbitrary (weight rows past N read as zero and are not stored).
- * Same kernel as the grouped GEMM with one expert.  workspace: lo_block_int8_linear_workspace_bytes(M); with
- * lo_block_int8_linear_split_workspace_bytes(M, N, K) bytes or more the K extent is dealt to several CTAs where the
+ * Same kernel as the grouped GEMM with one expert.  workspace: may be null; with
+ * lo_block_int8_linear_split_workspace_bytes(M, N, K) bytes or more (256-byte aligned) the K extent is dealt to several CTAs where the
  * output tiles alone would leave most of them idle and that is faster.  The result has the same bits either way: a
  * row of C depends on its row of A and on B alone, whatever M is.
  */
@@ -406,7 +406,8 @@ int lo_silu_mul_quant_int8_masked(const void *input, int64_t groups, int64_t gro
  *               128); a block that breaks the contract is skipped and code 20 is written to *status.
  *   masked:     A [E, max_m, K], masked_m i32 [E] = rows that exist per expert; C [E, max_m, N].
  * a_scale f32 [rows], B int8 [E, N, K] (plain layout), b_scale f32 [E, N].  N and K multiples of 128.
- * workspace: lo_m_grouped_gemm_workspace_bytes(total rows, E) bytes, 256-byte aligned.
+ * workspace: contiguous: lo_m_grouped_gemm_workspace_bytes(total rows, E) bytes, 256-byte aligned; masked: not used, may
+ * be null.
  * Replaces: op.m_grouped_w8a8_gemm_nt_contig_asm (python/lightop/gemmopt.py:744-751) and
  * op.m_grouped_marlin_w8a8_gemm_nt_masked_asm (python/lightop/gemmopt.py:604-617), which take weights
  * pre-shuffled for the reference's matrix cores; reference models test/w8a8/test_w8a8_deepgemm_contig.py:106-147

@@ -737,12 +737,12 @@ int run_linear(const int8_t *A, const float *a_scale, const int8_t *B, const flo
 }  // namespace
 }  // namespace lo
 
-extern "C" size_t lo_block_int8_linear_workspace_bytes(int64_t M) { return M <= 0 ? 0 : (size_t)lo::ALIGN_BYTES; }
+// (the undivided form writes nothing but C)
+extern "C" size_t lo_block_int8_linear_workspace_bytes(int64_t) { return 0; }
 
 extern "C" size_t lo_block_int8_linear_split_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K < 128) return 0;
-  const size_t parts = lo::plan_linear(M, N, K).partial_bytes;
-  return parts > 0 ? parts : (size_t)lo::ALIGN_BYTES;
+  return lo::plan_linear(M, N, K).partial_bytes;
 }
 
 extern "C" int lo_block_int8_linear(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale,
@@ -751,13 +751,11 @@ extern "C" int lo_block_int8_linear(const int8_t *A, const float *a_scale, const
   using namespace lo;
   const int rc = check_linear(M, N, K);
   if (rc != LO_OK || M == 0) return rc;
-  LO_REQUIRE(A && a_scale && B && b_scale && C && workspace, "block int8 linear: null pointer");
+  LO_REQUIRE(A && a_scale && B && b_scale && C, "block int8 linear: null pointer");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "block int8 linear: workspace must be 256-byte aligned");
   const LinearPlan L = plan_linear(M, N, K);
-  const size_t need = lo_block_int8_linear_workspace_bytes(M);
-  LO_REQUIRE(workspace_bytes >= need, "block int8 linear: workspace of %zu bytes, %zu needed", workspace_bytes, need);
   // the K extent is split where the workspace has room for the parts
-  int32_t *partial = L.n_split > 1 && workspace_bytes >= L.partial_bytes ? static_cast<int32_t *>(workspace) : nullptr;
+  int32_t *partial = L.n_split > 1 && workspace != nullptr && workspace_bytes >= L.partial_bytes ? static_cast<int32_t *>(workspace) : nullptr;
   return run_linear(A, a_scale, B, b_scale, M, N, K, C, L, partial, status, static_cast<cudaStream_t>(stream));
 }
 

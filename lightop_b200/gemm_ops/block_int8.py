@@ -39,7 +39,7 @@ def matmul_block_int8(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs: to
     if M:
         lib = _lib.load()
         nbytes = lib.lo_block_int8_linear_split_workspace_bytes(M, N, K)
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=A.device)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=A.device) if nbytes else None
         with _lib.on_device(A.device):
             st = lib.lo_block_int8_linear(_lib.ptr(a2), _lib.ptr(as2), _lib.ptr(B), _lib.ptr(bs2), M, N, K,
                                           _lib.ptr(C), _lib.ptr(ws), nbytes, _lib.ptr(device_status_word(A.device)),

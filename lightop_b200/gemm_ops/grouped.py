@@ -84,13 +84,11 @@ def m_grouped_w8a8_gemm_nt_masked(a: Tuple[torch.Tensor, torch.Tensor], b: Tuple
     if max_m == 0:
         return d
     lib = _lib.load()
-    ws_bytes = lib.lo_m_grouped_gemm_workspace_bytes(E * max_m, E)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=inp.device)
     status = device_status_word(inp.device)
     with _lib.on_device(inp.device):
         st = lib.lo_m_grouped_w8a8_gemm_nt_masked(_lib.ptr(inp), _lib.ptr(a_scale), _lib.ptr(w), _lib.ptr(b_scale),
                                                   _lib.ptr(d), _lib.ptr(masked_m.contiguous()), E, max_m, N, K,
-                                                  _lib.ptr(ws), ws_bytes, _lib.ptr(status),
+                                                  0, 0, _lib.ptr(status),
                                                   _lib.current_stream(inp.device))
     _lib.check(st, "m_grouped_w8a8_gemm_nt_masked")
     return d

@@ -78,6 +78,23 @@ def test_masked_layout(lo, E, max_m, masked, N, K):
     assert torch.equal(d.cpu(), ref)
 
 
+def test_masked_layout_keeps_no_scratch(lo):
+    from lightop_b200 import _lib
+    E, max_m, N, K = 2, 40, 128, 256
+    g = torch.Generator().manual_seed(6)
+    A = torch.randint(-127, 128, (E, max_m, K), generator=g, dtype=torch.int8).to(DEV)
+    As = (torch.rand(E, max_m, generator=g) * 0.05 + 1e-3).to(DEV)
+    B = torch.randint(-127, 128, (E, N, K), generator=g, dtype=torch.int8).to(DEV)
+    Bs = (torch.rand(E, N, generator=g) * 9e-4 + 1e-4).to(DEV)
+    mm = torch.tensor([40, 17], dtype=torch.int32, device=DEV)
+    d = torch.zeros(E, max_m, N, dtype=torch.bfloat16, device=DEV)
+    st = _lib.load().lo_m_grouped_w8a8_gemm_nt_masked(A.data_ptr(), As.data_ptr(), B.data_ptr(), Bs.data_ptr(), d.data_ptr(), mm.data_ptr(), E, max_m,
+                                                      N, K, 0, 0, 0, torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    ref = OC.grouped_matmul_masked(A.cpu(), As.cpu(), B.cpu(), Bs.cpu(), mm.cpu(), torch.zeros(E, max_m, N, dtype=torch.bfloat16))
+    assert torch.equal(d.cpu(), ref)
+
+
 def test_masked_silu_mul_quant(lo):
     g = torch.Generator().manual_seed(4)
     E, T, d = 4, 40, 256

@@ -184,3 +184,19 @@ def test_split_linear_has_the_bits_of_the_undivided_form(M, N, K):
     torch.cuda.synchronize()
     lo.check_device_status()
     assert torch.equal(out[0], out[1])
+
+
+def test_undivided_linear_keeps_no_scratch():
+    import lightop_b200 as lo
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    M, N, K = 5, 256, 384
+    g = torch.Generator().manual_seed(3)
+    q, s = lo.quant.per_token_group_quant_int8(torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV), 128)
+    B = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8).to(DEV)
+    b_s = (torch.rand(2, 3, generator=g) * 9e-3 + 1e-3).to(DEV)
+    assert lib.lo_block_int8_linear_split_workspace_bytes(M, N, K) == 0
+    c = torch.zeros(M, N, dtype=torch.bfloat16, device=DEV)
+    assert lib.lo_block_int8_linear(q.data_ptr(), s.data_ptr(), B.data_ptr(), b_s.data_ptr(), M, N, K, c.data_ptr(), 0, 0, 0,
+                                    torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(c, lo.gemm_ops.matmul_block_int8(q, B, s, b_s, [128, 128], torch.bfloat16))
