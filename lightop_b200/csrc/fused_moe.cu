@@ -380,17 +380,19 @@ extern "C" int lo_fused_moe_block_int8_noalloc(const void *x, const int8_t *w1, 
 namespace lo {
 namespace {
 // Chunk sizes of the per-channel layer, by the rows an expert gets on average.  A chunk is one pass over the expert's weights and
-// one MMA N extent (an N = 256 MMA costs about 1.3 x an N = 128 one); the GEMM is instantiated per chunk cap, and narrow caps leave
-// shared memory for more weight slots and tensor memory for more accumulators.  Layer times at the DeepSeek-V3 shape:
-//   <= 56 rows per expert : 64-row chunks, 12 weight slots and 8 accumulators (against 128 rows: 1680 / 1760 us at 4 rows per
-//                           expert, 1780 / 1890 at 16, 1860 / 2040 at 32, 2040 / 2240 at 56; from 64 rows on it loses, 10 to 25 %
-//                           at 93, where most experts need a second chunk)
-//   57 .. 104             : 128-row chunks (at 93: 2480 us, with 256 rows 2550)
-//   105 .. 136            : 160-row chunks (at 128: 2600 us, with 128 rows 3150, with 256 rows 2740)
-//   above                 : 256-row chunks (at 187: 3080 us, with 160 rows 4190)
+// one MMA N extent (an N = 256 MMA costs about 1.3 x an N = 128 one); the GEMM is instantiated per chunk cap.  Weight slots and
+// accumulators: 9 and 8 with 64 rows, 9 and 4 with 128, 8 and 3 with 160, 5 and 2 with 256.  Layer times in us, DeepSeek-V3
+// shape, caps of 64 / 128 / 160 / 256 rows:
+//   rows per expert     16                            56                            93                            128                           160
+//   even routing        1736 / 1793 / 1780 / 1833     1984 / 2060 / 2044 / 2072     3003 / 2372 / 2325 / 2351     3647 / 3068 / 2491 / 2514     4689 / 3960 / 3158 / 2674
+//   Zipf (1.2) routing   746 /  723 /  713 /  702     1789 / 1525 / 1433 / 1324     2597 / 2099 / 1930 / 1749     3492 / 2605 / 2392 / 2199     4174 / 3092 / 2841 / 2552
+//   <= 56 rows per expert : 64-row chunks, for the even case (Qwen3 shape: 407 / 397 / 397 / 410 at 16 rows, 483 / 487 / 480 /
+//                           489 at 56).  With a few hot experts every wider cap is faster; the routing is not known on the host.
+//   57 .. 136             : 160-row chunks, ahead of 128 in both (and no slower than 256 with even routing)
+//   above                 : 256-row chunks
 inline int channel_chunk_rows_for(int64_t rows, int experts) {
   const int64_t avg = rows / experts;
-  return avg <= 56 ? CHUNK_ROWS_SMALL : (avg <= 104 ? CHUNK_ROWS : (avg <= 136 ? CHUNK_ROWS_WIDE : 256));
+  return avg <= 56 ? CHUNK_ROWS_SMALL : (avg <= 136 ? CHUNK_ROWS_WIDE : 256);
 }
 struct ChannelLayout {
   int32_t *header;      // [0] num_tokens_post_pad, [1] num_chunks
