@@ -54,16 +54,18 @@ FusedLayout carve_fused(void *ws, int64_t M, int num_experts_for_align, int topk
   return L;
 }
 
-// Chunk sizes of the block-scaled layer, by the rows an expert gets on average (rows / experts), measured at the
-// DeepSeek-V3 shape.  The GEMM is instantiated per chunk cap and the caps differ in what fits beside the operands:
-// chunks of <= 64 rows leave room for 12 weight slots and 8 partial buffers, <= 128 rows for 7 and 4, <= 160 rows for 5
-// and 3.
-//   <= 48 rows per expert : 64-row chunks.  A weight-streaming call wants the deep rings, and the few experts that do
-//                           get more rows simply have a second chunk (-8 % from 96 to 512 tokens, -4 % at 1536).
-//   49 .. 119             : 128-row chunks (-9 % at 64 rows per expert, -2 % at 112 against the 160-row table).
-//   >= 120                : 160-row chunks, the widest whose partial buffers still number three: at 128 rows per expert
-//                           half of the experts have a few rows more than 128, and a second chunk means a second pass
-//                           over the expert's weights (-17 % at 128 rows per expert against the 128-row table).
+// Chunk sizes of the block-scaled layer, by the rows an expert gets on average (rows / experts).  The GEMM is instantiated per
+// chunk cap and the caps differ in what fits beside the operands: 8 weight slots and 8 partial buffers with 64 rows, 7 and 4
+// with 128, 5 and 3 with 160.  Layer times in us, DeepSeek-V3 shape, caps of 64 / 128 / 160 rows:
+//   rows per expert     16                     48                     64                     112                    128                    187
+//   even routing        1688 / 1765 / 1861     1830 / 2040 / 2257     2455 / 2196 / 2499     3386 / 2837 / 3084     4002 / 3633 / 3236     5393 / 4801 / 5213
+//   Zipf (1.2) routing   761 /  777 /  890     1472 / 1384 / 1599     1901 / 1820 / 2112     3080 / 2816 / 3050     3438 / 3042 / 3331     4804 / 4165 / 4344
+//   <= 48 rows per expert : 64-row chunks.  A weight-streaming call wants the deep rings, and the few experts that do get
+//                           more rows have a second chunk (at 56 still 1944 / 2048 / 2319 with even routing).
+//   49 .. 119             : 128-row chunks
+//   >= 120                : 160-row chunks: with 128 rows per expert half of the experts have a few rows more than 128, and a
+//                           second chunk means a second pass over the expert's weights.  That holds up to about 150 rows per
+//                           expert (144: 4661 / 4305 / 3802); above, and with skewed routing, 128-row chunks are ahead again.
 constexpr int CHUNK_ROWS = 128;
 constexpr int CHUNK_ROWS_WIDE = 160;
 constexpr int CHUNK_ROWS_SMALL = 64;

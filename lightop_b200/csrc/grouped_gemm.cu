@@ -39,8 +39,9 @@
 //
 // What it measured (DeepSeek-V3 shape, one layer, sustained at the 1000 W power cap; before = a per-step hand-over of scales
 // through the issuer, a thread on one channel and 16 tokens, two issuer warps and the output in the promotion warps):
-// 64 tokens 1764 -> 1470 us, 777 tokens 2290 -> 1880 us, 4096 tokens 3850 -> 3340 us.  The board is at its power cap in all of
-// these (SM clock 1.35 to 1.5 GHz), so what a change saves in cycles comes back as time only in part.
+// 64 tokens 1764 -> 1480 us, 777 tokens 2290 -> 1880 us, 4096 tokens 3850 -> 3340 us on one board (others: 1460, 1770, 2950 to 3150
+// now).  The board is at its power cap in all of these (SM clock 1.35 to 1.5 GHz), so what a change saves in cycles comes back
+// as time only in part.
 //
 // Per-channel mode (one scale per token and one per output channel instead of 128x128 blocks) uses the same feed without the
 // promotion: a tensor-memory buffer is the int32 accumulator of a whole item, summed over every K block by the tensor core, and
@@ -108,7 +109,7 @@ template <int MODE, int A_ROWS> struct Cfg {
   static constexpr int STAGING_BYTES = MODE == GEMM_CHANNEL ? 0 : A_ROWS * OUT_ROW_BYTES;
   static constexpr int FIXED_BYTES = 10 * 1024;   // scale tables, barriers, alignment slack (checked below)
   static constexpr int NW_FIT = (SMEM_LIMIT - FIXED_BYTES - STAGING_BYTES - NA * A_TILE_BYTES) / W_TILE_BYTES;
-  static constexpr int NW = NW_FIT > 12 ? 12 : NW_FIT;
+  static constexpr int NW = NW_FIT;
   // tensor memory is cut into partial buffers of A_ROWS columns, one int32 accumulator each (at most 8 are used):
   // the partial of one 128-wide K block in the block-scaled modes (the fp32 running sums live in the registers of
   // the promotion warps), the accumulator of a whole item in the per-channel mode
@@ -116,6 +117,15 @@ template <int MODE, int A_ROWS> struct Cfg {
   // Ring of scale-product tables: SC_BATCHES batches of SC_STEPS K-block steps each
   static constexpr int SC_SLOTS = MODE == GEMM_CHANNEL ? 1 : SC_BATCHES * SC_STEPS;
 };
+
+// The figures that the chunk rules of the layers give as their reasons.
+template <int MODE, int A_ROWS> constexpr bool ring_depths(int weight_slots, int buffers) {
+  return Cfg<MODE, A_ROWS>::NW == weight_slots && Cfg<MODE, A_ROWS>::NBUF == buffers;
+}
+static_assert(ring_depths<GEMM_SINGLE, 32>(11, 8) && ring_depths<GEMM_SINGLE, 64>(8, 8) && ring_depths<GEMM_SINGLE, 128>(7, 4) &&
+              ring_depths<GEMM_SINGLE, T_WIDE>(5, 3), "block-scaled: weight slots and partial buffers as the chunk rule states them");
+static_assert(ring_depths<GEMM_CHANNEL, 64>(9, 8) && ring_depths<GEMM_CHANNEL, 128>(9, 4) && ring_depths<GEMM_CHANNEL, T_WIDE>(8, 3) &&
+              ring_depths<GEMM_CHANNEL, 256>(5, 2), "per channel: weight slots and accumulators as the chunk rule states them");
 
 template <int MODE, int A_ROWS> struct Smem {
   using C = Cfg<MODE, A_ROWS>;

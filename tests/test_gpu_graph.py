@@ -79,3 +79,49 @@ def test_gate_graph_replay(lo):
         w_ref, ids_ref = OG.fused_gate(src, bias.cpu(), 8, 4, 8, 0, 2.5)
         assert torch.equal(ids.cpu(), ids_ref)
         torch.testing.assert_close(w.cpu(), w_ref, rtol=2e-5, atol=2e-6)
+
+
+@pytest.mark.parametrize("before", ["nothing", "copy", "fill", "join"])
+def test_dependent_launch_first_in_a_captured_graph(lo, before):
+    # the first kernel of these operators is a dependent launch: captured with no kernel ahead of it, but a copy, a fill or two
+    # joined streams
+    M, K, N = 64, 1024, 256
+    g = torch.Generator(device=DEV).manual_seed(3)
+    src = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    x = src.clone()
+    ids_src = torch.randint(0, 8, (M, 2), generator=g, device=DEV, dtype=torch.int32)
+    ids = ids_src.clone()
+    q_src, s = lo.quant.per_token_group_quant_int8(src, 128)
+    q = q_src.clone()
+    B = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    b_s = torch.rand(N // 128, K // 128, generator=g, device=DEV)
+    side = torch.cuda.Stream()
+
+    def ahead():
+        if before == "copy":
+            x.copy_(src), ids.copy_(ids_src), q.copy_(q_src)
+        elif before == "fill":
+            x.zero_(), ids.zero_(), q.zero_()
+        elif before == "join":
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                ids.copy_(ids_src)
+                q.copy_(q_src)
+            x.copy_(src)
+            torch.cuda.current_stream().wait_stream(side)
+
+    ops = {"token_quant": lambda: lo.quant.per_token_quant_int8(x), "align": lambda: lo.moe.moe_align_block_size(ids, 16, 8)[2:],
+           "linear": lambda: (lo.gemm_ops.matmul_block_int8(q, B, s, b_s, [128, 128], torch.bfloat16),)}
+    for name, op in ops.items():
+        ahead()
+        ref = op()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ahead()
+            out = op()
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(ref, out)), name
+    lo.check_device_status()

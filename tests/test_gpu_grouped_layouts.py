@@ -78,6 +78,36 @@ def test_masked_layout(lo, E, max_m, masked, N, K):
     assert torch.equal(d.cpu(), ref)
 
 
+@pytest.mark.parametrize("max_m", [129, 144, 145, 160])
+def test_masked_layout_of_129_to_160_rows(lo, max_m):
+    # the 160-row instantiation (a 128-row box and a second one); counts below zero and above max_m are taken as none and all
+    E, N, K = 5, 256, 384
+    g = torch.Generator().manual_seed(max_m)
+    A = torch.randint(-127, 128, (E, max_m, K), generator=g, dtype=torch.int8)
+    As = torch.rand(E, max_m, 1, generator=g) * 0.05 + 1e-3
+    B = torch.randint(-127, 128, (E, N, K), generator=g, dtype=torch.int8)
+    Bs = torch.rand(E, N, 1, generator=g) * 9e-4 + 1e-4
+    mm = torch.tensor([max_m, -3, max_m + 40, 1, 129], dtype=torch.int32)
+    d = torch.full((E, max_m, N), -5.0, dtype=torch.bfloat16, device=DEV)
+    lo.gemm_ops.m_grouped_w8a8_gemm_nt_masked((A.to(DEV), As.to(DEV)), (B.to(DEV), Bs.to(DEV)), d, mm.to(DEV), 64)
+    torch.cuda.synchronize()
+    lo.check_device_status()
+    ref = OC.grouped_matmul_masked(A, As, B, Bs, mm.clamp(0, max_m), torch.full((E, max_m, N), -5.0, dtype=torch.bfloat16))
+    assert torch.equal(d.cpu(), ref)
+
+
+@pytest.mark.parametrize("M", [129, 145, 160])
+def test_contiguous_layout_of_129_to_160_rows(lo, M):
+    # the same instantiation through the chunk table: a full 128-row block and a short last one of another expert
+    A, As, B, Bs, _ = _contig_case(2, [M], 1, 256, 384, seed=M)
+    m_idx = torch.cat([torch.zeros(128, dtype=torch.int32), torch.ones(M - 128, dtype=torch.int32)])
+    out = torch.full((M, 256), 3.0, dtype=torch.bfloat16, device=DEV)
+    lo.gemm_ops.m_grouped_w8a8_gemm_nt_contig_asm((A.to(DEV), As.to(DEV)), (B.to(DEV), Bs.to(DEV)), out, m_idx.to(DEV))
+    torch.cuda.synchronize()
+    lo.check_device_status()
+    assert torch.equal(out.cpu(), OC.grouped_matmul_contig(A, As, B, Bs, m_idx, torch.full((M, 256), 3.0, dtype=torch.bfloat16)))
+
+
 def test_masked_layout_keeps_no_scratch(lo):
     from lightop_b200 import _lib
     E, max_m, N, K = 2, 40, 128, 256

@@ -140,6 +140,64 @@ def _stage2_from_workspace(lo, M, E, k, H, I, x, w1, w2, w1_s, w2_s, w, ids):
     return out.cpu(), header, xq, xs, sorted_ids, act_q, act_s
 
 
+def test_epilogue_quotients_against_cuda_division(lo):
+    # SiLU and re-quantisation of the gate_up epilogue use inline quotients (Markstein's correction of a reciprocal).  Every bf16
+    # gate from 2^-30 to 2^60 of either sign, next to 128 up values, against the device's IEEE division: the same scales and codes.
+    H, I = 256, 128
+    bits = torch.arange(0, 1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    gates = bits[(bits.float().abs() >= 2.0 ** -30) & (bits.float().abs() < 2.0 ** 60)]
+    M = gates.numel()
+    x = torch.zeros(M, H, dtype=torch.bfloat16)
+    x[:, 0], x[:, 128] = gates, 1.0
+    w1 = torch.zeros(1, 2 * I, H, dtype=torch.int8)
+    w1[0, :I, 0] = 1                                                     # gate: the first K block, the same for all channels
+    w1[0, I:, 128] = torch.arange(-64, 64, dtype=torch.int8)             # up: the second K block
+    w1_s = torch.tensor([[[1.0, 1.0], [1.0, 0.037]]])
+    _, _, xq, xs, _, act_q, act_s = _stage2_from_workspace(lo, M, 1, 1, H, I, x, w1, torch.zeros(1, H, I, dtype=torch.int8), w1_s, torch.ones(1, 2, 1),
+                                                           torch.ones(M, 1), torch.zeros(M, 1, dtype=torch.int32))
+    xq, xs = xq[:M].to(DEV).float(), xs[:M].to(DEV)
+    g = (xq[:, :1] * xs[:, :1]).to(torch.bfloat16).float()
+    up = (xq[:, 128:129] * w1[0, I:, 128].to(DEV).float() * (xs[:, 1:] * 0.037)).to(torch.bfloat16).float()
+    silu = (g / (1.0 + torch.exp(-g))).to(torch.bfloat16).float()
+    act = (silu * up).to(torch.bfloat16).float()
+    eps = torch.tensor(1e-10).to(torch.bfloat16).float().to(DEV)
+    scale = torch.maximum(act.abs().amax(dim=1, keepdim=True), eps) / torch.tensor(127.0, device=DEV)
+    q = torch.trunc(torch.clamp(act / scale, -128, 127)).to(torch.int8)
+    assert M > 20000 and int((q != 0).sum()) > M * 32
+    assert torch.equal(act_s[:M], scale.cpu()), int((act_s[:M] != scale.cpu()).sum())
+    assert torch.equal(act_q[:M], q.cpu()), int((act_q[:M] != q.cpu()).sum())
+
+
+@pytest.mark.parametrize("mode", ["block", "channel"])
+@pytest.mark.parametrize("M", [16, 640])
+def test_layer_directly_behind_a_library_gemm(lo, mode, M):
+    # the activations come from the kernel just ahead in the stream: the quantisation, which reads them ahead of its own wait, must
+    # find them complete
+    E, k, H, I = 8, 2, 1024, 256
+    w1, w2, w1_s, w2_s = synthetic.make_weights(E, H, I, seed=5, device=DEV)
+    kw = dict(use_int8_w8a8=True, block_shape=[128, 128])
+    if mode == "channel":
+        w1_s, w2_s = synthetic.make_channel_scales(E, H, I, seed=5, device=DEV)
+        kw = dict(use_int8_w8a8=True, per_channel_quant=True)
+    g = torch.Generator(device=DEV).manual_seed(M)
+    ids = torch.randint(0, E, (M, k), generator=g, device=DEV, dtype=torch.int32)
+    w = torch.rand(M, k, generator=g, device=DEV)
+    proj = torch.randn(4096, H, generator=g, device=DEV).to(torch.bfloat16)
+    x = torch.zeros(M, H, dtype=torch.bfloat16, device=DEV)
+    ins = [torch.randn(M, 4096, generator=g, device=DEV).to(torch.bfloat16) for _ in range(12)]
+    torch.cuda.synchronize()
+    got = []
+    for a in ins:
+        torch.mm(a, proj, out=x)
+        got.append(lo.moe.fused_experts_impl_int8(x, w1, w2, w, ids, None, w1_scale=w1_s, w2_scale=w2_s, **kw))
+    torch.cuda.synchronize()
+    for a, y in zip(ins, got):
+        torch.mm(a, proj, out=x)
+        torch.cuda.synchronize()
+        assert torch.equal(y, lo.moe.fused_experts_impl_int8(x, w1, w2, w, ids, None, w1_scale=w1_s, w2_scale=w2_s, **kw))
+    lo.check_device_status()
+
+
 @pytest.mark.parametrize("channels", [(5,), (0,), (127,), (34,), (4, 5, 6, 7), (64, 67), tuple(range(128))])
 @pytest.mark.parametrize("M", [3, 70])
 def test_a_nan_in_a_quantisation_group(lo, M, channels):
