@@ -19,7 +19,8 @@ def matmul_block_int8(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs: to
     (python/lightop/_lmslim_native/layers/gemm/int8_utils.py:298-403).  ``A [..., K]`` int8,
     ``As [..., K/128]`` fp32, ``B [N, K]`` int8, ``Bs [ceil(N/128), K/128]`` fp32.  The kernel writes
     bf16; another ``output_dtype`` is produced by a cast of that result.  ``config`` (Triton tile
-    sizes in the reference) is accepted and ignored.
+    sizes in the reference) is accepted and ignored.  A row of the result depends on its own row of ``A`` and on ``B``
+    alone: it has the same bits in any batch.
     """
     assert len(block_size) == 2 and block_size[0] == 128 and block_size[1] == 128, "only [128, 128] blocks"
     _lib.require_cuda(A, B, As, Bs, bias)
