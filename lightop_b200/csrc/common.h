@@ -78,9 +78,10 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
                  int chunk_max, cudaStream_t stream);
 
 // Group quantisation of bf16 rows [M, H] written straight into the expert-sorted layout:
-// the int8 row and its scales of token t go to every position inv_pos[t * topk + j] >= 0.  quant.cu
+// the int8 row and its scales of token t go to every position inv_pos[t * topk + j] >= 0.  some_absent: tokens without any
+// position are to be expected (an expert map), and are not read.  quant.cu
 int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, const int32_t *inv_pos, float eps,
-                               int8_t *q_sorted, float *s_sorted, cudaStream_t stream);
+                               int8_t *q_sorted, float *s_sorted, bool some_absent, cudaStream_t stream);
 
 // Group quantisation of rows of any supported type, for a dependent launch of the kernel that follows.  quant.cu
 int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group_size, float eps, int8_t *q, float *s,
@@ -185,6 +186,21 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
   cfg.numAttrs = 1;
   g_launch_count.fetch_add(1, std::memory_order_relaxed);
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// Reciprocal refined by one Newton step, and the quotient a / b from it with the remainder folded back in (Markstein's method,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990)
+// (q = a*y, then q + (a - b*q)*y): the IEEE round-to-nearest quotient for finite operands whose quotient and reciprocal
+// are normal numbers.  Inline, so the divisions of a thread overlap; the library division is a subroutine call each: two of them
+// per output made the GEMM's epilogue a fifth of its time, and one per element two thirds of the group quantiser's.
+__device__ __forceinline__ float rcp_refined(float b) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+}
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+  const float q = __fmul_rn(a, y);
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
 // Lanes of the warp that hold the same expert as this lane (lanes without an expert match one another).

@@ -174,7 +174,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   // 2. activations -> int8 + per-128 scales, written once per routed slot into sorted order so
   //    that every chunk of the grouped GEMM is a run of consecutive rows (one TMA box)
   prof_mark(1, st);
-  rc = launch_group_quant_scatter(x, M, H, topk, L.inv_pos, 1e-10f, L.xq, L.xs, st);
+  rc = launch_group_quant_scatter(x, M, H, topk, L.inv_pos, 1e-10f, L.xq, L.xs, expert_map != nullptr, st);
   if (rc != LO_OK) return rc;
 
   // 3. gate_up GEMM, SiLU*mul and re-quantisation in the epilogue -> act_q/act_s in sorted order

@@ -419,30 +419,15 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   return r;
 }
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-// Reciprocal refined by one Newton step, and the quotient a / b from it with the remainder folded back in (Markstein's method,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990)
-// (q = a*y, then q + (a - b*q)*y): the IEEE round-to-nearest quotient for operands whose quotient and reciprocal
-// are normal numbers, which holds for every division of the epilogues (denominators in [1, 1e38] or a group
-// scale of at least 1e-10 / 127).  Inline, so the sixteen divisions of a piece overlap; the library division is
-// a subroutine call each, and two of them per output made the epilogue a fifth of the kernel's time.
-__device__ __forceinline__ float rcp_refined(float b) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
-}
 // a / b from the approximate reciprocal, corrected by the remainder once: within a unit in the last place or better of the
-// quotient, whose next use is a rounding to bf16.  The same operand ranges.
+// quotient, whose next use is a rounding to bf16.  The operand ranges of div_by() in common.h, which holds for every division of the
+// epilogues (denominators in [1, 1e38] or a group scale of at least 1e-10 / 127).
 __device__ __forceinline__ float div_fast(float a, float b) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
   const float q = __fmul_rn(a, y);
   return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
-__device__ __forceinline__ float div_by(float a, float b, float y) {
-  const float q = __fmul_rn(a, y);
-  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-}
-
 struct KParams {
   const float *a_scale;     // [positions, KB]
   const float *b_scale;

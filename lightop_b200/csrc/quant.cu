@@ -5,8 +5,8 @@
 //   amax  = max |x| over the group, clamped from below by eps rounded to x's type
 //   scale = amax / 127                 (IEEE fp32 division)
 //   q     = trunc(clamp(x / scale, -128, 127))   (IEEE fp32 division, then round toward zero)
-// Memory-bound streaming kernel: LANES lanes own one group, each lane moves 16
-// bytes of 2-byte input (or 32 bytes of fp32) and stores 8 int8 in one 8-byte store.
+// Memory-bound streaming kernel: LANES lanes own one group, each lane moves 32
+// bytes of 2-byte input (or 64 bytes of fp32) and stores 16 int8.
 #include "common.h"
 
 namespace lo {
@@ -45,81 +45,128 @@ template <> struct Load8<float> {
   }
 };
 
-// LANES lanes x 8 elements = one group.
+// Four quotients to four bytes: truncation toward zero, a NaN to -128.
+__device__ __forceinline__ uint32_t pack4_rz(const float (&r)[4]) {
+  int q[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) q[i] = __float2int_rz(fmaxf(r[i], -128.0f));
+  uint32_t hi, lo;      // (saturating: 127 from above)
+  asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(q[3]), "r"(q[2]));
+  asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(lo) : "r"(q[1]), "r"(q[0]), "r"(hi));
+  return lo;
+}
+
+// A thread's sixteen elements of a group of LANES x 16: maximum over the group's lanes, scale, codes.  Every lane of the warp
+// calls it.  Two-byte types take the quotient from the refined reciprocal wherever that is the IEEE quotient (a scale
+// that is finite and not near the ends of the range: all but groups with an infinity or, with a tiny eps, of next to nothing); with
+// the library's division and eight elements a thread the kernels were bound by their instructions: 4096 x 7168 alone 33 -> 22 us (the
+// bytes take 14), into eight sorted places 60 -> 49 us, 8192 rows of which a shard wants two thirds 82 -> 40 us.  Every bf16 and fp16 pair of maximum and element is compared with the library's division in the tests; fp32 elements keep it.
+template <typename T, int LANES>
+__device__ __forceinline__ float quantise16(const float (&v)[16], float eps_t, uint32_t (&packed)[4]) {
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+  for (int off = LANES / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  const float scale = __fdiv_rn(fmaxf(amax, eps_t), 127.0f);
+  const bool plain = sizeof(T) == 2 && scale >= 1e-30f && scale <= 1e37f;
+  if (plain) {
+    const float y = rcp_refined(scale);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      float r[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = div_by(v[4 * w + i], scale, y);
+      packed[w] = pack4_rz(r);
+    }
+  } else {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      float r[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = __fdiv_rn(v[4 * w + i], scale);
+      packed[w] = pack4_rz(r);
+    }
+  }
+  return scale;
+}
+
+// LANES lanes x 16 elements = one group.  (16 elements a thread halve the shuffles and the address arithmetic an element costs.)
 template <typename T, int LANES>
 __global__ void __launch_bounds__(256) group_quant_kernel(const T *__restrict__ x, int8_t *__restrict__ q,
                                                           float *__restrict__ s, int64_t num_groups,
-                                                          float eps_t) {
+                                                          float eps_t, int q16) {
   dependency_release();      // (a dependent kernel waits for the whole grid before it reads)
   const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t group = gthread / LANES;
-  const int lane_in_group = (int)(gthread % LANES);
   const bool active = group < num_groups;
-  float v[8];
-  float amax = 0.f;
+  float v[16];
   if (active) {
-    Load8<T>::load(x + group * (LANES * 8) + lane_in_group * 8, v);
+    Load8<T>::load(x + gthread * 16, *reinterpret_cast<float (*)[8]>(&v[0]));
+    Load8<T>::load(x + gthread * 16 + 8, *reinterpret_cast<float (*)[8]>(&v[8]));
+  } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    for (int i = 0; i < 16; ++i) v[i] = 0.f;
   }
-#pragma unroll
-  for (int off = LANES / 2; off > 0; off >>= 1)
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  uint32_t packed[4];
+  const float scale = quantise16<T, LANES>(v, eps_t, packed);
   if (!active) return;
-  amax = fmaxf(amax, eps_t);
-  const float scale = __fdiv_rn(amax, 127.0f);
-  uint32_t packed[2] = {0u, 0u};
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float r = __fdiv_rn(v[i], scale);
-    r = fminf(fmaxf(r, -128.0f), 127.0f);
-    const int qi = __float2int_rz(r);
-    packed[i >> 2] |= (uint32_t)(qi & 0xff) << (8 * (i & 3));
+  int8_t *dst = q + gthread * 16;
+  if (q16) {
+    *reinterpret_cast<uint4 *>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  } else {
+    *reinterpret_cast<uint2 *>(dst) = make_uint2(packed[0], packed[1]);
+    *reinterpret_cast<uint2 *>(dst + 8) = make_uint2(packed[2], packed[3]);
   }
-  *reinterpret_cast<uint2 *>(q + group * (LANES * 8) + lane_in_group * 8) = make_uint2(packed[0], packed[1]);
-  if (lane_in_group == 0) s[group] = scale;
+  if (gthread % LANES == 0) s[group] = scale;
 }
 
 // bf16 rows [M, H], group 128: quantise once, store to each of the token's sorted positions.
+// Without an expert map every token has positions: the rows are loaded and quantised while the alignment kernel is still at
+// work.  With one (`some_absent`) tokens may have none, and those are passed over: the positions are read first.
 __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfloat16 *__restrict__ x, int64_t M,
-                                                                  int64_t groups_per_row, int topk,
+                                                                  int groups_per_row, int topk,
                                                                   const int32_t *__restrict__ inv_pos, float eps_t,
                                                                   int8_t *__restrict__ q_sorted,
-                                                                  float *__restrict__ s_sorted) {
+                                                                  float *__restrict__ s_sorted, int some_absent) {
   const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t group = gthread / 16;
-  const int lane_in_group = (int)(gthread % 16);
-  const bool active = group < M * groups_per_row;
-  float v[8];
-  float amax = 0.f;
-  if (active) {
-    Load8<__nv_bfloat16>::load(x + group * 128 + lane_in_group * 8, v);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  const uint32_t group = (uint32_t)(gthread / 8);            // (2^32 groups would be a terabyte of activations)
+  const uint32_t row = group / (uint32_t)groups_per_row;
+  const int gi = (int)(group - row * (uint32_t)groups_per_row);
+  const int64_t token = row;
+  const bool active = token < M;
+  const int32_t *pos_of = inv_pos + token * topk;
+  if (some_absent) dependency_wait();
+  bool wanted = active;
+  if (some_absent && active) {
+    wanted = false;
+    for (int j = 0; j < topk; ++j) wanted |= pos_of[j] >= 0;
   }
+  float v[16];
+  if (wanted) {
+    Load8<__nv_bfloat16>::load(x + gthread * 16, *reinterpret_cast<float (*)[8]>(&v[0]));
+    Load8<__nv_bfloat16>::load(x + gthread * 16 + 8, *reinterpret_cast<float (*)[8]>(&v[8]));
+  } else {
 #pragma unroll
-  for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-  if (!active) return;          // (an exited block counts as released for the dependent launch)
-  amax = fmaxf(amax, eps_t);
-  const float scale = __fdiv_rn(amax, 127.0f);
-  uint32_t packed[2] = {0u, 0u};
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float r = __fdiv_rn(v[i], scale);
-    r = fminf(fmaxf(r, -128.0f), 127.0f);
-    packed[i >> 2] |= (uint32_t)(__float2int_rz(r) & 0xff) << (8 * (i & 3));
+    for (int i = 0; i < 16; ++i) v[i] = 0.f;
   }
-  const int64_t token = group / groups_per_row;
-  const int64_t gi = group % groups_per_row;
+  if (!__any_sync(0xffffffffu, wanted)) return;          // (an exited block counts as released for the dependent launch)
+  uint32_t packed[4];
+  const float scale = quantise16<__nv_bfloat16, 8>(v, eps_t, packed);
   // everything above reads the caller's activations only; the positions come from the align kernel before this one
-  dependency_wait();
+  if (!some_absent) dependency_wait();
   dependency_release();
+  if (!wanted) return;
+  const uint4 codes = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  const int64_t row_bytes = (int64_t)groups_per_row * 128;
+  int8_t *dst = q_sorted + gi * 128 + (gthread & 7) * 16;
+  const bool first = (gthread & 7) == 0;
+#pragma unroll 4
   for (int j = 0; j < topk; ++j) {
-    const int32_t pos = inv_pos[token * topk + j];
+    const int32_t pos = pos_of[j];
     if (pos < 0) continue;
-    *reinterpret_cast<uint2 *>(q_sorted + ((int64_t)pos * groups_per_row + gi) * 128 + lane_in_group * 8) =
-        make_uint2(packed[0], packed[1]);
-    if (lane_in_group == 0) s_sorted[(int64_t)pos * groups_per_row + gi] = scale;
+    *reinterpret_cast<uint4 *>(dst + pos * row_bytes) = codes;
+    if (first) s_sorted[(int64_t)pos * groups_per_row + gi] = scale;
   }
 }
 
@@ -149,15 +196,14 @@ __device__ __forceinline__ float block_max_256(float v, float *red) {
   return r;
 }
 
+// Eight codes: value x inv, rounded half to even, saturated, a NaN to -128.  Adding 1.5 x 2^23 rounds to an integer and leaves its
+// two's complement in the low byte (the conversion instruction runs at an eighth of the rate).
 __device__ __forceinline__ uint2 quant8_rn(const float (&v)[8], float inv) {
-  uint32_t packed[2] = {0u, 0u};
+  uint32_t b[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float r = __fmul_rn(v[i], inv);
-    r = fminf(fmaxf(r, -128.0f), 127.0f);
-    packed[i >> 2] |= (uint32_t)(__float2int_rn(r) & 0xff) << (8 * (i & 3));
-  }
-  return make_uint2(packed[0], packed[1]);
+  for (int i = 0; i < 8; ++i) b[i] = __float_as_uint(__fadd_rn(fminf(fmaxf(__fmul_rn(v[i], inv), -128.0f), 127.0f), 12582912.0f));
+  return make_uint2(__byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410),
+                    __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410));
 }
 
 template <typename T>
@@ -217,95 +263,124 @@ __global__ void __launch_bounds__(TOKEN_QUANT_THREADS) token_quant_kernel(const 
 // the SiLU: act = bf16(bf16(silu(gate)) * up); scale = max|act| / 127; q = rint(act * (127 / max)),
 // saturated; a row of zeros gets scale 0 and q 0.  Rows whose entry in row_ids is a padding
 // sentinel (< 0 or >= numel_valid) are skipped.
+// 128 threads a row, and a row's loads are on their way before anything is looked up for it: with 256 threads, the library's
+// division and the loads behind the look-ups a row's chain of latencies bound it: 24 000 rows of 2048 channels 139 us, now 99 (the
+// bytes take 38; what bounds it now are the instructions, an exponential and an exact quotient per element).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(TOKEN_QUANT_THREADS) silu_mul_token_quant_kernel(
+
+// g / (1 + exp(-g)), the IEEE quotient: the refined reciprocal is taken of the denominator times 2^-32, which keeps the
+// reciprocal normal up to the largest finite denominator.  What that form does not give has a denominator of 2 (next to zero, where
+// the quotient may be a subnormal), of 1 (large gates and infinity) or of infinity (g * 0: a signed zero or, for -inf, NaN).
+// The tests compare every bf16 gate with the library's division.
+__device__ __forceinline__ float silu_exact(float g) {
+  const float den = 1.0f + expf(-g);
+  const float b = den * 0x1p-32f;
+  const float q = div_by(g, b, rcp_refined(b)) * 0x1p-32f;
+  const float r = den == 2.0f ? g * 0.5f : (den == 1.0f ? g : q);
+  return den == INFINITY ? g * 0.0f : r;
+}
+// Eight activations, as bf16, of eight gates and up values; amax takes their largest magnitude.
+__device__ __forceinline__ uint4 act8(const uint4 &g, const uint4 &u, float &amax) {
+  const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
+  uint32_t out[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 sl = __floats2bfloat162_rn(silu_exact(__uint_as_float(gw[i] << 16)), silu_exact(__uint_as_float(gw[i] & 0xffff0000u)));
+    const float2 f = __bfloat1622float2(sl);
+    const __nv_bfloat162 a = __floats2bfloat162_rn(f.x * __uint_as_float(uw[i] << 16), f.y * __uint_as_float(uw[i] & 0xffff0000u));
+    out[i] = *reinterpret_cast<const uint32_t *>(&a);
+    amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(out[i] << 16)), fabsf(__uint_as_float(out[i] & 0xffff0000u))));
+  }
+  return make_uint4(out[0], out[1], out[2], out[3]);
+}
+__device__ __forceinline__ uint2 quant8_bf16(const uint4 &a, float inv) {
+  const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+  return quant8_rn(v, inv);
+}
+
+constexpr int SILU_THREADS = 128, SILU_VECS = 4;      // vectors of eight channels a thread keeps: rows of up to 4096 channels
+__global__ void __launch_bounds__(SILU_THREADS) silu_mul_token_quant_kernel(
     const __nv_bfloat16 *__restrict__ in, int64_t d, const int32_t *__restrict__ row_ids, int64_t numel_valid,
     const int32_t *__restrict__ num_rows_dev, int64_t group_rows, const int32_t *__restrict__ group_counts,
     int8_t *__restrict__ q, float *__restrict__ s) {
-  __shared__ float red[8];
+  __shared__ float red[SILU_THREADS / 32];
   const int64_t row = blockIdx.x;
   dependency_wait();
   dependency_release();
-  if (num_rows_dev && row >= *num_rows_dev) return;
-  // masked layout [groups, group_rows, 2d]: only the first group_counts[g] rows of a group exist
+  // masked layout [groups, group_rows, 2d]: only the first group_counts[g] rows of a group exist (most do not, so they are looked
+  // up before anything is loaded; of the sorted positions few are padding)
   if (group_counts && row % group_rows >= group_counts[row / group_rows]) return;
+  const uint4 *g = reinterpret_cast<const uint4 *>(in + row * 2 * d);
+  const int64_t vecs = d / 8;
+  const uint4 *u = g + vecs;
+  const bool kept = vecs <= SILU_VECS * SILU_THREADS;      // the row's activations stay in registers
+  uint4 gv[SILU_VECS], uv[SILU_VECS];
+  if (kept) {
+#pragma unroll
+    for (int v = 0; v < SILU_VECS; ++v) {
+      const int64_t i = threadIdx.x + v * SILU_THREADS;
+      if (i < vecs) {
+        gv[v] = g[i];
+        uv[v] = u[i];
+      }
+    }
+  }
+  if (num_rows_dev && row >= *num_rows_dev) return;
   if (row_ids) {
     const int32_t id = row_ids[row];
     if (id < 0 || id >= numel_valid) return;
   }
-  const __nv_bfloat16 *g = in + row * 2 * d;
-  const __nv_bfloat16 *u = g + d;
-  const int64_t vecs = d / 8;
   float amax = 0.f;
-  if (vecs <= 2 * TOKEN_QUANT_THREADS) {
-    // rows of up to 4096 channels: the activations stay in registers between the maximum and the
-    // quantisation (one read of the row, one evaluation of the SiLU)
-    float av[2][8];
+  if (kept) {
 #pragma unroll
-    for (int v = 0; v < 2; ++v) {
-      const int64_t i = threadIdx.x + (int64_t)v * TOKEN_QUANT_THREADS;
-      if (i < vecs) {
-        float gv[8], uv[8];
-        Load8<__nv_bfloat16>::load(g + i * 8, gv);
-        Load8<__nv_bfloat16>::load(u + i * 8, uv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float sl = __bfloat162float(__float2bfloat16_rn(__fdiv_rn(gv[j], 1.0f + expf(-gv[j]))));
-          av[v][j] = __bfloat162float(__float2bfloat16_rn(sl * uv[j]));
-          amax = fmaxf(amax, fabsf(av[v][j]));
-        }
-      }
+    for (int v = 0; v < SILU_VECS; ++v) {
+      if (threadIdx.x + v * SILU_THREADS < vecs) gv[v] = act8(gv[v], uv[v], amax);
     }
-    amax = block_max_256(amax, red);
-    const float inv = amax == 0.f ? 0.f : __fdiv_rn(127.0f, amax);
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-      const int64_t i = threadIdx.x + (int64_t)v * TOKEN_QUANT_THREADS;
-      if (i < vecs) *reinterpret_cast<uint2 *>(q + row * d + i * 8) = quant8_rn(av[v], inv);
-    }
-    if (threadIdx.x == 0) s[row] = __fdiv_rn(amax, 127.0f);
-    return;
+  } else {
+    for (int64_t i = threadIdx.x; i < vecs; i += SILU_THREADS) act8(g[i], u[i], amax);
   }
-  for (int64_t i = threadIdx.x; i < vecs; i += TOKEN_QUANT_THREADS) {
-    float gv[8], uv[8];
-    Load8<__nv_bfloat16>::load(g + i * 8, gv);
-    Load8<__nv_bfloat16>::load(u + i * 8, uv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sl = __bfloat162float(__float2bfloat16_rn(__fdiv_rn(gv[j], 1.0f + expf(-gv[j]))));
-      const float a = __bfloat162float(__float2bfloat16_rn(sl * uv[j]));
-      amax = fmaxf(amax, fabsf(a));
-    }
-  }
-  amax = block_max_256(amax, red);
+  for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
   const float inv = amax == 0.f ? 0.f : __fdiv_rn(127.0f, amax);
-  for (int64_t i = threadIdx.x; i < vecs; i += TOKEN_QUANT_THREADS) {
-    float gv[8], uv[8], av[8];
-    Load8<__nv_bfloat16>::load(g + i * 8, gv);
-    Load8<__nv_bfloat16>::load(u + i * 8, uv);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sl = __bfloat162float(__float2bfloat16_rn(__fdiv_rn(gv[j], 1.0f + expf(-gv[j]))));
-      av[j] = __bfloat162float(__float2bfloat16_rn(sl * uv[j]));
-    }
-    *reinterpret_cast<uint2 *>(q + row * d + i * 8) = quant8_rn(av, inv);
-  }
   if (threadIdx.x == 0) s[row] = __fdiv_rn(amax, 127.0f);
+  uint2 *dst = reinterpret_cast<uint2 *>(q + row * d);
+  if (kept) {
+#pragma unroll
+    for (int v = 0; v < SILU_VECS; ++v) {
+      const int64_t i = threadIdx.x + v * SILU_THREADS;
+      if (i < vecs) dst[i] = quant8_bf16(gv[v], inv);
+    }
+  } else {
+    for (int64_t i = threadIdx.x; i < vecs; i += SILU_THREADS) {
+      float again = 0.f;
+      dst[i] = quant8_bf16(act8(g[i], u[i], again), inv);
+    }
+  }
 }
 
 template <typename T>
 int launch_typed(const void *x, int64_t num_groups, int group_size, float eps_t, int8_t *q, float *s,
                  cudaStream_t stream) {
-  const int lanes = group_size / 8;
+  const int lanes = group_size / 16;
   const int threads = 256;
   const int64_t total_threads = num_groups * lanes;
   const int64_t blocks = ceil_div(total_threads, threads);
   if (blocks > 0x7fffffffLL) return fail(LO_ERR_INVALID_ARGUMENT, "group quant: too many groups");
   const T *xp = static_cast<const T *>(x);
-  switch (lanes) {
-    case 8: group_quant_kernel<T, 8><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t); break;
-    case 16: group_quant_kernel<T, 16><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t); break;
-    case 32: group_quant_kernel<T, 32><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t); break;
+  const int q16 = (reinterpret_cast<uintptr_t>(q) & 15) == 0 ? 1 : 0;      // (the caller's q may begin on 8 bytes only)
+  switch (group_size) {
+    case 64: group_quant_kernel<T, 4><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t, q16); break;
+    case 128: group_quant_kernel<T, 8><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t, q16); break;
+    case 256: group_quant_kernel<T, 16><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t, q16); break;
     default: return fail(LO_ERR_UNSUPPORTED, "group quant: group_size %d not in {64,128,256}", group_size);
   }
   LO_LAUNCH_OK("group_quant_kernel");
@@ -323,15 +398,15 @@ float round_eps_to_dtype(float eps, int dtype) {
 }
 
 int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, const int32_t *inv_pos, float eps,
-                               int8_t *q_sorted, float *s_sorted, cudaStream_t stream) {
+                               int8_t *q_sorted, float *s_sorted, bool some_absent, cudaStream_t stream) {
   if (M == 0) return LO_OK;
   LO_REQUIRE(H % 128 == 0, "group quant: hidden size must be a multiple of 128");
-  const int64_t total_threads = M * (H / 128) * 16;
+  const int64_t total_threads = M * (H / 128) * 8;
   const int64_t blocks = ceil_div(total_threads, 256);
   LO_REQUIRE(blocks <= 0x7fffffffLL, "group quant: too many groups");
   LO_CUDA_OK(launch_dependent(group_quant_scatter_kernel, dim3((unsigned)blocks), dim3(256), 0, stream,
-                              static_cast<const __nv_bfloat16 *>(x), M, H / 128, topk, inv_pos,
-                              round_eps_to_dtype(eps, LO_BF16), q_sorted, s_sorted));
+                              static_cast<const __nv_bfloat16 *>(x), M, (int)(H / 128), topk, inv_pos,
+                              round_eps_to_dtype(eps, LO_BF16), q_sorted, s_sorted, some_absent ? 1 : 0));
   return LO_OK;
 }
 
@@ -375,7 +450,7 @@ int launch_silu_mul_token_quant(const void *in, int64_t rows, int64_t d, const i
   if (rows == 0) return LO_OK;
   LO_REQUIRE(d >= 8 && d % 8 == 0, "silu-mul quant: width %lld must be a multiple of 8", (long long)d);
   LO_REQUIRE(rows <= 0x7fffffffLL, "silu-mul quant: too many rows");
-  LO_CUDA_OK(launch_dependent(silu_mul_token_quant_kernel, dim3((unsigned)rows), dim3(TOKEN_QUANT_THREADS), 0, stream,
+  LO_CUDA_OK(launch_dependent(silu_mul_token_quant_kernel, dim3((unsigned)rows), dim3(SILU_THREADS), 0, stream,
                               static_cast<const __nv_bfloat16 *>(in), d, row_ids, numel_valid, num_rows_dev,
                               group_rows > 0 ? group_rows : (int64_t)1, group_counts, q, s));
   return LO_OK;

@@ -1,0 +1,145 @@
+"""GPU tests of the streaming kernels where their instruction-saving forms could differ from the plain ones: quotients from a
+refined reciprocal against the library's division, and the top-k sum at the sizes where its split changes."""
+import pytest
+import torch
+
+from oracle import moe_block_int8 as O
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def lo():
+    import lightop_b200
+    return lightop_b200
+
+
+@pytest.mark.parametrize("dtype,bits", [(torch.bfloat16, 7), (torch.float16, 10)])
+@pytest.mark.parametrize("exponent", [0, -6, 9])
+def test_group_quant_every_pair_of_maximum_and_element(lo, dtype, bits, exponent):
+    """The code of an element depends on it and on its group's maximum only, and is the same for both times a power of two: every
+    mantissa of the maximum with every element of the nine octaves below it (what is smaller has code 0)."""
+    n = 1 << bits
+    mant = 1.0 + torch.arange(n, dtype=torch.float64) / n
+    elems = torch.cat([mant * 2.0 ** -e for e in range(9)])
+    elems = torch.cat([elems, -elems])
+    per = 127
+    rows = -(-elems.numel() // per)
+    body = torch.zeros(rows * per, dtype=torch.float64)
+    body[:elems.numel()] = elems
+    for top in mant.split(128):
+        x = torch.empty(top.numel(), rows, 128, dtype=torch.float64)
+        x[..., 0] = top[:, None]
+        b = body.view(1, rows, per).expand(top.numel(), rows, per)
+        x[..., 1:] = torch.where(b.abs() <= top[:, None, None], b, torch.zeros((), dtype=torch.float64))
+        x = (x * 2.0 ** exponent).to(dtype).reshape(-1, 128)
+        q_ref, s_ref = O.group_quant_int8(x, 128)
+        q, s = lo.quant.per_token_group_quant_int8(x.to(DEV), 128)
+        assert torch.equal(s.cpu(), s_ref) and torch.equal(q.cpu(), q_ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_group_quant_infinity_nan_and_the_ends_of_the_range(lo, dtype):
+    big = torch.finfo(dtype).max
+    x = torch.randn(8, 256, generator=torch.Generator().manual_seed(3)).to(dtype)
+    x[0, 5] = float("inf")
+    x[1, 130] = float("-inf")
+    x[2, 7] = float("nan")
+    x[3, :128] = 0
+    x[4, :128] = torch.finfo(dtype).tiny
+    x[5, 3], x[5, 4] = big, -big
+    x[6, 129] = float("nan")
+    x[6, 128] = float("inf")
+    q, s = lo.quant.per_token_group_quant_int8(x.to(DEV), 128)
+    # the kernel's rule: the maximum passes over NaN, the quotient is the IEEE one, NaN has the code -128
+    v = x.float().view(8, 2, 128)
+    eps = float(torch.tensor(1e-10).to(dtype))
+    amax = torch.where(v.isnan(), torch.zeros(()), v.abs()).amax(-1).clamp(min=eps)
+    scale = amax / 127.0
+    r = v / scale[..., None]
+    want = torch.where(r.isnan(), torch.full((), -128.0), r.clamp(-128, 127)).trunc().to(torch.int8)
+    assert torch.equal(s.cpu(), scale) and torch.equal(q.cpu().view(8, 2, 128), want)
+
+
+def test_group_quant_codes_that_begin_on_eight_bytes(lo):
+    from lightop_b200 import _lib
+    x = torch.randn(9, 256, generator=torch.Generator().manual_seed(4)).to(torch.bfloat16).to(DEV)
+    q, s = lo.quant.per_token_group_quant_int8(x, 128)
+    room = torch.zeros(9 * 256 + 16, dtype=torch.int8, device=DEV)
+    s2 = torch.empty_like(s)
+    assert _lib.load().lo_group_quant_int8(x.data_ptr(), _lib.LO_BF16, 18, 128, 1e-10, room.data_ptr() + 8, s2.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(room[8:8 + 9 * 256].view(9, 256), q) and torch.equal(s2, s)
+    assert not room[:8].any() and not room[-8:].any()
+
+
+def test_silu_quant_every_gate(lo):
+    """Every bf16 gate, with eight of one magnitude range to a row so that small results keep their codes."""
+    gates = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).to(DEV)
+    gates = gates[~gates.isnan()]
+    gates = torch.cat([gates, gates[:-gates.numel() % 8]]).view(-1, 8)
+    extra = torch.tensor([[float("inf"), 1, -1, 2, float("-inf"), 0, 5, float("nan")], [float("-inf")] * 8, [-3.0e38, -100, -90, -89, -88.5, -88, -87, -80]],
+                         dtype=torch.bfloat16, device=DEV)
+    gates = torch.cat([gates, extra])
+    up = torch.randn(gates.shape, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16).to(DEV)
+    q, s = lo.activation.fuse_silu_mul_quant(torch.cat([gates, up], 1).contiguous())
+    g = gates.float()
+    act = ((g / (1.0 + torch.exp(-g))).to(torch.bfloat16).float() * up.float()).to(torch.bfloat16).float()
+    amax = torch.where(act.isnan(), torch.zeros((), device=DEV), act.abs()).amax(-1, keepdim=True)
+    r = act * torch.where(amax == 0, torch.zeros((), device=DEV), torch.full_like(amax, 127.0) / amax)
+    want = torch.where(r.isnan(), torch.full((), -128.0, device=DEV), r.round().clamp(-128, 127)).to(torch.int8)
+    assert torch.equal(s.view(-1, 1), amax / torch.full_like(amax, 127.0))
+    assert torch.equal(q.view_as(want), want)
+
+
+# blocks of one vector a thread up to eight blocks a SM, of four above: both sides of the line, columns that do not fill the last
+# pass, slots that are all, some or not there, more than 32 of them
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,k,H", [(1, 8, 7168), (296, 8, 7168), (297, 8, 7168), (1185, 3, 2056), (1300, 2, 256), (5, 37, 264), (1200, 40, 136), (400, 9, 8200)])
+def test_moe_sum_split(lo, dtype, M, k, H):
+    g = torch.Generator(device=DEV).manual_seed(M + k)
+    a = torch.randn(M, k, H, generator=g, device=DEV).to(dtype)
+    mask = torch.rand(M, k, generator=g, device=DEV) < 0.3
+    mask[0] = False
+    mask[-1] = True
+    bias = torch.randn(M, H, generator=g, device=DEV).to(dtype)
+    for m in (None, mask):
+        for b, f in ((None, 1.0), (bias, 2.5)):
+            out = torch.empty(M, H, dtype=dtype, device=DEV)
+            lo.moe.moe_sum(a, out, bias=b, expert_mask=m, factor=f)
+            acc = torch.zeros(M, H, device=DEV)
+            for j in range(k):
+                acc = acc + (a[:, j].float() if m is None else torch.where(m[:, j:j + 1], a[:, j].float(), torch.zeros((), device=DEV)))
+            if b is None:
+                assert torch.equal(out, (acc * f).to(dtype))
+            else:      # one fused or two rounded operations: half a step of the product and of the sum, then of the result's type
+                want = acc.double() * f + b.double()
+                tol = 2.0 ** -23 * (acc.double() * f).abs() + 2.0 ** (-8 if dtype == torch.bfloat16 else -23) * want.abs() + 1e-30
+                assert bool(((out.double() - want).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("M", [7, 600])
+def test_layer_of_a_shard_passes_over_tokens_without_a_local_expert(lo, M):
+    """One expert of eight is local: most tokens have no position in the sorted rows, some have several slots."""
+    from lightop_b200 import synthetic
+    E, k, H, I = 8, 2, 256, 256
+    w1, w2, w1_s, w2_s = synthetic.make_weights(E, H, I, seed=1, device=DEV)
+    x, logits = synthetic.make_activations(M, H, E, seed=2, device=DEV)
+    weights = torch.empty(M, k, device=DEV)
+    ids = torch.empty(M, k, dtype=torch.int32, device=DEV)
+    lo.moe.topk_softmax(weights, ids, None, logits, True)
+    total = torch.zeros(M, H, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        emap = torch.full((E,), -1, dtype=torch.int32, device=DEV)
+        emap[e] = 0
+        y = lo.moe.fused_experts_impl_int8(x, w1[e:e + 1].contiguous(), w2[e:e + 1].contiguous(), weights, ids, torch.empty(M * k * H, dtype=torch.bfloat16, device=DEV),
+                                           use_int8_w8a8=True, block_shape=[128, 128], w1_scale=w1_s[e:e + 1].contiguous(), w2_scale=w2_s[e:e + 1].contiguous(),
+                                           global_num_experts=E, expert_map=emap)
+        assert not y[~(ids == e).any(1)].any()
+        total += y.double()
+    y = lo.moe.fused_experts_impl_int8(x, w1, w2, weights, ids, torch.empty(M * k * H, dtype=torch.bfloat16, device=DEV), use_int8_w8a8=True,
+                                       block_shape=[128, 128], w1_scale=w1_s, w2_scale=w2_s)
+    # every row once in each: the parts are rounded to bf16 where the whole is rounded once
+    assert float((total - y.double()).norm() / y.double().norm()) < 2 ** -8
