@@ -438,21 +438,28 @@ __global__ void __launch_bounds__(256) ep_gather_kernel(const __nv_bfloat16 *__r
   }
 }
 
-// One CTA per sorted position: copy the int8 row and its scales of token sorted_ids[pos] / top_k.
-__global__ void __launch_bounds__(128) permute_rows_kernel(const int8_t *__restrict__ A, const float *__restrict__ a_scale,
-                                                           int64_t rows_a, int64_t K, const int32_t *__restrict__ sorted_ids,
+// One warp per sorted position: copy the int8 row and its scales of token sorted_ids[pos] / top_k.  What a position's row depends on
+// is loaded at once, and a lane has four 16-byte loads of the row in flight.  (A block of 128 threads a position, with a load of
+// the count, one of the id and one of the row behind one another, took 13.7 us for 2400 rows of 4096 bytes.)
+constexpr int PERMUTE_WARPS = 4;
+__global__ void __launch_bounds__(PERMUTE_WARPS * 32) permute_rows_kernel(const int8_t *__restrict__ A, const float *__restrict__ a_scale,
+                                                           int64_t rows_a, int64_t K, const int32_t *__restrict__ sorted_ids, int64_t positions,
                                                            const int32_t *__restrict__ num_tokens_post_pad,
                                                            int64_t numel_valid, int top_k, int64_t kb,
                                                            int8_t *__restrict__ A_sorted,
                                                            float *__restrict__ a_scale_sorted, int64_t a_stride,
                                                            const int32_t *__restrict__ expert_ids, int block_size,
                                                            Chunk *__restrict__ chunks, int32_t *__restrict__ num_chunks) {
-  const int64_t pos = blockIdx.x;
+  const int64_t pos = (int64_t)blockIdx.x * PERMUTE_WARPS + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
   dependency_wait();
   dependency_release();
-  if (chunks != nullptr && threadIdx.x == 0) {
+  if (pos >= positions) return;
+  const int32_t post_pad = *num_tokens_post_pad;
+  const int32_t sid = sorted_ids[pos];
+  if (chunks != nullptr && lane == 0) {
     const int rows = block_size <= 128 ? block_size : 128;
-    const int64_t total = (int64_t)(*num_tokens_post_pad / block_size) * block_size;      // positions of whole blocks
+    const int64_t total = (int64_t)(post_pad / block_size) * block_size;      // positions of whole blocks
     if (pos % rows == 0 && pos < total) {
       Chunk ch;
       ch.expert = expert_ids[pos / block_size];
@@ -462,13 +469,11 @@ __global__ void __launch_bounds__(128) permute_rows_kernel(const int8_t *__restr
       chunks[pos / rows] = ch;
     }
     if (pos == 0) {
-      const int64_t there = ((int64_t)gridDim.x + rows - 1) / rows;
+      const int64_t there = (positions + rows - 1) / rows;
       *num_chunks = (int32_t)(total / rows < there ? total / rows : there);
     }
   }
-  if (pos >= *num_tokens_post_pad) return;
-  const int32_t sid = sorted_ids[pos];
-  if (sid < 0 || sid >= numel_valid) return;
+  if (pos >= post_pad || sid < 0 || sid >= numel_valid) return;
   const int64_t row = sid / top_k;
   if (row >= rows_a) return;
   // a_stride: bytes between two source rows (K for a plain matrix); without a scale array the scales follow the
@@ -476,8 +481,17 @@ __global__ void __launch_bounds__(128) permute_rows_kernel(const int8_t *__restr
   const uint4 *src = reinterpret_cast<const uint4 *>(A + row * a_stride);
   const float *src_s = a_scale ? a_scale + row * kb : reinterpret_cast<const float *>(A + row * a_stride + K);
   uint4 *dst = reinterpret_cast<uint4 *>(A_sorted + pos * K);
-  for (int64_t c = threadIdx.x; c < K / 16; c += blockDim.x) dst[c] = src[c];
-  for (int64_t c = threadIdx.x; c < kb; c += blockDim.x) a_scale_sorted[pos * kb + c] = src_s[c];
+  const int n = (int)(K / 16);
+  for (int c = lane; c < n; c += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c + 32 * u < n) v[u] = src[c + 32 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c + 32 * u < n) dst[c + 32 * u] = v[u];
+  }
+  for (int64_t c = lane; c < kb; c += 32) a_scale_sorted[pos * kb + c] = src_s[c];
 }
 
 }  // namespace
@@ -488,8 +502,8 @@ int launch_permute_rows(const int8_t *A, const float *a_scale, int64_t rows_a, i
                         int64_t a_stride, const int32_t *expert_ids, int block_size, Chunk *chunks, int32_t *num_chunks) {
   if (sorted_capacity <= 0) return LO_OK;
   LO_REQUIRE(sorted_capacity <= 0x7fffffffLL, "permute rows: too many positions");
-  LO_CUDA_OK(launch_dependent(permute_rows_kernel, dim3((unsigned)sorted_capacity), dim3(128), 0, stream, A, a_scale, rows_a, K, sorted_ids,
-                              num_tokens_post_pad, numel_valid, top_k, scales_per_row > 0 ? scales_per_row : K / 128, A_sorted,
+  LO_CUDA_OK(launch_dependent(permute_rows_kernel, dim3((unsigned)ceil_div(sorted_capacity, PERMUTE_WARPS)), dim3(PERMUTE_WARPS * 32), 0, stream, A, a_scale, rows_a, K,
+                              sorted_ids, sorted_capacity, num_tokens_post_pad, numel_valid, top_k, scales_per_row > 0 ? scales_per_row : K / 128, A_sorted,
                               a_scale_sorted, a_stride > 0 ? a_stride : K, expert_ids, block_size, chunks, num_chunks));
   return LO_OK;
 }
