@@ -203,6 +203,13 @@ __device__ __forceinline__ float div_by(float a, float b, float y) {
   return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
+// Order-preserving unsigned key of a float, for warp reductions in one instruction: -0 like 0, NaN like -inf (never preferred).
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t b = __float_as_uint(v == v ? v + 0.0f : -INFINITY);
+  return b ^ ((b >> 31) != 0u ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float key_value(uint32_t k) { return __uint_as_float(k ^ ((k >> 31) != 0u ? 0x80000000u : 0xffffffffu)); }
+
 // Lanes of the warp that hold the same expert as this lane (lanes without an expert match one another).
 // With many steps per warp the mask is built from one ballot per bit of the expert id: the match
 // instruction proper has a throughput of the order of one warp per ~64 cycles and SM here, which made it the

@@ -9,7 +9,10 @@ namespace {
 // ---------------------------------------------------------------------------
 // topk_softmax: one warp per row, experts strided over the lanes (expert =
 // lane + 32*i), k rounds of warp arg-max with erase.  Selection is done on the
-// logits (softmax is monotonic); ties go to the lower expert id.
+// logits (softmax is monotonic); ties go to the lower expert id.  A round is two warp reductions
+// in one instruction each, of keys that order like the logits and of the ids that have the
+// largest key (five shuffle steps of value and id were three times the instructions, which
+// bound the kernel: 8192 rows of 256 experts).
 // ---------------------------------------------------------------------------
 
 template <typename T> __device__ __forceinline__ float to_float(T v);
@@ -49,28 +52,27 @@ __global__ void __launch_bounds__(256) topk_softmax_kernel(const T *__restrict__
   float my_w = 0.f;   // lane j keeps the j-th selected probability
   int my_id = 0;
   float sel_sum = 0.f;
+  uint32_t key[VPL];
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) key[i] = order_key(v[i]);
+  const uint32_t erased = order_key(-INFINITY);
   for (int r = 0; r < k; ++r) {
-    float best = v[0];
-    int best_e = lane;
+    uint32_t best = key[0];
+    int best_i = 0;
 #pragma unroll
     for (int i = 1; i < VPL; ++i) {
-      if (v[i] > best) { best = v[i]; best_e = lane + 32 * i; }   // strict: keeps the lower id on ties
+      if (key[i] > best) { best = key[i]; best_i = i; }   // strict: keeps the lower id on ties
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, off);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
-    const float p = expf(best - mx) / denom;
+    const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+    const int best_e = (int)__reduce_min_sync(0xffffffffu, best == top ? (uint32_t)(lane + 32 * best_i) : 0xffffffffu);
+    const float p = expf(key_value(top) - mx) / denom;
     sel_sum += p;
     if (lane == r) { my_w = p; my_id = best_e; }
     // erase the winner in its owner lane
     if ((best_e & 31) == lane) {
-      const int slot = best_e >> 5;
 #pragma unroll
       for (int i = 0; i < VPL; ++i)
-        if (i == slot) v[i] = -INFINITY;
+        if (i == best_e >> 5) key[i] = erased;
     }
   }
   if (lane < k) {
@@ -302,7 +304,9 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_kernel(
 // i.e. still ascending flat index inside an expert: bit-identical to the single-CTA kernel.
 // ---------------------------------------------------------------------------
 constexpr int ALIGN_CLUSTER = 8;
-constexpr int64_t ALIGN_CLUSTER_MIN_IDS = 8192;   // below this the single CTA is as fast and costs one SM
+// One CTA against the cluster, in us: 2048 ids 10.1, 8.1; 2400 ids 11.6, 8.5; 4800 ids 15.8, 9.4; 6216 ids 17.5, 9.0.  Below, a warp has a
+// step or two and the exchange between the CTAs is what is left.
+constexpr int64_t ALIGN_CLUSTER_MIN_IDS = 2048;
 
 template <typename IdT>
 __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
