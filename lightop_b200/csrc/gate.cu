@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(GATE_WARPS * 32) fused_gate_kernel(
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int64_t row = (int64_t)blockIdx.x * GATE_WARPS + warp;
+  dependency_wait();
   dependency_release();      // the alignment kernel may get its block resident; it waits for this grid before it reads
   if (row >= M) return;
   float *s_row = gate_smem + (size_t)warp * 2 * E;
@@ -157,18 +158,15 @@ int launch_gate(const void *x, int x_dtype, const void *bias, int bias_dtype, in
   const size_t smem = (size_t)GATE_WARPS * 2 * E * sizeof(float);
   IdT *idp = static_cast<IdT *>(ids);
   const int vpl = (int)ceil_div(E, 32);
-#define LO_GATE_CASE(V)                                                                                         \
-  fused_gate_kernel<V, IdT><<<(unsigned)blocks, GATE_WARPS * 32, smem, st>>>(x, x_dtype, bias, bias_dtype, bias_row_stride, M, E, groups, \
-                                                                             topk_group, topk, n_shared, score_fn, \
-                                                                             renormalize, norm_eps, out_scale,     \
-                                                                             shared_div, num_valid, num_valid_dtype,\
-                                                                             padding_id, w, idp)
+#define LO_GATE_CASE(V)                                                                                             \
+  LO_CUDA_OK(launch_dependent(fused_gate_kernel<V, IdT>, dim3((unsigned)blocks), dim3(GATE_WARPS * 32), smem, st, x, x_dtype, bias, \
+                              bias_dtype, bias_row_stride, M, E, groups, topk_group, topk, n_shared, score_fn, renormalize, \
+                              norm_eps, out_scale, shared_div, num_valid, num_valid_dtype, padding_id, w, idp))
   if (vpl <= 4) LO_GATE_CASE(4);
   else if (vpl <= 8) LO_GATE_CASE(8);
   else if (vpl <= 16) LO_GATE_CASE(16);
   else LO_GATE_CASE(32);
 #undef LO_GATE_CASE
-  LO_LAUNCH_OK("fused_gate_kernel");
   return LO_OK;
 }
 

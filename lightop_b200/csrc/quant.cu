@@ -96,6 +96,7 @@ template <typename T, int LANES>
 __global__ void __launch_bounds__(256) group_quant_kernel(const T *__restrict__ x, int8_t *__restrict__ q,
                                                           float *__restrict__ s, int64_t num_groups,
                                                           float eps_t, int q16) {
+  dependency_wait();
   dependency_release();      // (a dependent kernel waits for the whole grid before it reads)
   const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t group = gthread / LANES;
@@ -378,12 +379,11 @@ int launch_typed(const void *x, int64_t num_groups, int group_size, float eps_t,
   const T *xp = static_cast<const T *>(x);
   const int q16 = (reinterpret_cast<uintptr_t>(q) & 15) == 0 ? 1 : 0;      // (the caller's q may begin on 8 bytes only)
   switch (group_size) {
-    case 64: group_quant_kernel<T, 4><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t, q16); break;
-    case 128: group_quant_kernel<T, 8><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t, q16); break;
-    case 256: group_quant_kernel<T, 16><<<(unsigned)blocks, threads, 0, stream>>>(xp, q, s, num_groups, eps_t, q16); break;
+    case 64: LO_CUDA_OK(launch_dependent(group_quant_kernel<T, 4>, dim3((unsigned)blocks), dim3(threads), 0, stream, xp, q, s, num_groups, eps_t, q16)); break;
+    case 128: LO_CUDA_OK(launch_dependent(group_quant_kernel<T, 8>, dim3((unsigned)blocks), dim3(threads), 0, stream, xp, q, s, num_groups, eps_t, q16)); break;
+    case 256: LO_CUDA_OK(launch_dependent(group_quant_kernel<T, 16>, dim3((unsigned)blocks), dim3(threads), 0, stream, xp, q, s, num_groups, eps_t, q16)); break;
     default: return fail(LO_ERR_UNSUPPORTED, "group quant: group_size %d not in {64,128,256}", group_size);
   }
-  LO_LAUNCH_OK("group_quant_kernel");
   return LO_OK;
 }
 

@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(256) moe_sum_kernel(const T *__restrict__ in, 
   const int64_t t = blockIdx.y;
   const int lane = threadIdx.x & 31;
   dependency_wait();            // the rows come from the kernel before this one
+  dependency_release();
   if (num_local_tokens && t >= *num_local_tokens) return;
   // which of the slots base + 0 .. base + 31 count (the same in every lane)
   auto live_slots = [&](int base) {

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(256) topk_softmax_kernel(const T *__restrict__
                                                            IdT *__restrict__ ids, int32_t *__restrict__ src_rows) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  dependency_wait();
   dependency_release();      // the alignment kernel may get its block resident; it waits for this grid before it reads
   if (row >= M) return;
   const T *g = gating + row * E;
@@ -92,7 +93,7 @@ int launch_topk_vpl(const void *gating, int64_t M, int E, int k, int renorm, flo
   IdT *idp = static_cast<IdT *>(ids);
   const int vpl = (int)ceil_div(E, 32);
 #define LO_TOPK_CASE(V)                                                                        \
-  topk_softmax_kernel<T, IdT, V><<<(unsigned)blocks, warps * 32, 0, st>>>(g, M, E, k, renorm, w, idp, src)
+  LO_CUDA_OK(launch_dependent(topk_softmax_kernel<T, IdT, V>, dim3((unsigned)blocks), dim3(warps * 32), 0, st, g, M, E, k, renorm, w, idp, src))
   if (vpl <= 1) LO_TOPK_CASE(1);
   else if (vpl <= 2) LO_TOPK_CASE(2);
   else if (vpl <= 4) LO_TOPK_CASE(4);
@@ -100,7 +101,6 @@ int launch_topk_vpl(const void *gating, int64_t M, int E, int k, int renorm, flo
   else if (vpl <= 16) LO_TOPK_CASE(16);
   else LO_TOPK_CASE(32);
 #undef LO_TOPK_CASE
-  LO_LAUNCH_OK("topk_softmax_kernel");
   return LO_OK;
 }
 
