@@ -62,10 +62,11 @@ template <> struct Vec8<float> {
 // One block row per token.  Each warp finds out once which of the token's slots count (a lane each, up to 32 at a time), then every
 // thread adds their rows in slot order, VPT vectors of eight columns at a time with several rows in flight.  (A thread that looked
 // at id, map and row of one slot after the other spent its time on the latencies: 8192 tokens with one local slot in eight took
-// 103 us for 234 MB, now 72; 64 tokens of eight slots 8.0, now 4.7.)  VPT = 4: one pass of a block over 8192 columns, the latency of finding the slots is paid once a token;
+// 103 us for 234 MB, now 59 (72 with two blocks a SM
+// instead of three); 64 tokens of eight slots 8.0, now 4.7.)  VPT = 4: one pass of a block over 8192 columns, the latency of finding the slots is paid once a token;
 // VPT = 1: more blocks a token where there are few tokens.
 template <typename T, typename IdT, int VPT>
-__global__ void __launch_bounds__(256) moe_sum_kernel(const T *__restrict__ in, T *__restrict__ out,
+__global__ void __launch_bounds__(256, VPT == 4 && sizeof(T) == 2 ? 3 : 1) moe_sum_kernel(const T *__restrict__ in, T *__restrict__ out,
                                                       const T *__restrict__ bias, int64_t M, int topk, int64_t H8,
                                                       float factor, const uint8_t *__restrict__ mask,
                                                       const int32_t *__restrict__ num_local_tokens,
