@@ -355,34 +355,58 @@ __device__ __forceinline__ void tmem_ld_wait16(uint32_t (&r)[16]) {
                  "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                :: "memory");
 }
-// Partial sums in the layout of an MMA accumulator fragment, 16 registers a thread at a time ("unit"):
-// two pieces (32 columns) of one half of the warp's channels (16 lanes, taddr points at the first of them): register 4c + r is
-// channel 8(r >> 1) + lane / 4, token 8c + 2(lane % 4) + (r & 1) ...
-__device__ __forceinline__ void tmem_ld_two(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr)
-               : "memory");
+// Partial sums, 16 registers a thread at a time ("unit"), four threads to a channel: two pieces (32 columns) of one half of the
+// warp's channels (16 lanes, taddr points at the first of them).  Register 8v + r is piece v, and of that piece
+//   ROW4  (16x128b loads): channel 8(r & 1) + lane / 4, token 4(r >> 1) + lane % 4
+//   !ROW4 (16x256b loads, the layout of an MMA accumulator fragment): channel 8((r >> 1) & 1) + lane / 4,
+//         token 8(r >> 2) + 2(lane % 4) + (r & 1)
+// In a loop of loads alone the first form moves 128 bytes per clock and scheduler, the second 64.  Layers take the first: 4096 tokens
+// 3348 -> 3318 us a pass, 8192 tokens of a shard 860 -> 842, Zipf routing the same; dense calls the second (4096 x 4096 x 7168 203 us a
+// pass against 207.5 with the first).
+template <bool ROW4> __device__ __forceinline__ void tmem_ld_two(uint32_t taddr, uint32_t (&r)[16]) {
+  if (ROW4)
+    asm volatile("tcgen05.ld.sync.aligned.16x128b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr)
+                 : "memory");
+  else
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr)
+                 : "memory");
 }
-// ... or one piece (16 columns) of both halves: register 8h + 4c + r is channel 16h + 8(r >> 1) + lane / 4, token as above.
-__device__ __forceinline__ void tmem_ld_one(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr + (16u << 16)) : "memory");
+// ... or one piece (16 columns) of both halves: register 8k + r is half k (channels 16k ..), r as above.
+template <bool ROW4> __device__ __forceinline__ void tmem_ld_one(uint32_t taddr, uint32_t (&r)[16]) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    uint32_t *h = &r[8 * k];
+    if (ROW4)
+      asm volatile("tcgen05.ld.sync.aligned.16x128b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]), "=r"(h[4]), "=r"(h[5]), "=r"(h[6]), "=r"(h[7]) : "r"(taddr + (uint32_t)k * (16u << 16)) : "memory");
+    else
+      asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]), "=r"(h[4]), "=r"(h[5]), "=r"(h[6]), "=r"(h[7]) : "r"(taddr + (uint32_t)k * (16u << 16)) : "memory");
+  }
 }
-// Place of token t of a piece in its 16-entry row of the scale table: the four scales a thread needs of a piece are one
-// 16-byte load.
-__device__ __forceinline__ int scale_place(int t) { return (t & ~15) | ((t >> 1) & 3) << 2 | ((t >> 3) & 1) << 1 | (t & 1); }
+// A thread's four tokens of a piece, j = 0 .. 3, with i = lane % 4; and the place of token t of a piece in its 16-entry row of the scale
+// table: the four scales of a thread are one 16-byte load, in the order of j.
+template <bool ROW4> __device__ __forceinline__ int token_of(int i, int j) { return ROW4 ? 4 * j + i : (j >> 1) * 8 + 2 * i + (j & 1); }
+template <bool ROW4> __device__ __forceinline__ int scale_place(int t) {
+  return ROW4 ? (t & ~15) | (t & 3) << 2 | ((t >> 2) & 3) : (t & ~15) | ((t >> 1) & 3) << 2 | ((t >> 3) & 1) << 1 | (t & 1);
+}
+// Row of an eight-token block that column c of a transposed matrix store is: a thread's pair of values is columns 2i and 2i + 1.
+template <bool ROW4> __device__ __forceinline__ int block_row(int c) { return ROW4 ? (c >> 1) + 4 * (c & 1) : c; }
 
-// acc = fma(float(raw), scale product, acc) on eight values, one half of a piece: s = the scale products of tokens 2i, 2i + 1,
-// 8 + 2i, 9 + 2i, i = lane % 4.  The 128-long int8 dot is below 2^21 in magnitude, so the conversion is exact; one rounding per
-// K block.  Two tokens of one channel at a time: the packed multiply-add takes the registers in pairs as they come.
-__device__ __forceinline__ void promote8(float *acc, const uint32_t *raw, const float (&s)[4]) {
+// acc = fma(float(raw), scale product, acc) on eight values, one half of a piece: s[j] = the scale product of token j of this thread.
+// The 128-long int8 dot is below 2^21 in magnitude, so the conversion is exact; one rounding per
+// K block.  Two tokens of one channel at a time: acc[4c + 2h + e] is channel 8h + lane / 4, token 2c + e of the thread's four.
+template <bool ROW4> __device__ __forceinline__ void promote8(float *acc, const uint32_t *raw, const float (&s)[4]) {
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
-    const float f0 = __int2float_rn((int32_t)raw[j]), f1 = __int2float_rn((int32_t)raw[j + 1]);
+    const int a = ROW4 ? (j & 4) + ((j >> 1) & 1) : j, b = ROW4 ? a + 2 : j + 1;
+    const float f0 = __int2float_rn((int32_t)raw[a]), f1 = __int2float_rn((int32_t)raw[b]);
     asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%0, %1};\n\t"
         "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
         : "+f"(acc[j]), "+f"(acc[j + 1]) : "f"(f0), "f"(f1), "f"(s[(j >> 1) & 2]), "f"(s[((j >> 1) & 2) + 1]));
@@ -533,6 +557,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   constexpr int PHASES = CF::PHASES;
   constexpr int NCG = CF::NCG;
   constexpr int EPI_WARPS = CF::EPI_WARPS;
+  constexpr bool ROW4 = FORM == TABLE;                           // see tmem_ld_two
   constexpr bool RESPLIT = CF::SPLIT_REGS && FORM != SPLIT;      // (a split K extent has no running sums)
   extern __shared__ uint8_t smem_raw[];
   SM &sm = *reinterpret_cast<SM *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -712,7 +737,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (t < T) {
               const float live = t < cur.ch.rows ? 1.f : 0.f;
 #pragma unroll
-              for (int i = 0; i < SC_STEPS; ++i) sc[i * A_ROWS + scale_place(t)] = live != 0.f ? __fmul_rn(a_cur[u][i], b_cur[i]) : 0.f;
+              for (int i = 0; i < SC_STEPS; ++i) sc[i * A_ROWS + scale_place<ROW4>(t)] = live != 0.f ? __fmul_rn(a_cur[u][i], b_cur[i]) : 0.f;
             }
           }
           __syncwarp();
@@ -1063,7 +1088,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         const uint32_t wait_ns = my_p == 0 ? 256u : LO_SLEEP_PROMO;
         // this lane's row of the staging tile for the matrix stores and loads of a piece: lanes 8m .. 8m + 7 address the
         // token rows of block m, blocks 0 / 1 are channels 0..7 / 8..15 of tokens 0..7, blocks 2 / 3 of tokens 8..15
-        const uint32_t stg_mine = smem_u32(&sm.staging[0]) + (uint32_t)(col_begin + (lane >> 4) * 8 + (lane & 7)) * OUT_ROW_BYTES +
+        const uint32_t stg_mine = smem_u32(&sm.staging[0]) + (uint32_t)(col_begin + (lane >> 4) * 8 + block_row<ROW4>(lane & 7)) * OUT_ROW_BYTES +
                                   (uint32_t)(q * 32 + ((lane >> 3) & 1) * 8) * 2u;
         // fp32 routed weight of token t of the chunk (0 where there is no row)
         auto weight_of = [&](int t) {
@@ -1092,8 +1117,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             constexpr int SETS = PC > 1 && (PC & 1) ? 3 : 2;
             uint32_t raw[SETS][16];
             auto load_unit = [&](int u, uint32_t part, uint32_t (&r)[16]) {
-              if ((PC & 1) && u == U - 1) tmem_ld_one(part + 16u * (PC - 1), r);
-              else tmem_ld_two(part + 32u * (u >> 1) + ((u & 1) ? 16u << 16 : 0u), r);
+              if ((PC & 1) && u == U - 1) tmem_ld_one<ROW4>(part + 16u * (PC - 1), r);
+              else tmem_ld_two<ROW4>(part + 32u * (u >> 1) + ((u & 1) ? 16u << 16 : 0u), r);
             };
             uint32_t dn = step & (uint32_t)(ND - 1), dph = (step >> 4) & 1u;      // the step's place in the rings of ND
             if (!__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; return; }
@@ -1151,11 +1176,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                   }
                   if (PC > 0) {
                     if (single) {
-                      promote8(&acc[PC > 0 ? PC - 1 : 0][0], &raw[set][0], s0);
-                      promote8(&acc[PC > 0 ? PC - 1 : 0][8], &raw[set][8], s0);
+                      promote8<ROW4>(&acc[PC > 0 ? PC - 1 : 0][0], &raw[set][0], s0);
+                      promote8<ROW4>(&acc[PC > 0 ? PC - 1 : 0][8], &raw[set][8], s0);
                     } else {
-                      promote8(&acc[u & ~1][8 * (u & 1)], &raw[set][0], s0);
-                      promote8(&acc[(u | 1) < NP ? (u | 1) : 0][8 * (u & 1)], &raw[set][8], s1);
+                      promote8<ROW4>(&acc[u & ~1][8 * (u & 1)], &raw[set][0], s0);
+                      promote8<ROW4>(&acc[(u | 1) < NP ? (u | 1) : 0][8 * (u & 1)], &raw[set][8], s1);
                     }
                   }
                 }
@@ -1186,7 +1211,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
               if (pc < my_p) {
                 float w[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) w[i] = weight_of(col_begin + pc * 16 + (i >> 1) * 8 + (lane & 3) * 2 + (i & 1));
+                for (int i = 0; i < 4; ++i) w[i] = weight_of(col_begin + pc * 16 + token_of<ROW4>(lane & 3, i));
 #pragma unroll
                 for (int j = 0; j < 16; ++j) acc[pc][j] *= w[((j >> 1) & 2) + (j & 1)];
               }
