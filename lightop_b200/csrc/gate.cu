@@ -3,7 +3,7 @@
 // moe_fused_gate, per token (one warp per token, experts strided over the lanes):
 //   p[e]      = sigmoid(x[e])                          (fp32)
 //   s[e]      = p[e] + bias[e]                         (selection score)
-//   group g   = experts [g*S, (g+1)*S), S = E / groups; group score = sum of its two largest s
+//   group g   = experts [g*S, (g+1)*S), S = E / groups; group score = sum of its two largest s (of its only s where S = 1)
 //   keep the topk_group best groups (ties: lower group), mask the others out
 //   pick the k_routed = topk - shared best s among the kept experts (ties: lower expert id),
 //   in descending order
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(GATE_WARPS * 32) fused_gate_kernel(
         if (v > m1) { m2 = m1; m1 = v; }
         else if (v > m2) { m2 = v; }
       }
-      gscore = m1 + m2;
+      gscore = S == 1 ? m1 : m1 + m2;      // (a group of one expert has no second score: m2 is still -inf)
     }
     uint32_t keep = 0u;           // bit g: group g survives
     uint32_t gkey = order_key(gscore);
@@ -102,8 +102,8 @@ __global__ void __launch_bounds__(GATE_WARPS * 32) fused_gate_kernel(
       keep |= 1u << best_g;
       if (lane == best_g) gkey = erased;
     }
-    // lanes >= groups hold -inf and a lane index >= groups; a winner among them would mean fewer than
-    // topk_group finite groups, which the argument checks exclude for finite inputs
+    // Lanes >= groups hold the key of -inf.  With finite scores every group's key is above it, so the topk_group <= groups winners are
+    // groups; a row with NaN or infinities may lose rounds to keys that are equal to it.
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       const int e = lane + 32 * i;

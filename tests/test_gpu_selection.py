@@ -62,3 +62,17 @@ def test_grouped_gate_with_ties(lo, E, groups, keep, k):
 def test_align_around_the_cluster(lo, numel_rows, k, E):
     g = torch.Generator().manual_seed(numel_rows + E)
     _check_align(lo, torch.randint(0, E, (numel_rows, k), generator=g, dtype=torch.int32), E, 16)
+
+
+@pytest.mark.parametrize("E,keep,k,shared", [(8, 2, 2, 0), (32, 8, 8, 0), (32, 32, 6, 0), (2, 1, 1, 0), (16, 5, 6, 1)])
+def test_grouped_gate_with_groups_of_one_expert(lo, E, keep, k, shared):
+    """The score of such a group is its expert's: the groups kept are the best experts."""
+    x = torch.randn(130, E, generator=torch.Generator().manual_seed(E + keep))
+    bias = torch.linspace(-0.5, 0.5, E)
+    w, ids = lo.moe.moe_fused_gate(x.to(DEV), bias.to(DEV), E, keep, k, shared, 2.5, False)
+    s = torch.sigmoid(x.to(DEV)).cpu()
+    order = torch.sort(s + bias, dim=1, descending=True, stable=True).indices[:, :k - shared]
+    assert torch.equal(ids.cpu().long()[:, :k - shared], order)
+    p = torch.gather(s, 1, order)
+    torch.testing.assert_close(w.cpu()[:, :k - shared], p / p.sum(1, keepdim=True), rtol=2e-5, atol=2e-6)
+    assert bool((ids.cpu()[:, k - shared:] == E).all())
