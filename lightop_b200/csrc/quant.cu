@@ -314,9 +314,11 @@ __global__ void __launch_bounds__(SILU_THREADS) silu_mul_token_quant_kernel(
   const int64_t row = blockIdx.x;
   dependency_wait();
   dependency_release();
-  // masked layout [groups, group_rows, 2d]: only the first group_counts[g] rows of a group exist (most do not, so they are looked
-  // up before anything is loaded; of the sorted positions few are padding)
+  // The grid is the capacity.  Rows that do not exist are passed over before anything of them is loaded: in the masked layout [groups,
+  // group_rows, 2d] all but the first group_counts[g] rows of a group, in the sorted one all from *num_rows_dev on.  What is left there
+  // is the padding of the experts' blocks, whose ids are looked up beside the loads.
   if (group_counts && row % group_rows >= group_counts[row / group_rows]) return;
+  if (num_rows_dev && row >= *num_rows_dev) return;
   const uint4 *g = reinterpret_cast<const uint4 *>(in + row * 2 * d);
   const int64_t vecs = d / 8;
   const uint4 *u = g + vecs;
@@ -332,7 +334,6 @@ __global__ void __launch_bounds__(SILU_THREADS) silu_mul_token_quant_kernel(
       }
     }
   }
-  if (num_rows_dev && row >= *num_rows_dev) return;
   if (row_ids) {
     const int32_t id = row_ids[row];
     if (id < 0 || id >= numel_valid) return;

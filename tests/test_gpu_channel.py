@@ -235,3 +235,24 @@ def test_fused_channel_chunk_rule(lo, counts):
     y = _run_fused(lo, x, w1, w2, w1_s, w2_s, w, ids)
     _, mean_rel = assert_out_close(y, OC.fused_moe_channel_int8(x, w1, w2, w1_s, w2_s, w, ids), f"per-channel {counts}")
     assert mean_rel < 2e-3
+
+
+@pytest.mark.parametrize("M", [1, 7, 600])
+def test_fused_channel_of_a_shard_of_eight(lo, M):
+    """One expert of eight is local: most of the positions that the grid covers do not exist, most tokens have no row."""
+    E, k, H, I = 8, 2, 256, 384
+    w1, w2, _, _ = synthetic.make_weights(E, H, I, seed=8)
+    w1_s, w2_s = synthetic.make_channel_scales(E, H, I, seed=8)
+    x, logits = synthetic.make_activations(M, H, E, seed=9)
+    w, ids = O.route_topk_softmax(logits, k, renormalize=True)
+    total = torch.zeros(M, H, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        emap = torch.full((E,), -1, dtype=torch.int32)
+        emap[e] = 0
+        y = _run_fused(lo, x, w1[e:e + 1], w2[e:e + 1], w1_s[e:e + 1], w2_s[e:e + 1], w, ids, expert_map=emap.to(DEV),
+                       global_num_experts=E)
+        assert not y[~(ids == e).any(1).to(DEV)].any()
+        total += y.double()
+    whole = _run_fused(lo, x, w1, w2, w1_s, w2_s, w, ids)
+    # the parts are rounded to bf16 where the whole is rounded once
+    assert float((total - whole.double()).norm() / whole.double().norm()) < 2 ** -8

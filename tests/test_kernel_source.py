@@ -43,3 +43,11 @@ def test_vector_stores_to_the_callers_output_look_at_its_address():
     assert any(s.startswith("p.vec_store = ") and "& 7) == 0" in s and "a.C) & 15) == 0" in s for s in st)
     i = next(i for i, s in enumerate(st) if "*reinterpret_cast<uint4 *>(dst) = v" in s)
     assert st[i - 1] == "if (p.vec_store)"
+
+
+def test_silu_quantiser_loads_no_row_that_does_not_exist():
+    # the grid is the capacity (with an expert map mostly rows that do not exist): both counts are looked at before a load of the row
+    st = _statements("quant.cu")
+    first_load = next(i for i, s in enumerate(st) if s == "gv[v] = g[i]")
+    assert any(s.startswith("if (num_rows_dev && row >= *num_rows_dev) return") for s in st[:first_load])
+    assert any(s.startswith("if (group_counts && row % group_rows >= group_counts[row / group_rows]) return") for s in st[:first_load])
