@@ -57,17 +57,21 @@ __device__ __forceinline__ uint32_t pack4_rz(const float (&r)[4]) {
 }
 
 // A thread's sixteen elements of a group of LANES x 16: maximum over the group's lanes, scale, codes.  Every lane of the warp
-// calls it.  Two-byte types take the quotient from the refined reciprocal wherever that is the IEEE quotient (a scale
-// that is finite and not near the ends of the range: all but groups with an infinity or, with a tiny eps, of next to nothing); with
-// the library's division and eight elements a thread the kernels were bound by their instructions: 4096 x 7168 alone 33 -> 22 us (the
-// bytes take 14), into eight sorted places 60 -> 49 us, 8192 rows of which a shard wants two thirds 82 -> 40 us.  Every bf16 and fp16 pair of maximum and element is compared with the library's division in the tests; fp32 elements keep it.
+// calls it; the ones without a group (the last block's, absent tokens') give zeros for the maximum and get no codes: zeros over a
+// scale of zero or of eps take the longest way through the library's division, which made 1 x 7168 fp32 3.2 us instead of 1.9.
+// Two-byte types take the quotient from the refined reciprocal wherever the scale is finite and not near the ends of the range
+// (all but groups with an infinity or, with a tiny eps, of next to nothing).  The codes are those of the IEEE quotient: every pair
+// of maximum and element of bf16 and fp16 is compared with the library's division in the tests; fp32 elements keep that one.
+// With the library's division and eight elements a thread the kernels were bound by their instructions: 4096 x 7168 bf16 alone
+// 33 -> 22 us (the bytes take 14), into eight sorted places 60 -> 49, 8192 rows of which a shard wants two thirds 82 -> 40.
 template <typename T, int LANES>
-__device__ __forceinline__ float quantise16(const float (&v)[16], float eps_t, uint32_t (&packed)[4]) {
+__device__ __forceinline__ float quantise16(const float (&v)[16], float eps_t, bool active, uint32_t (&packed)[4]) {
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
 #pragma unroll
   for (int off = LANES / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  if (!active) return 0.f;
   const float scale = __fdiv_rn(fmaxf(amax, eps_t), 127.0f);
   const bool plain = sizeof(T) == 2 && scale >= 1e-30f && scale <= 1e37f;
   if (plain) {
@@ -110,7 +114,7 @@ __global__ void __launch_bounds__(256) group_quant_kernel(const T *__restrict__ 
     for (int i = 0; i < 16; ++i) v[i] = 0.f;
   }
   uint32_t packed[4];
-  const float scale = quantise16<T, LANES>(v, eps_t, packed);
+  const float scale = quantise16<T, LANES>(v, eps_t, active, packed);
   if (!active) return;
   int8_t *dst = q + gthread * 16;
   if (q16) {
@@ -153,7 +157,7 @@ __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfl
   }
   if (!__any_sync(0xffffffffu, wanted)) return;          // (an exited block counts as released for the dependent launch)
   uint32_t packed[4];
-  const float scale = quantise16<__nv_bfloat16, 8>(v, eps_t, packed);
+  const float scale = quantise16<__nv_bfloat16, 8>(v, eps_t, wanted, packed);
   // everything above reads the caller's activations only; the positions come from the align kernel before this one
   if (!some_absent) dependency_wait();
   dependency_release();

@@ -51,3 +51,12 @@ def test_silu_quantiser_loads_no_row_that_does_not_exist():
     first_load = next(i for i, s in enumerate(st) if s == "gv[v] = g[i]")
     assert any(s.startswith("if (num_rows_dev && row >= *num_rows_dev) return") for s in st[:first_load])
     assert any(s.startswith("if (group_counts && row % group_rows >= group_counts[row / group_rows]) return") for s in st[:first_load])
+
+
+def test_lanes_without_a_group_take_no_quotient():
+    # they join the group's maximum and return before the first division (theirs would be the slowest one of the warp)
+    st = _statements("quant.cu")
+    start = next(i for i, s in enumerate(st) if "float quantise" in s)
+    leave = next(i for i in range(start, len(st)) if st[i].startswith("if (!active) return"))
+    assert any("__shfl_xor_sync" in s for s in st[start:leave])
+    assert not any("__fdiv_rn" in s or "div_by" in s for s in st[start:leave])
