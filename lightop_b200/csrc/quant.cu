@@ -5,8 +5,8 @@
 //   amax  = max |x| over the group, clamped from below by eps rounded to x's type
 //   scale = amax / 127                 (IEEE fp32 division)
 //   q     = trunc(clamp(x / scale, -128, 127))   (IEEE fp32 division, then round toward zero)
-// Memory-bound streaming kernel: LANES lanes own one group, each lane moves 32
-// bytes of 2-byte input (or 64 bytes of fp32) and stores 16 int8.
+// Memory-bound streaming kernel: a few lanes own one group, each lane moves 32 bytes of
+// input (64 of fp32 in large calls) and stores as many int8 as it has elements.
 #include "common.h"
 
 namespace lo {
@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t pack4_rz(const float (&r)[4]) {
   return lo;
 }
 
-// A thread's sixteen elements of a group of LANES x 16: maximum over the group's lanes, scale, codes.  Every lane of the warp
+// A thread's N elements (16 or 8) of a group of LANES x N: maximum over the group's lanes, scale, codes.  Every lane of the warp
 // calls it; the ones without a group (the last block's, absent tokens') give zeros for the maximum and get no codes: zeros over a
 // scale of zero or of eps take the longest way through the library's division, which made 1 x 7168 fp32 3.2 us instead of 1.9.
 // Two-byte types take the quotient from the refined reciprocal wherever the scale is finite and not near the ends of the range
@@ -64,11 +64,11 @@ __device__ __forceinline__ uint32_t pack4_rz(const float (&r)[4]) {
 // of maximum and element of bf16 and fp16 is compared with the library's division in the tests; fp32 elements keep that one.
 // With the library's division and eight elements a thread the kernels were bound by their instructions: 4096 x 7168 bf16 alone
 // 33 -> 22 us (the bytes take 14), into eight sorted places 60 -> 49, 8192 rows of which a shard wants two thirds 82 -> 40.
-template <typename T, int LANES>
-__device__ __forceinline__ float quantise16(const float (&v)[16], float eps_t, bool active, uint32_t (&packed)[4]) {
+template <typename T, int LANES, int N>
+__device__ __forceinline__ float quantise(const float (&v)[N], float eps_t, bool active, uint32_t (&packed)[N / 4]) {
   float amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  for (int i = 0; i < N; ++i) amax = fmaxf(amax, fabsf(v[i]));
 #pragma unroll
   for (int off = LANES / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
   if (!active) return 0.f;
@@ -77,7 +77,7 @@ __device__ __forceinline__ float quantise16(const float (&v)[16], float eps_t, b
   if (plain) {
     const float y = rcp_refined(scale);
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int w = 0; w < N / 4; ++w) {
       float r[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) r[i] = div_by(v[4 * w + i], scale, y);
@@ -85,7 +85,7 @@ __device__ __forceinline__ float quantise16(const float (&v)[16], float eps_t, b
     }
   } else {
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int w = 0; w < N / 4; ++w) {
       float r[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) r[i] = __fdiv_rn(v[4 * w + i], scale);
@@ -95,8 +95,9 @@ __device__ __forceinline__ float quantise16(const float (&v)[16], float eps_t, b
   return scale;
 }
 
-// LANES lanes x 16 elements = one group.  (16 elements a thread halve the shuffles and the address arithmetic an element costs.)
-template <typename T, int LANES>
+// LANES lanes x N elements = one group.  Sixteen elements a thread halve the shuffles and the address arithmetic an element costs;
+// fp32, which the library's division binds in either form, has twice the warps with eight: see launch_group_quant().
+template <typename T, int LANES, int N>
 __global__ void __launch_bounds__(256) group_quant_kernel(const T *__restrict__ x, int8_t *__restrict__ q,
                                                           float *__restrict__ s, int64_t num_groups,
                                                           float eps_t, int q16) {
@@ -105,23 +106,25 @@ __global__ void __launch_bounds__(256) group_quant_kernel(const T *__restrict__ 
   const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t group = gthread / LANES;
   const bool active = group < num_groups;
-  float v[16];
-  if (active) {
-    Load8<T>::load(x + gthread * 16, *reinterpret_cast<float (*)[8]>(&v[0]));
-    Load8<T>::load(x + gthread * 16 + 8, *reinterpret_cast<float (*)[8]>(&v[8]));
+  float v[N];
+#pragma unroll
+  for (int i = 0; i < N; i += 8) {
+    float (&part)[8] = *reinterpret_cast<float (*)[8]>(&v[i]);
+    if (active) Load8<T>::load(x + gthread * N + i, part);
+    else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) part[j] = 0.f;
+    }
+  }
+  uint32_t packed[N / 4];
+  const float scale = quantise<T, LANES, N>(v, eps_t, active, packed);
+  if (!active) return;
+  int8_t *dst = q + gthread * N;
+  if (N == 16 && q16) {
+    *reinterpret_cast<uint4 *>(dst) = make_uint4(packed[0], packed[1], packed[N / 4 - 2], packed[N / 4 - 1]);
   } else {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = 0.f;
-  }
-  uint32_t packed[4];
-  const float scale = quantise16<T, LANES>(v, eps_t, active, packed);
-  if (!active) return;
-  int8_t *dst = q + gthread * 16;
-  if (q16) {
-    *reinterpret_cast<uint4 *>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-  } else {
-    *reinterpret_cast<uint2 *>(dst) = make_uint2(packed[0], packed[1]);
-    *reinterpret_cast<uint2 *>(dst + 8) = make_uint2(packed[2], packed[3]);
+    for (int w = 0; w < N / 4; w += 2) *reinterpret_cast<uint2 *>(dst + 4 * w) = make_uint2(packed[w], packed[w + 1]);
   }
   if (gthread % LANES == 0) s[group] = scale;
 }
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfl
   }
   if (!__any_sync(0xffffffffu, wanted)) return;          // (an exited block counts as released for the dependent launch)
   uint32_t packed[4];
-  const float scale = quantise16<__nv_bfloat16, 8>(v, eps_t, wanted, packed);
+  const float scale = quantise<__nv_bfloat16, 8, 16>(v, eps_t, wanted, packed);
   // everything above reads the caller's activations only; the positions come from the align kernel before this one
   if (!some_absent) dependency_wait();
   dependency_release();
@@ -373,22 +376,24 @@ __global__ void __launch_bounds__(SILU_THREADS) silu_mul_token_quant_kernel(
   }
 }
 
-template <typename T>
+template <typename T, int N>
 int launch_typed(const void *x, int64_t num_groups, int group_size, float eps_t, int8_t *q, float *s,
                  cudaStream_t stream) {
-  const int lanes = group_size / 16;
+  const int lanes = group_size / N;
   const int threads = 256;
   const int64_t total_threads = num_groups * lanes;
   const int64_t blocks = ceil_div(total_threads, threads);
   if (blocks > 0x7fffffffLL) return fail(LO_ERR_INVALID_ARGUMENT, "group quant: too many groups");
   const T *xp = static_cast<const T *>(x);
   const int q16 = (reinterpret_cast<uintptr_t>(q) & 15) == 0 ? 1 : 0;      // (the caller's q may begin on 8 bytes only)
+  auto kernel = group_quant_kernel<T, 128 / N, N>;
   switch (group_size) {
-    case 64: LO_CUDA_OK(launch_dependent(group_quant_kernel<T, 4>, dim3((unsigned)blocks), dim3(threads), 0, stream, xp, q, s, num_groups, eps_t, q16)); break;
-    case 128: LO_CUDA_OK(launch_dependent(group_quant_kernel<T, 8>, dim3((unsigned)blocks), dim3(threads), 0, stream, xp, q, s, num_groups, eps_t, q16)); break;
-    case 256: LO_CUDA_OK(launch_dependent(group_quant_kernel<T, 16>, dim3((unsigned)blocks), dim3(threads), 0, stream, xp, q, s, num_groups, eps_t, q16)); break;
+    case 64: kernel = group_quant_kernel<T, 64 / N, N>; break;
+    case 128: break;
+    case 256: kernel = group_quant_kernel<T, 256 / N, N>; break;
     default: return fail(LO_ERR_UNSUPPORTED, "group quant: group_size %d not in {64,128,256}", group_size);
   }
+  LO_CUDA_OK(launch_dependent(kernel, dim3((unsigned)blocks), dim3(threads), 0, stream, xp, q, s, num_groups, eps_t, q16));
   return LO_OK;
 }
 
@@ -415,13 +420,19 @@ int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, co
   return LO_OK;
 }
 
+constexpr int64_t FP32_SMALL = 1 << 24;
 int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group_size, float eps, int8_t *q, float *s,
                        cudaStream_t st) {
   const float eps_t = round_eps_to_dtype(eps, x_dtype);
   switch (x_dtype) {
-    case LO_BF16: return launch_typed<__nv_bfloat16>(x, num_groups, group_size, eps_t, q, s, st);
-    case LO_F16: return launch_typed<__half>(x, num_groups, group_size, eps_t, q, s, st);
-    case LO_F32: return launch_typed<float>(x, num_groups, group_size, eps_t, q, s, st);
+    case LO_BF16: return launch_typed<__nv_bfloat16, 16>(x, num_groups, group_size, eps_t, q, s, st);
+    case LO_F16: return launch_typed<__half, 16>(x, num_groups, group_size, eps_t, q, s, st);
+    case LO_F32:
+      // Eight elements a thread up to 2^24 elements, sixteen above (the input no longer stays in L2, loads count more than warps).
+      // Eight, sixteen, us: 257 x 7168 2.8, 3.8; 1024 x 2048 2.9, 4.0; 1024 x 7168 5.9, 6.3; 4096 x 2048 6.6, 6.9; 4096 x 7168 23.9,
+      // 22.9 (from HBM 32.8, 30.9).
+      return num_groups * group_size <= FP32_SMALL ? launch_typed<float, 8>(x, num_groups, group_size, eps_t, q, s, st)
+                                                   : launch_typed<float, 16>(x, num_groups, group_size, eps_t, q, s, st);
     default: return fail(LO_ERR_UNSUPPORTED, "group quant: unsupported input dtype code %d", x_dtype);
   }
 }

@@ -75,6 +75,21 @@ def test_group_quant_codes_that_begin_on_eight_bytes(lo):
     assert not room[:8].any() and not room[-8:].any()
 
 
+@pytest.mark.parametrize("group", [64, 128, 256])
+def test_group_quant_fp32_on_both_sides_of_the_wide_form(lo, group):
+    """Eight elements a thread up to 2^24 elements, sixteen above: a large call has the bits of its parts."""
+    K = 7168
+    x = torch.randn(2341, K, generator=torch.Generator(device=DEV).manual_seed(group), device=DEV)
+    x[5, :group] = 0
+    assert x.numel() > 1 << 24 and x[:2340].numel() <= 1 << 24
+    q, s = lo.quant.per_token_group_quant_int8(x, group)
+    for part in (slice(0, 2340), slice(2333, 2341)):
+        q2, s2 = lo.quant.per_token_group_quant_int8(x[part], group)
+        assert torch.equal(q[part], q2) and torch.equal(s[part], s2)
+    q_ref, s_ref = O.group_quant_int8(x[:9].cpu(), group)
+    assert torch.equal(q[:9].cpu(), q_ref) and torch.equal(s[:9].cpu(), s_ref)
+
+
 def test_silu_quant_every_gate(lo):
     """Every bf16 gate, with eight of one magnitude range to a row so that small results keep their codes."""
     gates = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).to(DEV)
