@@ -271,9 +271,13 @@ __global__ void __launch_bounds__(TOKEN_QUANT_THREADS) token_quant_kernel(const 
 // the SiLU: act = bf16(bf16(silu(gate)) * up); scale = max|act| / 127; q = rint(act * (127 / max)),
 // saturated; a row of zeros gets scale 0 and q 0.  Rows whose entry in row_ids is a padding
 // sentinel (< 0 or >= numel_valid) are skipped.
-// 128 threads a row, and a row's loads are on their way before anything is looked up for it: with 256 threads, the library's
-// division and the loads behind the look-ups a row's chain of latencies bound it: 24 000 rows of 2048 channels 139 us, now 99 (the
-// bytes take 38; what bounds it now are the instructions, an exponential and an exact quotient per element).
+// A row's loads are on their way before its id is looked up: with the library's division and the loads behind the look-ups a row's
+// chain of latencies bound it: 24 000 rows of 2048 channels 139 us, now 99 (the bytes take 38; what bounds it now are the
+// instructions, an exponential and an exact quotient per element).  Threads a row, in us with 128 and 256:
+//   1 x 2048: 2.4, 2.1    148 x 4096: 3.2, 2.7    296 x 1408: 2.6, 2.4    444 x 1408: 2.7, 3.1    2368 x 2048: 8.4, 10.0
+//   64 x 8192: 7.6, 3.5    4000 x 8192: 79, 45    16 x 18432: 15.0, 9.9    2000 x 18432: 94, 93
+// 256 up to two rows a SM, where a row's chain is all there is, and for rows of more than 4096 channels, half of which would not
+// stay in the registers of 128; 128 else, where the blocks fill the SMs and fewer warps wait at a row's barrier.
 // ---------------------------------------------------------------------------
 
 // g / (1 + exp(-g)), the IEEE quotient: the refined reciprocal is taken of the denominator times 2^-32, which keeps the
@@ -312,12 +316,13 @@ __device__ __forceinline__ uint2 quant8_bf16(const uint4 &a, float inv) {
   return quant8_rn(v, inv);
 }
 
-constexpr int SILU_THREADS = 128, SILU_VECS = 4;      // vectors of eight channels a thread keeps: rows of up to 4096 channels
-__global__ void __launch_bounds__(SILU_THREADS) silu_mul_token_quant_kernel(
+constexpr int SILU_VECS = 4;      // vectors of eight channels a thread keeps: rows of up to 32 channels a thread stay in registers
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) silu_mul_token_quant_kernel(
     const __nv_bfloat16 *__restrict__ in, int64_t d, const int32_t *__restrict__ row_ids, int64_t numel_valid,
     const int32_t *__restrict__ num_rows_dev, int64_t group_rows, const int32_t *__restrict__ group_counts,
     int8_t *__restrict__ q, float *__restrict__ s) {
-  __shared__ float red[SILU_THREADS / 32];
+  __shared__ float red[THREADS / 32];
   const int64_t row = blockIdx.x;
   dependency_wait();
   dependency_release();
@@ -329,12 +334,12 @@ __global__ void __launch_bounds__(SILU_THREADS) silu_mul_token_quant_kernel(
   const uint4 *g = reinterpret_cast<const uint4 *>(in + row * 2 * d);
   const int64_t vecs = d / 8;
   const uint4 *u = g + vecs;
-  const bool kept = vecs <= SILU_VECS * SILU_THREADS;      // the row's activations stay in registers
+  const bool kept = vecs <= SILU_VECS * THREADS;      // the row's activations stay in registers
   uint4 gv[SILU_VECS], uv[SILU_VECS];
   if (kept) {
 #pragma unroll
     for (int v = 0; v < SILU_VECS; ++v) {
-      const int64_t i = threadIdx.x + v * SILU_THREADS;
+      const int64_t i = threadIdx.x + v * THREADS;
       if (i < vecs) {
         gv[v] = g[i];
         uv[v] = u[i];
@@ -349,27 +354,29 @@ __global__ void __launch_bounds__(SILU_THREADS) silu_mul_token_quant_kernel(
   if (kept) {
 #pragma unroll
     for (int v = 0; v < SILU_VECS; ++v) {
-      if (threadIdx.x + v * SILU_THREADS < vecs) gv[v] = act8(gv[v], uv[v], amax);
+      if (threadIdx.x + v * THREADS < vecs) gv[v] = act8(gv[v], uv[v], amax);
     }
   } else {
-    for (int64_t i = threadIdx.x; i < vecs; i += SILU_THREADS) act8(g[i], u[i], amax);
+    for (int64_t i = threadIdx.x; i < vecs; i += THREADS) act8(g[i], u[i], amax);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
   __syncthreads();
-  amax = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+  amax = red[0];
+#pragma unroll
+  for (int w = 1; w < THREADS / 32; ++w) amax = fmaxf(amax, red[w]);
   const float inv = amax == 0.f ? 0.f : __fdiv_rn(127.0f, amax);
   if (threadIdx.x == 0) s[row] = __fdiv_rn(amax, 127.0f);
   uint2 *dst = reinterpret_cast<uint2 *>(q + row * d);
   if (kept) {
 #pragma unroll
     for (int v = 0; v < SILU_VECS; ++v) {
-      const int64_t i = threadIdx.x + v * SILU_THREADS;
+      const int64_t i = threadIdx.x + v * THREADS;
       if (i < vecs) dst[i] = quant8_bf16(gv[v], inv);
     }
   } else {
-    for (int64_t i = threadIdx.x; i < vecs; i += SILU_THREADS) {
+    for (int64_t i = threadIdx.x; i < vecs; i += THREADS) {
       float again = 0.f;
       dst[i] = quant8_bf16(act8(g[i], u[i], again), inv);
     }
@@ -466,7 +473,8 @@ int launch_silu_mul_token_quant(const void *in, int64_t rows, int64_t d, const i
   if (rows == 0) return LO_OK;
   LO_REQUIRE(d >= 8 && d % 8 == 0, "silu-mul quant: width %lld must be a multiple of 8", (long long)d);
   LO_REQUIRE(rows <= 0x7fffffffLL, "silu-mul quant: too many rows");
-  LO_CUDA_OK(launch_dependent(silu_mul_token_quant_kernel, dim3((unsigned)rows), dim3(SILU_THREADS), 0, stream,
+  const bool wide = d > 128 * 8 * SILU_VECS || rows <= 2 * (int64_t)sm_count();
+  LO_CUDA_OK(launch_dependent(wide ? silu_mul_token_quant_kernel<256> : silu_mul_token_quant_kernel<128>, dim3((unsigned)rows), dim3(wide ? 256 : 128), 0, stream,
                               static_cast<const __nv_bfloat16 *>(in), d, row_ids, numel_valid, num_rows_dev,
                               group_rows > 0 ? group_rows : (int64_t)1, group_counts, q, s));
   return LO_OK;

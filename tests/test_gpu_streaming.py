@@ -109,6 +109,22 @@ def test_silu_quant_every_gate(lo):
     assert torch.equal(q.view_as(want), want)
 
 
+# both numbers of threads a row (by rows and by width), widths that fill the last vector a thread keeps in part, and rows too wide to
+# be kept, which are read and evaluated twice
+@pytest.mark.parametrize("rows,d", [(3, 8), (3, 1544), (700, 1544), (700, 4096), (5, 4104), (700, 4104), (5, 8192), (3, 8200), (310, 8200), (2, 18432)])
+def test_silu_quant_widths(lo, rows, d):
+    g = torch.Generator(device=DEV).manual_seed(rows + d)
+    x = (torch.randn(rows, 2 * d, generator=g, device=DEV) * 4).to(torch.bfloat16)
+    x[1] = 0
+    q, s = lo.activation.fuse_silu_mul_quant(x)
+    gate, up = x[:, :d].float(), x[:, d:].float()
+    act = ((gate / (1.0 + torch.exp(-gate))).to(torch.bfloat16).float() * up).to(torch.bfloat16).float()
+    amax = act.abs().amax(-1, keepdim=True)
+    r = act * torch.where(amax == 0, torch.zeros((), device=DEV), torch.full_like(amax, 127.0) / amax)
+    assert torch.equal(s.view(-1, 1), amax / torch.full_like(amax, 127.0))
+    assert torch.equal(q, r.round().clamp(-128, 127).to(torch.int8))
+
+
 # blocks of one vector a thread up to eight blocks a SM, of four above: both sides of the line, columns that do not fill the last
 # pass, slots that are all, some or not there, more than 32 of them
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
