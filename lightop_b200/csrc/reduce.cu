@@ -440,10 +440,14 @@ __global__ void __launch_bounds__(256) ep_gather_kernel(const __nv_bfloat16 *__r
   }
 }
 
-// One warp per sorted position: copy the int8 row and its scales of token sorted_ids[pos] / top_k.  What a position's row depends on
+// WPR warps per sorted position: copy the int8 row and its scales of token sorted_ids[pos] / top_k.  What a position's row depends on
 // is loaded at once, and a lane has four 16-byte loads of the row in flight.  (A block of 128 threads a position, with a load of
 // the count, one of the id and one of the row behind one another, took 13.7 us for 2400 rows of 4096 bytes.)
+// One warp a position where the positions fill the GPU, four (rows of 8192 bytes in one round of loads) where there are too few to
+// hide a row's rounds behind one another's.  Copy and a small GEMM, one and four warps, us: 64 positions of 16384 bytes 31.4, 30.1;
+// 152 of 7168 17.3, 16.5; 992 of 7168 19.9, 18.4; 992 of 2048 10.0, 9.8; 1504 of 7168 19.3, 19.6; 4320 of 1536 12.9, 15.5.
 constexpr int PERMUTE_WARPS = 4;
+template <int WPR>
 __global__ void __launch_bounds__(PERMUTE_WARPS * 32) permute_rows_kernel(const int8_t *__restrict__ A, const float *__restrict__ a_scale,
                                                            int64_t rows_a, int64_t K, const int32_t *__restrict__ sorted_ids, int64_t positions,
                                                            const int32_t *__restrict__ num_tokens_post_pad,
@@ -452,8 +456,9 @@ __global__ void __launch_bounds__(PERMUTE_WARPS * 32) permute_rows_kernel(const 
                                                            float *__restrict__ a_scale_sorted, int64_t a_stride,
                                                            const int32_t *__restrict__ expert_ids, int block_size,
                                                            Chunk *__restrict__ chunks, int32_t *__restrict__ num_chunks) {
-  const int64_t pos = (int64_t)blockIdx.x * PERMUTE_WARPS + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+  constexpr int LANES = 32 * WPR;
+  const int64_t pos = (int64_t)blockIdx.x * (PERMUTE_WARPS / WPR) + threadIdx.x / LANES;
+  const int lane = threadIdx.x % LANES;
   dependency_wait();
   dependency_release();
   if (pos >= positions) return;
@@ -484,16 +489,16 @@ __global__ void __launch_bounds__(PERMUTE_WARPS * 32) permute_rows_kernel(const 
   const float *src_s = a_scale ? a_scale + row * kb : reinterpret_cast<const float *>(A + row * a_stride + K);
   uint4 *dst = reinterpret_cast<uint4 *>(A_sorted + pos * K);
   const int n = (int)(K / 16);
-  for (int c = lane; c < n; c += 128) {
+  for (int c = lane; c < n; c += 4 * LANES) {
     uint4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (c + 32 * u < n) v[u] = src[c + 32 * u];
+      if (c + LANES * u < n) v[u] = src[c + LANES * u];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (c + 32 * u < n) dst[c + 32 * u] = v[u];
+      if (c + LANES * u < n) dst[c + LANES * u] = v[u];
   }
-  for (int64_t c = lane; c < kb; c += 32) a_scale_sorted[pos * kb + c] = src_s[c];
+  for (int64_t c = lane; c < kb; c += LANES) a_scale_sorted[pos * kb + c] = src_s[c];
 }
 
 }  // namespace
@@ -504,7 +509,9 @@ int launch_permute_rows(const int8_t *A, const float *a_scale, int64_t rows_a, i
                         int64_t a_stride, const int32_t *expert_ids, int block_size, Chunk *chunks, int32_t *num_chunks) {
   if (sorted_capacity <= 0) return LO_OK;
   LO_REQUIRE(sorted_capacity <= 0x7fffffffLL, "permute rows: too many positions");
-  LO_CUDA_OK(launch_dependent(permute_rows_kernel, dim3((unsigned)ceil_div(sorted_capacity, PERMUTE_WARPS)), dim3(PERMUTE_WARPS * 32), 0, stream, A, a_scale, rows_a, K,
+  const bool few = sorted_capacity <= 8 * (int64_t)sm_count();
+  LO_CUDA_OK(launch_dependent(few ? permute_rows_kernel<4> : permute_rows_kernel<1>, dim3((unsigned)(few ? sorted_capacity : ceil_div(sorted_capacity, PERMUTE_WARPS))),
+                              dim3(PERMUTE_WARPS * 32), 0, stream, A, a_scale, rows_a, K,
                               sorted_ids, sorted_capacity, num_tokens_post_pad, numel_valid, top_k, scales_per_row > 0 ? scales_per_row : K / 128, A_sorted,
                               a_scale_sorted, a_stride > 0 ? a_stride : K, expert_ids, block_size, chunks, num_chunks));
   return LO_OK;

@@ -174,3 +174,31 @@ def test_layer_of_a_shard_passes_over_tokens_without_a_local_expert(lo, M):
                                        block_shape=[128, 128], w1_scale=w1_s, w2_scale=w2_s)
     # every row once in each: the parts are rounded to bf16 where the whole is rounded once
     assert float((total - y.double()).norm() / y.double().norm()) < 2 ** -8
+
+
+# four warps copy a position's row up to eight positions a SM, one above: the same ids in front of more positions that do not exist
+@pytest.mark.parametrize("K", [128, 1152, 8192, 16384])
+@pytest.mark.parametrize("channel", [True, False])
+def test_row_copy_on_both_sides_of_the_number_of_warps(lo, K, channel):
+    M, E, k, N = 40, 4, 2, 128
+    g = torch.Generator(device=DEV).manual_seed(K)
+    ids = torch.rand(M, E, generator=g, device=DEV).topk(k, dim=1).indices.to(torch.int32)
+    aq = torch.randint(-127, 128, (M, K), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (E, N, K), generator=g, device=DEV, dtype=torch.int8)
+    a_s = torch.rand(M, 1 if channel else K // 128, generator=g, device=DEV) + 0.5
+    w_s = torch.rand(E, N if channel else 1, 1 if channel else K // 128, generator=g, device=DEV) + 0.5
+    sorted_ids, expert_ids, num_post = lo.moe.moe_align_block_size(ids, 16, E)
+    outs = []
+    for more in (0, 1600):
+        s = torch.cat([sorted_ids, sorted_ids.new_full((more,), M * k)])
+        e = torch.cat([expert_ids, expert_ids.new_zeros(more // 16)])
+        out = torch.full((M, k, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        lo.moe.moe_gemm_w8a8(aq, w, out, a_s, w_s, None, s, e, num_post, k, {"BLOCK_SIZE_M": 16})
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    # the whole sum of a row, with the scales as they are in exact arithmetic
+    want = torch.stack([(aq.double().view(M, -1, K // a_s.shape[1]) * a_s.double()[..., None]).view(M, K) @
+                        (w[e].double().view(N, -1, K // w_s.shape[2]) * w_s[e].double()[..., None]).view(N, K).t() for e in range(E)], 1)
+    want = torch.gather(want, 1, ids.long()[..., None].expand(M, k, N))
+    # K / 128 fp32 products and sums, then one rounding to bf16
+    assert float((outs[0].double() - want).norm() / want.norm()) < 2 ** -8
