@@ -78,10 +78,10 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
                  int chunk_max, cudaStream_t stream);
 
 // Group quantisation of bf16 rows [M, H] written straight into the expert-sorted layout:
-// the int8 row and its scales of token t go to every position inv_pos[t * topk + j] >= 0.  some_absent: tokens without any
-// position are to be expected (an expert map), and are not read.  quant.cu
+// the int8 row and its scales of token t go to every position inv_pos[t * topk + j] >= 0.  positions_first: the rows
+// of tokens without any position are not read, at the price of waiting for the alignment first (same results).  quant.cu
 int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, const int32_t *inv_pos, float eps,
-                               int8_t *q_sorted, float *s_sorted, bool some_absent, cudaStream_t stream);
+                               int8_t *q_sorted, float *s_sorted, bool positions_first, cudaStream_t stream);
 
 // Group quantisation of rows of any supported type, for a dependent launch of the kernel that follows.  quant.cu
 int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group_size, float eps, int8_t *q, float *s,

@@ -130,13 +130,13 @@ __global__ void __launch_bounds__(256) group_quant_kernel(const T *__restrict__ 
 }
 
 // bf16 rows [M, H], group 128: quantise once, store to each of the token's sorted positions.
-// Without an expert map every token has positions: the rows are loaded and quantised while the alignment kernel is still at
-// work.  With one (`some_absent`) tokens may have none, and those are passed over: the positions are read first.
+// The rows are loaded and quantised while the alignment kernel is still at work.  Where many tokens are to be expected without any
+// position (`positions_first`), the positions are read before that and those tokens' rows are passed over.
 __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfloat16 *__restrict__ x, int64_t M,
                                                                   int groups_per_row, int topk,
                                                                   const int32_t *__restrict__ inv_pos, float eps_t,
                                                                   int8_t *__restrict__ q_sorted,
-                                                                  float *__restrict__ s_sorted, int some_absent) {
+                                                                  float *__restrict__ s_sorted, int positions_first) {
   const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t group = (uint32_t)(gthread / 8);            // (2^32 groups would be a terabyte of activations)
   const uint32_t row = group / (uint32_t)groups_per_row;
@@ -144,9 +144,9 @@ __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfl
   const int64_t token = row;
   const bool active = token < M;
   const int32_t *pos_of = inv_pos + token * topk;
-  if (some_absent) dependency_wait();
+  if (positions_first) dependency_wait();
   bool wanted = active;
-  if (some_absent && active) {
+  if (positions_first && active) {
     wanted = false;
     for (int j = 0; j < topk; ++j) wanted |= pos_of[j] >= 0;
   }
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfl
   uint32_t packed[4];
   const float scale = quantise<__nv_bfloat16, 8, 16>(v, eps_t, wanted, packed);
   // everything above reads the caller's activations only; the positions come from the align kernel before this one
-  if (!some_absent) dependency_wait();
+  if (!positions_first) dependency_wait();
   dependency_release();
   if (!wanted) return;
   const uint4 codes = make_uint4(packed[0], packed[1], packed[2], packed[3]);
@@ -415,7 +415,7 @@ float round_eps_to_dtype(float eps, int dtype) {
 }
 
 int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, const int32_t *inv_pos, float eps,
-                               int8_t *q_sorted, float *s_sorted, bool some_absent, cudaStream_t stream) {
+                               int8_t *q_sorted, float *s_sorted, bool positions_first, cudaStream_t stream) {
   if (M == 0) return LO_OK;
   LO_REQUIRE(H % 128 == 0, "group quant: hidden size must be a multiple of 128");
   const int64_t total_threads = M * (H / 128) * 8;
@@ -423,7 +423,7 @@ int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, co
   LO_REQUIRE(blocks <= 0x7fffffffLL, "group quant: too many groups");
   LO_CUDA_OK(launch_dependent(group_quant_scatter_kernel, dim3((unsigned)blocks), dim3(256), 0, stream,
                               static_cast<const __nv_bfloat16 *>(x), M, (int)(H / 128), topk, inv_pos,
-                              round_eps_to_dtype(eps, LO_BF16), q_sorted, s_sorted, some_absent ? 1 : 0));
+                              round_eps_to_dtype(eps, LO_BF16), q_sorted, s_sorted, positions_first ? 1 : 0));
   return LO_OK;
 }
 

@@ -202,3 +202,25 @@ def test_row_copy_on_both_sides_of_the_number_of_warps(lo, K, channel):
     want = torch.gather(want, 1, ids.long()[..., None].expand(M, k, N))
     # K / 128 fp32 products and sums, then one rounding to bf16
     assert float((outs[0].double() - want).norm() / want.norm()) < 2 ** -8
+
+
+def test_layer_of_a_shard_reads_positions_or_rows_first(lo, monkeypatch):
+    """One expert of eight is local and the absent tokens' rows are more than 8 MB: positions first.  The same tokens in smaller calls:
+    rows first.  Every row has the same bits."""
+    from lightop_b200 import synthetic
+    M, E, k, H, I = 11003, 8, 2, 512, 128
+    w1, w2, w1_s, w2_s = synthetic.make_weights(E, H, I, seed=3, device=DEV)
+    x, logits = synthetic.make_activations(M, H, E, seed=4, device=DEV)
+    weights = torch.empty(M, k, device=DEV)
+    ids = torch.empty(M, k, dtype=torch.int32, device=DEV)
+    lo.moe.topk_softmax(weights, ids, None, logits, True)
+    emap = torch.full((E,), -1, dtype=torch.int32, device=DEV)
+    emap[3] = 0
+
+    def layer():
+        return lo.moe.fused_experts_impl_int8(x, w1[3:4].contiguous(), w2[3:4].contiguous(), weights, ids, None, use_int8_w8a8=True, block_shape=[128, 128],
+                                              w1_scale=w1_s[3:4].contiguous(), w2_scale=w2_s[3:4].contiguous(), global_num_experts=E, expert_map=emap)
+    y = layer()
+    assert not y[~(ids == 3).any(1)].any() and bool(y[(ids == 3).any(1)].any(1).all())
+    monkeypatch.setenv("LMSLIM_FUSED_MOE_CHUNK_SIZE", "2999")
+    assert torch.equal(layer(), y)
