@@ -71,10 +71,12 @@ __global__ void __launch_bounds__(256, VPT == 4 && sizeof(T) == 2 ? 3 : 1) moe_s
                                                       float factor, const uint8_t *__restrict__ mask,
                                                       const int32_t *__restrict__ num_local_tokens,
                                                       const IdT *__restrict__ ids, const int32_t *__restrict__ expert_map,
-                                                      int num_experts, int num_local) {
+                                                      int num_experts, int num_local, uint32_t per_token) {
   using V = Vec8<T>;
   constexpr int ROWS = VPT == 1 ? 8 : 2;      // rows in flight
-  const int64_t t = blockIdx.y;
+  // `per_token` blocks a token, next to one another in one dimension of the grid (the others end at 65535)
+  const uint32_t token = blockIdx.x / per_token, part = blockIdx.x - token * per_token;
+  const int64_t t = token;
   const int lane = threadIdx.x & 31;
   dependency_wait();            // the rows come from the kernel before this one
   dependency_release();
@@ -98,7 +100,7 @@ __global__ void __launch_bounds__(256, VPT == 4 && sizeof(T) == 2 ? 3 : 1) moe_s
   };
   const unsigned first = live_slots(0);
   const V *in_v = reinterpret_cast<const V *>(in) + t * topk * H8;
-  for (int64_t c0 = (int64_t)blockIdx.x * (blockDim.x * VPT); c0 < H8; c0 += (int64_t)gridDim.x * (blockDim.x * VPT)) {
+  for (int64_t c0 = (int64_t)part * (blockDim.x * VPT); c0 < H8; c0 += (int64_t)per_token * (blockDim.x * VPT)) {
     float acc[VPT][8];
     V b[VPT];
 #pragma unroll
@@ -170,12 +172,12 @@ int launch_sum(const void *in, void *out, const void *bias, int64_t M, int topk,
   // Four vectors a thread where slots may be missing and the blocks of one vector a thread would not all be on the GPU at once
   // (eight a SM).  With every slot there one vector a thread has as many loads in flight and more warps (2999 tokens of 8 slots: 93 against 100 us).
   const bool wide = (mask != nullptr || expert_map != nullptr) && M * narrow > 8 * (int64_t)sm_count();
-  const int64_t per_row = wide ? ceil_div(H8, 1024) : narrow;
-  dim3 grid((unsigned)(per_row > 65535 ? 65535 : per_row), (unsigned)M);
+  const int64_t per_token = wide ? ceil_div(H8, 1024) : narrow;
+  LO_REQUIRE(M * per_token <= 0x7fffffffLL, "moe_sum: too many tokens");
   auto kernel = wide ? moe_sum_kernel<T, IdT, 4> : moe_sum_kernel<T, IdT, 1>;
-  LO_CUDA_OK(launch_dependent(kernel, grid, dim3(256), 0, st, static_cast<const T *>(in),
+  LO_CUDA_OK(launch_dependent(kernel, dim3((unsigned)(M * per_token)), dim3(256), 0, st, static_cast<const T *>(in),
                               static_cast<T *>(out), static_cast<const T *>(bias), M, topk, H8, factor, mask, nlt,
-                              static_cast<const IdT *>(ids), expert_map, num_experts, num_local));
+                              static_cast<const IdT *>(ids), expert_map, num_experts, num_local, (uint32_t)per_token));
   return LO_OK;
 }
 
@@ -417,10 +419,11 @@ template <typename IdT>
 __global__ void __launch_bounds__(256) ep_gather_kernel(const __nv_bfloat16 *__restrict__ a, const IdT *__restrict__ ids,
                                                         const float *__restrict__ w, const int32_t *__restrict__ inv_perm,
                                                         const int32_t *__restrict__ expert_map,
-                                                        __nv_bfloat16 *__restrict__ out, int k, int64_t H8) {
+                                                        __nv_bfloat16 *__restrict__ out, int k, int64_t H8, uint32_t per_token) {
   using V = Vec8<__nv_bfloat16>;
-  const int64_t t = blockIdx.y;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < H8; c += (int64_t)gridDim.x * blockDim.x) {
+  const uint32_t token = blockIdx.x / per_token, part = blockIdx.x - token * per_token;      // as in moe_sum_kernel
+  const int64_t t = token;
+  for (int64_t c = (int64_t)part * blockDim.x + threadIdx.x; c < H8; c += (int64_t)per_token * blockDim.x) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j = 0; j < k; ++j) {
       // a slot that the scatter dropped has no row (and its id may lie outside the map): look at that first
@@ -691,14 +694,15 @@ extern "C" int lo_ep_gather(const void *a, const void *topk_ids, int ids_dtype, 
   LO_REQUIRE(a && topk_ids && topk_weights && inv_perm && out, "ep_gather: null pointer");
   LO_REQUIRE(aligned16(a, out), "ep_gather: rows and result must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t H8 = H / 8;
-  dim3 grid((unsigned)(ceil_div(H8, 256)), (unsigned)T);
+  const int64_t H8 = H / 8, per_token = ceil_div(H8, 256);
+  LO_REQUIRE(T * per_token <= 0x7fffffffLL, "ep_gather: too many tokens");
+  const unsigned grid = (unsigned)(T * per_token);
   if (ids_dtype == LO_I64)
     ep_gather_kernel<int64_t><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(a), static_cast<const int64_t *>(topk_ids),
-                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), k, H8);
+                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), k, H8, (uint32_t)per_token);
   else if (ids_dtype == LO_I32)
     ep_gather_kernel<int32_t><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(a), static_cast<const int32_t *>(topk_ids),
-                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), k, H8);
+                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), k, H8, (uint32_t)per_token);
   else
     return fail(LO_ERR_UNSUPPORTED, "ep_gather: unsupported id dtype code %d", ids_dtype);
   LO_LAUNCH_OK("ep_gather_kernel");

@@ -224,3 +224,23 @@ def test_layer_of_a_shard_reads_positions_or_rows_first(lo, monkeypatch):
     assert not y[~(ids == 3).any(1)].any() and bool(y[(ids == 3).any(1)].any(1).all())
     monkeypatch.setenv("LMSLIM_FUSED_MOE_CHUNK_SIZE", "2999")
     assert torch.equal(layer(), y)
+
+
+@pytest.mark.parametrize("H", [8, 2056])
+def test_reductions_of_more_than_65535_tokens(lo, H):
+    T, k = 65541, 2
+    g = torch.Generator(device=DEV).manual_seed(H)
+    a = torch.randn(T, k, H, generator=g, device=DEV).to(torch.bfloat16)
+    mask = torch.rand(T, k, generator=g, device=DEV) < 0.5
+    out = torch.empty(T, H, dtype=torch.bfloat16, device=DEV)
+    lo.moe.moe_sum(a, out)
+    assert torch.equal(out, (a[:, 0].float() + a[:, 1].float()).to(torch.bfloat16))
+    lo.moe.moe_sum(a, out, expert_mask=mask)
+    m = mask.float()[..., None]
+    assert torch.equal(out, (a[:, 0].float() * m[:, 0] + a[:, 1].float() * m[:, 1]).to(torch.bfloat16))
+    ids = torch.zeros(T, k, dtype=torch.int32, device=DEV)
+    inv = torch.randperm(T * k, generator=g, device=DEV).to(torch.int32).view(T, k)
+    w = torch.tensor([1.0, 2.0], device=DEV).expand(T, k).contiguous()      # (products by powers of two are exact: one rounding)
+    lo.moe.ep_gather(a.view(T * k, H), ids, w, inv, None, out)
+    rows = a.view(T * k, H)[inv.long()].float()
+    assert torch.equal(out, (rows[:, 0] + 2.0 * rows[:, 1]).to(torch.bfloat16))
