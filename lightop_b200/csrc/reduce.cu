@@ -56,40 +56,46 @@ template <> struct Vec8<float> {
   }
 };
 
+// Grid of `parts` blocks a token (or group of tokens), next to one another, and the tokens over the other two dimensions, which end at
+// 65535 each; grid_token() of a block may lie beyond the last one.
+inline dim3 token_grid(int64_t parts, int64_t tokens) {
+  const int64_t z = ceil_div(tokens, 65535);
+  return dim3((unsigned)parts, (unsigned)ceil_div(tokens, z), (unsigned)z);
+}
+__device__ __forceinline__ int64_t grid_token() { return (int64_t)blockIdx.z * gridDim.y + blockIdx.y; }
+
 // skip rule of one (token, slot):
 //   mask     : optional bool [M, topk]
 //   ids/map  : optional routing ids + expert_map; the slot is skipped when its expert is not local
-// One block row per token.  Each warp finds out once which of the token's slots count (a lane each, up to 32 at a time), then every
-// thread adds their rows in slot order, VPT vectors of eight columns at a time with several rows in flight.  (A thread that looked
-// at id, map and row of one slot after the other spent its time on the latencies: 8192 tokens with one local slot in eight took
-// 103 us for 234 MB, now 59 (72 with two blocks a SM
-// instead of three); 64 tokens of eight slots 8.0, now 4.7.)  VPT = 4: one pass of a block over 8192 columns, the latency of finding the slots is paid once a token;
-// VPT = 1: more blocks a token where there are few tokens.
-template <typename T, typename IdT, int VPT>
-__global__ void __launch_bounds__(256, VPT == 4 && sizeof(T) == 2 ? 3 : 1) moe_sum_kernel(const T *__restrict__ in, T *__restrict__ out,
+// A token has blockDim.x threads (whole warps) of one or more blocks, and a block as many tokens as fit.  Each warp finds out once
+// which of the token's slots count (a lane each, up to 32 at a time), then every thread adds their rows in slot order, VPT vectors of
+// eight columns at a time with ROWS rows in flight.  (A thread that looked at id, map and row of one slot after the other spent its
+// time on the latencies: 8192 tokens with one local slot in eight took 103 us for 234 MB, 64 tokens of eight slots 8.0.)
+// Bound by the latency of two dependent loads in small calls, by loads in flight (rows a thread times warps a SM) in large ones:
+// launch_sum() has the forms and what they take.
+template <typename T, typename IdT, int VPT, int ROWS, int BLOCKS_PER_SM>
+__global__ void __launch_bounds__(256, BLOCKS_PER_SM) moe_sum_kernel(const T *__restrict__ in, T *__restrict__ out,
                                                       const T *__restrict__ bias, int64_t M, int topk, int64_t H8,
                                                       float factor, const uint8_t *__restrict__ mask,
                                                       const int32_t *__restrict__ num_local_tokens,
                                                       const IdT *__restrict__ ids, const int32_t *__restrict__ expert_map,
-                                                      int num_experts, int num_local, uint32_t per_token) {
+                                                      int num_experts, int num_local) {
   using V = Vec8<T>;
-  constexpr int ROWS = VPT == 1 ? 8 : 2;      // rows in flight
-  // `per_token` blocks a token, next to one another in one dimension of the grid (the others end at 65535)
-  const uint32_t token = blockIdx.x / per_token, part = blockIdx.x - token * per_token;
-  const int64_t t = token;
+  const uint32_t t = (uint32_t)(grid_token() * blockDim.y + threadIdx.y);      // (M < 2^31; four bytes: registers are short in the forms of eight blocks a SM)
   const int lane = threadIdx.x & 31;
   dependency_wait();            // the rows come from the kernel before this one
   dependency_release();
-  if (num_local_tokens && t >= *num_local_tokens) return;
+  if (t >= M) return;
+  if (num_local_tokens && (int64_t)t >= *num_local_tokens) return;
   // which of the slots base + 0 .. base + 31 count (the same in every lane)
   auto live_slots = [&](int base) {
     const int j = base + lane;
     bool ok = j < topk;
-    if (ok && mask) ok = mask[t * topk + j] != 0;
+    if (ok && mask) ok = mask[(int64_t)t * topk + j] != 0;
     if (ok && ids) {
       // the rule of the alignment kernel (load_expert): an id outside [0, num_experts), or one that maps
       // outside the local experts, was dropped there and its row was never written
-      const long long e = (long long)ids[t * topk + j];
+      const long long e = (long long)ids[(int64_t)t * topk + j];
       ok = e >= 0 && e < num_experts;
       if (ok && expert_map) {
         const int m = expert_map[e];
@@ -98,68 +104,65 @@ __global__ void __launch_bounds__(256, VPT == 4 && sizeof(T) == 2 ? 3 : 1) moe_s
     }
     return __ballot_sync(0xffffffffu, ok);
   };
+  // (the token's blocks hold all of its columns: one pass)
+  const uint32_t cols = (uint32_t)H8, c0 = blockIdx.x * (blockDim.x * VPT) + threadIdx.x;
+  const V *in_v = reinterpret_cast<const V *>(in) + (int64_t)t * topk * H8 + c0;
+  constexpr bool EARLY_BIAS = VPT == 1 && ROWS == 8;      // (registers to spare)
+  float acc[VPT][8];
+  V b;
+  if (EARLY_BIAS && bias && c0 < cols) b = reinterpret_cast<const V *>(bias)[(int64_t)t * H8 + c0];
+#pragma unroll
+  for (int v = 0; v < VPT; ++v)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
   const unsigned first = live_slots(0);
-  const V *in_v = reinterpret_cast<const V *>(in) + t * topk * H8;
-  for (int64_t c0 = (int64_t)part * (blockDim.x * VPT); c0 < H8; c0 += (int64_t)per_token * (blockDim.x * VPT)) {
-    float acc[VPT][8];
-    V b[VPT];
+  for (int base = 0; base < topk; base += 32) {
+    unsigned live = base == 0 ? first : live_slots(base);
+    while (live) {
+      V row[ROWS][VPT];
+      bool on[ROWS];
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int64_t c = c0 + v * blockDim.x + threadIdx.x;
+      for (int u = 0; u < ROWS; ++u) {
+        on[u] = live != 0;
+        const int j = base + __ffs(live) - 1;
+        live &= live - 1;
+        if (on[u]) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
-      if (bias && VPT == 1 && c < H8) b[v] = reinterpret_cast<const V *>(bias)[t * H8 + c];
-    }
-    for (int base = 0; base < topk; base += 32) {
-      unsigned live = base == 0 ? first : live_slots(base);
-      while (live) {
-        V row[ROWS][VPT];
-        bool on[ROWS];
-#pragma unroll
-        for (int u = 0; u < ROWS; ++u) {
-          on[u] = live != 0;
-          const int j = base + __ffs(live) - 1;
-          live &= live - 1;
-          if (on[u]) {
-#pragma unroll
-            for (int v = 0; v < VPT; ++v) {
-              const int64_t c = c0 + v * blockDim.x + threadIdx.x;
-              if (c < H8) row[u][v] = in_v[(int64_t)j * H8 + c];
-            }
-          }
+          for (int v = 0; v < VPT; ++v)
+            if (c0 + v * blockDim.x < cols) row[u][v] = in_v[(int64_t)j * H8 + v * blockDim.x];
         }
+      }
 #pragma unroll
-        for (int u = 0; u < ROWS; ++u) {
-          if (on[u]) {
+      for (int u = 0; u < ROWS; ++u) {
+        if (on[u]) {
 #pragma unroll
-            for (int v = 0; v < VPT; ++v) {
-              float f[8];
-              row[u][v].to_float(f);
+          for (int v = 0; v < VPT; ++v) {
+            float f[8];
+            row[u][v].to_float(f);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) acc[v][i] += f[i];
-            }
+            for (int i = 0; i < 8; ++i) acc[v][i] += f[i];
           }
         }
       }
     }
+  }
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int64_t c = c0 + v * blockDim.x + threadIdx.x;
-      if (c >= H8) break;
-      if (bias) {
-        float f[8];
-        if (VPT > 1) b[v] = reinterpret_cast<const V *>(bias)[t * H8 + c];
-        b[v].to_float(f);
+  for (int v = 0; v < VPT; ++v) {
+    const uint32_t c = c0 + v * blockDim.x;
+    if (c >= cols) break;
+    if (bias) {
+      float f[8];
+      if (!EARLY_BIAS) b = reinterpret_cast<const V *>(bias)[(int64_t)t * H8 + c];
+      b.to_float(f);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[v][i] = acc[v][i] * factor + f[i];
-      } else {
+      for (int i = 0; i < 8; ++i) acc[v][i] = acc[v][i] * factor + f[i];
+    } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[v][i] = acc[v][i] * factor;
-      }
-      V o;
-      o.from_float(acc[v]);
-      reinterpret_cast<V *>(out)[t * H8 + c] = o;
+      for (int i = 0; i < 8; ++i) acc[v][i] = acc[v][i] * factor;
     }
+    V o;
+    o.from_float(acc[v]);
+    reinterpret_cast<V *>(out)[(int64_t)t * H8 + c] = o;
   }
 }
 
@@ -168,16 +171,40 @@ int launch_sum(const void *in, void *out, const void *bias, int64_t M, int topk,
                const uint8_t *mask, const int32_t *nlt, const void *ids, const int32_t *expert_map,
                cudaStream_t st, int num_experts = 0x7fffffff, int num_local = 0x7fffffff) {
   const int64_t H8 = H / 8;
-  const int64_t narrow = ceil_div(H8, 256);
-  // Four vectors a thread where slots may be missing and the blocks of one vector a thread would not all be on the GPU at once
-  // (eight a SM).  With every slot there one vector a thread has as many loads in flight and more warps (2999 tokens of 8 slots: 93 against 100 us).
-  const bool wide = (mask != nullptr || expert_map != nullptr) && M * narrow > 8 * (int64_t)sm_count();
-  const int64_t per_token = wide ? ceil_div(H8, 1024) : narrow;
-  LO_REQUIRE(M * per_token <= 0x7fffffffLL, "moe_sum: too many tokens");
-  auto kernel = wide ? moe_sum_kernel<T, IdT, 4> : moe_sum_kernel<T, IdT, 1>;
-  LO_CUDA_OK(launch_dependent(kernel, dim3((unsigned)(M * per_token)), dim3(256), 0, st, static_cast<const T *>(in),
-                              static_cast<T *>(out), static_cast<const T *>(bias), M, topk, H8, factor, mask, nlt,
-                              static_cast<const IdT *>(ids), expert_map, num_experts, num_local, (uint32_t)per_token));
+  // Forms, by the number of full blocks of one vector a thread (256 threads) that the call is, in us behind a kernel that wrote the
+  // rows (bf16, eight slots; eight rows in flight / four, five blocks a SM / four, eight blocks a SM / one row of four vectors; all of one
+  // build, the present one is up to 0.5 us faster):
+  //                            every slot there              one slot in eight
+  //   64 x 7168 (224)          2.8 /  3.0 /  3.2 /  5.8      2.4 /  2.3 /  2.4 /  3.3
+  //   600 x 1024 (300)         3.1 /  3.2 /  3.6 /  5.1      2.5 /  2.6 /  2.8 /  4.2
+  //   297 x 4096 (594)         5.0 /  4.4 /  4.8 /  5.8      3.4 /  2.9 /  3.0 /  3.6
+  //   600 x 5120 (1500)        9.8 /  9.1 /  9.5 /  9.4      7.7 /  6.6 /  6.1 /  6.2
+  //   1024 x 4096 (2048)      12.0 / 10.6 / 10.0 / 10.3      8.6 /  6.3 /  5.6 /  6.2
+  //   2048 x 4096 (4096)      25.9 / 25.1 / 24.0 / 26.8     16.7 / 11.6 /  9.7 /  9.5
+  //   8192 x 7168 (28672)      154 /  158 /  154 /  161       98 /   75 /   54 /   45
+  // The last form is for calls in which many slots may be missing (a mask, or a map of few local experts): a token has a row or two
+  // then and their latency is all there is.  It needs a token's warps to have four vectors each.
+  // Elements of four bytes have half the columns in flight a register, and eight rows would fit two blocks a SM: two rows,
+  // with six blocks a SM and, above six full blocks, eight (297 x 4096 5.9, 6.5; 2048 x 1024 8.7, 8.2; one slot in eight of
+  // 2048 x 7168 23.3, 21.3).
+  const int64_t full = M * H8 / 256, sms = sm_count();
+  const bool sparse = mask != nullptr || (expert_map != nullptr && 4 * (int64_t)num_local <= num_experts);
+  auto kernel = moe_sum_kernel<T, IdT, 1, 8, 1>;
+  int64_t vpt = 1;
+  if constexpr (sizeof(T) == 4) {
+    if (full > 6 * sms) kernel = moe_sum_kernel<T, IdT, 1, 2, 8>;
+    else if (full > 2 * sms) kernel = moe_sum_kernel<T, IdT, 1, 2, 6>;
+  } else {
+    if (full > 20 * sms && sparse && H8 >= 128) kernel = moe_sum_kernel<T, IdT, 4, 1, 4>, vpt = 4;
+    else if (full > 12 * sms) kernel = moe_sum_kernel<T, IdT, 1, 4, 8>;
+    else if (full > 2 * sms) kernel = moe_sum_kernel<T, IdT, 1, 4, 5>;
+  }
+  // as few blocks a token as hold its columns, as few warps in them, and as many tokens a block as 256 threads hold
+  const int64_t per_token = ceil_div(H8, 256 * vpt);
+  const int64_t threads = round_up(ceil_div(H8, per_token * vpt), 32), tokens = 256 / threads;
+  LO_CUDA_OK(launch_dependent(kernel, token_grid(per_token, ceil_div(M, tokens)), dim3((unsigned)threads, (unsigned)tokens), 0, st,
+                              static_cast<const T *>(in), static_cast<T *>(out), static_cast<const T *>(bias), M, topk, H8, factor, mask,
+                              nlt, static_cast<const IdT *>(ids), expert_map, num_experts, num_local));
   return LO_OK;
 }
 
@@ -419,11 +446,11 @@ template <typename IdT>
 __global__ void __launch_bounds__(256) ep_gather_kernel(const __nv_bfloat16 *__restrict__ a, const IdT *__restrict__ ids,
                                                         const float *__restrict__ w, const int32_t *__restrict__ inv_perm,
                                                         const int32_t *__restrict__ expert_map,
-                                                        __nv_bfloat16 *__restrict__ out, int k, int64_t H8, uint32_t per_token) {
+                                                        __nv_bfloat16 *__restrict__ out, int64_t T, int k, int64_t H8) {
   using V = Vec8<__nv_bfloat16>;
-  const uint32_t token = blockIdx.x / per_token, part = blockIdx.x - token * per_token;      // as in moe_sum_kernel
-  const int64_t t = token;
-  for (int64_t c = (int64_t)part * blockDim.x + threadIdx.x; c < H8; c += (int64_t)per_token * blockDim.x) {
+  const int64_t t = grid_token();
+  if (t >= T) return;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < H8; c += (int64_t)gridDim.x * blockDim.x) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j = 0; j < k; ++j) {
       // a slot that the scatter dropped has no row (and its id may lie outside the map): look at that first
@@ -694,15 +721,14 @@ extern "C" int lo_ep_gather(const void *a, const void *topk_ids, int ids_dtype, 
   LO_REQUIRE(a && topk_ids && topk_weights && inv_perm && out, "ep_gather: null pointer");
   LO_REQUIRE(aligned16(a, out), "ep_gather: rows and result must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t H8 = H / 8, per_token = ceil_div(H8, 256);
-  LO_REQUIRE(T * per_token <= 0x7fffffffLL, "ep_gather: too many tokens");
-  const unsigned grid = (unsigned)(T * per_token);
+  const int64_t H8 = H / 8;
+  const dim3 grid = token_grid(ceil_div(H8, 256), T);
   if (ids_dtype == LO_I64)
     ep_gather_kernel<int64_t><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(a), static_cast<const int64_t *>(topk_ids),
-                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), k, H8, (uint32_t)per_token);
+                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), T, k, H8);
   else if (ids_dtype == LO_I32)
     ep_gather_kernel<int32_t><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(a), static_cast<const int32_t *>(topk_ids),
-                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), k, H8, (uint32_t)per_token);
+                                                   topk_weights, inv_perm, expert_map, static_cast<__nv_bfloat16 *>(out), T, k, H8);
   else
     return fail(LO_ERR_UNSUPPORTED, "ep_gather: unsupported id dtype code %d", ids_dtype);
   LO_LAUNCH_OK("ep_gather_kernel");

@@ -125,8 +125,8 @@ def test_silu_quant_widths(lo, rows, d):
     assert torch.equal(q, r.round().clamp(-128, 127).to(torch.int8))
 
 
-# blocks of one vector a thread up to eight blocks a SM, of four above: both sides of the line, columns that do not fill the last
-# pass, slots that are all, some or not there, more than 32 of them
+# the forms' lines (two and twelve full blocks a SM) from both sides, columns that do not fill the last block, slots that are all, some or
+# not there, more than 32 of them
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,k,H", [(1, 8, 7168), (296, 8, 7168), (297, 8, 7168), (1185, 3, 2056), (1300, 2, 256), (5, 37, 264), (1200, 40, 136), (400, 9, 8200)])
 def test_moe_sum_split(lo, dtype, M, k, H):
@@ -244,3 +244,51 @@ def test_reductions_of_more_than_65535_tokens(lo, H):
     lo.moe.ep_gather(a.view(T * k, H), ids, w, inv, None, out)
     rows = a.view(T * k, H)[inv.long()].float()
     assert torch.equal(out, (rows[:, 0] + 2.0 * rows[:, 1]).to(torch.bfloat16))
+
+
+# several tokens a block and a last block that is not full, every form (up to two, up to twelve, more, and more than twenty full blocks
+# a SM, fp32 up to six), columns that leave threads of a token's last warp or block without any
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,k,H", [(1, 1, 8), (67, 8, 256), (301, 8, 1024), (607, 3, 1032), (299, 8, 5120), (9001, 5, 264), (9601, 2, 264), (15001, 2, 264), (5801, 2, 1056), (1700, 33, 4112)])
+def test_moe_sum_forms(lo, dtype, M, k, H):
+    g = torch.Generator(device=DEV).manual_seed(M + H)
+    a = torch.randn(M, k, H, generator=g, device=DEV).to(dtype)
+    mask = torch.rand(M, k, generator=g, device=DEV) < 0.4
+    valid = torch.tensor([M - M // 3], dtype=torch.int32, device=DEV)
+    for m in (None, mask):
+        acc = torch.zeros(M, H, device=DEV)
+        for j in range(k):
+            acc = acc + (a[:, j].float() if m is None else torch.where(m[:, j:j + 1], a[:, j].float(), torch.zeros((), device=DEV)))
+        out = torch.full((M, H), 7.0, dtype=dtype, device=DEV)
+        lo.moe.moe_sum(a, out, expert_mask=m, num_local_tokens=valid, factor=0.5)
+        n = int(valid)
+        assert torch.equal(out[:n], (acc[:n] * 0.5).to(dtype)) and bool((out[n:] == 7.0).all())
+        none = torch.full_like(out, 7.0)
+        lo.moe.moe_sum(a, none, expert_mask=m, num_local_tokens=-valid)
+        assert bool((none == 7.0).all())
+
+
+@pytest.mark.parametrize("M,H", [(5501, 1152), (6003, 1024), (300, 1024), (9601, 512)])
+def test_layer_sum_with_few_local_experts(lo, monkeypatch, M, H):
+    """One expert of eight is local: the form of four vectors a thread above twenty full blocks a SM, the others below and for narrow
+    rows.  The same tokens in smaller calls have the same bits."""
+    from lightop_b200 import synthetic
+    E, k, I = 8, 2, 128
+    w1, w2, w1_s, w2_s = synthetic.make_weights(E, H, I, seed=5, device=DEV)
+    x, logits = synthetic.make_activations(M, H, E, seed=6, device=DEV)
+    weights = torch.empty(M, k, device=DEV)
+    ids = torch.empty(M, k, dtype=torch.int32, device=DEV)
+    lo.moe.topk_softmax(weights, ids, None, logits, True)
+    emap = torch.full((E,), -1, dtype=torch.int32, device=DEV)
+    emap[2] = 0
+    shared = torch.randn(M, H, generator=torch.Generator(device=DEV).manual_seed(7), device=DEV).to(torch.bfloat16)
+
+    def layer(ids):
+        return lo.moe.fused_experts_impl_int8(x, w1[2:3].clone(), w2[2:3].clone(), weights, ids, None, use_int8_w8a8=True, block_shape=[128, 128],
+                                              w1_scale=w1_s[2:3].clone(), w2_scale=w2_s[2:3].clone(), global_num_experts=E, expert_map=emap,
+                                              routed_scaling_factor=2.5, shared_output=shared)
+    y = layer(ids)
+    assert torch.equal(y[~(ids == 2).any(1)], shared[~(ids == 2).any(1)])
+    assert torch.equal(layer(ids.long()), y)
+    monkeypatch.setenv("LMSLIM_FUSED_MOE_CHUNK_SIZE", "97")
+    assert torch.equal(layer(ids), y)
