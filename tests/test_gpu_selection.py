@@ -76,3 +76,39 @@ def test_grouped_gate_with_groups_of_one_expert(lo, E, keep, k, shared):
     p = torch.gather(s, 1, order)
     torch.testing.assert_close(w.cpu()[:, :k - shared], p / p.sum(1, keepdim=True), rtol=2e-5, atol=2e-6)
     assert bool((ids.cpu()[:, k - shared:] == E).all())
+
+
+@pytest.mark.parametrize("E,groups,keep,k", [(256, 8, 4, 8), (256, 16, 4, 8), (256, 1, 1, 8), (64, 2, 1, 6)])
+def test_gate_passes_over_nan(lo, E, groups, keep, k):
+    """A NaN counts as -inf: it is taken only where nothing else is left, and the other experts' order and weights stay."""
+    g = torch.Generator().manual_seed(E + groups)
+    x = torch.randn(66, E, generator=g)
+    x[torch.rand(66, E, generator=g) < 0.3] = float("nan")
+    x[0] = float("nan")
+    w, ids = lo.moe.moe_fused_gate(x.to(DEV), torch.zeros(E, device=DEV), groups, keep, k, 0, 2.5, False)
+    w, ids = w.cpu(), ids.cpu().long()
+    assert bool(((ids >= 0) & (ids < E)).all())
+    s = torch.sigmoid(x.to(DEV)).cpu()
+    s = torch.where(s.isnan(), torch.full((), float("-inf")), s)[1:]
+    top2 = s.view(65, groups, -1).topk(2, dim=2).values.sum(2)
+    kept = torch.sort(top2, dim=1, descending=True, stable=True).indices[:, :keep]
+    mask = torch.zeros(65, groups, dtype=torch.bool).scatter_(1, kept, True).repeat_interleave(E // groups, 1)
+    order = torch.sort(torch.where(mask, s, torch.full((), float("-inf"))), dim=1, descending=True, stable=True).indices[:, :k]
+    assert torch.equal(ids[1:], order)
+    p = torch.gather(s, 1, order)
+    torch.testing.assert_close(w[1:], p / p.sum(1, keepdim=True), rtol=2e-5, atol=2e-6)
+
+
+def test_topk_softmax_passes_over_nan(lo):
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(66, 256, generator=g)
+    x[torch.rand(66, 256, generator=g) < 0.3] = float("nan")
+    x[0] = float("nan")
+    weights = torch.empty(66, 8, device=DEV)
+    ids = torch.empty(66, 8, dtype=torch.int32, device=DEV)
+    lo.moe.topk_softmax(weights, ids, None, x.to(DEV), False)
+    ids = ids.cpu().long()
+    assert bool(((ids >= 0) & (ids < 256)).all())
+    s = torch.where(x.isnan(), torch.full((), float("-inf")), x)
+    assert torch.equal(ids[1:], torch.sort(s, dim=1, descending=True, stable=True).indices[1:, :8])
+    assert bool(weights.isnan().all())      # (a NaN is in the row's denominator)
