@@ -189,9 +189,12 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 }
 
 // Reciprocal refined by one Newton step, and the quotient a / b from it with the remainder folded back in (Markstein's method,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990)
-// (q = a*y, then q + (a - b*q)*y): the IEEE round-to-nearest quotient for finite operands whose quotient and reciprocal
-// are normal numbers.  Inline, so the divisions of a thread overlap; the library division is a subroutine call each: two of them
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): q = a*y, then q + (a - b*q)*y.
+// Not the IEEE quotient of any two fp32 numbers: the reciprocal need not be the rounded one, and the remainder is inexact where it is
+// subnormal.  What the tests establish, exhaustively, is what the callers use: the truncated or rounded codes of bf16 and fp16
+// elements over their group's scale (in the range that the caller checks), and the SiLU of every bf16 gate after its rounding to
+// bf16.  fp32 elements take the library's division.
+// Inline, so the divisions of a thread overlap; the library division is a subroutine call each: two of them
 // per output made the GEMM's epilogue a fifth of its time, and one per element two thirds of the group quantiser's.
 __device__ __forceinline__ float rcp_refined(float b) {
   float y;

@@ -360,9 +360,13 @@ __device__ __forceinline__ void tmem_ld_wait16(uint32_t (&r)[16]) {
 //   ROW4  (16x128b loads): channel 8(r & 1) + lane / 4, token 4(r >> 1) + lane % 4
 //   !ROW4 (16x256b loads, the layout of an MMA accumulator fragment): channel 8((r >> 1) & 1) + lane / 4,
 //         token 8(r >> 2) + 2(lane % 4) + (r & 1)
-// In a loop of loads alone the first form moves 128 bytes per clock and scheduler, the second 64.  Layers take the first: 4096 tokens
-// 3348 -> 3318 us a pass, 8192 tokens of a shard 860 -> 842, Zipf routing the same; dense calls the second (4096 x 4096 x 7168 203 us a
-// pass against 207.5 with the first).
+// In a loop of loads alone the first form moves 128 bytes per clock and scheduler, the second 64.  Calls with a chunk table (layers,
+// expert rows, the grouped GEMM on its own) take the first, dense calls the second.  First, second, in us a pass, medians of three
+// turns on one board whose turns differ by 0.1 to 2.5 % (the stand-alone GEMM's by up to 8):
+//   layer of 1024 tokens 1877, 1891    2048 2301, 2354    4096 3177, 3233    Qwen3 2048 805, 822 (Zipf 913, 916)    64, 777: the same
+//   8192 tokens of a shard 785, 799    4096 expert rows 433, 441    16384 1429, 1454    grouped GEMM of 4096 rows 318, 325
+//   dense 4096 x 4096 x 7168 173.6, 169.4    1000 x 4096 x 7168 50.5, 48.8    4096 x 7168 x 2048 104.0, 103.2    smaller: the same
+// Why the dense ones lose is not known.
 template <bool ROW4> __device__ __forceinline__ void tmem_ld_two(uint32_t taddr, uint32_t (&r)[16]) {
   if (ROW4)
     asm volatile("tcgen05.ld.sync.aligned.16x128b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -444,8 +448,8 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 }
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 // a / b from the approximate reciprocal, corrected by the remainder once: within a unit in the last place or better of the
-// quotient, whose next use is a rounding to bf16.  The operand ranges of div_by() in common.h, which holds for every division of the
-// epilogues (denominators in [1, 1e38] or a group scale of at least 1e-10 / 127).
+// quotient, whose next use is a rounding to bf16.  Here as with div_by() (common.h) the reciprocal has to be a normal number, which it
+// is for every division of the epilogues: their denominators are in [1, 1e38] or a group scale of at least 1e-10 / 127.
 __device__ __forceinline__ float div_fast(float a, float b) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));

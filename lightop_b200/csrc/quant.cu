@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(TOKEN_QUANT_THREADS) token_quant_kernel(const 
 // stay in the registers of 128; 128 else, where the blocks fill the SMs and fewer warps wait at a row's barrier.
 // ---------------------------------------------------------------------------
 
-// g / (1 + exp(-g)), the IEEE quotient: the refined reciprocal is taken of the denominator times 2^-32, which keeps the
+// g / (1 + exp(-g)), after its rounding to bf16 the same as with the library's division: the refined reciprocal is taken of the denominator times 2^-32, which keeps the
 // reciprocal normal up to the largest finite denominator.  What that form does not give has a denominator of 2 (next to zero, where
 // the quotient may be a subnormal), of 1 (large gates and infinity) or of infinity (g * 0: a signed zero or, for -inf, NaN).
 // The tests compare every bf16 gate with the library's division.
@@ -474,7 +474,8 @@ int launch_silu_mul_token_quant(const void *in, int64_t rows, int64_t d, const i
   LO_REQUIRE(d >= 8 && d % 8 == 0, "silu-mul quant: width %lld must be a multiple of 8", (long long)d);
   LO_REQUIRE(rows <= 0x7fffffffLL, "silu-mul quant: too many rows");
   const bool wide = d > 128 * 8 * SILU_VECS || rows <= 2 * (int64_t)sm_count();
-  LO_CUDA_OK(launch_dependent(wide ? silu_mul_token_quant_kernel<256> : silu_mul_token_quant_kernel<128>, dim3((unsigned)rows), dim3(wide ? 256 : 128), 0, stream,
+  auto kernel = wide ? silu_mul_token_quant_kernel<256> : silu_mul_token_quant_kernel<128>;
+  LO_CUDA_OK(launch_dependent(kernel, dim3((unsigned)rows), dim3(wide ? 256 : 128), 0, stream,
                               static_cast<const __nv_bfloat16 *>(in), d, row_ids, numel_valid, num_rows_dev,
                               group_rows > 0 ? group_rows : (int64_t)1, group_counts, q, s));
   return LO_OK;

@@ -81,7 +81,8 @@ __global__ void __launch_bounds__(256, BLOCKS_PER_SM) moe_sum_kernel(const T *__
                                                       const IdT *__restrict__ ids, const int32_t *__restrict__ expert_map,
                                                       int num_experts, int num_local) {
   using V = Vec8<T>;
-  const uint32_t t = (uint32_t)(grid_token() * blockDim.y + threadIdx.y);      // (M < 2^31; four bytes: registers are short in the forms of eight blocks a SM)
+  // (M < 2^31; four bytes, as registers are short in the forms of eight blocks a SM)
+  const uint32_t t = (uint32_t)(grid_token() * blockDim.y + threadIdx.y);
   const int lane = threadIdx.x & 31;
   dependency_wait();            // the rows come from the kernel before this one
   dependency_release();
@@ -540,10 +541,11 @@ int launch_permute_rows(const int8_t *A, const float *a_scale, int64_t rows_a, i
   if (sorted_capacity <= 0) return LO_OK;
   LO_REQUIRE(sorted_capacity <= 0x7fffffffLL, "permute rows: too many positions");
   const bool few = sorted_capacity <= 8 * (int64_t)sm_count();
-  LO_CUDA_OK(launch_dependent(few ? permute_rows_kernel<4> : permute_rows_kernel<1>, dim3((unsigned)(few ? sorted_capacity : ceil_div(sorted_capacity, PERMUTE_WARPS))),
-                              dim3(PERMUTE_WARPS * 32), 0, stream, A, a_scale, rows_a, K,
-                              sorted_ids, sorted_capacity, num_tokens_post_pad, numel_valid, top_k, scales_per_row > 0 ? scales_per_row : K / 128, A_sorted,
-                              a_scale_sorted, a_stride > 0 ? a_stride : K, expert_ids, block_size, chunks, num_chunks));
+  auto kernel = few ? permute_rows_kernel<4> : permute_rows_kernel<1>;
+  const unsigned blocks = (unsigned)(few ? sorted_capacity : ceil_div(sorted_capacity, PERMUTE_WARPS));
+  LO_CUDA_OK(launch_dependent(kernel, dim3(blocks), dim3(PERMUTE_WARPS * 32), 0, stream, A, a_scale, rows_a, K, sorted_ids,
+                              sorted_capacity, num_tokens_post_pad, numel_valid, top_k, scales_per_row > 0 ? scales_per_row : K / 128,
+                              A_sorted, a_scale_sorted, a_stride > 0 ? a_stride : K, expert_ids, block_size, chunks, num_chunks));
   return LO_OK;
 }
 
