@@ -60,3 +60,21 @@ def test_lanes_without_a_group_take_no_quotient():
     leave = next(i for i in range(start, len(st)) if st[i].startswith("if (!active) return"))
     assert any("__shfl_xor_sync" in s for s in st[start:leave])
     assert not any("__fdiv_rn" in s or "div_by" in s for s in st[start:leave])
+
+
+def test_what_lets_the_next_kernel_start_has_waited_itself():
+    # a kernel that released its successor before its own wait would let it (and what that one releases) run ahead of earlier work
+    import glob
+    seen = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        st = _statements(os.path.basename(path))
+        waited = False
+        for s in st:
+            if "__global__" in s:
+                waited = False
+            if s.endswith("dependency_wait()"):
+                waited = True
+            elif s.endswith("dependency_release()"):
+                assert waited, os.path.basename(path)
+                seen += 1
+    assert seen >= 9
