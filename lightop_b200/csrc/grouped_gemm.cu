@@ -62,9 +62,10 @@
 namespace lo {
 namespace {
 
-// Interval between two polls of a barrier, in nanoseconds, by role.  (Intervals from none to 2 us measured no different, in time
-// or in power.)
-constexpr uint32_t LO_SLEEP_PRODUCER = 128u, LO_SLEEP_SCALE = 128u, LO_SLEEP_MMA = 20u, LO_SLEEP_PROMO = 32u, LO_SLEEP_OUT = 256u;
+// Interval between two polls of a barrier, in nanoseconds: none.  try_wait parks the thread for a while by itself; a sleep on top of
+// it, or its form with a time hint, is more code in the loops of all roles (4096 tokens 3147 -> 3091 us without
+// either, Qwen3 2048 Zipf 935 -> 892, sharded 8192 797 -> 789; sleeps of 100 ns to 2 us by role lost half of it or all).
+constexpr uint32_t LO_SLEEP = 0u, LO_SLEEP_MMA = 0u;
 
 constexpr int TILE_N = 128;      // weight rows per accumulator (MMA M)
 constexpr int TILE_K = 128;      // int8 elements (= bytes) per K block
@@ -166,83 +167,42 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// One poll.  The suspend-time hint lets the hardware park the thread until the phase completes (or the
-// hint runs out) instead of returning at once: waiting warps then stop competing for issue slots
-// with the warps that have work (without it, polling made up most of the executed instructions).
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(200000u)
-      : "memory");
-  return ok != 0;
-}
-// Upper bound of one wait, in SM clock cycles (about 1.5 s at 1.9 GHz).
-constexpr long long WAIT_LIMIT_CYCLES = 3000000000ll;
-
-// Bounded wait.  Returns false when the CTA is aborting (this waiter timed out or another one
-// did); `code` identifies the waiter in the status word.  The clock is only consulted every
-// 256 failed polls, so a wait that completes quickly costs nothing but the polls.  A waiter sleeps
-// `sleep_ns` between two polls: a polling warp is always eligible, and the scheduler it shares with
-// four others was observed to give it most of the issue slots (a promotion warp's dozen loop
-// instructions between two K blocks took several hundred cycles).  Waiters far off the critical path
-// (producers that run stages ahead, promotion warps without columns in a narrow chunk) sleep longer.
-template <class S>
-__device__ __forceinline__ bool mbar_wait(S &sm, uint64_t *bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP_PROMO) {
-  if (mbar_try_wait(bar, parity)) return true;
-  long long t0 = 0;
-  while (true) {
-    // the polls between two looks at the clock carry no bookkeeping but their count
-#pragma unroll 1
-    for (int i = 0; i < 256; ++i) {
-      __nanosleep(sleep_ns);
-      if (mbar_try_wait(bar, parity)) return true;
-    }
-    if (sm.abort_flag) return false;
-    const long long now = clock64();
-    if (t0 == 0) t0 = now;
-    if (now - t0 > WAIT_LIMIT_CYCLES) {
-      sm.abort_flag = 1;
-      if (status) atomicCAS(status, 0, code);
-      return false;
-    }
-  }
-}
-
-// The same wait and arrive for a barrier given by its shared-memory address.
+// One poll; the hardware may park the thread for a short while before it answers no.
 __device__ __forceinline__ bool mbar_try_wait_addr(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(200000u)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
+// Upper bound of one wait, in SM clock cycles (about 1.5 s at 1.9 GHz; below 2^32, so the low half of the clock measures it).
+constexpr uint32_t WAIT_LIMIT_CYCLES = 3000000000u;
+
+// Bounded wait.  Returns false when the CTA is aborting (this waiter timed out or another one did); `code` identifies the waiter
+// in the status word.  Short on purpose: it is inlined into the loops of all roles, which share the instruction caches.
 template <class S>
-__device__ __forceinline__ bool mbar_wait_addr(S &sm, uint32_t bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP_PROMO) {
+__device__ __forceinline__ bool mbar_wait_addr(S &sm, uint32_t bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP) {
   if (mbar_try_wait_addr(bar, parity)) return true;
-  long long t0 = 0;
-  while (true) {
+  const uint32_t t0 = (uint32_t)clock();
 #pragma unroll 1
-    for (int i = 0; i < 256; ++i) {
-      __nanosleep(sleep_ns);
-      if (mbar_try_wait_addr(bar, parity)) return true;
-    }
+  while (!mbar_try_wait_addr(bar, parity)) {
     if (sm.abort_flag) return false;
-    const long long now = clock64();
-    if (t0 == 0) t0 = now;
-    if (now - t0 > WAIT_LIMIT_CYCLES) {
+    if ((uint32_t)clock() - t0 > WAIT_LIMIT_CYCLES) {
       sm.abort_flag = 1;
       if (status) atomicCAS(status, 0, code);
       return false;
     }
+    if (sleep_ns > 0u) __nanosleep(sleep_ns);
   }
+  return true;
+}
+template <class S>
+__device__ __forceinline__ bool mbar_wait(S &sm, uint64_t *bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP) {
+  return mbar_wait_addr(sm, smem_u32(bar), parity, status, code, sleep_ns);
 }
 // One non-blocking look at a barrier: has the phase of this parity completed?
 __device__ __forceinline__ bool mbar_test_addr(uint32_t bar, uint32_t parity) {
@@ -637,7 +597,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             const int32_t row_g = (int32_t)(ch.expert * p.n_rows_per_expert + (int64_t)(ph * p.n_tiles + nt) * TILE_N);
             for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NW
-              if (it >= (uint32_t)NW && !mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 1, LO_SLEEP_PRODUCER)) { ok = false; break; }
+              if (it >= (uint32_t)NW && !mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 1)) { ok = false; break; }
               mbar_arrive_expect_tx(&sm.ready[it % ND], W_TILE_BYTES);
               tma_load_2d(sm.w[s], &w_map, kb * TILE_K, row_g, &sm.ready[it % ND], pol_w);
               s = s + 1 == NW ? 0 : s + 1;
@@ -664,7 +624,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           for (int ph = 0; ph < PHASES && ok; ++ph) {
             for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NA
-              if (it >= (uint32_t)NA && !mbar_wait(sm, &sm.done[(it - NA) % ND], ((it - NA) / ND) & 1u, p.status, 6, LO_SLEEP_PRODUCER)) { ok = false; break; }
+              if (it >= (uint32_t)NA && !mbar_wait(sm, &sm.done[(it - NA) % ND], ((it - NA) / ND) & 1u, p.status, 6)) { ok = false; break; }
               uint64_t *bar = &sm.ready[it % ND];
               mbar_arrive_expect_tx(bar, a_bytes);
               tma_load_2d(sm.a[s], &a_maps.m[mi], kb * TILE_K, ch.row0, bar, pol_a);
@@ -732,7 +692,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           if (nxt.valid) fetch(nxt, a_nxt, b_nxt);
           // the slot's previous batch has been read when the partial of its last step has been consumed
           if (n_batch >= (uint32_t)SC_BATCHES &&
-              !__all_sync(0xffffffffu, mbar_wait(sm, &sm.consumed[end_of[0] % ND], (end_of[0] / ND) & 1u, p.status, 4, LO_SLEEP_SCALE))) break;
+              !__all_sync(0xffffffffu, mbar_wait(sm, &sm.consumed[end_of[0] % ND], (end_of[0] / ND) & 1u, p.status, 4))) break;
           const int T = (cur.ch.rows + 15) & ~15;
           float *sc = &sm.sc[slot * SC_STEPS][0];
 #pragma unroll
@@ -851,7 +811,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       if constexpr (MODE == GEMM_GATE_UP) {
         // A row of the tile is one token's 128-channel quantisation group: |act| maximum over the warp (four channels
         // per lane), scale = max / 127, q = trunc(clamp(act / scale)), one 4-byte store per lane.
-        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9, LO_SLEEP_OUT))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9))) break;
         const int64_t I = (int64_t)p.n_tiles * TILE_N;
         int8_t *q_out = p.act_q + (int64_t)ch.row0 * I + (int64_t)nt * TILE_N + lane * 4;
         float *s_out = p.act_s + (int64_t)ch.row0 * p.n_tiles + nt;
@@ -914,7 +874,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             }
           }
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9, LO_SLEEP_OUT))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9))) break;
         const int64_t n0 = (int64_t)nt * TILE_N + (lane & 15) * 8;
         const int n_steps = (ch.rows + 2 * OUT_WARPS - 1) / (2 * OUT_WARPS);
 #pragma unroll 4
@@ -1088,8 +1048,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         const uint32_t part0 = tmem_base + lane_off + (uint32_t)col_begin;
         const uint32_t sc0 = smem_u32(&sm.sc[0][0]) + (uint32_t)col_begin * 4u + (uint32_t)(lane & 3) * 16u;
         const uint32_t done0 = smem_u32(&sm.done[0]), consumed0 = smem_u32(&sm.consumed[0]), scales0 = smem_u32(&sm.scales[0]);
-        // a warp without columns only has to keep step
-        const uint32_t wait_ns = my_p == 0 ? 256u : LO_SLEEP_PROMO;
         // this lane's row of the staging tile for the matrix stores and loads of a piece: lanes 8m .. 8m + 7 address the
         // token rows of block m, blocks 0 / 1 are channels 0..7 / 8..15 of tokens 0..7, blocks 2 / 3 of tokens 8..15
         const uint32_t stg_mine = smem_u32(&sm.staging[0]) + (uint32_t)(col_begin + (lane >> 4) * 8 + block_row<ROW4>(lane & 7)) * OUT_ROW_BYTES +
@@ -1125,7 +1083,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
               else tmem_ld_two<ROW4>(part + 32u * (u >> 1) + ((u & 1) ? 16u << 16 : 0u), r);
             };
             uint32_t dn = step & (uint32_t)(ND - 1), dph = (step >> 4) & 1u;      // the step's place in the rings of ND
-            if (!__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; return; }
+            if (!__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5))) { ok = false; return; }
             tc_fence_after();
             if (PC > 0) load_unit(0, part0 + buf * (uint32_t)A_ROWS, raw[0]);
             uint32_t sc_at = 0;
@@ -1173,7 +1131,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                     if (kb0 + i + 1 < KB) {
                       // warp-uniform outcome: the accesses to tensor memory are warp-collective
                       if (!__all_sync(0xffffffffu, next_done) &&
-                          !__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5, wait_ns))) { ok = false; return; }
+                          !__all_sync(0xffffffffu, mbar_wait_addr(sm, done0 + 8u * dn, dph, p.status, 5))) { ok = false; return; }
                       tc_fence_after();
                       if (PC > 0) load_unit(0, part0 + buf * (uint32_t)A_ROWS, raw[next_set]);
                     }
