@@ -262,9 +262,10 @@ size_t lo_block_int8_linear_split_workspace_bytes(int64_t M, int64_t N, int64_t 
 
 /*
  * The same linear on activations that are not quantised yet: x [M,K] of type x_dtype (LO_BF16 / LO_F16 / LO_F32,
- * 16-byte aligned) goes through lo_group_quant_int8 (group 128, eps 1e-10) into the workspace first.
+ * 16-byte aligned) goes through lo_group_quant_int8 (group 128, eps 1e-10) into the workspace first; up to four rows and a few
+ * million weights are one kernel without a workspace, with the same bits.
  * Replaces: apply_w8a8_block_int8_linear (python/lightop/_lmslim_native/layers/gemm/int8_utils.py:406-429).
- * workspace: lo_block_int8_linear_dynamic_workspace_bytes(M, N, K).
+ * workspace: lo_block_int8_linear_dynamic_workspace_bytes(M, N, K); may be null where that is 0.
  */
 size_t lo_block_int8_linear_dynamic_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int lo_block_int8_linear_dynamic(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N,

@@ -84,6 +84,10 @@ int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, co
                                int8_t *q_sorted, float *s_sorted, bool positions_first, cudaStream_t stream);
 
 // Group quantisation of rows of any supported type, for a dependent launch of the kernel that follows.  quant.cu
+// Linear of a few rows in one kernel (quant.cu): whether it takes the call, and the call.
+bool linear_rows_fit(int64_t M, int64_t N, int64_t K, int x_dtype);
+int launch_linear_rows(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K, float eps, void *C,
+                       cudaStream_t st);
 int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group_size, float eps, int8_t *q, float *s,
                        cudaStream_t stream);
 

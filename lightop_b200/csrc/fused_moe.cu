@@ -797,7 +797,8 @@ DynLinearLayout carve_dyn_linear(void *ws, int64_t M, int64_t K, const LinearPla
 }  // namespace lo
 
 extern "C" size_t lo_block_int8_linear_dynamic_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K < 128) return 0;
+  // (the one-kernel form keeps no scratch; where it depends on the type of x whether it takes the call, the answer serves all types)
+  if (M <= 0 || N <= 0 || K < 128 || lo::linear_rows_fit(M, N, K, LO_F32)) return 0;
   return lo::carve_dyn_linear(nullptr, M, K, lo::plan_linear(M, N, K)).bytes;
 }
 
@@ -807,9 +808,16 @@ extern "C" int lo_block_int8_linear_dynamic(const void *x, int x_dtype, const in
   using namespace lo;
   int rc = check_linear(M, N, K);
   if (rc != LO_OK || M == 0) return rc;
-  LO_REQUIRE(x && B && b_scale && C && workspace, "block int8 linear: null pointer");
+  const bool rows = linear_rows_fit(M, N, K, x_dtype);
+  LO_REQUIRE(x && B && b_scale && C && (workspace || rows), "block int8 linear: null pointer");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0, "group quant: x must be 16-byte and q 8-byte aligned");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "block int8 linear: workspace must be 256-byte aligned");
+  if (rows) {
+    // (the operands that the grouped GEMM refuses are refused here too)
+    LO_REQUIRE(aligned16(B, b_scale), "grouped gemm: operands and scales must be 16-byte aligned");
+    LO_REQUIRE((reinterpret_cast<uintptr_t>(C) & 1) == 0, "grouped gemm: the output must be aligned to its bf16 elements");
+    return launch_linear_rows(x, x_dtype, B, b_scale, M, N, K, 1e-10f, C, static_cast<cudaStream_t>(stream));
+  }
   const LinearPlan L = plan_linear(M, N, K);
   DynLinearLayout D = carve_dyn_linear(workspace, M, K, L);
   LO_REQUIRE(workspace_bytes >= D.bytes, "block int8 linear: workspace of %zu bytes, %zu needed", workspace_bytes, D.bytes);

@@ -404,6 +404,143 @@ int launch_typed(const void *x, int64_t num_groups, int group_size, float eps_t,
   return LO_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Dense block-INT8 linear of one to four rows in one kernel: quantisation, dot products, promotion.
+//
+// With so few rows the linear is a read of the weights; the tensor cores' tile (128 outputs, one CTA) leaves most SMs without work or
+// needs the K extent dealt out and a second kernel behind it, and quantisation is a launch of its own in front.  Here a CTA owns a
+// few outputs over the whole K extent: it quantises the rows itself (every CTA the same ones, from L2), takes the int32 dot
+// product of every 128-wide K block with dp4a, and carries the fp32 chain over the K blocks in their order: the arithmetic and
+// the bits of the quantiser and of the tensor-core forms.
+//
+// Bound by latency: one read of weights (the first loads in flight before the rows are quantised), the quantisation, the chain.  512
+// threads a CTA instead of 256 shorten the quantisation: 1 x 576 x 7168 5.2 -> 4.0 us, 1 x 4096 x 7168 14.0 -> 11.3.
+// ---------------------------------------------------------------------------
+constexpr int ROW_THREADS = 512, ROW_WARPS = ROW_THREADS / 32;
+constexpr int ROWS_MAX = 4;
+constexpr int ROW_AHEAD = 4;         // 16-byte weight loads a lane has in flight
+constexpr int KB_UNIT = 4;       // K blocks that a warp takes with one load: eight lanes each
+
+// Shared memory: codes [ROWS][K], scales [ROWS][KB], dot products as fp32 [outs][ROWS][KB].
+constexpr size_t rows_smem(int rows, int64_t KB, int outs) { return (size_t)rows * KB * 128 + (size_t)rows * KB * 4 + (size_t)outs * rows * KB * 4; }
+constexpr size_t ROWS_SMEM_PLAIN = 48 * 1024;      // what a kernel gets without asking
+
+template <typename T, int ROWS>
+__global__ void __launch_bounds__(ROW_THREADS) linear_rows_kernel(const T *__restrict__ x, const int8_t *__restrict__ B,
+                                                              const float *__restrict__ b_scale, int M, int N, int KB, int outs,
+                                                              float eps_t, __nv_bfloat16 *__restrict__ C) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint8_t *codes = smem;                                                  // [ROWS][KB * 128]
+  float *scale = reinterpret_cast<float *>(smem + ROWS * KB * 128);       // [ROWS][KB]: token scale, then times the weight block's
+  float *dots = scale + ROWS * KB;                                        // [outs][ROWS][KB]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n0 = blockIdx.x * outs;
+  const int64_t K = (int64_t)KB * 128;
+  const int units_per_row = (KB + KB_UNIT - 1) / KB_UNIT, units = outs * units_per_row;
+  dependency_wait();
+  dependency_release();      // (a dependent kernel waits for the whole grid before it reads)
+
+  // unit u: four K blocks of one output's weights, 512 consecutive bytes
+  auto load = [&](int u) {
+    const int r = u / units_per_row, kb = (u - r * units_per_row) * KB_UNIT + (lane >> 3);
+    if (u >= units || kb >= KB || n0 + r >= N) return make_uint4(0u, 0u, 0u, 0u);
+    return __ldg(reinterpret_cast<const uint4 *>(B + (int64_t)(n0 + r) * K + kb * 128 + (lane & 7) * 16));
+  };
+  uint4 w[ROW_AHEAD];
+#pragma unroll
+  for (int i = 0; i < ROW_AHEAD; ++i) w[i] = load(warp + i * ROW_WARPS);
+
+  // the rows, sixteen elements a thread (rows that do not exist: zero codes)
+  const int parts = ROWS * KB * 8, present = M * KB * 8;
+  for (int i0 = warp * 32; i0 < parts; i0 += ROW_THREADS) {
+    const int i = i0 + lane;
+    const bool active = i < present;
+    float v[16];
+    if (active) {
+      Load8<T>::load(x + (int64_t)i * 16, *reinterpret_cast<float (*)[8]>(&v[0]));
+      Load8<T>::load(x + (int64_t)i * 16 + 8, *reinterpret_cast<float (*)[8]>(&v[8]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = 0.f;
+    }
+    uint32_t packed[4] = {0u, 0u, 0u, 0u};
+    const float s = quantise<T, 8, 16>(v, eps_t, active, packed);
+    if (i < parts) {
+      *reinterpret_cast<uint4 *>(codes + i * 16) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+      // (a CTA's outputs lie in one block of 128 weight rows: their number is a power of two, at most 32)
+      if ((i & 7) == 0) {
+        const int g = i >> 3, kb = g % KB;
+        scale[g] = active ? __fmul_rn(s, __ldg(b_scale + (int64_t)(n0 / 128) * KB + kb)) : 0.f;
+      }
+    }
+  }
+  __syncthreads();
+
+  auto dot_unit = [&](int u, const uint4 &wv) {
+    const int r = u / units_per_row, kb = (u - r * units_per_row) * KB_UNIT + (lane >> 3);
+    int d[ROWS];
+#pragma unroll
+    for (int m = 0; m < ROWS; ++m) {
+      const uint4 a = kb < KB ? *reinterpret_cast<const uint4 *>(codes + (m * KB + kb) * 128 + (lane & 7) * 16) : make_uint4(0u, 0u, 0u, 0u);
+      d[m] = __dp4a((int)a.x, (int)wv.x, __dp4a((int)a.y, (int)wv.y, __dp4a((int)a.z, (int)wv.z, __dp4a((int)a.w, (int)wv.w, 0))));
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+      for (int m = 0; m < ROWS; ++m) d[m] += __shfl_xor_sync(0xffffffffu, d[m], off);
+    if ((lane & 7) == 0 && kb < KB) {
+#pragma unroll
+      for (int m = 0; m < ROWS; ++m) dots[(r * ROWS + m) * KB + kb] = __int2float_rn(d[m]);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < ROW_AHEAD; ++i)
+    if (warp + i * ROW_WARPS < units) dot_unit(warp + i * ROW_WARPS, w[i]);
+  for (int u0 = warp + ROW_AHEAD * ROW_WARPS; u0 < units; u0 += ROW_AHEAD * ROW_WARPS) {
+#pragma unroll
+    for (int i = 0; i < ROW_AHEAD; ++i) w[i] = load(u0 + i * ROW_WARPS);
+#pragma unroll
+    for (int i = 0; i < ROW_AHEAD; ++i)
+      if (u0 + i * ROW_WARPS < units) dot_unit(u0 + i * ROW_WARPS, w[i]);
+  }
+  __syncthreads();
+
+  // acc = fma(float(dot), a_s * b_s, acc) over the K blocks in their order
+  if (threadIdx.x < outs * ROWS) {
+    const int r = threadIdx.x / ROWS, m = threadIdx.x - r * ROWS;
+    if (m < M && n0 + r < N) {
+      const float *d = dots + threadIdx.x * KB, *s = scale + m * KB;
+      float acc = 0.f;
+#pragma unroll 8
+      for (int kb = 0; kb < KB; ++kb) acc = __fmaf_rn(d[kb], s[kb], acc);
+      C[(int64_t)m * N + n0 + r] = __float2bfloat16_rn(acc);
+    }
+  }
+}
+
+// Outputs a CTA: a power of two, two CTAs a SM where the outputs allow it.
+inline int rows_outs(int64_t N) {
+  int outs = 4;
+  while (outs < 32 && N > (int64_t)outs * 2 * sm_count()) outs *= 2;
+  return outs;
+}
+
+template <typename T>
+int launch_rows(const void *x, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K, float eps_t, void *C, cudaStream_t st) {
+  const int KB = (int)(K / 128);
+  const int outs = rows_outs(N);
+  const dim3 grid((unsigned)ceil_div(N, outs));
+  const T *xt = static_cast<const T *>(x);
+  __nv_bfloat16 *c = static_cast<__nv_bfloat16 *>(C);
+#define LO_ROWS_CASE(R) \
+  LO_CUDA_OK(launch_dependent(linear_rows_kernel<T, R>, grid, dim3(ROW_THREADS), rows_smem(R, KB, outs), st, xt, B, b_scale, (int)M, (int)N, KB, outs, eps_t, c))
+  if (M <= 1) LO_ROWS_CASE(1);
+  else if (M <= 2) LO_ROWS_CASE(2);
+  else LO_ROWS_CASE(ROWS_MAX);
+#undef LO_ROWS_CASE
+  return LO_OK;
+}
+
 }  // namespace
 
 // eps rounded to the element type of x, the way a torch clamp(min=eps) on a tensor of
@@ -440,6 +577,35 @@ int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group
       // 22.9 (from HBM 32.8, 30.9).
       return num_groups * group_size <= FP32_SMALL ? launch_typed<float, 8>(x, num_groups, group_size, eps_t, q, s, st)
                                                    : launch_typed<float, 16>(x, num_groups, group_size, eps_t, q, s, st);
+    default: return fail(LO_ERR_UNSUPPORTED, "group quant: unsupported input dtype code %d", x_dtype);
+  }
+}
+
+// Up to two rows and 30 million weights, three or four rows and 4.5 million: beyond, what every CTA spends on the same quantisation and on
+// dp4a is more than the launches it saves.  Device time in us of the kernels before (quantisation, GEMM, promotion where split) and
+// of this one, weights from HBM; a pass from Python is 16 to 18 us before and 11 to 12 now wherever the device takes less:
+//   1 row   576 x 7168 10.7, 4.0   1536 x 1536 6.8, 3.3   2048 x 4096 11.1, 4.9   7168 x 2048 8.4, 7.0   4096 x 7168 16.3, 11.3
+//   2 rows  576 x 7168 10.9, 5.1   1536 x 1536 6.8, 3.7   2048 x 4096 11.0, 6.5   7168 x 2048 8.4, 8.1   4096 x 7168 16.7, 14.0
+//   4 rows  576 x 7168 10.9, 7.3   1536 x 1536 6.8, 5.4   2304 x 1280  6.8, 5.5
+//   left to the others: 1 x 16384 x 2048 10.2, 13.0   1 x 7168 x 18432 34.9, 43.9   4 x 2048 x 4096 11.0, 12.0   4 x 1024 x 7168 12.2, 13.3
+// fp32 rows, whose quotients the library's division takes, less: 1 x 4096 x 7168 19.3, 15.8   2 x 1024 x 7168 15.0, 12.5   4 x 576 x 7168 14.2,
+// 12.7 but 2 x 7168 x 2048 12.7, 13.1   3 x 2304 x 1280 9.5, 10.3.
+bool linear_rows_fit(int64_t M, int64_t N, int64_t K, int x_dtype) {
+  if (M < 1 || M > ROWS_MAX || N < 1 || N >= (1LL << 31) || K > (1LL << 20)) return false;
+  const bool fp32 = x_dtype == LO_F32;
+  if (M > 2 && fp32 && N > 4 * sm_count()) return false;
+  const int64_t most = M > 2 ? 4500000 : (M == 2 && fp32 ? 14000000 : 30000000);
+  const int rows = M <= 2 ? (int)M : ROWS_MAX;
+  return N * K <= most && rows_smem(rows, K / 128, rows_outs(N)) <= ROWS_SMEM_PLAIN;
+}
+
+int launch_linear_rows(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K, float eps, void *C,
+                       cudaStream_t st) {
+  const float eps_t = round_eps_to_dtype(eps, x_dtype);
+  switch (x_dtype) {
+    case LO_BF16: return launch_rows<__nv_bfloat16>(x, B, b_scale, M, N, K, eps_t, C, st);
+    case LO_F16: return launch_rows<__half>(x, B, b_scale, M, N, K, eps_t, C, st);
+    case LO_F32: return launch_rows<float>(x, B, b_scale, M, N, K, eps_t, C, st);
     default: return fail(LO_ERR_UNSUPPORTED, "group quant: unsupported input dtype code %d", x_dtype);
   }
 }

@@ -83,7 +83,7 @@ def _dynamic_linear(x: torch.Tensor, w: torch.Tensor, block_size: List[int], w_s
     dev = x.device
     C = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=dev)
     nbytes = lib.lo_block_int8_linear_dynamic_workspace_bytes(M, N, K)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
     with _lib.on_device(dev):
         st = lib.lo_block_int8_linear_dynamic(_lib.ptr(x), _lib.dtype_code(x.dtype), _lib.ptr(w), _lib.ptr(bs), M, N, K,
                                               _lib.ptr(C), _lib.ptr(ws), nbytes, _lib.ptr(device_status_word(dev)),
