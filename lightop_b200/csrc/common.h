@@ -84,6 +84,12 @@ int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, co
                                int8_t *q_sorted, float *s_sorted, bool positions_first, cudaStream_t stream);
 
 // Group quantisation of rows of any supported type, for a dependent launch of the kernel that follows.  quant.cu
+// Alignment (segments of 16, chunk table) and launch_group_quant_scatter() in one kernel, for up to ROUTE_SMALL_IDS (token, slot) pairs.  quant.cu
+constexpr int ROUTE_SMALL_IDS = 256;
+bool route_quant_small_fits(int64_t M, int64_t H, int topk);
+int launch_route_quant_small(const void *x, int64_t M, int64_t H, int topk, const void *topk_ids, int ids_dtype, int num_experts,
+                             const int32_t *expert_map, float eps, int8_t *q_sorted, float *s_sorted, int32_t *sorted_ids, int64_t sorted_capacity,
+                             int32_t *num_tokens_post_pad, Chunk *chunks, int32_t *num_chunks, int64_t chunk_capacity, int chunk_max, cudaStream_t stream);
 // Linear of a few rows in one kernel (quant.cu): whether it takes the call, and the call.
 bool linear_rows_fit(int64_t M, int64_t N, int64_t K, int x_dtype);
 int launch_linear_rows(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K, float eps, void *C,
@@ -208,6 +214,20 @@ __device__ __forceinline__ float rcp_refined(float b) {
 __device__ __forceinline__ float div_by(float a, float b, float y) {
   const float q = __fmul_rn(a, y);
   return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// Expert of (token, slot) number i, through the map where map_mode is 1; -1 where there is none.
+template <typename IdT>
+__device__ __forceinline__ int load_expert(const IdT *ids, int64_t i, int64_t numel, int E,
+                                           const int32_t *expert_map, int map_mode) {
+  if (i >= numel) return -1;
+  long long e = (long long)ids[i];
+  if (e < 0 || e >= E) return -1;
+  if (map_mode == 1) {
+    e = expert_map[e];
+    if (e < 0 || e >= E) return -1;
+  }
+  return (int)e;
 }
 
 // Order-preserving unsigned key of a float, for warp reductions in one instruction: -0 like 0, NaN like -inf (never preferred).

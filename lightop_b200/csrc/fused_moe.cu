@@ -176,19 +176,27 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   int rc;
 
   const int chunk_max = chunk_rows_for(numel, align_E);
-  // 1. expert-major stable order, chunk table, position of every (token, slot)
   prof_mark(0, st);
-  rc = launch_align(topk_ids, ids_dtype, numel, align_E, FUSED_ALIGN_BLOCK, expert_map, expert_map ? 1 : 0,
-                    L.sorted_ids, L.sorted_cap, nullptr, 0, L.header, L.chunks, L.header + 1, L.chunk_cap, L.inv_pos,
-                    chunk_max, st);
-  if (rc != LO_OK) return rc;
+  if (route_quant_small_fits(M, H, topk)) {
+    // 1 and 2 in one kernel: a launch and the wait of one kernel for the other less
+    prof_mark(1, st);
+    rc = launch_route_quant_small(x, M, H, topk, topk_ids, ids_dtype, align_E, expert_map, 1e-10f, L.xq, L.xs, L.sorted_ids, L.sorted_cap,
+                                  L.header, L.chunks, L.header + 1, L.chunk_cap, chunk_max, st);
+    if (rc != LO_OK) return rc;
+  } else {
+    // 1. expert-major stable order, chunk table, position of every (token, slot)
+    rc = launch_align(topk_ids, ids_dtype, numel, align_E, FUSED_ALIGN_BLOCK, expert_map, expert_map ? 1 : 0,
+                      L.sorted_ids, L.sorted_cap, nullptr, 0, L.header, L.chunks, L.header + 1, L.chunk_cap, L.inv_pos,
+                      chunk_max, st);
+    if (rc != LO_OK) return rc;
 
-  // 2. activations -> int8 + per-128 scales, written once per routed slot into sorted order so
-  //    that every chunk of the grouped GEMM is a run of consecutive rows (one TMA box)
-  prof_mark(1, st);
-  rc = launch_group_quant_scatter(x, M, H, topk, L.inv_pos, 1e-10f, L.xq, L.xs,
-                                  expert_map != nullptr && positions_first(M, H, topk, E_local, align_E), st);
-  if (rc != LO_OK) return rc;
+    // 2. activations -> int8 + per-128 scales, written once per routed slot into sorted order so
+    //    that every chunk of the grouped GEMM is a run of consecutive rows (one TMA box)
+    prof_mark(1, st);
+    rc = launch_group_quant_scatter(x, M, H, topk, L.inv_pos, 1e-10f, L.xq, L.xs,
+                                    expert_map != nullptr && positions_first(M, H, topk, E_local, align_E), st);
+    if (rc != LO_OK) return rc;
+  }
 
   // 3. gate_up GEMM, SiLU*mul and re-quantisation in the epilogue -> act_q/act_s in sorted order
   prof_mark(2, st);

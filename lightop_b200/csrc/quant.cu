@@ -179,6 +179,123 @@ __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfl
 }
 
 // ---------------------------------------------------------------------------
+// Alignment and quantisation of a small call in one kernel.
+//
+// As kernels of their own the two are a launch each around a few hundred ids, and the second waits for one CTA of the first.  Here
+// every CTA works the positions out for itself: experts of all ids in shared memory, one id a thread, rank = earlier ids of the
+// same expert (counted by comparison), segments from one scan over the experts' counts.  CTA 0 writes the tables that the GEMMs
+// read; the others quantise a share of one token's row each and store it at the token's positions.  Same order, tables, codes
+// and scales as the two kernels.  Bound by latency (ids, count, scan, store).
+// ---------------------------------------------------------------------------
+constexpr int ROUTE_THREADS = 256, ROUTE_SEGMENT = 16;
+static_assert(ROUTE_SMALL_IDS == ROUTE_THREADS, "one id a thread");
+
+template <typename IdT>
+__global__ void __launch_bounds__(ROUTE_THREADS) route_quant_kernel(
+    const __nv_bfloat16 *__restrict__ x, int groups_per_row, int blocks_per_row, int topk, const IdT *__restrict__ ids, int numel, int E,
+    const int32_t *__restrict__ expert_map, int map_mode, float eps_t, int8_t *__restrict__ q_sorted, float *__restrict__ s_sorted,
+    int32_t *__restrict__ sorted_ids, int64_t sorted_capacity, int32_t *__restrict__ num_tokens_post_pad, Chunk *__restrict__ chunks,
+    int32_t *__restrict__ num_chunks, int64_t chunk_capacity, int chunk_max) {
+  __shared__ __align__(16) int32_t expert_of[ROUTE_SMALL_IDS];
+  __shared__ int32_t pos_of[ROUTE_SMALL_IDS];
+  __shared__ __align__(16) uint32_t count[1024];       // ids per expert
+  __shared__ __align__(16) uint32_t offset[1024];      // before the expert: padded rows in the low half, chunks in the high half
+  __shared__ uint32_t warp_tot[ROUTE_THREADS / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  *reinterpret_cast<uint4 *>(&count[tid * 4]) = make_uint4(0u, 0u, 0u, 0u);
+  dependency_wait();
+  dependency_release();
+  // a share of a token's row: eight lanes a group, sixteen elements a lane
+  const int share = (int)blockIdx.x - 1, token = share / blocks_per_row;
+  const int part = (share - token * blocks_per_row) * ROUTE_THREADS + tid;
+  const bool active = share >= 0 && part < groups_per_row * 8;
+  float v[16];
+  if (active) {
+    const __nv_bfloat16 *src = x + ((int64_t)token * groups_per_row * 8 + part) * 16;
+    Load8<__nv_bfloat16>::load(src, *reinterpret_cast<float (*)[8]>(&v[0]));
+    Load8<__nv_bfloat16>::load(src + 8, *reinterpret_cast<float (*)[8]>(&v[8]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = 0.f;
+  }
+  const int e = load_expert<IdT>(ids, tid, numel, E, expert_map, map_mode);
+  expert_of[tid] = e;
+  if (blockIdx.x == 0)
+    for (int64_t i = tid; i < sorted_capacity; i += ROUTE_THREADS) sorted_ids[i] = numel;
+  __syncthreads();
+  int rank = 0;
+  if (e >= 0) {
+    atomicAdd(&count[e], 1u);
+    for (int i = 0; i < tid; i += 4) {
+      const int4 o = *reinterpret_cast<const int4 *>(&expert_of[i]);
+      rank += (o.x == e) + (i + 1 < tid && o.y == e) + (i + 2 < tid && o.z == e) + (i + 3 < tid && o.w == e);
+    }
+  }
+  __syncthreads();
+  // exclusive scan over the experts, four a thread (E <= 1024)
+  {
+    const uint4 c4 = *reinterpret_cast<const uint4 *>(&count[tid * 4]);
+    const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+    uint32_t own[4], sum = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      own[i] = sum;
+      sum += (c[i] + ROUTE_SEGMENT - 1) / ROUTE_SEGMENT * ROUTE_SEGMENT + ((c[i] + chunk_max - 1) / chunk_max << 16);
+    }
+    uint32_t run = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, run, off);
+      if (lane >= off) run += t;
+    }
+    if (lane == 31) warp_tot[warp] = run;
+    __syncthreads();
+    uint32_t base = run - sum;
+#pragma unroll
+    for (int w = 0; w < ROUTE_THREADS / 32; ++w) base += w < warp ? warp_tot[w] : 0u;
+    *reinterpret_cast<uint4 *>(&offset[tid * 4]) = make_uint4(base + own[0], base + own[1], base + own[2], base + own[3]);
+    if (blockIdx.x == 0 && tid == ROUTE_THREADS - 1) {
+      const uint32_t total = base + sum;
+      *num_tokens_post_pad = (int32_t)(total & 0xffffu);
+      *num_chunks = (int64_t)(total >> 16) < chunk_capacity ? (int32_t)(total >> 16) : (int32_t)chunk_capacity;
+    }
+  }
+  __syncthreads();
+  const int pos = e >= 0 ? (int)(offset[e] & 0xffffu) + rank : -1;
+  if (blockIdx.x == 0) {
+    if (pos >= 0 && pos < sorted_capacity) sorted_ids[pos] = tid;
+    for (int x0 = tid; x0 < E; x0 += ROUTE_THREADS) {
+      // equal chunks, rounded up to segments, as the alignment kernel cuts them
+      const int c = (int)count[x0], nch = (c + chunk_max - 1) / chunk_max;
+      const int per = nch > 0 ? ((c + nch - 1) / nch + ROUTE_SEGMENT - 1) / ROUTE_SEGMENT * ROUTE_SEGMENT : 0;
+      int ci = (int)(offset[x0] >> 16);
+      for (int r = 0; r < c; r += per, ++ci)
+        if (ci < chunk_capacity) {
+          Chunk ch;
+          ch.expert = x0;
+          ch.row0 = (int)(offset[x0] & 0xffffu) + r;
+          ch.rows = c - r < per ? c - r : per;
+          ch.pad = (c - r - 1) / per;
+          chunks[ci] = ch;
+        }
+    }
+    return;
+  }
+  pos_of[tid] = pos;
+  __syncthreads();
+  uint32_t packed[4];
+  const float scale = quantise<__nv_bfloat16, 8, 16>(v, eps_t, active, packed);
+  if (!active) return;
+  const uint4 codes = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  for (int j = 0; j < topk; ++j) {
+    const int64_t p = pos_of[token * topk + j];
+    if (p < 0) continue;
+    *reinterpret_cast<uint4 *>(q_sorted + p * groups_per_row * 128 + part * 16) = codes;
+    if ((part & 7) == 0) s_sorted[p * groups_per_row + (part >> 3)] = scale;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Per-token (whole-row) INT8 quantisation, the activation format of the per-channel W8A8 mode.
 //
 // Arithmetic of the reference's kernel (python/lightop/_lmslim_native/layers/gemm/int8_utils.py:21-44):
@@ -561,6 +678,33 @@ int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, co
   LO_CUDA_OK(launch_dependent(group_quant_scatter_kernel, dim3((unsigned)blocks), dim3(256), 0, stream,
                               static_cast<const __nv_bfloat16 *>(x), M, (int)(H / 128), topk, inv_pos,
                               round_eps_to_dtype(eps, LO_BF16), q_sorted, s_sorted, positions_first ? 1 : 0));
+  return LO_OK;
+}
+
+// Up to 256 ids and one CTA a SM for the rows; every CTA repeats the counting, so more of them take longer than one that counts for all.
+// Layers in a graph in us, as two kernels and as one (experts 256, narrow, unless said):
+//   top-8 of 1 x 7168 44.9, 42.2   8 x 7168 71.5, 69.2   32 x 7168 170.2, 169.6 (one shard of eight 50.2, 49.4)   4 x 4096, Qwen3 widths 107.2, 103.9
+//   top-2 of 32 x 256 17.7, 15.7   128 x 2048 27.8, 26.4     top-1 of 256 x 1024 (256 CTAs) 26.6, 26.6   256 x 7168 (512) 50.5, 53.0
+bool route_quant_small_fits(int64_t M, int64_t H, int topk) {
+  return M * topk <= ROUTE_SMALL_IDS && M * ceil_div(H / 128 * 8, ROUTE_THREADS) <= sm_count();
+}
+int launch_route_quant_small(const void *x, int64_t M, int64_t H, int topk, const void *topk_ids, int ids_dtype, int num_experts,
+                             const int32_t *expert_map, float eps, int8_t *q_sorted, float *s_sorted, int32_t *sorted_ids, int64_t sorted_capacity,
+                             int32_t *num_tokens_post_pad, Chunk *chunks, int32_t *num_chunks, int64_t chunk_capacity, int chunk_max, cudaStream_t stream) {
+  LO_REQUIRE(M >= 1 && topk >= 1 && M * topk <= ROUTE_SMALL_IDS && H % 128 == 0 && num_experts >= 1 && num_experts <= 1024, "route and quantise: bad shape");
+  const int groups = (int)(H / 128), per_row = (int)ceil_div(groups * 8, ROUTE_THREADS);
+  const dim3 grid((unsigned)(1 + M * per_row));
+  const int map_mode = expert_map ? 1 : 0;
+  const float eps_t = round_eps_to_dtype(eps, LO_BF16);
+  const __nv_bfloat16 *xt = static_cast<const __nv_bfloat16 *>(x);
+  if (ids_dtype == LO_I32)
+    LO_CUDA_OK(launch_dependent(route_quant_kernel<int32_t>, grid, dim3(ROUTE_THREADS), 0, stream, xt, groups, per_row, topk, static_cast<const int32_t *>(topk_ids),
+                                (int)(M * topk), num_experts, expert_map, map_mode, eps_t, q_sorted, s_sorted, sorted_ids, sorted_capacity, num_tokens_post_pad,
+                                chunks, num_chunks, chunk_capacity, chunk_max));
+  else
+    LO_CUDA_OK(launch_dependent(route_quant_kernel<int64_t>, grid, dim3(ROUTE_THREADS), 0, stream, xt, groups, per_row, topk, static_cast<const int64_t *>(topk_ids),
+                                (int)(M * topk), num_experts, expert_map, map_mode, eps_t, q_sorted, s_sorted, sorted_ids, sorted_capacity, num_tokens_post_pad,
+                                chunks, num_chunks, chunk_capacity, chunk_max));
   return LO_OK;
 }
 

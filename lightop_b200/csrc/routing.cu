@@ -132,19 +132,6 @@ int launch_topk_ids(const void *gating, int64_t M, int E, int k, int renorm, flo
 constexpr int ALIGN_WARPS = 32;
 
 template <typename IdT>
-__device__ __forceinline__ int load_expert(const IdT *ids, int64_t i, int64_t numel, int E,
-                                           const int32_t *expert_map, int map_mode) {
-  if (i >= numel) return -1;
-  long long e = (long long)ids[i];
-  if (e < 0 || e >= E) return -1;
-  if (map_mode == 1) {
-    e = expert_map[e];
-    if (e < 0 || e >= E) return -1;
-  }
-  return (int)e;
-}
-
-template <typename IdT>
 __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_kernel(
     const IdT *__restrict__ ids, int64_t numel, int E, int block_size, const int32_t *__restrict__ expert_map,
     int map_mode, int32_t *__restrict__ sorted_ids, int64_t sorted_capacity, int32_t *__restrict__ expert_ids,
