@@ -2,6 +2,7 @@
 // (histogram + prefix scan + stable scatter) with the grouped-GEMM chunk table.
 #include "common.h"
 #include <cooperative_groups.h>
+#include <type_traits>
 
 namespace lo {
 namespace {
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// The same alignment for many ids, as a thread-block CLUSTER of ALIGN_CLUSTER CTAs (one launch).
+// The same alignment for many ids, as a thread-block CLUSTER of 8 or 16 CTAs (one launch).
 // The single-CTA kernel above is bound by the instruction issue rate of its one SM (about 140
 // instructions per warp step over 32 k ids at the prefill size).  Here CTA r of the cluster takes the r-th
 // contiguous slice of the ids; the CTAs exchange their per-expert counts through distributed shared
@@ -290,12 +291,17 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_kernel(
 //   CTA + seen so far by this warp + rank inside the warp step,
 // i.e. still ascending flat index inside an expert: bit-identical to the single-CTA kernel.
 // ---------------------------------------------------------------------------
-constexpr int ALIGN_CLUSTER = 8;
-// One CTA against the cluster, in us: 2048 ids 10.1, 8.1; 2400 ids 11.6, 8.5; 4800 ids 15.8, 9.4; 6216 ids 17.5, 9.0.  Below, a warp has a
+constexpr int ALIGN_CLUSTER = 8, ALIGN_CLUSTER_WIDE = 16;
+constexpr int ALIGN_BATCH = 128;      // ids a warp has in flight
+// One CTA against the cluster of 8, in us: 2048 ids 10.1, 8.1; 2400 ids 11.6, 8.5; 4800 ids 15.8, 9.4; 6216 ids 17.5, 9.0.  Below, a warp has a
 // step or two and the exchange between the CTAs is what is left.
 constexpr int64_t ALIGN_CLUSTER_MIN_IDS = 2048;
+// Cluster of 8 with one id after the other, with batches of loads, and cluster of 16 with batches, in us (256 experts, in a graph): 2400 ids
+// (128 experts) 6.3, 6.2, 6.1; 6216 ids 7.3, 7.3, 6.9; 16384 9.3, 8.9, 7.8; 32768 13.0, 11.6, 9.7; 65536 18.2, 15.1, 12.1; 262144 53.9, 44.1, 25.0.
+// With 1024 experts the sixteen tables cost more: 2049 ids 8.8, 8.7, 11.0; 131072 31.7, 28.8, 20.6.
+constexpr int64_t ALIGN_WIDE_MIN_IDS = 6144;
 
-template <typename IdT>
+template <typename IdT, int C>
 __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
     const IdT *__restrict__ ids, int64_t numel, int E, int block_size, const int32_t *__restrict__ expert_map,
     int map_mode, int32_t *__restrict__ sorted_ids, int64_t sorted_capacity, int32_t *__restrict__ expert_ids,
@@ -303,7 +309,6 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
     int32_t *__restrict__ num_chunks, int64_t chunk_capacity, int32_t *__restrict__ inv_pos, int chunk_max) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  const int C = (int)cluster.num_blocks();
   const int r = (int)cluster.block_rank();
   extern __shared__ int32_t smem[];
   int32_t *hist = smem;                       // [ALIGN_WARPS][E] per-warp counts, then exclusive prefixes inside this CTA
@@ -313,6 +318,7 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
   int32_t *warp_tot = chunk_off + (E + 1);    // [2][32]
   int32_t *cta_cnt = warp_tot + 64;           // [E] ids per expert in this CTA's slice (read by the other CTAs)
   int32_t *before = cta_cnt + E;              // [E] ids per expert in lower-ranked CTAs
+  int16_t *experts = reinterpret_cast<int16_t *>(before + E);      // [ALIGN_WARPS][ALIGN_BATCH] experts of the ids at hand
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < ALIGN_WARPS * E; i += blockDim.x) hist[i] = 0;
@@ -334,27 +340,56 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
   const int id_bits = seg_len >= 256 ? 32 - __clz(E > 1 ? E - 1 : 1) : 0;
   int32_t *my_hist = hist + warp * E;
 
-  for (int64_t base = seg_begin; base < seg_end; base += 32) {
-    const int e = load_expert<IdT>(ids, base + lane, seg_end, E, expert_map, map_mode);
-    if (e >= 0) atomicAdd(&my_hist[e], 1);
+  int16_t *mine = experts + warp * ALIGN_BATCH;
+  // A batch of ids: all loads of the ids, then all look-ups in the map, in flight together; lane l keeps the places l, l + 32, ...
+  auto fetch = [&](int64_t base) {
+    constexpr int N = ALIGN_BATCH / 32;
+    long long id[N];
+    int e[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const int64_t i = base + j * 32 + lane;
+      id[j] = i < seg_end ? (long long)ids[i] : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      e[j] = id[j] < 0 || id[j] >= E ? -1 : (int)id[j];
+      if (map_mode == 1 && e[j] >= 0) e[j] = expert_map[e[j]];
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) mine[j * 32 + lane] = (int16_t)(e[j] < 0 || e[j] >= E ? -1 : e[j]);
+  };
+  for (int64_t base = seg_begin; base < seg_end; base += ALIGN_BATCH) {
+    fetch(base);
+#pragma unroll 1
+    for (int j = lane; j < ALIGN_BATCH; j += 32)
+      if (mine[j] >= 0) atomicAdd(&my_hist[mine[j]], 1);
   }
   __syncthreads();
   for (int e = tid; e < E; e += blockDim.x) {
     int run = 0;
-    for (int w = 0; w < ALIGN_WARPS; ++w) {
-      const int c = hist[w * E + e];
-      hist[w * E + e] = run;
-      run += c;
+#pragma unroll 1
+    for (int w0 = 0; w0 < ALIGN_WARPS; w0 += 8) {
+      int c[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) c[w] = hist[(w0 + w) * E + e];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        hist[(w0 + w) * E + e] = run;
+        run += c[w];
+      }
     }
     cta_cnt[e] = run;
   }
   cluster.sync();      // every CTA's counts are published (and the sentinel fill is complete everywhere)
   for (int e = tid; e < E; e += blockDim.x) {
-    int total = 0, lower = 0;
+    int total = 0, lower = 0, v[C];
+#pragma unroll
+    for (int rr = 0; rr < C; ++rr) v[rr] = cluster.map_shared_rank(cta_cnt, rr)[e];
+#pragma unroll
     for (int rr = 0; rr < C; ++rr) {
-      const int v = cluster.map_shared_rank(cta_cnt, rr)[e];
-      total += v;
-      if (rr < r) lower += v;
+      total += v[rr];
+      if (rr < r) lower += v[rr];
     }
     count[e] = total;
     before[e] = lower;
@@ -432,25 +467,83 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
     }
   }
 
-  // stable scatter of this CTA's slice
-  for (int64_t base = seg_begin; base < seg_end; base += 32) {
-    const int e = load_expert<IdT>(ids, base + lane, seg_end, E, expert_map, map_mode);
-    const unsigned peers = peers_of(e, id_bits);
-    const int rank = __popc(peers & ((1u << lane) - 1u));
-    int prior = 0;
-    if (e >= 0) prior = my_hist[e];
-    __syncwarp();
-    if (e >= 0) {
-      const int64_t pos = (int64_t)seg_off[e] + before[e] + prior + rank;
-      if (pos < sorted_capacity) sorted_ids[pos] = (int32_t)(base + lane);
-      if (inv_pos) inv_pos[base + lane] = (int32_t)pos;
-      if (lane == (__ffs(peers) - 1)) my_hist[e] = prior + __popc(peers);
-    } else if (inv_pos && base + lane < seg_end) {
-      inv_pos[base + lane] = -1;
+  // stable scatter of this CTA's slice (the experts of a segment of one batch are still in shared memory)
+  for (int64_t batch = seg_begin; batch < seg_end; batch += ALIGN_BATCH) {
+    if (seg_len > ALIGN_BATCH) fetch(batch);
+#pragma unroll 1
+    for (int j = lane; j < ALIGN_BATCH && batch + j - lane < seg_end; j += 32) {
+      const int e = mine[j];
+      const unsigned peers = peers_of(e, id_bits);
+      const int rank = __popc(peers & ((1u << lane) - 1u));
+      int prior = 0;
+      if (e >= 0) prior = my_hist[e];
+      __syncwarp();
+      if (e >= 0) {
+        const int64_t pos = (int64_t)seg_off[e] + before[e] + prior + rank;
+        if (pos < sorted_capacity) sorted_ids[pos] = (int32_t)(batch + j);
+        if (inv_pos) inv_pos[batch + j] = (int32_t)pos;
+        if (lane == (__ffs(peers) - 1)) my_hist[e] = prior + __popc(peers);
+      } else if (inv_pos && batch + j < seg_end) {
+        inv_pos[batch + j] = -1;
+      }
+      __syncwarp();
     }
-    __syncwarp();
   }
   cluster.sync();      // no CTA leaves while another may still read its counts
+}
+
+template <int C> cudaLaunchConfig_t cluster_config(cudaLaunchAttribute (&attr)[2], size_t smem, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C, 1, 1);
+  cfg.blockDim = dim3(ALIGN_WARPS * 32, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cfg;
+}
+
+template <typename IdT, int C, typename... Args> int launch_cluster(size_t smem, cudaStream_t stream, Args... args) {
+  auto kernel = align_cluster_kernel<IdT, C>;
+  // (both belong to the (kernel, device) pair: set whenever a launch needs them, whichever device is current)
+  if (C > 8) LO_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  if (smem > 48 * 1024) LO_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = cluster_config<C>(attr, smem, stream);
+  g_launch_count.fetch_add(1, std::memory_order_relaxed);
+  LO_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return LO_OK;
+}
+
+constexpr size_t cluster_smem(int E) {
+  return sizeof(int32_t) * ((size_t)ALIGN_WARPS * E + 5 * (size_t)E + 2 + 64) + sizeof(int16_t) * ALIGN_WARPS * ALIGN_BATCH;
+}
+
+// Whether the device has room for a cluster of 16 (a size that a part with smaller clusters of SMs need not have): asked once a device.
+bool wide_cluster_fits() {
+  static std::atomic<int8_t> known[64];      // 0: not asked, 1: yes, 2: no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  int8_t k = known[dev].load(std::memory_order_relaxed);
+  if (k == 0) {
+    auto kernel = align_cluster_kernel<int32_t, ALIGN_CLUSTER_WIDE>;
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = cluster_config<ALIGN_CLUSTER_WIDE>(attr, cluster_smem(1024), nullptr);
+    int clusters = 0;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem(1024)) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+    if (!ok) (void)cudaGetLastError();
+    k = ok ? 1 : 2;
+    known[dev].store(k, std::memory_order_relaxed);
+  }
+  return k == 1;
 }
 
 }  // namespace
@@ -469,40 +562,19 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
   const size_t smem = sizeof(int32_t) * ((size_t)ALIGN_WARPS * num_experts + 3 * (size_t)num_experts + 2 + 64);
   cudaError_t e;
   if (numel >= ALIGN_CLUSTER_MIN_IDS && (ids_dtype == LO_I32 || ids_dtype == LO_I64)) {
-    // many ids: one cluster of ALIGN_CLUSTER CTAs
-    const size_t csmem = smem + sizeof(int32_t) * 2 * (size_t)num_experts;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ALIGN_CLUSTER, 1, 1);
-    cfg.blockDim = dim3(ALIGN_WARPS * 32, 1, 1);
-    cfg.dynamicSmemBytes = csmem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ALIGN_CLUSTER;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    if (ids_dtype == LO_I32) {
-      if (csmem > 48 * 1024)
-        LO_CUDA_OK(cudaFuncSetAttribute(align_cluster_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
-      g_launch_count.fetch_add(1, std::memory_order_relaxed);
-      LO_CUDA_OK(cudaLaunchKernelEx(&cfg, align_cluster_kernel<int32_t>, static_cast<const int32_t *>(topk_ids), numel,
-                                    num_experts, block_size, expert_map, map_mode, sorted_ids, sorted_capacity, expert_ids,
-                                    expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos,
-                                    chunk_max));
-    } else {
-      if (csmem > 48 * 1024)
-        LO_CUDA_OK(cudaFuncSetAttribute(align_cluster_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
-      g_launch_count.fetch_add(1, std::memory_order_relaxed);
-      LO_CUDA_OK(cudaLaunchKernelEx(&cfg, align_cluster_kernel<int64_t>, static_cast<const int64_t *>(topk_ids), numel,
-                                    num_experts, block_size, expert_map, map_mode, sorted_ids, sorted_capacity, expert_ids,
-                                    expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos,
-                                    chunk_max));
-    }
-    return LO_OK;
+    // many ids: one cluster
+    const size_t csmem = cluster_smem(num_experts);
+    auto launch = [&](auto *typed) -> int {
+      using IdT = typename std::remove_const<typename std::remove_pointer<decltype(typed)>::type>::type;
+      auto with = [&](auto width) -> int {
+        return launch_cluster<IdT, decltype(width)::value>(csmem, stream, typed, numel, num_experts, block_size, expert_map, map_mode, sorted_ids,
+                                                           sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks,
+                                                           chunk_capacity, inv_pos, chunk_max);
+      };
+      return numel >= ALIGN_WIDE_MIN_IDS && wide_cluster_fits() ? with(std::integral_constant<int, ALIGN_CLUSTER_WIDE>{})
+                                                                : with(std::integral_constant<int, ALIGN_CLUSTER>{});
+    };
+    return ids_dtype == LO_I32 ? launch(static_cast<const int32_t *>(topk_ids)) : launch(static_cast<const int64_t *>(topk_ids));
   }
   if (ids_dtype == LO_I32) {
     // the opt-in belongs to the (kernel, device) pair: set whenever a launch needs it, whichever device is current
