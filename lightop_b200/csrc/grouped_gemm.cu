@@ -62,10 +62,13 @@
 namespace lo {
 namespace {
 
-// Interval between two polls of a barrier, in nanoseconds: none.  try_wait parks the thread for a while by itself; a sleep on top of
-// it, or its form with a time hint, is more code in the loops of all roles (4096 tokens 3147 -> 3091 us without
-// either, Qwen3 2048 Zipf 935 -> 892, sharded 8192 797 -> 789; sleeps of 100 ns to 2 us by role lost half of it or all).
-constexpr uint32_t LO_SLEEP = 0u, LO_SLEEP_MMA = 0u;
+// How a wait polls, by the chunk cap of the instantiation (see Smem::POLL).  The plain form is the shortest in the loops of all roles, which
+// share the instruction caches: with sleeps and hints in their place 4096 tokens took 3147 us instead of 3091, Qwen3 2048 Zipf 935 instead of
+// 892, sharded 8192 797 instead of 789.  Where the weights bound the kernel, the board's power does: 32 tokens in a graph 1066 plain, 1055
+// with sleeps; 64 tokens (cap 64) 1419 plain, 1422 to 1424 with sleeps, 1415 with a hint.
+enum Poll { PLAIN, HINT, SLEEP };
+// SLEEP: interval between two polls in nanoseconds, by role
+constexpr uint32_t LO_SLEEP_PRODUCER = 128u, LO_SLEEP_SCALE = 128u, LO_SLEEP_MMA = 20u, LO_SLEEP_PROMO = 32u, LO_SLEEP_OUT = 256u;
 
 constexpr int TILE_N = 128;      // weight rows per accumulator (MMA M)
 constexpr int TILE_K = 128;      // int8 elements (= bytes) per K block
@@ -130,6 +133,7 @@ static_assert(ring_depths<GEMM_CHANNEL, 64>(9, 8) && ring_depths<GEMM_CHANNEL, 1
 
 template <int MODE, int A_ROWS> struct Smem {
   using C = Cfg<MODE, A_ROWS>;
+  static constexpr int POLL = A_ROWS <= 32 ? SLEEP : (A_ROWS <= 64 && MODE != GEMM_CHANNEL ? HINT : PLAIN);
   // operand tiles first: each is a multiple of 1024 bytes, base is 1024-aligned
   uint8_t w[C::NW][W_TILE_BYTES];
   uint8_t a[C::NA][C::A_TILE_BYTES];
@@ -167,16 +171,25 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// One poll; the hardware may park the thread for a short while before it answers no.
-__device__ __forceinline__ bool mbar_try_wait_addr(uint32_t bar, uint32_t parity) {
+// One poll; the hardware may park the thread for a short while, or for up to the hint's time, before it answers no.
+template <int POLL> __device__ __forceinline__ bool mbar_try_wait_addr(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if (POLL == HINT)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(200000u)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 // Upper bound of one wait, in SM clock cycles (about 1.5 s at 1.9 GHz; below 2^32, so the low half of the clock measures it).
@@ -185,23 +198,23 @@ constexpr uint32_t WAIT_LIMIT_CYCLES = 3000000000u;
 // Bounded wait.  Returns false when the CTA is aborting (this waiter timed out or another one did); `code` identifies the waiter
 // in the status word.  Short on purpose: it is inlined into the loops of all roles, which share the instruction caches.
 template <class S>
-__device__ __forceinline__ bool mbar_wait_addr(S &sm, uint32_t bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP) {
-  if (mbar_try_wait_addr(bar, parity)) return true;
+__device__ __forceinline__ bool mbar_wait_addr(S &sm, uint32_t bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP_PROMO) {
+  if (mbar_try_wait_addr<S::POLL>(bar, parity)) return true;
   const uint32_t t0 = (uint32_t)clock();
 #pragma unroll 1
-  while (!mbar_try_wait_addr(bar, parity)) {
+  while (!mbar_try_wait_addr<S::POLL>(bar, parity)) {
     if (sm.abort_flag) return false;
     if ((uint32_t)clock() - t0 > WAIT_LIMIT_CYCLES) {
       sm.abort_flag = 1;
       if (status) atomicCAS(status, 0, code);
       return false;
     }
-    if (sleep_ns > 0u) __nanosleep(sleep_ns);
+    if (S::POLL == SLEEP) __nanosleep(sleep_ns);
   }
   return true;
 }
 template <class S>
-__device__ __forceinline__ bool mbar_wait(S &sm, uint64_t *bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP) {
+__device__ __forceinline__ bool mbar_wait(S &sm, uint64_t *bar, uint32_t parity, int32_t *status, int code, uint32_t sleep_ns = LO_SLEEP_PROMO) {
   return mbar_wait_addr(sm, smem_u32(bar), parity, status, code, sleep_ns);
 }
 // One non-blocking look at a barrier: has the phase of this parity completed?
@@ -597,7 +610,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             const int32_t row_g = (int32_t)(ch.expert * p.n_rows_per_expert + (int64_t)(ph * p.n_tiles + nt) * TILE_N);
             for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NW
-              if (it >= (uint32_t)NW && !mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 1)) { ok = false; break; }
+              if (it >= (uint32_t)NW && !mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 1, LO_SLEEP_PRODUCER)) { ok = false; break; }
               mbar_arrive_expect_tx(&sm.ready[it % ND], W_TILE_BYTES);
               tma_load_2d(sm.w[s], &w_map, kb * TILE_K, row_g, &sm.ready[it % ND], pol_w);
               s = s + 1 == NW ? 0 : s + 1;
@@ -624,7 +637,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           for (int ph = 0; ph < PHASES && ok; ++ph) {
             for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NA
-              if (it >= (uint32_t)NA && !mbar_wait(sm, &sm.done[(it - NA) % ND], ((it - NA) / ND) & 1u, p.status, 6)) { ok = false; break; }
+              if (it >= (uint32_t)NA && !mbar_wait(sm, &sm.done[(it - NA) % ND], ((it - NA) / ND) & 1u, p.status, 6, LO_SLEEP_PRODUCER)) { ok = false; break; }
               uint64_t *bar = &sm.ready[it % ND];
               mbar_arrive_expect_tx(bar, a_bytes);
               tma_load_2d(sm.a[s], &a_maps.m[mi], kb * TILE_K, ch.row0, bar, pol_a);
@@ -700,7 +713,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           if (nxt.valid) fetch(nxt, a_nxt, b_nxt);
           // the slot's previous batch has been read when the partial of its last step has been consumed
           if (n_batch >= (uint32_t)SC_BATCHES &&
-              !__all_sync(0xffffffffu, mbar_wait(sm, &sm.consumed[end_of[0] % ND], (end_of[0] / ND) & 1u, p.status, 4))) break;
+              !__all_sync(0xffffffffu, mbar_wait(sm, &sm.consumed[end_of[0] % ND], (end_of[0] / ND) & 1u, p.status, 4, LO_SLEEP_SCALE))) break;
           const int T = (cur.ch.rows + 15) & ~15;
           float *sc = &sm.sc[slot * SC_STEPS][0];
 #pragma unroll
@@ -822,7 +835,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       if constexpr (MODE == GEMM_GATE_UP) {
         // A row of the tile is one token's 128-channel quantisation group: |act| maximum over the warp (four channels
         // per lane), scale = max / 127, q = trunc(clamp(act / scale)), one 4-byte store per lane.
-        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9, LO_SLEEP_OUT))) break;
         const int64_t I = (int64_t)p.n_tiles * TILE_N;
         int8_t *q_out = p.act_q + (int64_t)ch.row0 * I + (int64_t)nt * TILE_N + lane * 4;
         float *s_out = p.act_s + (int64_t)ch.row0 * p.n_tiles + nt;
@@ -885,7 +898,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             }
           }
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.stg_full, par, p.status, 9, LO_SLEEP_OUT))) break;
         const int64_t n0 = (int64_t)nt * TILE_N + (lane & 15) * 8;
         const int n_steps = (ch.rows + 2 * OUT_WARPS - 1) / (2 * OUT_WARPS);
 #pragma unroll 4
