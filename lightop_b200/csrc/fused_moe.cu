@@ -56,16 +56,19 @@ FusedLayout carve_fused(void *ws, int64_t M, int num_experts_for_align, int topk
 
 // Chunk sizes of the block-scaled layer, by the rows an expert gets on average (rows / experts).  The GEMM is instantiated per
 // chunk cap and the caps differ in what fits beside the operands: 8 weight slots and 8 partial buffers with 64 rows, 7 and 4
-// with 128, 5 and 3 with 160.  Layer times in us, DeepSeek-V3 shape, caps of 64 / 128 / 160 rows:
-//   rows per expert     16                     48                     64                     112                    128                    187
-//   even routing        1688 / 1765 / 1861     1830 / 2040 / 2257     2455 / 2196 / 2499     3386 / 2837 / 3084     4002 / 3633 / 3236     5393 / 4801 / 5213
-//   Zipf (1.2) routing   761 /  777 /  890     1472 / 1384 / 1599     1901 / 1820 / 2112     3080 / 2816 / 3050     3438 / 3042 / 3331     4804 / 4165 / 4344
+// with 128, 5 and 3 with 160.  Layer times in us, caps of 64 / 128 / 160 rows:
+//   rows per expert               48                     56                     64                    100                   112                   120
+//   Qwen3 shape, even routing     423 /  454 /  472      460 /  482 /  503      544 /  485 /  520     742 /  625 /  643     770 /  640 /  663     827 /  723 /  673
+//   DeepSeek-V3, even            1876 / 2006 / 2073     2026 / 2066 / 2143                           3461 / 2648 / 2735    3568 / 2807 / 2791    3686 / 2987 / 2848
+//   rows per expert              128                    156 (shard)            181                   203 (shard)           256
+//   Qwen3 shape (shards: DeepSeek-V3, one of eight), even   929 / 815 / 739    650 / 607 / 556     1193 / 1099 / 1122     825 / 698 / 700     1568 / 1402 / 1336
+//   Qwen3, Zipf (1.2) routing     892 /  845 /  880                                                                                           1529 / 1383 / 1398
 //   <= 48 rows per expert : 64-row chunks.  A weight-streaming call wants the deep rings, and the few experts that do get
-//                           more rows have a second chunk (at 56 still 1944 / 2048 / 2319 with even routing).
+//                           more rows have a second chunk (with even routing up to 56).
 //   49 .. 119             : 128-row chunks
 //   >= 120                : 160-row chunks: with 128 rows per expert half of the experts have a few rows more than 128, and a
-//                           second chunk means a second pass over the expert's weights.  That holds up to about 150 rows per
-//                           expert (144: 4661 / 4305 / 3802); above, and with skewed routing, 128-row chunks are ahead again.
+//                           second chunk means a second pass over the expert's weights.  With skewed routing 128-row chunks are up to 4 %
+//                           ahead, with about 190 rows per expert (two chunks of fewer than 128 rows either way) up to 2 %.
 constexpr int CHUNK_ROWS = 128;
 constexpr int CHUNK_ROWS_WIDE = 160;
 constexpr int CHUNK_ROWS_SMALL = 64;
