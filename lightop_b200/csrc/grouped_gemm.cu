@@ -41,8 +41,9 @@
 // through the issuer, a thread on one channel and 16 tokens, two issuer warps and the output in the promotion warps):
 // 64 tokens 1764 -> 1480 us, 777 tokens 2290 -> 1880 us, 4096 tokens 3850 -> 3340 us on one board (others: 1415, 1740, 2880 to 3000
 // now).  The board is at its power cap in all of these (SM clock 1.35 to 1.5 GHz), so what a change saves in cycles comes back
-// as time only in part.  What the roles execute counts twice: the loops of sixteen warps share the instruction caches, and shorter
-// waits and a scale loop of half the length made 4096 tokens 4 % and Zipf routing 7 % faster with the same arithmetic.
+// as time only in part.  Instructions besides the arithmetic cost at the cap as well: shorter waits and a scale loop of half the length
+// made 4096 tokens 4 % and Zipf routing 7 % faster there (at burst clocks the launches take the same time; down GEMM without an
+// instruction to issue 1.13 -> 0.90 warps per issue).
 //
 // Per-channel mode (one scale per token and one per output channel instead of 128x128 blocks) uses the same feed without the
 // promotion: a tensor-memory buffer is the int32 accumulator of a whole item, summed over every K block by the tensor core, and
@@ -63,8 +64,8 @@
 namespace lo {
 namespace {
 
-// How a wait polls, by the chunk cap of the instantiation (see Smem::POLL).  The plain form is the shortest in the loops of all roles, which
-// share the instruction caches: with sleeps and hints in their place 4096 tokens took 3147 us instead of 3091, Qwen3 2048 Zipf 935 instead of
+// How a wait polls, by the chunk cap of the instantiation (see Smem::POLL).  The plain form is the shortest in the loops of all roles,
+// which share the instruction caches and the power: with sleeps and hints in their place 4096 tokens took 3147 us instead of 3091, Qwen3 2048 Zipf 935 instead of
 // 892, sharded 8192 797 instead of 789.  Where the weights bound the kernel, the board's power does: 32 tokens in a graph 1066 plain, 1055
 // with sleeps; 64 tokens (cap 64) 1419 plain, 1422 to 1424 with sleeps, 1415 with a hint.
 enum Poll { PLAIN, HINT, SLEEP };
@@ -656,9 +657,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       // for the tables by themselves, four K-block steps at a time: a hand-over per step through the MMA issuer made this
       // warp's chain (wait, multiply, store, arrive: 900 cycles) the slowest of the kernel.  Scales come from L2 (the chunk's
       // scale rows are read by every output tile of the expert), one batch ahead, across the ends of passes and items.  Rows
-      // of scales whose length is a multiple of four are read with 16-byte loads, in a loop of its own: with the choice inside the
-      // loop its code was twice as long, and what this warp fetches of instructions the promotion warps on the same scheduler wait
-      // for (4096 tokens 3091 -> 3015 us, Qwen3 2048 Zipf 892 -> 867).
+      // of scales whose length is a multiple of four are read with 16-byte loads, in a loop of its own: with the choice inside the loop
+      // its code was twice as long, at the cost of the promotion warps on the same scheduler too
+      // (4096 tokens 3091 -> 3015 us, Qwen3 2048 Zipf 892 -> 867).
       if constexpr (MODE != GEMM_CHANNEL && FORM != SPLIT) {
         constexpr int NU = (A_ROWS + 31) / 32;
         const int64_t nblk = (p.n_rows_per_expert + TILE_N - 1) / TILE_N;
