@@ -535,6 +535,7 @@ int launch_typed(const void *x, int64_t num_groups, int group_size, float eps_t,
 // ---------------------------------------------------------------------------
 constexpr int ROW_THREADS = 512, ROW_WARPS = ROW_THREADS / 32;
 constexpr int ROWS_MAX = 4;
+constexpr int ROW_OUTS_MAX = 32;      // outputs of a CTA at most
 constexpr int ROW_AHEAD = 4;         // 16-byte weight loads a lane has in flight
 constexpr int KB_UNIT = 4;       // K blocks that a warp takes with one load: eight lanes each
 
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(ROW_THREADS) linear_rows_kernel(const T *__res
 // Outputs a CTA: a power of two, two CTAs a SM where the outputs allow it.
 inline int rows_outs(int64_t N) {
   int outs = 4;
-  while (outs < 32 && N > (int64_t)outs * 2 * sm_count()) outs *= 2;
+  while (outs < ROW_OUTS_MAX && N > (int64_t)outs * 2 * sm_count()) outs *= 2;
   return outs;
 }
 
@@ -732,12 +733,14 @@ int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group
 //   2 rows  576 x 7168 10.9, 5.1   1536 x 1536 6.8, 3.7   2048 x 4096 11.0, 6.5   7168 x 2048 8.4, 8.1   4096 x 7168 16.7, 14.0
 //   4 rows  576 x 7168 10.9, 7.3   1536 x 1536 6.8, 5.4   2304 x 1280  6.8, 5.5
 //   left to the others: 1 x 16384 x 2048 10.2, 13.0   1 x 7168 x 18432 34.9, 43.9   4 x 2048 x 4096 11.0, 12.0   4 x 1024 x 7168 12.2, 13.3
-// fp32 rows, whose quotients the library's division takes, less: 1 x 4096 x 7168 19.3, 15.8   2 x 1024 x 7168 15.0, 12.5   4 x 576 x 7168 14.2,
-// 12.7 but 2 x 7168 x 2048 12.7, 13.1   3 x 2304 x 1280 9.5, 10.3.
+// Only as many outputs as two CTAs a SM of 32 take at once; every further wave repeats the quantisation: 1 x 9344 x 1024 7.1, 4.6 but
+// 1 x 29184 x 1024 10.4, 12.4   1 x 200000 x 128 12.1, 49.7   3 x 33024 x 128 5.9, 17.5.
+// fp32 rows, whose quotients the library's division takes, less: 1 x 4096 x 7168 19.3, 16.8   1 x 9344 x 3072 14.6, 14.7   2 x 1024 x 7168 15.0, 12.5
+// but 2 x 7168 x 2048 12.7, 13.1   2 x 64 x 20480 14.0, 16.0   4 x 64 x 9216 11.1, 13.0   3 x 2304 x 1280 9.5, 10.3.
 bool linear_rows_fit(int64_t M, int64_t N, int64_t K, int x_dtype) {
-  if (M < 1 || M > ROWS_MAX || N < 1 || N >= (1LL << 31) || K > (1LL << 20)) return false;
+  if (M < 1 || M > ROWS_MAX || N < 1 || N > (int64_t)ROW_OUTS_MAX * 2 * sm_count() || K > (1LL << 20)) return false;
   const bool fp32 = x_dtype == LO_F32;
-  if (M > 2 && fp32 && N > 4 * sm_count()) return false;
+  if (fp32 && (M > 2 || (M == 2 && K > 8192))) return false;
   const int64_t most = M > 2 ? 4500000 : (M == 2 && fp32 ? 14000000 : 30000000);
   const int rows = M <= 2 ? (int)M : ROWS_MAX;
   return N * K <= most && rows_smem(rows, K / 128, rows_outs(N)) <= ROWS_SMEM_PLAIN;

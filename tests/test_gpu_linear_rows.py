@@ -30,21 +30,21 @@ def _both(x, B, b_s):
 # outputs: fewer than a CTA's, remainders of 4, 8, 16 and 32 outputs a CTA, across blocks of 128; K: one, five, eleven and 56 blocks (a warp
 # takes four at a time, its loads run 64 units ahead), and many
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
-@pytest.mark.parametrize("N,K", [(1, 128), (5, 640), (127, 1408), (129, 7168), (576, 7168), (1187, 384), (2373, 640), (4745, 128), (9001, 384)])
+@pytest.mark.parametrize("N,K", [(1, 128), (5, 640), (127, 1408), (129, 7168), (576, 7168), (1187, 384), (2373, 640), (4745, 128), (9001, 384), (9472, 128)])
 def test_one_kernel_has_the_bits_of_the_two_operators(M, N, K):
     one, two = _both(*_inputs(M, N, K, torch.bfloat16, M + N + K))
     assert torch.equal(one, two), int((one != two).sum())
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
-@pytest.mark.parametrize("M,N,K", [(1, 300, 2048), (2, 4096, 1280), (3, 129, 512), (1, 40, 32768)])
+@pytest.mark.parametrize("M,N,K", [(1, 300, 2048), (2, 4096, 1280), (2, 129, 512), (1, 40, 32768)])
 def test_other_input_types(M, N, K, dtype):
     one, two = _both(*_inputs(M, N, K, dtype, M + N + K))
     assert torch.equal(one, two)
 
 
 def test_rows_with_nan_infinity_zeros_and_tiny_values():
-    x, B, b_s = _inputs(4, 200, 1024, torch.float32, 5)
+    x, B, b_s = _inputs(4, 200, 1024, torch.bfloat16, 5)
     x[0, 130] = float("nan")
     x[1, 5], x[1, 700] = float("inf"), -float("inf")
     x[2] = 0.0
@@ -56,5 +56,5 @@ def test_rows_with_nan_infinity_zeros_and_tiny_values():
 def test_larger_calls_keep_the_other_form():
     from lightop_b200 import _lib
     size = _lib.load().lo_block_int8_linear_dynamic_workspace_bytes
-    assert size(5, 128, 128) > 0 and size(4, 1024, 7168) > 0 and size(1, 16384, 2048) > 0 and size(2, 128, 65536) > 0
-    assert size(1, 4096, 7168) == 0 and size(2, 1024, 7168) == 0 and size(4, 576, 7168) == 0
+    assert size(5, 128, 128) > 0 and size(4, 1024, 7168) > 0 and size(1, 9473, 128) > 0 and size(1, 16384, 2048) > 0 and size(2, 128, 65536) > 0
+    assert size(1, 4096, 7168) == 0 and size(2, 1024, 7168) == 0
