@@ -298,8 +298,9 @@ constexpr int ALIGN_BATCH = 128;      // ids a warp has in flight
 constexpr int64_t ALIGN_CLUSTER_MIN_IDS = 2048;
 // Cluster of 8 with one id after the other, with batches of loads, and cluster of 16 with batches, in us (256 experts, in a graph): 2400 ids
 // (128 experts) 6.3, 6.2, 6.1; 6216 ids 7.3, 7.3, 6.9; 16384 9.3, 8.9, 7.8; 32768 13.0, 11.6, 9.7; 65536 18.2, 15.1, 12.1; 262144 53.9, 44.1, 25.0.
-// With 1024 experts the sixteen tables cost more: 2049 ids 8.8, 8.7, 11.0; 131072 31.7, 28.8, 20.6.
-constexpr int64_t ALIGN_WIDE_MIN_IDS = 6144;
+// The CTAs clear, scan and exchange a count per expert, so with many experts sixteen of them pay from 24 ids an expert on: 1024 experts 2049
+// ids 8.8, 8.7, 11.0; 8192 9.9, -, 11.5; 16384 12.0, -, 12.8; 32768 15.4, -, 14.1; 131072 31.7, 28.8, 20.6.
+constexpr int64_t ALIGN_WIDE_MIN_IDS = 6144, ALIGN_WIDE_IDS_PER_EXPERT = 24;
 
 template <typename IdT, int C>
 __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32) align_cluster_kernel(
   for (int64_t base = seg_begin; base < seg_end; base += ALIGN_BATCH) {
     fetch(base);
 #pragma unroll 1
-    for (int j = lane; j < ALIGN_BATCH; j += 32)
+    for (int j = lane; j < ALIGN_BATCH && base + j - lane < seg_end; j += 32)
       if (mine[j] >= 0) atomicAdd(&my_hist[mine[j]], 1);
   }
   __syncthreads();
@@ -571,7 +572,7 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
                                                            sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks,
                                                            chunk_capacity, inv_pos, chunk_max);
       };
-      return numel >= ALIGN_WIDE_MIN_IDS && wide_cluster_fits() ? with(std::integral_constant<int, ALIGN_CLUSTER_WIDE>{})
+      return numel >= ALIGN_WIDE_MIN_IDS && numel >= ALIGN_WIDE_IDS_PER_EXPERT * num_experts && wide_cluster_fits() ? with(std::integral_constant<int, ALIGN_CLUSTER_WIDE>{})
                                                                 : with(std::integral_constant<int, ALIGN_CLUSTER>{});
     };
     return ids_dtype == LO_I32 ? launch(static_cast<const int32_t *>(topk_ids)) : launch(static_cast<const int64_t *>(topk_ids));

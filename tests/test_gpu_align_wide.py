@@ -21,7 +21,7 @@ def test_order_and_tables(M, k, E, dtype):
     _check_align(lo, ids, E, 16, expert_map=emap, ignore=True)
 
 
-@pytest.mark.parametrize("M,E", [(20000, 1024), (6144, 1), (30000, 3)])
+@pytest.mark.parametrize("M,E", [(20000, 1024), (24576, 1024), (6144, 1), (30000, 3)])
 def test_ends_of_the_number_of_experts(M, E):
     import lightop_b200 as lo
     ids = torch.randint(0, E, (M, 1), generator=torch.Generator().manual_seed(M), dtype=torch.int32)
