@@ -146,7 +146,8 @@ int lo_moe_grouped_gemm_i8_block(const int8_t *A, const float *a_scale, int64_t 
  * Replaces: fused_experts_impl_int8 with use_int8_w8a8=True, block_shape=[128,128],
  *           python/lightop/_lmslim_native/layers/fused_moe/int8.py:628-908 (one chunk).
  * x [M,H] bf16; w1 [E,2I,H] int8; w2 [E,H,I] int8; w1_scale [E,2I/128,H/128] f32;
- * w2_scale [E,H/128,I/128] f32; topk_weights [M,topk] f32; topk_ids [M,topk] (LO_I32/LO_I64);
+ * w2_scale [E,H/128,I/128] f32; topk_weights [M,topk] f32; topk_ids [M,topk] (LO_I32/LO_I64; a
+ * token may name the same expert in several slots);
  * expert_map i32 [global_num_experts] or NULL (ids mapping to -1 contribute nothing);
  * cache3 [M,topk,H] bf16 scratch (the caller's cache13); shared_output [M,H] bf16 or NULL;
  * out [M,H] bf16 = routed_scaling_factor * sum_j w_j * expert_j(x) (+ shared_output).

@@ -77,6 +77,16 @@ inline int chunk_rows_for(int64_t rows, int experts) {
   return avg >= 120 ? CHUNK_ROWS_WIDE : (avg <= 48 ? CHUNK_ROWS_SMALL : CHUNK_ROWS);
 }
 
+// Rows that a chunk of a call's table may hold: the smallest size the GEMM is instantiated for that holds min(rows, chunk_max).  The
+// alignment cuts the table at this size and the GEMM's instantiation is chosen by it, so that no chunk is wider than the instantiation that reads
+// it.  `rows` is the number of tokens, the most an expert gets where the experts of a token are distinct; nothing makes them so (a batch
+// of padding tokens may carry one id in every slot), and an expert with more rows then has more chunks.
+inline int table_chunk_rows(int64_t rows, int chunk_max) {
+  for (int cap : {32, CHUNK_ROWS_SMALL, CHUNK_ROWS, CHUNK_ROWS_WIDE})
+    if (rows <= cap || chunk_max <= cap) return cap;
+  return 256;
+}
+
 // Whether the quantiser of the block-scaled layer reads a token's positions before its row, so that rows of tokens without a local
 // expert are not read.  It then starts behind the alignment instead of beside it, which costs about 1 us: worth it where a fifth of
 // the tokens or more can be expected to have no local expert (ids spread evenly over the experts) and their rows are 8 MB or more.
@@ -178,7 +188,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   const int64_t numel = M * topk;
   int rc;
 
-  const int chunk_max = chunk_rows_for(numel, align_E);
+  const int chunk_max = table_chunk_rows(M, chunk_rows_for(numel, align_E));
   prof_mark(0, st);
   if (route_quant_small_fits(M, H, topk)) {
     // 1 and 2 in one kernel: a launch and the wait of one kernel for the other less
@@ -205,7 +215,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   prof_mark(2, st);
   GemmArgs g1{};
   g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap;
-  g1.max_chunk_rows = (int)(M < chunk_max ? M : chunk_max);   // an expert receives at most one row per token
+  g1.max_chunk_rows = chunk_max;
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = numel;
@@ -489,7 +499,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   LO_REQUIRE(workspace_bytes >= L.bytes, "channel moe: workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t numel = M * topk;
-  const int chunk_max = channel_chunk_rows_for(numel, align_E);
+  const int chunk_max = table_chunk_rows(M, channel_chunk_rows_for(numel, align_E));
   // 1. expert-major stable order, chunk table, position of every (token, slot)
   prof_mark(0, st);
   int rc = launch_align(topk_ids, ids_dtype, numel, align_E, FUSED_ALIGN_BLOCK, expert_map, expert_map ? 1 : 0,
@@ -504,7 +514,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   prof_mark(2, st);
   GemmArgs g1{};
   g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap;
-  g1.max_chunk_rows = (int)(M < chunk_max ? M : chunk_max);
+  g1.max_chunk_rows = chunk_max;
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(2 * I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = numel; g1.out_by_position = 1;
@@ -564,7 +574,7 @@ int expert_rows_impl(const int8_t *xq, const float *xs, int64_t x_stride, const 
   LO_REQUIRE(workspace_bytes >= L.bytes, "expert rows: workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // chunk sizes: the rule of lo_fused_moe_block_int8
-  const int chunk_max = chunk_rows_for(T, E_local);
+  const int chunk_max = table_chunk_rows(T, chunk_rows_for(T, E_local));
   // 1. expert-major stable order of the rows (ids outside [0, E_local) are dropped)
   int rc = launch_align(row_expert, LO_I32, T, E_local, FUSED_ALIGN_BLOCK, nullptr, 0, L.sorted_ids, L.sorted_cap,
                         nullptr, 0, L.header, L.chunks, L.header + 1, L.chunk_cap, nullptr, chunk_max, st);
@@ -573,7 +583,7 @@ int expert_rows_impl(const int8_t *xq, const float *xs, int64_t x_stride, const 
   rc = launch_permute_rows(xq, xs, T, H, L.sorted_ids, L.sorted_cap, L.header, T, 1, L.xq, L.xs, st, 0, x_stride);
   if (rc != LO_OK) return rc;
   GemmArgs g1{};
-  g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap; g1.max_chunk_rows = (int)(T < chunk_max ? T : chunk_max);
+  g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap; g1.max_chunk_rows = chunk_max;
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = T;
