@@ -227,6 +227,8 @@ __device__ __forceinline__ int local_expert(const IdT *ids, int64_t i, const int
 // from peer masks.  Runs as one CTA or, for many ids, as a cluster of EP_PLAN_CLUSTER CTAs that take
 // consecutive slices of the ids and exchange their per-expert counts through distributed shared memory.
 constexpr int EP_PLAN_CLUSTER = 8;
+constexpr int EP_PLAN_MAX_EXPERTS = 1024;      // experts, or ranks: the entry points refuse more
+constexpr size_t ep_plan_smem(int E) { return sizeof(int32_t) * (36 * (size_t)E + 1); }
 constexpr int64_t EP_PLAN_CLUSTER_MIN_IDS = 8192;
 
 template <typename IdT>
@@ -322,8 +324,9 @@ template <typename IdT>
 int launch_ep_plan(const void *ids, int64_t numel, const int32_t *expert_map, const int32_t *counts_in, int local_E,
                    int alignment, int32_t *m_indices, int64_t rows, int32_t *inv_perm, cudaStream_t st,
                    int32_t *counts_out = nullptr) {
-  const size_t smem = sizeof(int32_t) * (36 * (size_t)local_E + 1);
-  LO_CUDA_OK(cudaFuncSetAttribute(ep_plan_kernel<IdT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const size_t smem = ep_plan_smem(local_E);
+  // (the limit of the most experts, whatever this call needs: another thread's call with fewer must not lower it before the launch)
+  LO_CUDA_OK(cudaFuncSetAttribute(ep_plan_kernel<IdT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ep_plan_smem(EP_PLAN_MAX_EXPERTS)));
   const IdT *idp = static_cast<const IdT *>(ids);
   if (numel >= EP_PLAN_CLUSTER_MIN_IDS) {
     cudaLaunchConfig_t cfg = {};

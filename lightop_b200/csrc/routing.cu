@@ -510,20 +510,29 @@ template <int C> cudaLaunchConfig_t cluster_config(cudaLaunchAttribute (&attr)[2
   return cfg;
 }
 
-template <typename IdT, int C, typename... Args> int launch_cluster(size_t smem, cudaStream_t stream, Args... args) {
+// Dynamic shared memory of the two kernels.  The limits that a kernel is given are those of the most experts, whatever a call needs: they
+// belong to the (kernel, device) pair, and a limit of the call's own size could be lowered by another thread between here and the launch.
+constexpr int ALIGN_MAX_EXPERTS = 1024;
+constexpr size_t align_smem(int E) { return sizeof(int32_t) * ((size_t)ALIGN_WARPS * E + 3 * (size_t)E + 2 + 64); }
+constexpr size_t cluster_smem(int E) {
+  return sizeof(int32_t) * ((size_t)ALIGN_WARPS * E + 5 * (size_t)E + 2 + 64) + sizeof(int16_t) * ALIGN_WARPS * ALIGN_BATCH;
+}
+
+template <typename IdT, int C> cudaError_t allow_cluster(size_t smem) {
   auto kernel = align_cluster_kernel<IdT, C>;
-  // (both belong to the (kernel, device) pair: set whenever a launch needs them, whichever device is current)
-  if (C > 8) LO_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  if (smem > 48 * 1024) LO_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaError_t e = cudaSuccess;
+  if (C > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess && smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem(ALIGN_MAX_EXPERTS));
+  return e;
+}
+
+template <typename IdT, int C, typename... Args> int launch_cluster(size_t smem, cudaStream_t stream, Args... args) {
+  LO_CUDA_OK((allow_cluster<IdT, C>(smem)));
   cudaLaunchAttribute attr[2];
   const cudaLaunchConfig_t cfg = cluster_config<C>(attr, smem, stream);
   g_launch_count.fetch_add(1, std::memory_order_relaxed);
-  LO_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, args...));
+  LO_CUDA_OK(cudaLaunchKernelEx(&cfg, align_cluster_kernel<IdT, C>, args...));
   return LO_OK;
-}
-
-constexpr size_t cluster_smem(int E) {
-  return sizeof(int32_t) * ((size_t)ALIGN_WARPS * E + 5 * (size_t)E + 2 + 64) + sizeof(int16_t) * ALIGN_WARPS * ALIGN_BATCH;
 }
 
 // Whether the device has room for a cluster of 16 (a size that a part with smaller clusters of SMs need not have): asked once a device.
@@ -533,13 +542,11 @@ bool wide_cluster_fits() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
   int8_t k = known[dev].load(std::memory_order_relaxed);
   if (k == 0) {
-    auto kernel = align_cluster_kernel<int32_t, ALIGN_CLUSTER_WIDE>;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = cluster_config<ALIGN_CLUSTER_WIDE>(attr, cluster_smem(1024), nullptr);
+    const cudaLaunchConfig_t cfg = cluster_config<ALIGN_CLUSTER_WIDE>(attr, cluster_smem(ALIGN_MAX_EXPERTS), nullptr);
     int clusters = 0;
-    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem(1024)) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+    const bool ok = allow_cluster<int32_t, ALIGN_CLUSTER_WIDE>(cfg.dynamicSmemBytes) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, align_cluster_kernel<int32_t, ALIGN_CLUSTER_WIDE>, &cfg) == cudaSuccess && clusters > 0;
     if (!ok) (void)cudaGetLastError();
     k = ok ? 1 : 2;
     known[dev].store(k, std::memory_order_relaxed);
@@ -555,49 +562,35 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
                  Chunk *chunks, int32_t *num_chunks, int64_t chunk_capacity, int32_t *inv_pos,
                  int chunk_max, cudaStream_t stream) {
   if (chunk_max != 32 && chunk_max != 64 && chunk_max != 160 && chunk_max != 256) chunk_max = 128;
-  LO_REQUIRE(num_experts >= 1 && num_experts <= 1024, "moe_align: num_experts %d outside [1,1024]", num_experts);
+  LO_REQUIRE(num_experts >= 1 && num_experts <= ALIGN_MAX_EXPERTS, "moe_align: num_experts %d outside [1,1024]", num_experts);
   LO_REQUIRE(block_size >= 1, "moe_align: block_size must be positive");
   LO_REQUIRE(numel >= 0 && numel < (1LL << 30), "moe_align: numel out of range");
   LO_REQUIRE(map_mode == 0 || expert_map != nullptr, "moe_align: map_mode %d needs an expert_map", map_mode);
   LO_REQUIRE(sorted_ids && num_tokens_post_pad, "moe_align: null output");
-  const size_t smem = sizeof(int32_t) * ((size_t)ALIGN_WARPS * num_experts + 3 * (size_t)num_experts + 2 + 64);
-  cudaError_t e;
-  if (numel >= ALIGN_CLUSTER_MIN_IDS && (ids_dtype == LO_I32 || ids_dtype == LO_I64)) {
-    // many ids: one cluster
-    const size_t csmem = cluster_smem(num_experts);
-    auto launch = [&](auto *typed) -> int {
-      using IdT = typename std::remove_const<typename std::remove_pointer<decltype(typed)>::type>::type;
+  auto launch = [&](auto *typed) -> int {
+    using IdT = typename std::remove_const<typename std::remove_pointer<decltype(typed)>::type>::type;
+    if (numel >= ALIGN_CLUSTER_MIN_IDS) {
+      // many ids: one cluster
+      const size_t smem = cluster_smem(num_experts);
       auto with = [&](auto width) -> int {
-        return launch_cluster<IdT, decltype(width)::value>(csmem, stream, typed, numel, num_experts, block_size, expert_map, map_mode, sorted_ids,
+        return launch_cluster<IdT, decltype(width)::value>(smem, stream, typed, numel, num_experts, block_size, expert_map, map_mode, sorted_ids,
                                                            sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks,
                                                            chunk_capacity, inv_pos, chunk_max);
       };
-      return numel >= ALIGN_WIDE_MIN_IDS && numel >= ALIGN_WIDE_IDS_PER_EXPERT * num_experts && wide_cluster_fits() ? with(std::integral_constant<int, ALIGN_CLUSTER_WIDE>{})
-                                                                : with(std::integral_constant<int, ALIGN_CLUSTER>{});
-    };
-    return ids_dtype == LO_I32 ? launch(static_cast<const int32_t *>(topk_ids)) : launch(static_cast<const int64_t *>(topk_ids));
-  }
-  if (ids_dtype == LO_I32) {
-    // the opt-in belongs to the (kernel, device) pair: set whenever a launch needs it, whichever device is current
-    if (smem > 48 * 1024) {
-      e = cudaFuncSetAttribute(align_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return fail(LO_ERR_CUDA, "moe_align: smem opt-in failed: %s", cudaGetErrorString(e));
+      const bool wide = numel >= ALIGN_WIDE_MIN_IDS && numel >= ALIGN_WIDE_IDS_PER_EXPERT * num_experts && wide_cluster_fits();
+      return wide ? with(std::integral_constant<int, ALIGN_CLUSTER_WIDE>{}) : with(std::integral_constant<int, ALIGN_CLUSTER>{});
     }
-    LO_CUDA_OK(launch_dependent(align_kernel<int32_t>, dim3(1), dim3(ALIGN_WARPS * 32), smem, stream,
-        static_cast<const int32_t *>(topk_ids), numel, num_experts, block_size, expert_map, map_mode, sorted_ids,
-        sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos, chunk_max));
-  } else if (ids_dtype == LO_I64) {
-    if (smem > 48 * 1024) {
-      e = cudaFuncSetAttribute(align_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return fail(LO_ERR_CUDA, "moe_align: smem opt-in failed: %s", cudaGetErrorString(e));
-    }
-    LO_CUDA_OK(launch_dependent(align_kernel<int64_t>, dim3(1), dim3(ALIGN_WARPS * 32), smem, stream,
-        static_cast<const int64_t *>(topk_ids), numel, num_experts, block_size, expert_map, map_mode, sorted_ids,
-        sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity, inv_pos, chunk_max));
-  } else {
-    return fail(LO_ERR_UNSUPPORTED, "moe_align: unsupported id dtype code %d", ids_dtype);
-  }
-  return LO_OK;
+    const size_t smem = align_smem(num_experts);
+    if (smem > 48 * 1024)
+      LO_CUDA_OK(cudaFuncSetAttribute(align_kernel<IdT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)align_smem(ALIGN_MAX_EXPERTS)));
+    LO_CUDA_OK(launch_dependent(align_kernel<IdT>, dim3(1), dim3(ALIGN_WARPS * 32), smem, stream, typed, numel, num_experts, block_size, expert_map, map_mode,
+                                sorted_ids, sorted_capacity, expert_ids, expert_ids_capacity, num_tokens_post_pad, chunks, num_chunks, chunk_capacity,
+                                inv_pos, chunk_max));
+    return LO_OK;
+  };
+  if (ids_dtype == LO_I32) return launch(static_cast<const int32_t *>(topk_ids));
+  if (ids_dtype == LO_I64) return launch(static_cast<const int64_t *>(topk_ids));
+  return fail(LO_ERR_UNSUPPORTED, "moe_align: unsupported id dtype code %d", ids_dtype);
 }
 
 }  // namespace lo
