@@ -8,6 +8,7 @@
 // Memory-bound streaming kernel: a few lanes own one group, each lane moves 32 bytes of
 // input (64 of fp32 in large calls) and stores as many int8 as it has elements.
 #include "common.h"
+#include <type_traits>
 
 namespace lo {
 namespace {
@@ -531,9 +532,13 @@ int launch_typed(const void *x, int64_t num_groups, int group_size, float eps_t,
 // the bits of the quantiser and of the tensor-core forms.
 //
 // Bound by latency: one read of weights (the first loads in flight before the rows are quantised), the quantisation, the chain.  512
-// threads a CTA instead of 256 shorten the quantisation: 1 x 576 x 7168 5.2 -> 4.0 us, 1 x 4096 x 7168 14.0 -> 11.3.
+// threads a CTA instead of 256 shorten the quantisation: 1 x 576 x 7168 5.2 -> 4.0 us, 1 x 4096 x 7168 14.0 -> 11.3.  Two CTAs a SM
+// hold the registers to 64, at 12 to 24 bytes of spills.  By itself the form of four rows takes 79: one CTA a SM, which is the better form up to
+// one CTA a SM (4 x 576 x 7168 7.3, with 64 registers 7.5) and a second wave, with the quantisation repeated, beyond: 4 x 600 x 7168 12.5, with
+// 64 registers 8.8, 4 x 1187 x 3584 8.9, 6.7, 4 x 2304 x 1280 5.5, 4.2, 3 x 4745 x 896 7.0, 5.7.
 // ---------------------------------------------------------------------------
 constexpr int ROW_THREADS = 512, ROW_WARPS = ROW_THREADS / 32;
+constexpr int ROW_CTAS = 2;      // resident CTAs a SM where there are more CTAs than SMs: what the rules below count with
 constexpr int ROWS_MAX = 4;
 constexpr int ROW_OUTS_MAX = 32;      // outputs of a CTA at most
 constexpr int ROW_AHEAD = 4;         // 16-byte weight loads a lane has in flight
@@ -542,11 +547,12 @@ constexpr int KB_UNIT = 4;       // K blocks that a warp takes with one load: ei
 // Shared memory: codes [ROWS][K], scales [ROWS][KB], dot products as fp32 [outs][ROWS][KB].
 constexpr size_t rows_smem(int rows, int64_t KB, int outs) { return (size_t)rows * KB * 128 + (size_t)rows * KB * 4 + (size_t)outs * rows * KB * 4; }
 constexpr size_t ROWS_SMEM_PLAIN = 48 * 1024;      // what a kernel gets without asking
+static_assert(ROW_CTAS * (ROWS_SMEM_PLAIN + 1024) <= 227 * 1024, "shared memory of the resident CTAs of a SM");
 
-template <typename T, int ROWS>
-__global__ void __launch_bounds__(ROW_THREADS) linear_rows_kernel(const T *__restrict__ x, const int8_t *__restrict__ B,
-                                                              const float *__restrict__ b_scale, int M, int N, int KB, int outs,
-                                                              float eps_t, __nv_bfloat16 *__restrict__ C) {
+template <typename T, int ROWS, int CTAS>
+__global__ void __launch_bounds__(ROW_THREADS, CTAS) linear_rows_kernel(const T *__restrict__ x, const int8_t *__restrict__ B,
+                                                                    const float *__restrict__ b_scale, int M, int N, int KB, int outs,
+                                                                    float eps_t, __nv_bfloat16 *__restrict__ C) {
   extern __shared__ __align__(16) uint8_t smem[];
   uint8_t *codes = smem;                                                  // [ROWS][KB * 128]
   float *scale = reinterpret_cast<float *>(smem + ROWS * KB * 128);       // [ROWS][KB]: token scale, then times the weight block's
@@ -636,10 +642,10 @@ __global__ void __launch_bounds__(ROW_THREADS) linear_rows_kernel(const T *__res
   }
 }
 
-// Outputs a CTA: a power of two, two CTAs a SM where the outputs allow it.
+// Outputs a CTA: a power of two, one wave of CTAs where the outputs allow it.
 inline int rows_outs(int64_t N) {
   int outs = 4;
-  while (outs < ROW_OUTS_MAX && N > (int64_t)outs * 2 * sm_count()) outs *= 2;
+  while (outs < ROW_OUTS_MAX && N > (int64_t)outs * ROW_CTAS * sm_count()) outs *= 2;
   return outs;
 }
 
@@ -650,11 +656,13 @@ int launch_rows(const void *x, const int8_t *B, const float *b_scale, int64_t M,
   const dim3 grid((unsigned)ceil_div(N, outs));
   const T *xt = static_cast<const T *>(x);
   __nv_bfloat16 *c = static_cast<__nv_bfloat16 *>(C);
-#define LO_ROWS_CASE(R) \
-  LO_CUDA_OK(launch_dependent(linear_rows_kernel<T, R>, grid, dim3(ROW_THREADS), rows_smem(R, KB, outs), st, xt, B, b_scale, (int)M, (int)N, KB, outs, eps_t, c))
-  if (M <= 1) LO_ROWS_CASE(1);
-  else if (M <= 2) LO_ROWS_CASE(2);
-  else LO_ROWS_CASE(ROWS_MAX);
+#define LO_ROWS_CASE(R, CTAS) \
+  LO_CUDA_OK(launch_dependent(linear_rows_kernel<T, R, CTAS>, grid, dim3(ROW_THREADS), rows_smem(R, KB, outs), st, xt, B, b_scale, (int)M, (int)N, KB, outs, eps_t, c))
+  if (M <= 1) LO_ROWS_CASE(1, ROW_CTAS);
+  else if (M <= 2) LO_ROWS_CASE(2, ROW_CTAS);
+  else if constexpr (std::is_same<T, float>::value) return fail(LO_ERR_UNSUPPORTED, "linear of a few rows: more than two rows of fp32");      // linear_rows_fit() sends none
+  else if ((int)grid.x <= sm_count()) LO_ROWS_CASE(ROWS_MAX, 1);
+  else LO_ROWS_CASE(ROWS_MAX, ROW_CTAS);
 #undef LO_ROWS_CASE
   return LO_OK;
 }
@@ -738,7 +746,7 @@ int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group
 // fp32 rows, whose quotients the library's division takes, less: 1 x 4096 x 7168 19.3, 16.8   1 x 9344 x 3072 14.6, 14.7   2 x 1024 x 7168 15.0, 12.5
 // but 2 x 7168 x 2048 12.7, 13.1   2 x 64 x 20480 14.0, 16.0   4 x 64 x 9216 11.1, 13.0   3 x 2304 x 1280 9.5, 10.3.
 bool linear_rows_fit(int64_t M, int64_t N, int64_t K, int x_dtype) {
-  if (M < 1 || M > ROWS_MAX || N < 1 || N > (int64_t)ROW_OUTS_MAX * 2 * sm_count() || K > (1LL << 20)) return false;
+  if (M < 1 || M > ROWS_MAX || N < 1 || N > (int64_t)ROW_OUTS_MAX * ROW_CTAS * sm_count() || K > (1LL << 20)) return false;
   const bool fp32 = x_dtype == LO_F32;
   if (fp32 && (M > 2 || (M == 2 && K > 8192))) return false;
   const int64_t most = M > 2 ? 4500000 : (M == 2 && fp32 ? 14000000 : 30000000);

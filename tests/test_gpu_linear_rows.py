@@ -43,6 +43,13 @@ def test_other_input_types(M, N, K, dtype):
     assert torch.equal(one, two)
 
 
+# three and four rows of fp16: up to one CTA a SM, and more
+@pytest.mark.parametrize("M,N,K", [(3, 576, 1408), (4, 129, 7168), (3, 1187, 640), (4, 4745, 384), (4, 1, 128)])
+def test_fp16_rows(M, N, K):
+    one, two = _both(*_inputs(M, N, K, torch.float16, M + N + K))
+    assert torch.equal(one, two)
+
+
 def test_rows_with_nan_infinity_zeros_and_tiny_values():
     x, B, b_s = _inputs(4, 200, 1024, torch.bfloat16, 5)
     x[0, 130] = float("nan")

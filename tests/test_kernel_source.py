@@ -78,3 +78,16 @@ def test_what_lets_the_next_kernel_start_has_waited_itself():
                 assert waited, os.path.basename(path)
                 seen += 1
     assert seen >= 9
+
+
+def test_the_linear_of_a_few_rows_has_the_ctas_its_rules_count_with():
+    # outputs a CTA and the limit on the outputs assume ROW_CTAS CTAs a SM: the compiler has to be held to it wherever a call has more CTAs than
+    # there are SMs (a second wave repeats the quantisation)
+    with open(os.path.join(CSRC, "quant.cu")) as f:
+        text = f.read()
+    assert re.search(r"__launch_bounds__\(ROW_THREADS, CTAS\) linear_rows_kernel", text)
+    forms = re.findall(r"^(.*)\bLO_ROWS_CASE\((\w+), (\w+)\);", text, flags=re.M)
+    assert len(forms) == 4
+    for before, _, ctas in forms:
+        assert ctas == "ROW_CTAS" or "(int)grid.x <= sm_count()" in before
+    assert "N > (int64_t)outs * ROW_CTAS * sm_count()" in text and "N > (int64_t)ROW_OUTS_MAX * ROW_CTAS * sm_count()" in text
