@@ -734,24 +734,38 @@ int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group
   }
 }
 
-// Up to two rows and 30 million weights, three or four rows and 4.5 million: beyond, what every CTA spends on the same quantisation and on
-// dp4a is more than the launches it saves.  Device time in us of the kernels before (quantisation, GEMM, promotion where split) and
-// of this one, weights from HBM; a pass from Python is 16 to 18 us before and 11 to 12 now wherever the device takes less:
-//   1 row   576 x 7168 10.7, 4.0   1536 x 1536 6.8, 3.3   2048 x 4096 11.1, 4.9   7168 x 2048 8.4, 7.0   4096 x 7168 16.3, 11.3
-//   2 rows  576 x 7168 10.9, 5.1   1536 x 1536 6.8, 3.7   2048 x 4096 11.0, 6.5   7168 x 2048 8.4, 8.1   4096 x 7168 16.7, 14.0
-//   4 rows  576 x 7168 10.9, 7.3   1536 x 1536 6.8, 5.4   2304 x 1280  6.8, 5.5
-//   left to the others: 1 x 16384 x 2048 10.2, 13.0   1 x 7168 x 18432 34.9, 43.9   4 x 2048 x 4096 11.0, 12.0   4 x 1024 x 7168 12.2, 13.3
-// Only as many outputs as two CTAs a SM of 32 take at once; every further wave repeats the quantisation: 1 x 9344 x 1024 7.1, 4.6 but
-// 1 x 29184 x 1024 10.4, 12.4   1 x 200000 x 128 12.1, 49.7   3 x 33024 x 128 5.9, 17.5.
-// fp32 rows, whose quotients the library's division takes, less: 1 x 4096 x 7168 19.3, 16.8   1 x 9344 x 3072 14.6, 14.7   2 x 1024 x 7168 15.0, 12.5
-// but 2 x 7168 x 2048 12.7, 13.1   2 x 64 x 20480 14.0, 16.0   4 x 64 x 9216 11.1, 13.0   3 x 2304 x 1280 9.5, 10.3.
+// Whether the one-kernel form takes the call: up to 30 million weights with one or two rows (14 million with two of fp32), 4.5 million
+// with three or four, one wave of CTAs (further ones repeat the quantisation: 1 x 29184 x 1024 12.4 us against 10.4 of the other kernels, 3 x 33024
+// x 128 17.5 against 5.9), and K up to the line below.  A CTA's time is that of outs * K weights, dp4a and loads in turn; the other kernels
+// (quantisation, GEMM, promotion where split) give a CTA of 128 outputs to the tensor core, whose time grows with K alone and less steeply.  So
+// the line falls with the outputs a CTA, and where more rows or a dearer quantisation (fp32 quotients are the library's divisions) come on top.
+// Device time in us, weights from HBM, the other kernels and this one, around the lines:
+//   1 row, 16 outputs: 2400 x 10240 15.0, 13.9   2400 x 12288 16.8, 17.2     32: 8192 x 3584 11.5, 11.0   6144 x 4096 12.0, 11.8 (fp16 14.5, 15.2)   4800 x 6144 14.9, 15.1
+//   2 rows, 8 outputs: 1200 x 10240 12.9, 12.3   1200 x 12288 14.3, 14.8     16: 4096 x 7168 16.4, 14.1   2400 x 7168 14.0, 13.4   3072 x 8192 14.4, 17.0
+//           32: 7168 x 2048 8.9, 8.1   5120 x 2560 9.3, 9.6   7168 x 4096 12.2, 15.0   (the worst inside: 2400 x 6144 11.6, 11.7, of fp16 14.9, 15.3)
+//   1 row of fp32, 8: 1200 x 20480 22.6, 21.8   1200 x 24576 25.5, 25.6      16: 4096 x 7168 19.1, 16.8   3072 x 8192 17.4, 18.0
+//           32: 6144 x 2048 11.4, 10.8   8192 x 3072 13.5, 14.4
+//   2 rows of fp32, 8: 1536 x 6144 13.5, 13.6   1200 x 8192 15.0, 15.6       16: 2400 x 4096 13.5, 13.6   32: 6144 x 2048 12.0, 12.1
+//   Far from the lines: 1 x 576 x 7168 10.7, 4.0   1 x 1536 x 1536 6.8, 3.3   2 x 576 x 7168 10.9, 5.1   2 x 2048 x 4096 11.0, 6.5
+//   3 and 4 rows: 4 x 576 x 7168 11.0, 7.2   4 x 600 x 7168 11.3, 8.8   4 x 1536 x 1536 6.6, 4.2   3 x 4745 x 896 6.8, 5.7   4 x 9472 x 384 5.8, 4.4
+// A pass from Python is 16 to 18 us with the other kernels and 11 to 12 with this one wherever the device takes less.
+constexpr int64_t ROWS_ANY_K = 1LL << 20;
+constexpr int64_t ROWS_K[4][4] = {
+    // outputs a CTA: 4, 8, 16, 32
+    {ROWS_ANY_K, ROWS_ANY_K, 10240, 3584},      // one row of bf16 or fp16
+    {ROWS_ANY_K, 10240, 7168, 2048},            // two
+    {ROWS_ANY_K, 20480, 7168, 2048},            // one row of fp32
+    {8192, 5120, 3072, 1536},                   // two
+};
 bool linear_rows_fit(int64_t M, int64_t N, int64_t K, int x_dtype) {
-  if (M < 1 || M > ROWS_MAX || N < 1 || N > (int64_t)ROW_OUTS_MAX * ROW_CTAS * sm_count() || K > (1LL << 20)) return false;
+  if (M < 1 || M > ROWS_MAX || N < 1 || N > (int64_t)ROW_OUTS_MAX * ROW_CTAS * sm_count() || K > ROWS_ANY_K) return false;
   const bool fp32 = x_dtype == LO_F32;
-  if (fp32 && (M > 2 || (M == 2 && K > 8192))) return false;
+  if (fp32 && M > 2) return false;
+  const int outs = rows_outs(N);
+  if (M <= 2 && K > ROWS_K[(fp32 ? 2 : 0) + (M - 1)][outs == 4 ? 0 : (outs == 8 ? 1 : (outs == 16 ? 2 : 3))]) return false;
   const int64_t most = M > 2 ? 4500000 : (M == 2 && fp32 ? 14000000 : 30000000);
   const int rows = M <= 2 ? (int)M : ROWS_MAX;
-  return N * K <= most && rows_smem(rows, K / 128, rows_outs(N)) <= ROWS_SMEM_PLAIN;
+  return N * K <= most && rows_smem(rows, K / 128, outs) <= ROWS_SMEM_PLAIN;
 }
 
 int launch_linear_rows(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K, float eps, void *C,

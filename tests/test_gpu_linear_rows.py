@@ -60,8 +60,31 @@ def test_rows_with_nan_infinity_zeros_and_tiny_values():
     assert torch.equal(one.isnan(), two.isnan()) and torch.equal(one.nan_to_num(), two.nan_to_num())
 
 
-def test_larger_calls_keep_the_other_form():
+# both sides of every limit, by the kernels that a call launches: K by the outputs a CTA (4 up to 1184 outputs, 8 up to 2368, 16 up to 4736, 32), the number of
+# weights, of outputs and of rows, the shared memory
+BF16, F16, F32 = torch.bfloat16, torch.float16, torch.float32
+
+
+@pytest.mark.parametrize("M,N,inside,outside,dtypes", [
+    (1, 2400, 10240, 10368, (BF16, F16)), (1, 4800, 3584, 3712, (BF16, F16)), (1, 2368, 12544, 12672, (BF16,)), (1, 9472, 128, None, (BF16, F16, F32)),
+    (1, 9473, None, 128, (BF16, F16, F32)), (1, 128, 42496, 42624, (F16,)),
+    (2, 1200, 10240, 10368, (BF16, F16)), (2, 2400, 7168, 7296, (BF16, F16)), (2, 4800, 2048, 2176, (BF16, F16)),
+    (1, 1200, 20480, 20608, (F32,)), (1, 2400, 7168, 7296, (F32,)), (1, 4800, 2048, 2176, (F32,)),
+    (2, 64, 8192, 8320, (F32,)), (2, 1200, 5120, 5248, (F32,)), (2, 2400, 3072, 3200, (F32,)), (2, 4800, 1536, 1664, (F32,)), (2, 9216, 1408, 1536, (F32,)),
+    (3, 1024, 4352, 4480, (BF16, F16)), (4, 1024, 4352, 4480, (BF16, F16)), (4, 128, 10624, 10752, (BF16,)), (3, 128, None, 128, (F32,)), (5, 128, None, 128, (BF16, F16, F32))])
+def test_both_sides_of_the_limits(M, N, inside, outside, dtypes):
+    import lightop_b200 as lo
     from lightop_b200 import _lib
-    size = _lib.load().lo_block_int8_linear_dynamic_workspace_bytes
-    assert size(5, 128, 128) > 0 and size(4, 1024, 7168) > 0 and size(1, 9473, 128) > 0 and size(1, 16384, 2048) > 0 and size(2, 128, 65536) > 0
-    assert size(1, 4096, 7168) == 0 and size(2, 1024, 7168) == 0
+    lib = _lib.load()
+    for dtype in dtypes:
+        for K, one in ((inside, True), (outside, False)):
+            if K is None:
+                continue
+            x, B, b_s = _inputs(M, N, K, dtype, M + N + K)
+            before = lib.lo_launch_count()
+            y = lo.gemm_ops.apply_w8a8_block_int8_linear(x, B, [128, 128], b_s)
+            launches = lib.lo_launch_count() - before
+            assert (launches == 1) == one, (dtype, K, launches)
+            q, s = lo.quant.per_token_group_quant_int8(x, 128)
+            assert torch.equal(y, lo.gemm_ops.matmul_block_int8(q, B, s, b_s, [128, 128], torch.bfloat16).to(dtype)), (dtype, K)
+    lo.check_device_status()
