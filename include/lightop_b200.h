@@ -263,12 +263,15 @@ size_t lo_block_int8_linear_split_workspace_bytes(int64_t M, int64_t N, int64_t 
 
 /*
  * The same linear on activations that are not quantised yet: x [M,K] of type x_dtype (LO_BF16 / LO_F16 / LO_F32,
- * 16-byte aligned) goes through lo_group_quant_int8 (group 128, eps 1e-10) into the workspace first; up to four rows and a few
- * million weights are one kernel without a workspace, with the same bits.
+ * 16-byte aligned) goes through lo_group_quant_int8 (group 128, eps 1e-10) into the workspace first; up to four rows and, by their
+ * type and the shape, up to 30 million weights are one kernel without a workspace, with the same bits.
  * Replaces: apply_w8a8_block_int8_linear (python/lightop/_lmslim_native/layers/gemm/int8_utils.py:406-429).
- * workspace: lo_block_int8_linear_dynamic_workspace_bytes(M, N, K); may be null where that is 0.
+ * workspace: lo_block_int8_linear_dynamic_workspace_bytes(M, N, K), which serves every type of x, or
+ * lo_block_int8_linear_dynamic_scratch_bytes(M, N, K, x_dtype), which is 0 where the call is one kernel; the workspace may then be
+ * null.  256-byte aligned.
  */
 size_t lo_block_int8_linear_dynamic_workspace_bytes(int64_t M, int64_t N, int64_t K);
+size_t lo_block_int8_linear_dynamic_scratch_bytes(int64_t M, int64_t N, int64_t K, int x_dtype);
 int lo_block_int8_linear_dynamic(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N,
                                  int64_t K, void *C, void *workspace, size_t workspace_bytes, int32_t *status,
                                  void *stream);

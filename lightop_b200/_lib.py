@@ -78,6 +78,7 @@ PROTOTYPES = {
                                      c_void_p, c_size_t, c_void_p, c_void_p]),
     "lo_block_int8_linear_split_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64]),
     "lo_block_int8_linear_dynamic_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64]),
+    "lo_block_int8_linear_dynamic_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int]),
     "lo_block_int8_linear_dynamic": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_void_p,
                                              c_void_p, c_size_t, c_void_p, c_void_p]),
     "lo_moe_fused_gate": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int64, c_int, c_int, c_int, c_int, c_int, c_float,

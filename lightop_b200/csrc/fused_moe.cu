@@ -817,10 +817,15 @@ DynLinearLayout carve_dyn_linear(void *ws, int64_t M, int64_t K, const LinearPla
 }  // namespace
 }  // namespace lo
 
+// (enough for every call of these sizes, whichever kernels take it)
 extern "C" size_t lo_block_int8_linear_dynamic_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  // (the one-kernel form keeps no scratch; where it depends on the type of x whether it takes the call, the answer serves all types)
-  if (M <= 0 || N <= 0 || K < 128 || lo::linear_rows_fit(M, N, K, LO_F32)) return 0;
+  if (M <= 0 || N <= 0 || K < 128) return 0;
   return lo::carve_dyn_linear(nullptr, M, K, lo::plan_linear(M, N, K)).bytes;
+}
+
+// (the one-kernel form keeps no scratch, and the type of x has a say in whether it takes the call)
+extern "C" size_t lo_block_int8_linear_dynamic_scratch_bytes(int64_t M, int64_t N, int64_t K, int x_dtype) {
+  return lo::linear_rows_fit(M, N, K, x_dtype) ? 0 : lo_block_int8_linear_dynamic_workspace_bytes(M, N, K);
 }
 
 extern "C" int lo_block_int8_linear_dynamic(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M,

@@ -82,10 +82,11 @@ def _dynamic_linear(x: torch.Tensor, w: torch.Tensor, block_size: List[int], w_s
     lib = _lib.load()
     dev = x.device
     C = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=dev)
-    nbytes = lib.lo_block_int8_linear_dynamic_workspace_bytes(M, N, K)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+    code = _lib.dtype_code(x.dtype)
     with _lib.on_device(dev):
-        st = lib.lo_block_int8_linear_dynamic(_lib.ptr(x), _lib.dtype_code(x.dtype), _lib.ptr(w), _lib.ptr(bs), M, N, K,
+        nbytes = lib.lo_block_int8_linear_dynamic_scratch_bytes(M, N, K, code)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        st = lib.lo_block_int8_linear_dynamic(_lib.ptr(x), code, _lib.ptr(w), _lib.ptr(bs), M, N, K,
                                               _lib.ptr(C), _lib.ptr(ws), nbytes, _lib.ptr(device_status_word(dev)),
                                               _lib.current_stream(dev))
     _lib.check(st, "apply_w8a8_block_int8_linear")

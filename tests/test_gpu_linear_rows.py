@@ -88,3 +88,29 @@ def test_both_sides_of_the_limits(M, N, inside, outside, dtypes):
             q, s = lo.quant.per_token_group_quant_int8(x, 128)
             assert torch.equal(y, lo.gemm_ops.matmul_block_int8(q, B, s, b_s, [128, 128], torch.bfloat16).to(dtype)), (dtype, K)
     lo.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K,dtype,one", [(1, 576, 1408, BF16, True), (4, 576, 1408, F16, True), (4, 576, 1408, F32, False), (5, 128, 256, BF16, False)])
+def test_workspace_asked_for_is_the_workspace_needed(M, N, K, dtype, one):
+    # the query by type is 0 exactly where a null workspace is taken; a byte less than it is refused, and the size for all types serves every type
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    x, B, b_s = _inputs(M, N, K, dtype, 3)
+    need = lib.lo_block_int8_linear_dynamic_scratch_bytes(M, N, K, _lib.dtype_code(dtype))
+    every = lib.lo_block_int8_linear_dynamic_workspace_bytes(M, N, K)
+    assert (need == 0) == one and every > 0 and need in (0, every)
+    ws = torch.empty(every, dtype=torch.uint8, device=DEV)
+
+    def call(ptr, size):
+        c = torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV)
+        st = lib.lo_block_int8_linear_dynamic(x.data_ptr(), _lib.dtype_code(dtype), B.data_ptr(), b_s.data_ptr(), M, N, K, c.data_ptr(), ptr, size, 0,
+                                              torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return st, c
+
+    want = call(ws.data_ptr(), every)
+    assert want[0] == 0
+    st, c = call(0, 0)
+    assert (st == 0) == one and (st != 0 or torch.equal(c, want[1]))
+    if not one:
+        assert call(ws.data_ptr(), need - 1)[0] != 0
