@@ -268,7 +268,7 @@ size_t lo_block_int8_linear_split_workspace_bytes(int64_t M, int64_t N, int64_t 
  * Replaces: apply_w8a8_block_int8_linear (python/lightop/_lmslim_native/layers/gemm/int8_utils.py:406-429).
  * workspace: lo_block_int8_linear_dynamic_workspace_bytes(M, N, K), which serves every type of x, or
  * lo_block_int8_linear_dynamic_scratch_bytes(M, N, K, x_dtype), which is 0 where the call is one kernel; the workspace may then be
- * null.  256-byte aligned.
+ * null.  256-byte aligned.  C may overlap x; such a call needs the first of the two sizes.
  */
 size_t lo_block_int8_linear_dynamic_workspace_bytes(int64_t M, int64_t N, int64_t K);
 size_t lo_block_int8_linear_dynamic_scratch_bytes(int64_t M, int64_t N, int64_t K, int x_dtype);

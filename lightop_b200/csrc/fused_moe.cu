@@ -814,6 +814,10 @@ DynLinearLayout carve_dyn_linear(void *ws, int64_t M, int64_t K, const LinearPla
   D.bytes = c.off;
   return D;
 }
+inline bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + b_bytes && y < x + a_bytes;
+}
 }  // namespace
 }  // namespace lo
 
@@ -834,7 +838,8 @@ extern "C" int lo_block_int8_linear_dynamic(const void *x, int x_dtype, const in
   using namespace lo;
   int rc = check_linear(M, N, K);
   if (rc != LO_OK || M == 0) return rc;
-  const bool rows = linear_rows_fit(M, N, K, x_dtype);
+  // (every CTA of the one-kernel form reads x while others write C: a call in place takes the kernels that quantise first)
+  const bool rows = linear_rows_fit(M, N, K, x_dtype) && !overlap(x, (size_t)(M * K) * (x_dtype == LO_F32 ? 4 : 2), C, (size_t)(M * N) * 2);
   LO_REQUIRE(x && B && b_scale && C && (workspace || rows), "block int8 linear: null pointer");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0, "group quant: x must be 16-byte and q 8-byte aligned");
   LO_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & (ALIGN_BYTES - 1)) == 0, "block int8 linear: workspace must be 256-byte aligned");

@@ -114,3 +114,32 @@ def test_workspace_asked_for_is_the_workspace_needed(M, N, K, dtype, one):
     assert (st == 0) == one and (st != 0 or torch.equal(c, want[1]))
     if not one:
         assert call(ws.data_ptr(), need - 1)[0] != 0
+
+
+@pytest.mark.parametrize("M,K,at", [(1, 2048, 0), (4, 1024, 0), (2, 1024, 512), (2, 1024, -512)])
+def test_output_over_the_input(M, K, at):
+    # C on top of x (at elements off): the rows are read before anything is stored
+    from lightop_b200 import _lib
+    lib = _lib.load()
+    x, B, b_s = _inputs(M, K, K, BF16, 9)
+    every = lib.lo_block_int8_linear_dynamic_workspace_bytes(M, K, K)
+    ws = torch.empty(every, dtype=torch.uint8, device=DEV)
+    apart = torch.empty(M, K, dtype=torch.bfloat16, device=DEV)
+    both = torch.empty(M * K + 1024, dtype=torch.bfloat16, device=DEV)
+    mine = both[512:512 + M * K]
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(src, dst, w, size):
+        return lib.lo_block_int8_linear_dynamic(src, _lib.LO_BF16, B.data_ptr(), b_s.data_ptr(), M, K, K, dst, w, size, 0, stream)
+
+    assert call(x.data_ptr(), apart.data_ptr(), 0, 0) == 0
+    for _ in range(20):
+        mine.copy_(x.view(-1))
+        assert call(mine.data_ptr(), both.data_ptr() + (512 + at) * 2, ws.data_ptr(), every) == 0
+        assert torch.equal(both[512 + at:512 + at + M * K], apart.view(-1))
+    mine.copy_(x.view(-1))
+    assert call(mine.data_ptr(), both.data_ptr() + (512 + at) * 2, 0, 0) != 0 and torch.equal(mine, x.view(-1))
+    # side by side is apart
+    side = torch.empty(2 * M * K, dtype=torch.bfloat16, device=DEV)
+    side[:M * K].copy_(x.view(-1))
+    assert call(side.data_ptr(), side.data_ptr() + 2 * M * K, 0, 0) == 0 and torch.equal(side[M * K:], apart.view(-1))
