@@ -368,7 +368,8 @@ def gate_up_alg_bytes(M, k, H, I, experts_hit, channel=False):
 
 
 def stage_times(lightop_b200, _lib, step, reps: int):
-    """Per-kernel durations of the fused call (separate pass, events between its kernels)."""
+    """Per-kernel durations of the fused call (separate pass, events between its kernels).  Small calls align and quantise in one
+    kernel: "align" is then 0 and "group_quant_scatter" the time of both."""
     lib = _lib.load()
     lib.lo_profile_enable(1)
     stage = [0.0] * 5

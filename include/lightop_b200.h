@@ -428,9 +428,10 @@ int lo_m_grouped_w8a8_gemm_nt_masked(const int8_t *A, const float *a_scale, cons
 
 /*
  * Per-stage timing of lo_fused_moe_block_int8 for benchmarks: while enabled (per host thread), the
- * call records CUDA events between its five kernels (align, group quant, gate_up GEMM, down GEMM,
+ * call records CUDA events between its kernels (align, group quant, gate_up GEMM, down GEMM,
  * top-k sum); lo_profile_read waits for the last one and returns the five durations in
- * milliseconds (host array).  No counterpart in the reference, which times with
+ * milliseconds (host array).  A small call (up to 256 (token, slot) pairs) aligns and quantises in one
+ * kernel: its time is the second duration, and the first is 0.  No counterpart in the reference, which times with
  * triton.testing.do_bench around the whole call (test/moe_w8a8/moe_benchmark.py:918-932).
  */
 int lo_profile_enable(int on);

@@ -104,6 +104,7 @@ struct StageProfile {
   bool enabled = false;
   bool created = false;
   bool recorded = false;
+  bool joined = false;      // alignment and quantisation were one kernel: there is no event 1
   cudaEvent_t ev[6];
 };
 thread_local StageProfile g_prof;
@@ -131,7 +132,10 @@ extern "C" int lo_profile_read(float *ms5) {
   LO_REQUIRE(ms5 != nullptr, "profile read: null output");
   LO_REQUIRE(g_prof.created && g_prof.recorded, "profile read: no fused call was recorded on this thread");
   LO_CUDA_OK(cudaEventSynchronize(g_prof.ev[5]));
-  for (int i = 0; i < 5; ++i) LO_CUDA_OK(cudaEventElapsedTime(&ms5[i], g_prof.ev[i], g_prof.ev[i + 1]));
+  for (int i = 0; i < 5; ++i) {
+    if (g_prof.joined && i == 0) ms5[i] = 0.f;
+    else LO_CUDA_OK(cudaEventElapsedTime(&ms5[i], g_prof.ev[g_prof.joined && i == 1 ? 0 : i], g_prof.ev[i + 1]));
+  }
   return LO_OK;
 }
 
@@ -190,9 +194,9 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
 
   const int chunk_max = table_chunk_rows(M, chunk_rows_for(numel, align_E));
   prof_mark(0, st);
-  if (route_quant_small_fits(M, H, topk)) {
+  g_prof.joined = route_quant_small_fits(M, H, topk);
+  if (g_prof.joined) {
     // 1 and 2 in one kernel: a launch and the wait of one kernel for the other less
-    prof_mark(1, st);
     rc = launch_route_quant_small(x, M, H, topk, topk_ids, ids_dtype, align_E, expert_map, 1e-10f, L.xq, L.xs, L.sorted_ids, L.sorted_cap,
                                   L.header, L.chunks, L.header + 1, L.chunk_cap, chunk_max, st);
     if (rc != LO_OK) return rc;
@@ -502,6 +506,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   const int chunk_max = table_chunk_rows(M, channel_chunk_rows_for(numel, align_E));
   // 1. expert-major stable order, chunk table, position of every (token, slot)
   prof_mark(0, st);
+  g_prof.joined = false;
   int rc = launch_align(topk_ids, ids_dtype, numel, align_E, FUSED_ALIGN_BLOCK, expert_map, expert_map ? 1 : 0,
                         L.sorted_ids, L.sorted_cap, nullptr, 0, L.header, L.chunks, L.header + 1, L.chunk_cap,
                         L.inv_pos, chunk_max, st);
