@@ -83,8 +83,10 @@ int launch_align(const void *topk_ids, int ids_dtype, int64_t numel, int num_exp
 int launch_group_quant_scatter(const void *x, int64_t M, int64_t H, int topk, const int32_t *inv_pos, float eps,
                                int8_t *q_sorted, float *s_sorted, bool positions_first, cudaStream_t stream);
 
-// Group quantisation of rows of any supported type, for a dependent launch of the kernel that follows.  quant.cu
-// Alignment (segments of 16, chunk table) and launch_group_quant_scatter() in one kernel, for up to ROUTE_SMALL_IDS (token, slot) pairs.  quant.cu
+// Expert segments of the layers start on multiples of the MMA's N granule, whichever kernel orders the rows.
+constexpr int FUSED_ALIGN_BLOCK = 16;
+
+// Alignment (segments of FUSED_ALIGN_BLOCK, chunk table) and launch_group_quant_scatter() in one kernel, for up to ROUTE_SMALL_IDS (token, slot) pairs.  quant.cu
 constexpr int ROUTE_SMALL_IDS = 256;
 bool route_quant_small_fits(int64_t M, int64_t H, int topk);
 int launch_route_quant_small(const void *x, int64_t M, int64_t H, int topk, const void *topk_ids, int ids_dtype, int num_experts,
@@ -94,6 +96,7 @@ int launch_route_quant_small(const void *x, int64_t M, int64_t H, int topk, cons
 bool linear_rows_fit(int64_t M, int64_t N, int64_t K, int x_dtype);
 int launch_linear_rows(const void *x, int x_dtype, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K, float eps, void *C,
                        cudaStream_t st);
+// Group quantisation of rows of any supported type, for a dependent launch of the kernel that follows.  quant.cu
 int launch_group_quant(const void *x, int x_dtype, int64_t num_groups, int group_size, float eps, int8_t *q, float *s,
                        cudaStream_t stream);
 

@@ -9,7 +9,6 @@ float round_eps_to_dtype(float eps, int dtype);   // quant.cu
 namespace {
 
 constexpr int64_t ALIGN_BYTES = 256;
-constexpr int FUSED_ALIGN_BLOCK = 16;   // expert segments start on multiples of the MMA N granule
 
 struct Carver {
   uint8_t *base;
@@ -27,7 +26,7 @@ struct FusedLayout {
   float *xs;            // [sorted_cap, H/128]
   int32_t *header;      // [0] num_tokens_post_pad, [1] num_chunks
   int32_t *sorted_ids;
-  int32_t *inv_pos;     // [M*topk] position of every (token, slot), -1 if dropped
+  int32_t *inv_pos;     // [M*topk] position of every (token, slot), -1 if dropped; written and read by calls that align in a kernel of its own
   Chunk *chunks;
   int8_t *act_q;
   float *act_s;

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256) group_quant_scatter_kernel(const __nv_bfl
 // read; the others quantise a share of one token's row each and store it at the token's positions.  Same order, tables, codes
 // and scales as the two kernels.  Bound by latency (ids, count, scan, store).
 // ---------------------------------------------------------------------------
-constexpr int ROUTE_THREADS = 256, ROUTE_SEGMENT = 16;
+constexpr int ROUTE_THREADS = 256;
 static_assert(ROUTE_SMALL_IDS == ROUTE_THREADS, "one id a thread");
 
 template <typename IdT>
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_quant_kernel(
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       own[i] = sum;
-      sum += (c[i] + ROUTE_SEGMENT - 1) / ROUTE_SEGMENT * ROUTE_SEGMENT + ((c[i] + chunk_max - 1) / chunk_max << 16);
+      sum += (c[i] + FUSED_ALIGN_BLOCK - 1) / FUSED_ALIGN_BLOCK * FUSED_ALIGN_BLOCK + ((c[i] + chunk_max - 1) / chunk_max << 16);
     }
     uint32_t run = sum;
 #pragma unroll
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_quant_kernel(
     for (int x0 = tid; x0 < E; x0 += ROUTE_THREADS) {
       // equal chunks, rounded up to segments, as the alignment kernel cuts them
       const int c = (int)count[x0], nch = (c + chunk_max - 1) / chunk_max;
-      const int per = nch > 0 ? ((c + nch - 1) / nch + ROUTE_SEGMENT - 1) / ROUTE_SEGMENT * ROUTE_SEGMENT : 0;
+      const int per = nch > 0 ? ((c + nch - 1) / nch + FUSED_ALIGN_BLOCK - 1) / FUSED_ALIGN_BLOCK * FUSED_ALIGN_BLOCK : 0;
       int ci = (int)(offset[x0] >> 16);
       for (int r = 0; r < c; r += per, ++ci)
         if (ci < chunk_capacity) {

@@ -40,6 +40,30 @@ def _layer(M, k, E, H, I, ids, x, expert_map=None, E_local=None):
     return out, tables, lib.lo_launch_count() - before, (w1, w2, s1, s2, wgt)
 
 
+def check_tables(t, local_ids, E, q, s):
+    """Tables, rows and scales read back from a layer's workspace against the codes and scales of the tokens; ids outside [0, E) have no row."""
+    M, k = local_ids.shape
+    q, s, flat = q.cpu(), s.cpu(), local_ids.reshape(-1).tolist()
+    by_expert = [[] for _ in range(E)]
+    for i, v in enumerate(flat):
+        if 0 <= v < E:
+            by_expert[v].append(i)
+    avg = M * k // E
+    most = 160 if avg >= 120 else (64 if avg <= 48 else 128)
+    want, chunks = [], []
+    for e, mine in enumerate(by_expert):
+        n = -(-len(mine) // most)
+        per = -(-(-(-len(mine) // n)) // 16) * 16 if n else 0
+        chunks += [[e, len(want) + r, min(per, len(mine) - r), (len(mine) - r - 1) // per] for r in range(0, len(mine), per or 1)]
+        want += mine + [M * k] * (-len(mine) % 16)
+    assert t["n_pad"] == len(want) and t["sorted"].tolist() == want + [M * k] * (t["sorted"].numel() - len(want))
+    assert t["chunks"].tolist() == chunks
+    rows = torch.tensor(want)
+    real = rows < M * k
+    token = rows[real] // k
+    assert torch.equal(t["xq"][:len(want)][real], q[token]) and torch.equal(t["xs"][:len(want)][real], s[token])
+
+
 # one id; many ids of one expert (more than a segment, more than a chunk); no multiple of anything; rows of one share and of several
 # (256 lanes of sixteen elements); the largest call; ids outside the experts; as many experts as there can be
 @pytest.mark.parametrize("M,k,E,H,same,dtype", [(1, 1, 1, 128, False, torch.int32), (1, 8, 256, 7168, False, torch.int32), (17, 3, 9, 640, False, torch.int64),
@@ -55,22 +79,7 @@ def test_tables_rows_and_scales(M, k, E, H, same, dtype):
     x = torch.randn(M, H, generator=g).to(torch.bfloat16).to(DEV)
     _, t, launches, _ = _layer(M, k, E, H, 128, ids.to(DEV), x)
     assert launches == 4
-    q, s = lo.quant.per_token_group_quant_int8(x, 128)
-    q, s, flat = q.cpu(), s.cpu(), ids.reshape(-1).tolist()
-    want, chunks = [], []
-    for e in range(E):
-        mine = [i for i, v in enumerate(flat) if v == e]
-        avg = M * k // E
-        most = 160 if avg >= 120 else (64 if avg <= 48 else 128)
-        n = -(-len(mine) // most)
-        per = -(-(-(-len(mine) // n)) // 16) * 16 if n else 0
-        chunks += [[e, len(want) + r, min(per, len(mine) - r), (len(mine) - r - 1) // per] for r in range(0, len(mine), per or 1)]
-        want += mine + [M * k] * (-len(mine) % 16)
-    assert t["n_pad"] == len(want) and t["sorted"].tolist() == want + [M * k] * (t["sorted"].numel() - len(want))
-    assert t["chunks"].tolist() == chunks
-    for p, i in enumerate(want):
-        if i < M * k:
-            assert torch.equal(t["xq"][p], q[i // k]) and torch.equal(t["xs"][p], s[i // k])
+    check_tables(t, ids, E, *lo.quant.per_token_group_quant_int8(x, 128))
 
 
 @pytest.mark.parametrize("M", [32, 33])          # 256 ids are one kernel, 264 are two
