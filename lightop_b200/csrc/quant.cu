@@ -644,8 +644,9 @@ __global__ void __launch_bounds__(ROW_THREADS, CTAS) linear_rows_kernel(const T 
 
 // Outputs a CTA: a power of two, one wave of CTAs where the outputs allow it.
 inline int rows_outs(int64_t N) {
+  const int64_t ctas = (int64_t)ROW_CTAS * sm_count();
   int outs = 4;
-  while (outs < ROW_OUTS_MAX && N > (int64_t)outs * ROW_CTAS * sm_count()) outs *= 2;
+  while (outs < ROW_OUTS_MAX && N > outs * ctas) outs *= 2;
   return outs;
 }
 

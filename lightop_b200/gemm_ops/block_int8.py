@@ -86,8 +86,8 @@ def _dynamic_linear(x: torch.Tensor, w: torch.Tensor, block_size: List[int], w_s
     with _lib.on_device(dev):
         nbytes = lib.lo_block_int8_linear_dynamic_scratch_bytes(M, N, K, code)
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
-        st = lib.lo_block_int8_linear_dynamic(_lib.ptr(x), code, _lib.ptr(w), _lib.ptr(bs), M, N, K,
-                                              _lib.ptr(C), _lib.ptr(ws), nbytes, _lib.ptr(device_status_word(dev)),
+        st = lib.lo_block_int8_linear_dynamic(x.data_ptr(), code, w.data_ptr(), bs.data_ptr(), M, N, K, C.data_ptr(),
+                                              ws.data_ptr() if nbytes else 0, nbytes, device_status_word(dev).data_ptr(),
                                               _lib.current_stream(dev))
     _lib.check(st, "apply_w8a8_block_int8_linear")
     return C if x.dtype == torch.bfloat16 else C.to(x.dtype)

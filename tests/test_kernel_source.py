@@ -90,4 +90,4 @@ def test_the_linear_of_a_few_rows_has_the_ctas_its_rules_count_with():
     assert len(forms) == 4
     for before, _, ctas in forms:
         assert ctas == "ROW_CTAS" or "(int)grid.x <= sm_count()" in before
-    assert "N > (int64_t)outs * ROW_CTAS * sm_count()" in text and "N > (int64_t)ROW_OUTS_MAX * ROW_CTAS * sm_count()" in text
+    assert "ctas = (int64_t)ROW_CTAS * sm_count()" in text and "N > outs * ctas" in text and "N > (int64_t)ROW_OUTS_MAX * ROW_CTAS * sm_count()" in text
