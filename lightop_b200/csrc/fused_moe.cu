@@ -62,8 +62,13 @@ FusedLayout carve_fused(void *ws, int64_t M, int num_experts_for_align, int topk
 //   rows per expert              128                    156 (shard)            181                   203 (shard)           256
 //   Qwen3 shape (shards: DeepSeek-V3, one of eight), even   929 / 815 / 739    650 / 607 / 556     1193 / 1099 / 1122     825 / 698 / 700     1568 / 1402 / 1336
 //   Qwen3, Zipf (1.2) routing     892 /  845 /  880                                                                                           1529 / 1383 / 1398
-//   <= 48 rows per expert : 64-row chunks.  A weight-streaming call wants the deep rings, and the few experts that do get
-//                           more rows have a second chunk (with even routing up to 56).
+// Caps of 64 / 128 rows around the first line, on another board:
+//   rows per expert               32             40             48             56             64
+//   Qwen3 shape, Zipf (1.2)       353 /  356     423 /  424     465 /  458     500 /  484     548 /  532      even 56: 490 / 501, 64: 589 / 541
+//   DeepSeek-V3, Zipf (1.2)      1255 / 1207                   1659 / 1549    1892 / 1777                     even 56: 2335 / 2266
+//   <= 48 rows per expert : 64-row chunks.  A weight-streaming call wants the deep rings: 7 % with even routing.  With Zipf routing 128-row
+//                           chunks are up to 7 % ahead from 32 rows per expert on; the routing is not known on the host.  At 56 the two
+//                           are within 3 % either way with even routing, by board, and 128 is ahead with Zipf.
 //   49 .. 119             : 128-row chunks
 //   >= 120                : 160-row chunks: with 128 rows per expert half of the experts have a few rows more than 128, and a
 //                           second chunk means a second pass over the expert's weights.  With skewed routing 128-row chunks are up to 4 %

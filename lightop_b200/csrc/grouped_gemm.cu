@@ -39,10 +39,10 @@
 //
 // What it measured (DeepSeek-V3 shape, one layer, sustained at the 1000 W power cap; before = a per-step hand-over of scales
 // through the issuer, a thread on one channel and 16 tokens, two issuer warps and the output in the promotion warps):
-// 64 tokens 1764 -> 1480 us, 777 tokens 2290 -> 1880 us, 4096 tokens 3850 -> 3340 us on one board (others: 1415, 1740, 2880 to 3000
-// now).  The board is at its power cap in all of these (SM clock 1.35 to 1.5 GHz), so what a change saves in cycles comes back
+// 64 tokens 1764 -> 1480 us, 777 tokens 2290 -> 1880 us, 4096 tokens 3850 -> 3340 us on one board (others: 1415 to 1440, 1740 to 1840, 2880
+// to 3050 now).  The board is at its power cap in all of these (SM clock 1.35 to 1.5 GHz), so what a change saves in cycles comes back
 // as time only in part.  Instructions besides the arithmetic cost at the cap as well: shorter waits and a scale loop of half the length
-// made 4096 tokens 4 % and Zipf routing 7 % faster there (at burst clocks the launches take the same time; down GEMM without an
+// made 4096 tokens 4 to 6 % and Zipf routing 7 % faster there (at burst clocks the launches take the same time; down GEMM without an
 // instruction to issue 1.13 -> 0.90 warps per issue).
 //
 // Per-channel mode (one scale per token and one per output channel instead of 128x128 blocks) uses the same feed without the
@@ -67,7 +67,9 @@ namespace {
 // How a wait polls, by the chunk cap of the instantiation (see Smem::POLL).  The plain form is the shortest in the loops of all roles,
 // which share the instruction caches and the power: with sleeps and hints in their place 4096 tokens took 3147 us instead of 3091, Qwen3 2048 Zipf 935 instead of
 // 892, sharded 8192 797 instead of 789.  Where the weights bound the kernel, the board's power does: 32 tokens in a graph 1066 plain, 1055
-// with sleeps; 64 tokens (cap 64) 1419 plain, 1422 to 1424 with sleeps, 1415 with a hint.
+// with sleeps.  With a cap of 64 rows a hint saves 0.2 to 0.3 %, which three runs of each side in turn tell apart at the DeepSeek-V3 shape (40
+// tokens 1218.7 to 1221.6 with a hint, 1223.2 to 1223.9 plain; 64 1436.9 to 1437.5, 1440.1 to 1440.8; 256 1730.6 to 1733.1, 1736.3 to 1738.5);
+// the same sign within the spread for 777 tokens and at the Qwen3 shape (64 tokens 359.7 to 360.8, 359.7 to 363.1); sleeps cost 0.3 to 0.6 %.
 enum Poll { PLAIN, HINT, SLEEP };
 // SLEEP: interval between two polls in nanoseconds, by role
 constexpr uint32_t LO_SLEEP_PRODUCER = 128u, LO_SLEEP_SCALE = 128u, LO_SLEEP_MMA = 20u, LO_SLEEP_PROMO = 32u, LO_SLEEP_OUT = 256u;
