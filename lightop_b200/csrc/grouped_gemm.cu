@@ -18,7 +18,7 @@
 //
 // Warp roles in a CTA of 16 warps (block-scaled modes):
 //   warp 0       : weight producer: streams the weight tiles (HBM) into ring w[] by TMA
-//   warp 1       : MMA issuer.  Two lanes follow the two barriers of a step (operands ready, partial buffer free), poll in
+//   warp 1       : MMA issuer (of a pair of CTAs: rank 0's; the other's passes consumed[] on).  Two lanes follow the two barriers of a step (operands ready, partial buffer free), poll in
 //                  the same instruction and agree by a vote; one elected lane issues the four MMAs of the step and one
 //                  commit to done[].  Owns the tensor-memory allocation.
 //   warp 2       : scale producer: token scales times weight-block scale, tables of four steps at a time
@@ -49,6 +49,13 @@
 // promotion: a tensor-memory buffer is the int32 accumulator of a whole item, summed over every K block by the tensor core, and
 // 16 or 20 warps run an epilogue (int32 -> fp32, times token scale, times channel scale) while the MMAs of the next items fill
 // the other buffers.  The scale producer idles and there are no output warps in that mode.
+//
+// Pairs.  Wide chunks of calls with enough work run on clusters of two CTAs (see use_pairs()): two neighbouring tiles of a chunk are one MMA of
+// 256 rows (cta_group::2), for which each CTA loads its own weight tile and half of the chunk's token rows.  The rows of a chunk, which each
+// tile reads again from L2, cross to the SMs half as often, take half of the shared memory (the weight ring of 160-row chunks has 7 slots
+// instead of 5, per channel that of 256-row ones 9 instead of 5) and are read from there by one MMA instead of two.  Rank 0 issues for both: the loads of both CTAs complete on its ready[],
+// its commits arrive at done[] of both, and the other CTA's warp 1 passes on what its own promotion warps hand back.  Everything behind the
+// MMAs (promotion, scales, output) stays with each CTA's tile.
 //
 // Every wait is bounded: after about a second a waiter records a timeout in the
 // status word, raises a CTA-wide abort flag, and all roles fall through to the
@@ -96,7 +103,7 @@ constexpr int SMEM_LIMIT = 227 * 1024;          // dynamic shared memory a CTA c
 // A_ROWS is the largest chunk (token count) the instantiation accepts: with few tokens per call no
 // expert can receive more than that many rows, the activation tiles shrink and more weight tiles fit
 // into shared memory (more weight bytes in flight per SM).
-template <int MODE, int A_ROWS> struct Cfg {
+template <int MODE, int A_ROWS, bool PAIR = false> struct Cfg {
   // gate_up: an item is two passes over K on the same chunk, first the gate tile, then the up tile
   static constexpr int PHASES = MODE == GEMM_GATE_UP ? 2 : 1;
   // Column groups: the chunk's tokens are dealt, in pieces of 16, to this many sets of four warps (one warp per lane quarter
@@ -107,7 +114,8 @@ template <int MODE, int A_ROWS> struct Cfg {
   static constexpr int NUM_THREADS = (FIRST_EPI_WARP + EPI_WARPS + (MODE == GEMM_CHANNEL ? 0 : OUT_WARPS)) * 32;
   static constexpr bool SPLIT_REGS = MODE != GEMM_CHANNEL && A_ROWS > 64;
   static_assert(!SPLIT_REGS || NUM_THREADS == 512, "the register split is made for four warp groups");
-  static constexpr int A_TILE_BYTES = A_ROWS * TILE_K;
+  // a pair of CTAs shares a chunk's rows: each keeps half of them
+  static constexpr int A_TILE_BYTES = (PAIR ? A_ROWS / 2 : A_ROWS) * TILE_K;
   // Two rings.  Activation tiles come from L2 (the chunk's rows are read by every output tile of the expert): a
   // slot is refilled only after the MMAs that read it have completed, so the ring has to cover the load latency
   // plus the MMA queue, four K blocks at least.  Weight tiles come from HBM and get the shared memory that is left.
@@ -132,11 +140,12 @@ template <int MODE, int A_ROWS> constexpr bool ring_depths(int weight_slots, int
 }
 static_assert(ring_depths<GEMM_SINGLE, 32>(11, 8) && ring_depths<GEMM_SINGLE, 64>(8, 8) && ring_depths<GEMM_SINGLE, 128>(7, 4) &&
               ring_depths<GEMM_SINGLE, T_WIDE>(5, 3), "block-scaled: weight slots and partial buffers as the chunk rule states them");
+static_assert(Cfg<GEMM_SINGLE, T_WIDE, true>::NW == 7 && Cfg<GEMM_CHANNEL, 256, true>::NW == 9, "pairs: weight slots as the head of this file states them");
 static_assert(ring_depths<GEMM_CHANNEL, 64>(9, 8) && ring_depths<GEMM_CHANNEL, 128>(9, 4) && ring_depths<GEMM_CHANNEL, T_WIDE>(8, 3) &&
               ring_depths<GEMM_CHANNEL, 256>(5, 2), "per channel: weight slots and accumulators as the chunk rule states them");
 
-template <int MODE, int A_ROWS> struct Smem {
-  using C = Cfg<MODE, A_ROWS>;
+template <int MODE, int A_ROWS, bool PAIR = false> struct Smem {
+  using C = Cfg<MODE, A_ROWS, PAIR>;
   static constexpr int POLL = A_ROWS <= 32 ? SLEEP : (A_ROWS <= 64 && MODE != GEMM_CHANNEL ? HINT : PLAIN);
   // operand tiles first: each is a multiple of 1024 bytes, base is 1024-aligned
   uint8_t w[C::NW][W_TILE_BYTES];
@@ -153,6 +162,7 @@ template <int MODE, int A_ROWS> struct Smem {
   // promotion warps (the partial of the step is in its buffer).
   uint64_t done[ND];
   uint64_t consumed[ND];                   // block-scaled modes: the partial of the step has been read, its buffer is free
+  uint64_t peer_consumed[PAIR ? ND : 1];   // pairs, block-scaled modes, leader: consumed[] of the other CTA
   uint64_t scales[SC_BATCHES];             // block-scaled modes: the batch's scale products are in place
   uint64_t tmem_full[C::NBUF];             // per-channel mode: the accumulator of an item is complete
   uint64_t tmem_empty[C::NBUF];            // per-channel mode: the accumulator has been read
@@ -236,6 +246,33 @@ __device__ __forceinline__ bool mbar_test_addr(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ void mbar_arrive_addr(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// Barriers of the CTA that issues a pair's MMAs (rank 0 of the cluster), by their address in the cluster.  The arrival says that values have
+// left tensor memory, which their tcgen05.wait::ld has seen to; it publishes no data, and asks for no release at cluster scope: with one
+// (mbarrier.arrive.release.cluster) every step of a pair waited for it, 4096 tokens 2797 -> 5944 us.
+struct ClusterBarrier {
+  uint32_t addr;
+};
+__device__ __forceinline__ ClusterBarrier operator+(ClusterBarrier b, uint32_t bytes) { return ClusterBarrier{b.addr + bytes}; }
+__device__ __forceinline__ void mbar_arrive_addr(ClusterBarrier bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar.addr) : "memory");
+}
+template <bool PAIR> __device__ __forceinline__ auto issuer_barrier(uint32_t addr) {
+  if constexpr (PAIR) {
+    ClusterBarrier b;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(b.addr) : "r"(addr));
+    return b;
+  } else {
+    return addr;
+  }
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -256,13 +293,19 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
   return p;
 }
 
-// 2-D tiled TMA load global -> shared (this CTA), completion on an mbarrier.
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int32_t x, int32_t y, uint64_t *bar,
-                                            uint64_t policy) {
+// 2-D tiled TMA load global -> shared (this CTA), completion on an mbarrier of this CTA or of the pair's issuer.
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t bar, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
       " [%0], [%1, {%2, %3}], [%4], %5;"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy)
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int32_t x, int32_t y, ClusterBarrier bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint"
+      " [%0], [%1, {%2, %3}], [%4], %5;"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar.addr), "l"(policy)
       : "memory");
 }
 
@@ -285,32 +328,44 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
   return d;
 }
 
-// Instruction descriptor: int8 x int8 -> int32, both operands K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t make_idesc(uint32_t n) {
+// Instruction descriptor: int8 x int8 -> int32, both operands K-major, M = m, N = n.
+__device__ __forceinline__ uint32_t make_idesc(uint32_t m, uint32_t n) {
   uint32_t d = 0;
   d |= 2u << 4;            // accumulator format: S32
   d |= 1u << 7;            // A format: signed 8-bit
   d |= 1u << 10;           // B format: signed 8-bit
   d |= (n >> 3) << 17;     // N / 8
-  d |= (128u >> 4) << 24;  // M / 16
+  d |= (m >> 4) << 24;     // M / 16
   return d;
 }
 
-// The descriptors' upper halves are the same for every operand; the lower ones hold the start address.
+// The descriptors' upper halves are the same for every operand; the lower ones hold the start address.  PAIR: one MMA on the operands and the
+// tensor memory of both CTAs, at the same places in each.
+template <bool PAIR>
 __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint32_t adesc_lo, uint32_t bdesc_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
-      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %4, p;\n\t}"
-      ::"r"(tmem_d), "r"(adesc_lo), "r"(bdesc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
+  if (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], a, b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(adesc_lo), "r"(bdesc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(adesc_lo), "r"(bdesc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
-__device__ __forceinline__ void umma_commit_addr(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// An arrival at the barrier (of both CTAs of a pair) when the MMAs issued so far have completed.
+template <bool PAIR> __device__ __forceinline__ void umma_commit_addr(uint32_t bar) {
+  if (PAIR)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // 16 consecutive tensor-memory columns of this thread's lane.
@@ -468,7 +523,8 @@ struct KParams {
 };
 
 // Four tensor maps of the sorted activation matrix, box heights 16 / 32 / 64 / 128 rows.  A chunk of
-// more than 128 rows (per-channel mode only) is fetched as a 128-row box plus a second box for the rest.
+// more than 128 rows is fetched as a 128-row box plus a second box for the rest; the halves of a pair's chunk (a multiple of 16 rows each) as one
+// box or two that cover no other rows, where two can.
 struct AMaps {
   CUtensorMap m[4];
 };
@@ -481,7 +537,7 @@ __device__ __forceinline__ int a_map_index(int T) { return T <= 16 ? 0 : (T <= 3
 // Where the chunks come from is part of the instantiation (a branch for it in the common kernel cost the block-scaled loops
 // registers and 3 to 9 % at 4096 rows).
 enum Form { TABLE, DENSE, SPLIT };      // chunk table / one expert, from arithmetic / the same with the K extent of a tile split
-template <int MODE, int FORM> struct ItemCursor {
+template <int MODE, int FORM, bool PAIR> struct ItemCursor {
   const KParams &p;
   int num_chunks, n_tiles, ci, nt, step_c, step_t;
   int k0, kn;            // K blocks of the item taken last
@@ -503,16 +559,18 @@ template <int MODE, int FORM> struct ItemCursor {
     next = *reinterpret_cast<const int4 *>(p.chunks + ci);
   }
   __device__ __forceinline__ ItemCursor(const KParams &params, int n_chunks)
-      : p(params), num_chunks(n_chunks), n_tiles(FORM == SPLIT ? params.n_tiles * params.n_split : params.n_tiles),
+      : p(params), num_chunks(n_chunks), n_tiles(FORM == SPLIT ? params.n_tiles * params.n_split : (PAIR ? params.n_tiles / 2 : params.n_tiles)),
         k0(0), kn(params.KB), next(make_int4(-1, 0, 0, 0)) {
-    ci = (int)blockIdx.x / n_tiles; nt = (int)blockIdx.x % n_tiles;
-    step_c = (int)gridDim.x / n_tiles; step_t = (int)gridDim.x % n_tiles;
+    // a pair walks the items as one: two tiles of a chunk, one for each CTA
+    const int self = PAIR ? (int)blockIdx.x / 2 : (int)blockIdx.x, all = PAIR ? (int)gridDim.x / 2 : (int)gridDim.x;
+    ci = self / n_tiles; nt = self % n_tiles;
+    step_c = all / n_tiles; step_t = all % n_tiles;
     fetch();
   }
   __device__ __forceinline__ bool take(Chunk &ch, int &tile) {
     if (ci >= num_chunks) return false;
     ch.expert = next.x; ch.row0 = next.y; ch.rows = next.z; ch.pad = next.w;
-    tile = nt;
+    tile = PAIR ? 2 * nt + (int)(blockIdx.x & 1) : nt;
     if constexpr (FORM == SPLIT) {
       const int part = nt / p.n_tiles;
       tile = nt - part * p.n_tiles;
@@ -527,11 +585,11 @@ template <int MODE, int FORM> struct ItemCursor {
   }
 };
 
-template <int MODE, int A_ROWS, int FORM>
-__global__ void __launch_bounds__((Cfg<MODE, A_ROWS>::NUM_THREADS), 1)
+template <int MODE, int A_ROWS, int FORM, bool PAIR>
+__global__ void __launch_bounds__((Cfg<MODE, A_ROWS, PAIR>::NUM_THREADS), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ AMaps a_maps, const KParams p) {
-  using SM = Smem<MODE, A_ROWS>;
-  using CF = Cfg<MODE, A_ROWS>;
+  using SM = Smem<MODE, A_ROWS, PAIR>;
+  using CF = Cfg<MODE, A_ROWS, PAIR>;
   constexpr int NW = CF::NW;
   constexpr int NA = CF::NA;
   constexpr int NBUF = CF::NBUF;
@@ -548,6 +606,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   // roles, tensor-memory addresses, barrier addresses) is uniform across the warp
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;      // 0: the CTA that issues the pair's MMAs
 
   // ------------------------------ set-up -----------------------------------
   if (tid == 0) {
@@ -555,11 +614,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       mbar_init(&sm.ready[s], 2);            // the two producers
       mbar_init(&sm.done[s], 1);             // tcgen05.commit of the MMA thread
       mbar_init(&sm.consumed[s], EPI_WARPS * 32);      // every lane of the promotion warps
+      if (PAIR) mbar_init(&sm.peer_consumed[PAIR ? s : 0], 1);
     }
     for (int b = 0; b < SC_BATCHES; ++b) mbar_init(&sm.scales[b], 1);
     for (int b = 0; b < NBUF; ++b) {
       mbar_init(&sm.tmem_full[b], 1);
-      mbar_init(&sm.tmem_empty[b], EPI_WARPS);
+      mbar_init(&sm.tmem_empty[b], (PAIR ? 2 : 1) * EPI_WARPS);
     }
     mbar_init(&sm.stg_full, EPI_WARPS);
     mbar_init(&sm.stg_free, OUT_WARPS);
@@ -567,9 +627,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     fence_barrier_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(TMEM_COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(TMEM_COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   if (tid == 32) {
     // descriptors into the descriptor cache while the set-up runs
@@ -580,6 +646,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();      // the other CTA's barriers are there
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
 
@@ -602,10 +669,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       if (lane == 0) {
         const uint64_t pol_stream = policy_evict_first();
         const uint64_t pol_keep = policy_evict_normal();
+        const auto ready0 = issuer_barrier<PAIR>(smem_u32(&sm.ready[0]));
         uint32_t it = 0;
         int s = 0;
         bool ok = true;
-        for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
+        for (ItemCursor<MODE, FORM, PAIR> items(p, num_chunks); ok && items.take(ch, nt);) {
           if (ch.expert < 0) continue;
           // weight tiles are streamed (evict-first) unless another chunk of the same expert is about to read
           // them again: those stay in L2 under the normal policy
@@ -615,8 +683,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NW
               if (it >= (uint32_t)NW && !mbar_wait(sm, &sm.done[(it - NW) % ND], ((it - NW) / ND) & 1u, p.status, 1, LO_SLEEP_PRODUCER)) { ok = false; break; }
-              mbar_arrive_expect_tx(&sm.ready[it % ND], W_TILE_BYTES);
-              tma_load_2d(sm.w[s], &w_map, kb * TILE_K, row_g, &sm.ready[it % ND], pol_w);
+              const auto bar = ready0 + 8u * (it % ND);
+              if (rank == 0) mbar_arrive_expect_tx(&sm.ready[it % ND], (PAIR ? 2 : 1) * W_TILE_BYTES);
+              tma_load_2d(sm.w[s], &w_map, kb * TILE_K, row_g, bar, pol_w);
               s = s + 1 == NW ? 0 : s + 1;
             }
           }
@@ -628,25 +697,28 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       // it (a second one for the rows beyond 128).
       if (lane == 0) {
         const uint64_t pol_a = policy_evict_last();
+        const auto ready0 = issuer_barrier<PAIR>(smem_u32(&sm.ready[0]));
         uint32_t it = 0;
         int s = 0;
         bool ok = true;
-        for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
+        for (ItemCursor<MODE, FORM, PAIR> items(p, num_chunks); ok && items.take(ch, nt);) {
           if (ch.expert < 0) continue;
-          const int T = (ch.rows + 15) & ~15;
-          const int T0 = T > 128 ? 128 : T;                  // first box; the rest (if any) goes into a second one
-          const int mi = a_map_index(T0);
-          const int mi2 = T > 128 ? a_map_index(T - 128) : -1;
+          // one box, or two: the rows beyond 128, and for pairs, whose half of the rows is a multiple of 16, what is beyond a power of two
+          const int T = PAIR ? (ch.rows + 31) / 32 * 16 : (ch.rows + 15) & ~15;
+          const int mi = PAIR ? 27 - __clz(T) : a_map_index(T > 128 ? 128 : T);
+          const int T0 = PAIR || T > 128 ? 16 << mi : T;
+          const int mi2 = T > T0 ? a_map_index(T - T0) : -1;
           const uint32_t a_bytes = (16u << mi) * TILE_K + (mi2 >= 0 ? (16u << mi2) * TILE_K : 0u);
+          const int row0 = ch.row0 + (PAIR ? (int)rank * T : 0);
           for (int ph = 0; ph < PHASES && ok; ++ph) {
             for (int kb = FORM == SPLIT ? items.k0 : 0; kb < (FORM == SPLIT ? items.k0 + items.kn : KB); ++kb, ++it) {
               // slot s was read by step it - NA
               if (it >= (uint32_t)NA && !mbar_wait(sm, &sm.done[(it - NA) % ND], ((it - NA) / ND) & 1u, p.status, 6, LO_SLEEP_PRODUCER)) { ok = false; break; }
-              uint64_t *bar = &sm.ready[it % ND];
-              mbar_arrive_expect_tx(bar, a_bytes);
-              tma_load_2d(sm.a[s], &a_maps.m[mi], kb * TILE_K, ch.row0, bar, pol_a);
-              if constexpr (A_ROWS > 128) {
-                if (mi2 >= 0) tma_load_2d(sm.a[s] + 128 * TILE_K, &a_maps.m[mi2], kb * TILE_K, ch.row0 + 128, bar, pol_a);
+              const auto bar = ready0 + 8u * (it % ND);
+              if (rank == 0) mbar_arrive_expect_tx(&sm.ready[it % ND], (PAIR ? 2u : 1u) * a_bytes);
+              tma_load_2d(sm.a[s], &a_maps.m[mi], kb * TILE_K, row0, bar, pol_a);
+              if constexpr (PAIR || A_ROWS > 128) {
+                if (mi2 >= 0) tma_load_2d(sm.a[s] + T0 * TILE_K, &a_maps.m[mi2], kb * TILE_K, row0 + T0, bar, pol_a);
               }
               s = s + 1 == NA ? 0 : s + 1;
             }
@@ -667,7 +739,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         const int64_t nblk = (p.n_rows_per_expert + TILE_N - 1) / TILE_N;
         auto produce = [&](auto by_four) {
         constexpr bool vec = decltype(by_four)::value;
-        ItemCursor<MODE, FORM> items(p, num_chunks);
+        ItemCursor<MODE, FORM, PAIR> items(p, num_chunks);
         struct Batch { Chunk ch; int nt, ph, kb; bool valid; };     // K blocks kb .. kb + 3 of a pass over an item
         float a_cur[NU][4], b_cur[4], a_nxt[NU][4], b_nxt[4];
         auto next_item = [&](Batch &b) {
@@ -751,6 +823,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         if ((KB & 3) == 0) produce(std::true_type{});
         else produce(std::false_type{});
       }
+    } else if (PAIR && rank != 0) {
+      // ============ second CTA of a pair, warp 1: passes the partial buffers that its promotion warps hand back on to the issuer ============
+      // (One arrival a step across the cluster instead of one of every lane.  Per-channel accumulators are handed back once an item, by the
+      // epilogue warps themselves.)
+      if (MODE != GEMM_CHANNEL && lane == 0) {
+        const uint32_t consumed0 = smem_u32(&sm.consumed[0]);
+        const auto peer0 = issuer_barrier<PAIR>(smem_u32(&sm.peer_consumed[0]));
+        uint32_t it = 0;
+        bool ok = true;
+        for (ItemCursor<MODE, FORM, PAIR> items(p, num_chunks); ok && items.take(ch, nt);) {
+          if (ch.expert < 0) continue;
+#pragma unroll 1
+          for (uint32_t u = 0; u < (uint32_t)(PHASES * KB); ++u, ++it) {
+            const uint32_t at = 8u * (it & (uint32_t)(ND - 1));
+            if (!mbar_wait_addr(sm, consumed0 + at, (it >> 4) & 1u, p.status, 11, LO_SLEEP_MMA)) { ok = false; break; }
+            tc_fence_after();
+            tc_fence_before();
+            mbar_arrive_addr(peer0 + at);
+          }
+        }
+      }
     } else {
       // ============================ MMA issuer (warp 1) ================================
       // A step of this role is a chain of dependent instructions and barrier round trips, which takes longer than the
@@ -769,13 +862,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       const uint32_t done0 = smem_u32(&sm.done[0]);
       // this lane's barrier of step u is number (u + my_off) % ND of its ring; a buffer is waited for with the step that
       // used it before (the steps before the first one read as complete: parity 1 of a fresh barrier)
-      const uint32_t my_base = smem_u32(lane == 0 ? &sm.ready[0] : &sm.consumed[0]);
+      constexpr int WAITERS = PAIR && MODE != GEMM_CHANNEL ? 3 : 2;      // pairs: lane 2 has the other CTA's partial buffer
+      const uint32_t my_base = smem_u32(lane == 0 ? &sm.ready[0] : (lane == 1 ? &sm.consumed[0] : &sm.peer_consumed[0]));
       const uint32_t my_off = lane == 0 ? 0u : 0u - (uint32_t)NBUF;
       uint32_t acc_par = 1;              // per-channel mode: phase of the accumulator ring
-      bool ok = true, seen = lane > 1;
-      for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
+      bool ok = true, seen = lane >= WAITERS;
+      for (ItemCursor<MODE, FORM, PAIR> items(p, num_chunks); ok && items.take(ch, nt);) {
         if (ch.expert < 0) continue;
-        const uint32_t idesc = make_idesc((uint32_t)((__shfl_sync(0xffffffffu, ch.rows, 0) + 15) & ~15));
+        // (a pair's N is a multiple of 32)
+        constexpr uint32_t GRAN = PAIR ? 32u : 16u;
+        const uint32_t idesc = make_idesc(PAIR ? 256u : 128u, ((uint32_t)__shfl_sync(0xffffffffu, ch.rows, 0) + GRAN - 1u) & ~(GRAN - 1u));
         const uint32_t steps = (uint32_t)(FORM == SPLIT ? items.kn : PHASES * KB);
 #pragma unroll 1
         for (uint32_t u = 0; u < steps; ++u, ++it) {
@@ -783,7 +879,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (!seen) {
               uint32_t bar = my_base + 8u * ((it + my_off) & (uint32_t)(ND - 1)), par = ((it + my_off) >> 4) & 1u;
               if (MODE == GEMM_CHANNEL && lane == 1) { bar = smem_u32(&sm.tmem_empty[sb]); par = acc_par; }
-              seen = mbar_wait_addr(sm, bar, par, p.status, 3 + lane, LO_SLEEP_MMA);
+              seen = mbar_wait_addr(sm, bar, par, p.status, lane == 2 ? 10 : 3 + lane, LO_SLEEP_MMA);
             }
             if (!__all_sync(0xffffffffu, seen)) { ok = false; break; }
             __syncwarp();      // what one lane has seen holds for the lane that issues (a vote does not order memory)
@@ -793,7 +889,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           // the early look at the next step
           const uint32_t nx = it + 1u + my_off;
           if (MODE == GEMM_CHANNEL) seen = lane > 1 || (lane == 1 && !last) || (lane == 0 && mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u));
-          else seen = lane > 1 || mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u);
+          else seen = lane >= WAITERS || mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u);
           // descriptor start addresses are in 16-byte units
           const uint32_t adesc = desc_w0 + sw * (uint32_t)(W_TILE_BYTES >> 4);
           const uint32_t bdesc = desc_a0 + sa * (uint32_t)(CF::A_TILE_BYTES >> 4);
@@ -801,10 +897,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           if (elect_one()) {
 #pragma unroll
             for (int k4 = 0; k4 < TILE_K / 32; ++k4)
-              umma_i8(d, adesc + (uint32_t)(k4 * 2), bdesc + (uint32_t)(k4 * 2), desc_hi, idesc,
+              umma_i8<PAIR>(d, adesc + (uint32_t)(k4 * 2), bdesc + (uint32_t)(k4 * 2), desc_hi, idesc,
                       (MODE == GEMM_CHANNEL ? (u | (uint32_t)k4) : (uint32_t)k4) != 0u ? 1u : 0u);
-            umma_commit_addr(done0 + 8u * (it & (uint32_t)(ND - 1)));
-            if (MODE == GEMM_CHANNEL && last) umma_commit(&sm.tmem_full[sb]);
+            umma_commit_addr<PAIR>(done0 + 8u * (it & (uint32_t)(ND - 1)));
+            if (MODE == GEMM_CHANNEL && last) umma_commit_addr<PAIR>(smem_u32(&sm.tmem_full[sb]));
           }
           __syncwarp();
           sw = sw + 1 == (uint32_t)NW ? 0u : sw + 1;
@@ -823,7 +919,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     const int ow = warp - (FIRST_EPI_WARP + EPI_WARPS);
     uint32_t par = 0;
     // (the parts of a split K extent leave the kernel as int32 sums, straight from the promotion warps)
-    for (ItemCursor<MODE, FORM> items(p, FORM == SPLIT ? 0 : num_chunks); items.take(ch, nt);) {
+    for (ItemCursor<MODE, FORM, PAIR> items(p, FORM == SPLIT ? 0 : num_chunks); items.take(ch, nt);) {
       if (ch.expert < 0) {
         // block of a non-local expert: its output rows are zero
         if (MODE == GEMM_SINGLE && p.C != nullptr) {
@@ -944,7 +1040,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     uint32_t sc_slot = 0, sc_par = 0;            // ring of scale batches
     uint32_t buf = 0, step = 0;                  // block-scaled modes: partial buffer and count of the K-block step
     bool ok = true;
-    for (ItemCursor<MODE, FORM> items(p, num_chunks); ok && items.take(ch, nt);) {
+    for (ItemCursor<MODE, FORM, PAIR> items(p, num_chunks); ok && items.take(ch, nt);) {
       if (ch.expert < 0) {
         // block of a non-local expert: its output rows are zero (the block-scaled modes leave that to the output warps)
         if (MODE == GEMM_CHANNEL && p.C != nullptr) {
@@ -994,6 +1090,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         const bool n_ok = n_glob < p.n_store;
         const float bs = n_glob < p.n_rows_per_expert ? __ldg(p.b_scale + (int64_t)ch.expert * p.n_rows_per_expert + n_glob) : 0.f;
         const uint32_t b = ab % NBUF;
+        const auto empty = issuer_barrier<PAIR>(smem_u32(&sm.tmem_empty[b]));      // the accumulator goes back to the warp that issues the MMAs
         const uint32_t aph = (ab / NBUF) & 1u;
         ++ab;
         if (!__all_sync(0xffffffffu, mbar_wait(sm, &sm.tmem_full[b], aph, p.status, 5))) { ok = false; break; }
@@ -1008,7 +1105,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             // every value this warp needs is in registers: hand the buffer back before the stores
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.tmem_empty[b]);
+            if (lane == 0) mbar_arrive_addr(empty);
           }
           // piece pc holds tokens 16 * pc .. 16 * pc + 15 of this group: register set pc / 2, lanes 16 * (pc & 1) ..
           const int32_t sid_u = pick(sid_r, pc >> 1);
@@ -1031,7 +1128,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         }
         if (my_p == 0) {
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.tmem_empty[b]);
+          if (lane == 0) mbar_arrive_addr(empty);
         }
       } else if constexpr (FORM == SPLIT) {
         // ---------------- a part of the K extent: the int32 sum of every K block as it is ----------------
@@ -1282,9 +1379,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     while (clock64() - t0 < 400000ll) {
     }
   }
+  if (PAIR) cluster_sync();      // neither CTA leaves, or frees its tensor memory, while the other may use it
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
 
@@ -1330,20 +1429,21 @@ int make_tile_map(CUtensorMap *map, const int8_t *base, int64_t rows, int64_t K,
   return LO_OK;
 }
 
-template <int MODE, int A_ROWS, int FORM = TABLE>
+template <int MODE, int A_ROWS, int FORM = TABLE, bool PAIR = false>
 int launch_mode(const GemmArgs &a, cudaStream_t stream) {
-  using SM = Smem<MODE, A_ROWS>;
+  using SM = Smem<MODE, A_ROWS, PAIR>;
+  using CF = Cfg<MODE, A_ROWS, PAIR>;
   static_assert(sizeof(SM) + 1024 <= SMEM_LIMIT, "shared-memory layout exceeds what a CTA can be given");
   static_assert(ND == 16, "the promotion warps take the completion-ring phase from bit 4 of the step count");
-  static_assert(Cfg<MODE, A_ROWS>::NW >= 4, "too few weight stages");
-  static_assert(Cfg<MODE, A_ROWS>::NW < ND && Cfg<MODE, A_ROWS>::NA < ND && Cfg<MODE, A_ROWS>::NBUF < ND, "completion ring too short");
+  static_assert(CF::NW >= 4, "too few weight stages");
+  static_assert(CF::NW < ND && CF::NA < ND && CF::NBUF < ND, "completion ring too short");
   const size_t smem_bytes = sizeof(SM) + 1024;
   // the attribute belongs to the (kernel, device) pair: set it once per device this thread launches on
   static thread_local uint64_t configured_devices = 0;
   int dev = 0;
   LO_CUDA_OK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !((configured_devices >> dev) & 1u)) {
-    LO_CUDA_OK(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, A_ROWS, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
+    LO_CUDA_OK(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, A_ROWS, FORM, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
     if (dev >= 0 && dev < 64) configured_devices |= (uint64_t)1 << dev;
   }
   CUtensorMap wmap;
@@ -1367,9 +1467,24 @@ int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   p.n_split = a.partial != nullptr ? (int)ceil_div(p.KB, a.split_steps) : 1; p.split_steps = a.split_steps; p.partial = a.partial;
   const int grid = sm_count();
   if (grid <= 0) return fail(LO_ERR_CUDA, "no CUDA device");
-  LO_CUDA_OK(launch_dependent(grouped_gemm_kernel<MODE, A_ROWS, FORM>, dim3(grid), dim3(Cfg<MODE, A_ROWS>::NUM_THREADS), smem_bytes, stream, wmap,
-                              amaps, p));
+  LO_CUDA_OK(launch_dependent_clusters(PAIR ? 2 : 1, grouped_gemm_kernel<MODE, A_ROWS, FORM, PAIR>, dim3(PAIR ? grid & ~1 : grid),
+                                       dim3(CF::NUM_THREADS), smem_bytes, stream, wmap, amaps, p));
   return LO_OK;
+}
+
+// Whether a call with wide chunks runs on pairs of CTAs: tiles come in twos (a pair with one tile idle would waste half of it), and
+// every SM has enough K-block steps to make up for the start, which waits for the other CTA, and for the slower of two CTAs in every step.
+// One CTA / pairs, in us, by the steps of an SM (at least; a call with a chunk table has a chunk an expert or more):
+//   dense linear    20 (2000 x 2304 x 1280) 17.0 / 18.3    60 (600 x 4096 x 7168) 44.4 / 44.9     97 (1000 x 4096 x 7168) 52.1 / 51.8
+//                  145 (1500 x 4096 x 7168) 77.8 / 76.5   194 (2000 x 4096 x 7168) 104.3 / 102.7    387 (4096 x 4096 x 7168) 204 / 197
+//   layers          83 (Qwen3, 4096 tokens of a shard of eight) 200.7 / 202.2    664 (Qwen3 2048, Zipf) 862 / 830    3100 (DeepSeek-V3 4096) 3065 / 3011
+//   per channel      5 (32 experts of 1024 x 384) 154.2 / 154.1    42 and 83 (masked, 16 of 4096 x 1536) 76.9 / 75.3    1550 and 3100 (DeepSeek-V3 2999) 2417 / 2334
+constexpr int PAIR_MIN_STEPS = 96, PAIR_MIN_STEPS_CHANNEL = 32;
+bool use_pairs(GemmMode mode, const GemmArgs &a) {
+  if (a.n_tiles % 2 != 0 || a.partial != nullptr || sm_count() < 2) return false;
+  const int64_t chunks = a.chunks != nullptr ? a.E : a.fixed_chunks;
+  const int64_t steps = chunks * a.n_tiles * (mode == GEMM_GATE_UP ? 2 : 1) * (a.K / TILE_K) / sm_count();
+  return steps >= (mode == GEMM_CHANNEL ? PAIR_MIN_STEPS_CHANNEL : PAIR_MIN_STEPS);
 }
 
 }  // namespace
@@ -1395,13 +1510,14 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
              "grouped gemm: the K extent is split for dense calls only");
   // no chunk can hold more rows than max_chunk_rows (a bound the caller derives from the token count)
   const int cap = a.max_chunk_rows <= 0 ? T_MAX : a.max_chunk_rows;
+  const bool pair = use_pairs(mode, a);
   if (mode == GEMM_GATE_UP) {
     LO_REQUIRE(a.n_rows_per_expert == 2 * (int64_t)a.n_tiles * TILE_N, "grouped gemm: gate_up needs N = 2*I");
     LO_REQUIRE(cap <= T_WIDE, "grouped gemm: block-scaled chunks hold at most 160 rows");
     if (cap <= 32) return launch_mode<GEMM_GATE_UP, 32>(a, stream);
     if (cap <= 64) return launch_mode<GEMM_GATE_UP, 64>(a, stream);
-    if (cap <= 128) return launch_mode<GEMM_GATE_UP, 128>(a, stream);
-    return launch_mode<GEMM_GATE_UP, T_WIDE>(a, stream);
+    if (cap <= 128) return pair ? launch_mode<GEMM_GATE_UP, 128, TABLE, true>(a, stream) : launch_mode<GEMM_GATE_UP, 128>(a, stream);
+    return pair ? launch_mode<GEMM_GATE_UP, T_WIDE, TABLE, true>(a, stream) : launch_mode<GEMM_GATE_UP, T_WIDE>(a, stream);
   }
   LO_REQUIRE((int64_t)a.n_tiles * TILE_N >= a.n_rows_per_expert && (int64_t)(a.n_tiles - 1) * TILE_N < a.n_rows_per_expert,
              "grouped gemm: tile count mismatch");
@@ -1409,9 +1525,9 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
     LO_REQUIRE(cap <= 256, "grouped gemm: per-channel chunks hold at most 256 rows");
     if (cap <= 32) return launch_mode<GEMM_CHANNEL, 32>(a, stream);
     if (cap <= 64) return launch_mode<GEMM_CHANNEL, 64>(a, stream);
-    if (cap <= 128) return launch_mode<GEMM_CHANNEL, 128>(a, stream);
-    if (cap <= T_WIDE) return launch_mode<GEMM_CHANNEL, T_WIDE>(a, stream);
-    return launch_mode<GEMM_CHANNEL, 256>(a, stream);
+    if (cap <= 128) return pair ? launch_mode<GEMM_CHANNEL, 128, TABLE, true>(a, stream) : launch_mode<GEMM_CHANNEL, 128>(a, stream);
+    if (cap <= T_WIDE) return pair ? launch_mode<GEMM_CHANNEL, T_WIDE, TABLE, true>(a, stream) : launch_mode<GEMM_CHANNEL, T_WIDE>(a, stream);
+    return pair ? launch_mode<GEMM_CHANNEL, 256, TABLE, true>(a, stream) : launch_mode<GEMM_CHANNEL, 256>(a, stream);
   }
   LO_REQUIRE(cap <= T_WIDE, "grouped gemm: block-scaled chunks hold at most 160 rows");
   if (a.partial != nullptr) {
@@ -1422,12 +1538,12 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
   if (a.chunks == nullptr) {
     if (cap <= 32) return launch_mode<GEMM_SINGLE, 32, DENSE>(a, stream);
     if (cap <= 64) return launch_mode<GEMM_SINGLE, 64, DENSE>(a, stream);
-    return launch_mode<GEMM_SINGLE, 128, DENSE>(a, stream);
+    return pair ? launch_mode<GEMM_SINGLE, 128, DENSE, true>(a, stream) : launch_mode<GEMM_SINGLE, 128, DENSE>(a, stream);
   }
   if (cap <= 32) return launch_mode<GEMM_SINGLE, 32>(a, stream);
   if (cap <= 64) return launch_mode<GEMM_SINGLE, 64>(a, stream);
-  if (cap <= 128) return launch_mode<GEMM_SINGLE, 128>(a, stream);
-  return launch_mode<GEMM_SINGLE, T_WIDE>(a, stream);
+  if (cap <= 128) return pair ? launch_mode<GEMM_SINGLE, 128, TABLE, true>(a, stream) : launch_mode<GEMM_SINGLE, 128>(a, stream);
+  return pair ? launch_mode<GEMM_SINGLE, T_WIDE, TABLE, true>(a, stream) : launch_mode<GEMM_SINGLE, T_WIDE>(a, stream);
 }
 
 }  // namespace lo
