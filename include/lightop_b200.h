@@ -425,6 +425,11 @@ int lo_m_grouped_w8a8_gemm_nt_contig(const int8_t *A, const float *a_scale, cons
 int lo_m_grouped_w8a8_gemm_nt_masked(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale,
                                      void *C, const int32_t *masked_m, int E, int64_t max_m, int64_t N, int64_t K,
                                      void *workspace, size_t workspace_bytes, int32_t *status, void *stream);
+/* The same with a hint, the rows an expert can be expected to have (0: not known).  Any value gives the same results; it decides on the
+ * kernel's form (pairs of CTAs pay from a few rows on). */
+int lo_m_grouped_w8a8_gemm_nt_masked_expected(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale,
+                                     void *C, const int32_t *masked_m, int E, int64_t max_m, int64_t expected_m, int64_t N, int64_t K,
+                                     void *workspace, size_t workspace_bytes, int32_t *status, void *stream);
 
 /*
  * Per-stage timing of lo_fused_moe_block_int8 for benchmarks: while enabled (per host thread), the

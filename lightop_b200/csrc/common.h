@@ -139,6 +139,7 @@ struct GemmArgs {
   const float *a_scale;     // [rows_a, K/128]
   int64_t rows_a;
   int max_chunk_rows;       // upper bound of Chunk::rows (0 = 128); selects the shared-memory staging depth
+  int64_t expected_rows;    // rows an expert can be expected to have, capped at a chunk's (0 = not known); decides on pairs of CTAs
   const int8_t *B;          // [E, n_rows_per_expert, K] int8
   const float *b_scale;     // [E, n_rows_per_expert/128, K/128]
   int E;
@@ -174,6 +175,9 @@ struct GemmArgs {
 };
 
 int launch_grouped_gemm(GemmMode mode, const GemmArgs &args, cudaStream_t stream);
+// Whether a call of at least this many chunks, of about this many rows, runs on pairs of CTAs where its chunks may be wider than 64
+// rows.  grouped_gemm.cu
+bool grouped_gemm_on_pairs(GemmMode mode, int64_t chunks, int64_t rows, int n_tiles, int64_t K);
 
 #ifdef __CUDACC__
 // Programmatic dependent launch.  A kernel launched with launch_dependent() may start while the kernel before it

@@ -55,29 +55,28 @@ FusedLayout carve_fused(void *ws, int64_t M, int num_experts_for_align, int topk
 
 // Chunk sizes of the block-scaled layer, by the rows an expert gets on average (rows / experts).  The GEMM is instantiated per
 // chunk cap and the caps differ in what fits beside the operands: 8 weight slots and 8 partial buffers with 64 rows, 7 and 4
-// with 128, 5 and 3 with 160.  Layer times in us, caps of 64 / 128 / 160 rows:
-//   rows per expert               48                     56                     64                    100                   112                   120
-//   Qwen3 shape, even routing     423 /  454 /  472      460 /  482 /  503      544 /  485 /  520     742 /  625 /  643     770 /  640 /  663     827 /  723 /  673
-//   DeepSeek-V3, even            1876 / 2006 / 2073     2026 / 2066 / 2143                           3461 / 2648 / 2735    3568 / 2807 / 2791    3686 / 2987 / 2848
-//   rows per expert              128                    156 (shard)            181                   203 (shard)           256
-//   Qwen3 shape (shards: DeepSeek-V3, one of eight), even   929 / 815 / 739    650 / 607 / 556     1193 / 1099 / 1122     825 / 698 / 700     1568 / 1402 / 1336
-//   Qwen3, Zipf (1.2) routing     892 /  845 /  880                                                                                           1529 / 1383 / 1398
-// Caps of 64 / 128 rows around the first line, on another board:
-//   rows per expert               32             40             48             56             64
-//   Qwen3 shape, Zipf (1.2)       353 /  356     423 /  424     465 /  458     500 /  484     548 /  532      even 56: 490 / 501, 64: 589 / 541
-//   DeepSeek-V3, Zipf (1.2)      1255 / 1207                   1659 / 1549    1892 / 1777                     even 56: 2335 / 2266
-//   <= 48 rows per expert : 64-row chunks.  A weight-streaming call wants the deep rings: 7 % with even routing.  With Zipf routing 128-row
+// with 128, 7 and 3 with 160 on pairs of CTAs (5 and 3 on single ones).  Layer times in us, caps of 64 (single CTAs) / 128 / 160 rows (pairs):
+//   rows per expert          32                    48                    56                    64                    100                   120                   128
+//   DeepSeek-V3, even       1836 / 1931 / 1974     1988 / 2080 / 2140     2244 / 2134 / 2235     2682 / 2245 / 2314     3613 / 2665 / 2717     3950 / 3127 / 2927     4226 / 3543 / 3034
+//   Zipf (1.2) routing      1228 / 1178 / 1200     1614 / 1506 / 1492     1877 / 1723 / 1694     2018 / 1842 / 1836     2812 / 2560 / 2513     3274 / 2886 / 2817     3446 / 3035 / 2946
+//   Qwen3, even              417 /  448 /  459      450 /  480 /  510      493 /  498 /  524      579 /  531 /  553      786 /  630 /  653      852 /  731 /  699      942 /  842 /  730
+//   Zipf                     359 /  369 /  374      454 /  445 /  451      487 /  470 /  496      542 /  520 /  523      729 /  684 /  699      853 /  801 /  797      894 /  842 /  813
+//   <= 48 rows per expert : 64-row chunks.  A weight-streaming call wants the deep rings: 4 to 7 % with even routing.  With Zipf routing 128-row
 //                           chunks are up to 7 % ahead from 32 rows per expert on; the routing is not known on the host.  At 56 the two
-//                           are within 3 % either way with even routing, by board, and 128 is ahead with Zipf.
+//                           are within 5 % either way with even routing, by shape, and 128 is ahead with Zipf.
 //   49 .. 119             : 128-row chunks
-//   >= 120                : 160-row chunks: with 128 rows per expert half of the experts have a few rows more than 128, and a
-//                           second chunk means a second pass over the expert's weights.  With skewed routing 128-row chunks are up to 4 %
-//                           ahead, with about 190 rows per expert (two chunks of fewer than 128 rows either way) up to 2 %.
+//   176 .. 232            : 128-row chunks: nearly every expert has two chunks with either cap, and the narrower ones have the deeper rings.
+//                           128 / 160 rows, even routing: Qwen3 168 rows 1028 / 1003, 176 1052 / 1066, 184 1067 / 1106, 216 1190 / 1233, 232 1234 /
+//                           1265, 240 1253 / 1255; 7168 tokens of a shard with 32 experts (224) 719 / 743, 5376 (168) 610 / 612, 8192 (256) 828 / 789;
+//                           Zipf 176 1012 / 1023, 224 1238 / 1197
+//   otherwise >= 120      : 160-row chunks: with 128 rows per expert half of the experts have a few rows more than 128, and a
+//                           second chunk means a second pass over the expert's weights (256 rows: 1374 / 1313, Zipf 1368 / 1322).
 constexpr int CHUNK_ROWS = 128;
 constexpr int CHUNK_ROWS_WIDE = 160;
 constexpr int CHUNK_ROWS_SMALL = 64;
 inline int chunk_rows_for(int64_t rows, int experts) {
   const int64_t avg = rows / experts;
+  if (avg >= 176 && avg <= 232) return CHUNK_ROWS;
   return avg >= 120 ? CHUNK_ROWS_WIDE : (avg <= 48 ? CHUNK_ROWS_SMALL : CHUNK_ROWS);
 }
 
@@ -223,7 +222,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   prof_mark(2, st);
   GemmArgs g1{};
   g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap;
-  g1.max_chunk_rows = chunk_max;
+  g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(numel, align_E);
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = numel;
@@ -240,7 +239,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   prof_mark(3, st);
   GemmArgs g2{};
   g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap;
-  g2.max_chunk_rows = g1.max_chunk_rows; g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
+  g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows; g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
   g2.n_rows_per_expert = H; g2.K = I; g2.n_tiles = (int)(H / 128);
   g2.sorted_ids = L.sorted_ids; g2.numel_valid = numel;
   g2.chunks = L.chunks; g2.num_chunks = L.header + 1;
@@ -316,7 +315,7 @@ int grouped_gemm_on_blocks(GemmMode mode, const int8_t *A, const float *a_scale,
   if (rc != LO_OK) return rc;
   GemmArgs g{};
   g.A = W.a_sorted; g.a_scale = W.as_sorted; g.rows_a = sorted_capacity;
-  g.max_chunk_rows = block_size < 128 ? block_size : 128; g.B = B; g.b_scale = b_scale; g.E = E;
+  g.max_chunk_rows = block_size < 128 ? block_size : 128; g.expected_rows = ceil_div(numel_valid, E); g.B = B; g.b_scale = b_scale; g.E = E;
   g.n_rows_per_expert = N; g.K = K; g.n_tiles = (int)(N / 128);
   g.sorted_ids = sorted_ids; g.numel_valid = numel_valid;
   g.chunks = W.chunks; g.num_chunks = W.num_chunks;
@@ -424,19 +423,21 @@ extern "C" int lo_fused_moe_block_int8_noalloc(const void *x, const int8_t *w1, 
 namespace lo {
 namespace {
 // Chunk sizes of the per-channel layer, by the rows an expert gets on average.  A chunk is one pass over the expert's weights and
-// one MMA N extent (an N = 256 MMA costs about 1.3 x an N = 128 one); the GEMM is instantiated per chunk cap.  Weight slots and
-// accumulators: 9 and 8 with 64 rows, 9 and 4 with 128, 8 and 3 with 160, 5 and 2 with 256.  Layer times in us, DeepSeek-V3
-// shape, caps of 64 / 128 / 160 / 256 rows:
-//   rows per expert     16                            56                            93                            128                           160
-//   even routing        1736 / 1793 / 1780 / 1833     1984 / 2060 / 2044 / 2072     3003 / 2372 / 2325 / 2351     3647 / 3068 / 2491 / 2514     4689 / 3960 / 3158 / 2674
-//   Zipf (1.2) routing   746 /  723 /  713 /  702     1789 / 1525 / 1433 / 1324     2597 / 2099 / 1930 / 1749     3492 / 2605 / 2392 / 2199     4174 / 3092 / 2841 / 2552
-//   <= 56 rows per expert : 64-row chunks, for the even case (Qwen3 shape: 407 / 397 / 397 / 410 at 16 rows, 483 / 487 / 480 /
-//                           489 at 56).  With a few hot experts every wider cap is faster; the routing is not known on the host.
-//   57 .. 136             : 160-row chunks, ahead of 128 in both (and no slower than 256 with even routing)
+// one MMA N extent; the GEMM is instantiated per chunk cap, and on pairs of CTAs the wider caps keep the weight rings as deep as the narrow
+// ones (weight slots and accumulators: 9 and 8 with 64 rows; pairs 9 and 4 with 128, 9 and 3 with 160, 9 and 2 with 256; single CTAs 9 and 4, 8 and 3,
+// 5 and 2).  Layer times in us, caps of 64 (single CTAs) / 128 / 160 / 256 rows (pairs):
+//   rows per expert          16                            48                            56                            93                            128
+//   DeepSeek-V3, even        1747 / 1752 / 1758 / 1851     1941 / 1929 / 1952 / 2080     2085 / 1984 / 2011 / 2127     3142 / 2246 / 2248 / 2372     3825 / 3006 / 2574 / 2614
+//   Zipf (1.2) routing        822 /  726 /  722 /  736     1571 / 1270 / 1229 / 1215     1789 / 1441 / 1384 / 1353     2576 / 2016 / 1864 / 1808     3294 / 2509 / 2319 / 2211
+//   Qwen3, even               408 /  407 /  408 /  410      462 /  454 /  459 /  469      501 /  467 /  470 /  486      756 /  551 /  548 /  565      907 /  714 /  635 /  629
+//   Zipf                      258 /  251 /  247 /  248      444 /  402 /  383 /  387      484 /  418 /  414 /  410      694 /  580 /  548 /  540      886 /  721 /  680 /  666
+//   <= 136 rows per expert: 160-row chunks: as fast as narrower ones where the rows are spread evenly (within 1 %), up to 28 % faster where
+//                           a few experts are hot; the routing is not known on the host.  At 2 rows per expert (66 tokens) the same.
 //   above                 : 256-row chunks
-inline int channel_chunk_rows_for(int64_t rows, int experts) {
+// On single CTAs a weight-streaming call wants the narrow chunks (up to 56 rows per expert 64-row ones are up to 4 % ahead with even routing).
+inline int channel_chunk_rows_for(int64_t rows, int experts, bool pairs) {
   const int64_t avg = rows / experts;
-  return avg <= 56 ? CHUNK_ROWS_SMALL : (avg <= 136 ? CHUNK_ROWS_WIDE : 256);
+  return avg <= 56 && !pairs ? CHUNK_ROWS_SMALL : (avg <= 136 ? CHUNK_ROWS_WIDE : 256);
 }
 struct ChannelLayout {
   int32_t *header;      // [0] num_tokens_post_pad, [1] num_chunks
@@ -507,7 +508,10 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   LO_REQUIRE(workspace_bytes >= L.bytes, "channel moe: workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t numel = M * topk;
-  const int chunk_max = table_chunk_rows(M, channel_chunk_rows_for(numel, align_E));
+  const int64_t per_expert = ceil_div(numel, align_E);
+  const bool pairs = grouped_gemm_on_pairs(GEMM_CHANNEL, E_local, per_expert, (int)(2 * I / 128), H) &&
+                     grouped_gemm_on_pairs(GEMM_CHANNEL, E_local, per_expert, (int)(H / 128), I);
+  const int chunk_max = table_chunk_rows(M, channel_chunk_rows_for(numel, align_E, pairs));
   // 1. expert-major stable order, chunk table, position of every (token, slot)
   prof_mark(0, st);
   g_prof.joined = false;
@@ -523,7 +527,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   prof_mark(2, st);
   GemmArgs g1{};
   g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap;
-  g1.max_chunk_rows = chunk_max;
+  g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(numel, align_E);
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(2 * I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = numel; g1.out_by_position = 1;
@@ -540,7 +544,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   // 4. down GEMM, routed weight in the epilogue -> cache3[token, slot, :]
   prof_mark(3, st);
   GemmArgs g2{};
-  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows;
+  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows;
   g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
   g2.n_rows_per_expert = H; g2.K = I; g2.n_tiles = (int)(H / 128);
   g2.sorted_ids = L.sorted_ids; g2.numel_valid = numel;
@@ -592,7 +596,7 @@ int expert_rows_impl(const int8_t *xq, const float *xs, int64_t x_stride, const 
   rc = launch_permute_rows(xq, xs, T, H, L.sorted_ids, L.sorted_cap, L.header, T, 1, L.xq, L.xs, st, 0, x_stride);
   if (rc != LO_OK) return rc;
   GemmArgs g1{};
-  g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap; g1.max_chunk_rows = chunk_max;
+  g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap; g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(T, E_local);
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = T;
@@ -604,7 +608,7 @@ int expert_rows_impl(const int8_t *xq, const float *xs, int64_t x_stride, const 
   rc = launch_grouped_gemm(GEMM_GATE_UP, g1, st);
   if (rc != LO_OK) return rc;
   GemmArgs g2{};
-  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows;
+  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows;
   g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
   g2.n_rows_per_expert = H; g2.K = I; g2.n_tiles = (int)(H / 128);
   g2.sorted_ids = L.sorted_ids; g2.numel_valid = T;
@@ -768,7 +772,7 @@ int check_linear(int64_t M, int64_t N, int64_t K) {
 int run_linear(const int8_t *A, const float *a_scale, const int8_t *B, const float *b_scale, int64_t M, int64_t N, int64_t K,
                void *C, const LinearPlan &L, int32_t *partial, int32_t *status, cudaStream_t st) {
   GemmArgs g{};
-  g.A = A; g.a_scale = a_scale; g.rows_a = M; g.max_chunk_rows = L.chunk_rows;
+  g.A = A; g.a_scale = a_scale; g.rows_a = M; g.max_chunk_rows = L.chunk_rows; g.expected_rows = L.chunk_rows;
   g.B = B; g.b_scale = b_scale; g.E = 1;
   g.n_rows_per_expert = N; g.n_store = N; g.K = K; g.n_tiles = L.n_tiles;
   g.numel_valid = M; g.fixed_chunks = L.n_chunks;

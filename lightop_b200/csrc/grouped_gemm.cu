@@ -50,7 +50,7 @@
 // 16 or 20 warps run an epilogue (int32 -> fp32, times token scale, times channel scale) while the MMAs of the next items fill
 // the other buffers.  The scale producer idles and there are no output warps in that mode.
 //
-// Pairs.  Wide chunks of calls with enough work run on clusters of two CTAs (see use_pairs()): two neighbouring tiles of a chunk are one MMA of
+// Pairs.  Wide chunks of calls with enough work run on clusters of two CTAs (see grouped_gemm_on_pairs()): two neighbouring tiles of a chunk are one MMA of
 // 256 rows (cta_group::2), for which each CTA loads its own weight tile and half of the chunk's token rows.  The rows of a chunk, which each
 // tile reads again from L2, cross to the SMs half as often, take half of the shared memory (the weight ring of 160-row chunks has 7 slots
 // instead of 5, per channel that of 256-row ones 9 instead of 5) and are read from there by one MMA instead of two.  Rank 0 issues for both: the loads of both CTAs complete on its ready[],
@@ -1472,22 +1472,24 @@ int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   return LO_OK;
 }
 
-// Whether a call with wide chunks runs on pairs of CTAs: tiles come in twos (a pair with one tile idle would waste half of it), and
-// every SM has enough K-block steps to make up for the start, which waits for the other CTA, and for the slower of two CTAs in every step.
-// One CTA / pairs, in us, by the steps of an SM (at least; a call with a chunk table has a chunk an expert or more):
-//   dense linear    20 (2000 x 2304 x 1280) 17.0 / 18.3    60 (600 x 4096 x 7168) 44.4 / 44.9     97 (1000 x 4096 x 7168) 52.1 / 51.8
-//                  145 (1500 x 4096 x 7168) 77.8 / 76.5   194 (2000 x 4096 x 7168) 104.3 / 102.7    387 (4096 x 4096 x 7168) 204 / 197
-//   layers          83 (Qwen3, 4096 tokens of a shard of eight) 200.7 / 202.2    664 (Qwen3 2048, Zipf) 862 / 830    3100 (DeepSeek-V3 4096) 3065 / 3011
-//   per channel      5 (32 experts of 1024 x 384) 154.2 / 154.1    42 and 83 (masked, 16 of 4096 x 1536) 76.9 / 75.3    1550 and 3100 (DeepSeek-V3 2999) 2417 / 2334
-constexpr int PAIR_MIN_STEPS = 96, PAIR_MIN_STEPS_CHANNEL = 32;
-bool use_pairs(GemmMode mode, const GemmArgs &a) {
-  if (a.n_tiles % 2 != 0 || a.partial != nullptr || sm_count() < 2) return false;
-  const int64_t chunks = a.chunks != nullptr ? a.E : a.fixed_chunks;
-  const int64_t steps = chunks * a.n_tiles * (mode == GEMM_GATE_UP ? 2 : 1) * (a.K / TILE_K) / sm_count();
-  return steps >= (mode == GEMM_CHANNEL ? PAIR_MIN_STEPS_CHANNEL : PAIR_MIN_STEPS);
-}
-
+// Whether a call with wide chunks runs on pairs of CTAs: tiles come in twos (a pair with one tile idle would waste half of it), and what a
+// pair saves, half of the loads of the chunk's rows, has to make up for its start, which waits for the other CTA (0.5 us), and for the slower of
+// two CTAs in every step.  So the rule counts the rows that an SM loads: K-block steps (a call with a chunk table has a chunk an expert or more) times
+// rows a chunk.  One CTA / pairs, in us, by steps x rows in thousands:
+//   dense linear     7 (600 x 4096 x 7168) 44.4 / 44.9      8 (1200 x 7168 x 2048) 33.3 / 34.4     12 (1000 x 4096 x 7168) 52.1 / 51.8
+//                   18 (1500 x 4096 x 7168) 77.8 / 76.5    25 (2000 x 4096 x 7168) 104.3 / 102.7   50 (4096 x 4096 x 7168) 204 / 197
+//   layers          11 (Qwen3, 4096 tokens of a shard of eight) 200.7 / 202.2    42 (Qwen3 700, Zipf) 431 / 424    85 (Qwen3 2048, Zipf) 887 / 838
+//                  400 (DeepSeek-V3 4096) 3160 / 3112
+//   per channel, masked layout (both GEMMs), experts of 7168 x 2048: 32 with 1 row 158.7 / 161.2    6 rows 214.6 / 217.8    16 231.7 / 231.3 (6, 3)
+//                   24 243.5 / 239.2 (9, 5)     100 319.7 / 316.1        of 4096 x 1536: 32 with 24 rows 113.8 / 115.5 (4, 2)   16 with 80 76.9 / 75.3 (7, 3)
+constexpr int64_t PAIR_MIN_ROWS = 12000, PAIR_MIN_ROWS_CHANNEL = 7000;
 }  // namespace
+
+bool grouped_gemm_on_pairs(GemmMode mode, int64_t chunks, int64_t rows, int n_tiles, int64_t K) {
+  if (n_tiles % 2 != 0 || sm_count() < 2) return false;
+  const int64_t steps = chunks * n_tiles * (mode == GEMM_GATE_UP ? 2 : 1) * (K / TILE_K) / sm_count();
+  return steps * rows >= (mode == GEMM_CHANNEL ? PAIR_MIN_ROWS_CHANNEL : PAIR_MIN_ROWS);
+}
 
 int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
   LO_REQUIRE(a.K % TILE_K == 0 && a.K >= TILE_K, "grouped gemm: K=%lld must be a positive multiple of 128", (long long)a.K);
@@ -1510,7 +1512,7 @@ int launch_grouped_gemm(GemmMode mode, const GemmArgs &a, cudaStream_t stream) {
              "grouped gemm: the K extent is split for dense calls only");
   // no chunk can hold more rows than max_chunk_rows (a bound the caller derives from the token count)
   const int cap = a.max_chunk_rows <= 0 ? T_MAX : a.max_chunk_rows;
-  const bool pair = use_pairs(mode, a);
+  const bool pair = a.partial == nullptr && grouped_gemm_on_pairs(mode, a.chunks != nullptr ? a.E : a.fixed_chunks, a.expected_rows < cap ? a.expected_rows : cap, a.n_tiles, a.K);
   if (mode == GEMM_GATE_UP) {
     LO_REQUIRE(a.n_rows_per_expert == 2 * (int64_t)a.n_tiles * TILE_N, "grouped gemm: gate_up needs N = 2*I");
     LO_REQUIRE(cap <= T_WIDE, "grouped gemm: block-scaled chunks hold at most 160 rows");

@@ -120,7 +120,7 @@ extern "C" int lo_m_grouped_w8a8_gemm_nt_contig(const int8_t *A, const float *a_
   contig_plan_kernel<<<(unsigned)ceil_div(threads, 256), 256, 0, st>>>(m_indices, M, E, W.chunks, W.num_chunks, status);
   LO_LAUNCH_OK("contig_plan_kernel");
   GemmArgs g = channel_args(A, a_scale, M, B, b_scale, E, N, K, C, (int)(M < 256 ? M : 256), status);
-  g.chunks = W.chunks; g.num_chunks = W.num_chunks;
+  g.chunks = W.chunks; g.num_chunks = W.num_chunks; g.expected_rows = ceil_div(M, E);
   return launch_grouped_gemm(GEMM_CHANNEL, g, st);
 }
 
@@ -128,6 +128,14 @@ extern "C" int lo_m_grouped_w8a8_gemm_nt_masked(const int8_t *A, const float *a_
                                                 const float *b_scale, void *C, const int32_t *masked_m, int E,
                                                 int64_t max_m, int64_t N, int64_t K, void *workspace,
                                                 size_t workspace_bytes, int32_t *status, void *stream) {
+  return lo_m_grouped_w8a8_gemm_nt_masked_expected(A, a_scale, B, b_scale, C, masked_m, E, max_m, 0, N, K, workspace, workspace_bytes, status,
+                                                   stream);
+}
+
+extern "C" int lo_m_grouped_w8a8_gemm_nt_masked_expected(const int8_t *A, const float *a_scale, const int8_t *B,
+                                                         const float *b_scale, void *C, const int32_t *masked_m, int E,
+                                                         int64_t max_m, int64_t expected_m, int64_t N, int64_t K, void *workspace,
+                                                         size_t workspace_bytes, int32_t *status, void *stream) {
   using namespace lo;
   LO_REQUIRE(E >= 1 && max_m >= 0, "grouped gemm (masked): bad shape");
   if (max_m == 0) return LO_OK;
@@ -140,6 +148,6 @@ extern "C" int lo_m_grouped_w8a8_gemm_nt_masked(const int8_t *A, const float *a_
   // the chunks follow from the row counts: the kernel forms them itself
   const int cap = (int)(max_m < 256 ? max_m : 256);
   GemmArgs g = channel_args(A, a_scale, (int64_t)E * max_m, B, b_scale, E, N, K, C, cap, status);
-  g.masked_m = masked_m; g.max_m = max_m; g.fixed_chunks = E * (int)ceil_div(max_m, cap);
+  g.masked_m = masked_m; g.max_m = max_m; g.expected_rows = expected_m > 0 ? expected_m : 0; g.fixed_chunks = E * (int)ceil_div(max_m, cap);
   return launch_grouped_gemm(GEMM_CHANNEL, g, st);
 }

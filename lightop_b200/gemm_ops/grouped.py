@@ -67,7 +67,8 @@ def m_grouped_w8a8_gemm_nt_masked(a: Tuple[torch.Tensor, torch.Tensor], b: Tuple
 
     Signature of the reference (python/lightop/gemmopt.py:604-617): ``a = (int8 [E, max_m, K], fp32
     [E, max_m, 1])``, ``b = (int8 [E, N, K], fp32 [E, N, 1])``, ``d`` bf16 ``[E, max_m, N]``, ``masked_m``
-    int32 ``[E]``.  ``expected_m_per_group`` (a tile-selection hint there) and ``config`` are ignored.
+    int32 ``[E]``.  ``expected_m_per_group`` is a hint as there, the rows an expert can be expected to have (any value gives the
+    same results; what is not an integer counts as not known); ``config`` is ignored.
     Weights in the plain layout (the reference's kernel takes them pre-shuffled).
     """
     inp, a_scale, w, b_scale, E, N, K = _operands(a, b)
@@ -86,9 +87,10 @@ def m_grouped_w8a8_gemm_nt_masked(a: Tuple[torch.Tensor, torch.Tensor], b: Tuple
     lib = _lib.load()
     status = device_status_word(inp.device)
     with _lib.on_device(inp.device):
-        st = lib.lo_m_grouped_w8a8_gemm_nt_masked(_lib.ptr(inp), _lib.ptr(a_scale), _lib.ptr(w), _lib.ptr(b_scale),
-                                                  _lib.ptr(d), _lib.ptr(masked_m.contiguous()), E, max_m, N, K,
-                                                  0, 0, _lib.ptr(status),
-                                                  _lib.current_stream(inp.device))
+        expected = min(max(expected_m_per_group, 0), max_m) if isinstance(expected_m_per_group, int) else 0
+        st = lib.lo_m_grouped_w8a8_gemm_nt_masked_expected(_lib.ptr(inp), _lib.ptr(a_scale), _lib.ptr(w), _lib.ptr(b_scale),
+                                                           _lib.ptr(d), _lib.ptr(masked_m.contiguous()), E, max_m, expected, N, K,
+                                                           0, 0, _lib.ptr(status),
+                                                           _lib.current_stream(inp.device))
     _lib.check(st, "m_grouped_w8a8_gemm_nt_masked")
     return d

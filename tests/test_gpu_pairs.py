@@ -16,7 +16,7 @@ def _int8(g, *shape):
     return torch.randint(-127, 128, shape, generator=g, device=DEV, dtype=torch.int8)
 
 
-@pytest.mark.parametrize("M,tiles,K", [(65, 130, 14336), (96, 128, 14336), (97, 128, 14336), (112, 128, 14336), (200, 66, 14336),
+@pytest.mark.parametrize("M,tiles,K", [(65, 256, 14336), (96, 256, 14336), (97, 256, 14336), (112, 256, 14336), (200, 130, 14336),
                                        (1000, 34, 7168), (3999, 10, 6272)])
 def test_dense_linear(M, tiles, K):
     import lightop_b200 as lo
@@ -37,7 +37,7 @@ def test_dense_linear(M, tiles, K):
 @pytest.mark.parametrize("block,channel", [(128, False), (128, True), (256, True)])
 def test_grouped_gemm(block, channel):
     import lightop_b200 as lo
-    E, tiles, K = len(COUNTS), 12, 7168
+    E, tiles, K = len(COUNTS), 16, 7168
     g = torch.Generator(device=DEV).manual_seed(block)
     ids = torch.cat([torch.full((c,), e, dtype=torch.int32, device=DEV) for e, c in enumerate(COUNTS)])
     ids = ids[torch.randperm(len(ids), generator=g, device=DEV)].view(-1, 1)
@@ -65,7 +65,7 @@ def test_grouped_gemm(block, channel):
 @pytest.mark.parametrize("channel", [False, True])
 def test_layer(counts, channel):
     import lightop_b200 as lo
-    E, H, I = len(counts), 7168, 1536
+    E, H, I = len(counts), 7168, 2048
     w1, w2, w1_s, w2_s = synthetic.make_weights(E, H, I, seed=1, device=DEV)
     if channel:
         w1_s, w2_s = synthetic.make_channel_scales(E, H, I, seed=1, device=DEV)
@@ -84,3 +84,23 @@ def test_layer(counts, channel):
         if len(rows):
             assert torch.equal(y[rows], run(rows, e, e + 1)), counts[e]
     lo.check_device_status()
+
+
+@pytest.mark.parametrize("max_m", [128, 160, 300])
+def test_masked_layout_by_hint(max_m):
+    # the hint decides on the form: none, too few rows for pairs, enough, more than there can be, and what is no number
+    import lightop_b200 as lo
+    E, N, K = 24, 2048, 7168
+    g = torch.Generator(device=DEV).manual_seed(max_m)
+    a, w = (_int8(g, E, max_m, K), torch.rand(E, max_m, 1, generator=g, device=DEV)), (_int8(g, E, N, K), torch.rand(E, N, 1, generator=g, device=DEV))
+    rows = torch.tensor([min(c, max_m) for c in COUNTS], dtype=torch.int32, device=DEV)
+    outs = []
+    for hint in (0, 1, 100, 1 << 70, -5, None):
+        d = torch.full((E, max_m, N), -5.0, dtype=torch.bfloat16, device=DEV)
+        lo.gemm_ops.m_grouped_w8a8_gemm_nt_masked(a, w, d, rows, hint)
+        outs.append(d)
+    torch.cuda.synchronize()
+    lo.check_device_status()
+    assert all(torch.equal(outs[0], d) for d in outs[1:])
+    for e in range(E):
+        assert bool((outs[0][e, int(rows[e]):] == -5.0).all()) and not bool((outs[0][e, :int(rows[e])] == -5.0).all(1).any())
