@@ -10,6 +10,11 @@ from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_void_
 
 import torch
 
+try:
+    from . import _host as host      # csrc/host.cpp
+except ImportError as e:
+    raise ImportError("lightop_b200/_host.so is missing or unusable: build it with `python lightop_b200/build.py` (there is no fallback)") from e
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # LIGHTOP_B200_LIB overrides the location of the shared library (e.g. an instrumented build)
 LIB_PATH = os.environ.get("LIGHTOP_B200_LIB") or os.path.join(_HERE, "liblightop_b200.so")
@@ -136,6 +141,7 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
+    host.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in PROTOTYPES}, check)
     _lib = lib
     return lib
 

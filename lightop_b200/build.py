@@ -1,17 +1,21 @@
 """Build step of the C-ABI library: nvcc for sm_100a only, in-tree output.
 
 ``python lightop_b200/build.py`` (run by path: importing the package needs the built library) compiles ``csrc/*.cu`` into
-``lightop_b200/liblightop_b200.so``.  nvcc cross-compiles without a GPU.
+``lightop_b200/liblightop_b200.so`` and ``csrc/host.cpp`` (the host side of small calls, against the installed torch) into
+``lightop_b200/_host.so``.  nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "liblightop_b200.so")
+HOST = os.path.join(HERE, "_host.so")
 SOURCES = ["common.cu", "quant.cu", "routing.cu", "gate.cu", "reduce.cu", "grouped_gemm.cu", "fused_moe.cu", "grouped_layouts.cu", "peer.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -25,18 +29,29 @@ def _nvcc() -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(HOST):
         return True
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "lightop_b200.h")]
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
+
+
+def _host_command() -> list:
+    # (found without importing torch: a first import of it takes a while)
+    torch_dir = list(importlib.util.find_spec("torch").submodule_search_locations)[0]
+    cuda_dir = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    include = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+               os.path.join(cuda_dir, "include"), sysconfig.get_path("include")]
+    lib = os.path.join(torch_dir, "lib")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", *[f"-I{d}" for d in include], os.path.join(CSRC, "host.cpp"),
+            "-o", HOST, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{lib}"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
     objs = []
-    procs = []
+    procs = [("host.cpp", subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True))]
     for src in SOURCES:
         obj = os.path.join(CSRC, src.replace(".cu", ".o"))
         cmd = [_nvcc(), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
@@ -47,7 +62,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     for src, pr in procs:
         out, _ = pr.communicate()
         if pr.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {src}:\n{out}")
+            raise RuntimeError(f"the compiler failed on {src}:\n{out}")
         if verbose and out:
             print(out)
     link = [_nvcc(), "-shared", "-o", LIB, *objs, "-cudart", "static"]

@@ -70,6 +70,10 @@ def gemm_w8a8_asm(a, b, scale_a, scale_b, block_size, out_dtype, layout="TN"):
 
 def _dynamic_linear(x: torch.Tensor, w: torch.Tensor, block_size: List[int], w_s: torch.Tensor) -> Optional[torch.Tensor]:
     """Quantisation and GEMM in one native call; None for the forms that the two separate operators take or refuse."""
+    if type(x) is torch.Tensor and x.is_cuda:
+        C = _lib.host.linear(x, w, block_size, w_s, device_status_word(x.device))
+        if C is not None:
+            return C
     if list(block_size) != [128, 128] or w.dim() != 2 or x.dim() == 0 or x.dtype not in (torch.bfloat16, torch.float16, torch.float32):
         return None
     N, K = w.shape

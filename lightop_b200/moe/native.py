@@ -55,6 +55,15 @@ def fused_experts_impl_int8(hidden_states: torch.Tensor,
     ``routed_scaling_factor`` as in ``moe_sum`` (int8.py:882-888).  ``cache13`` is the
     caller's bf16 scratch of at least ``M * topk * hidden`` elements; None allocates it.
     """
+    if (use_int8_w8a8 and activation == "silu" and type(hidden_states) is torch.Tensor and hidden_states.is_cuda
+            and not (use_fp8_w8a8 or use_int8_w8a16 or use_int4_w4a16)
+            and w1_zp is None and w2_zp is None and a1_scale is None and a2_scale is None and i_q is None and i_s is None):
+        # the usual form, in one step; what it does not take (None) goes on below
+        out = _lib.host.fused_experts(hidden_states, w1, w2, topk_weights, topk_ids, cache13, w1_scale, w2_scale, expert_map, shared_output,
+                                      block_shape, per_channel_quant, global_num_experts, apply_router_weight_on_input,
+                                      routed_scaling_factor, inplace, device_status_word(hidden_states.device))
+        if out is not None:
+            return out
     assert use_int8_w8a8 or use_fp8_w8a8
     assert hidden_states.shape[1] == w1.shape[2], "Hidden size mismatch"
     assert topk_weights.shape == topk_ids.shape, "topk shape mismatch"

@@ -26,6 +26,8 @@ def topk_softmax(topk_weights: torch.Tensor, topk_indices: torch.Tensor,
     ``[M,k]``; ``topk_indices`` int32 / uint32 / int64 ``[M,k]`` in descending score order;
     ``token_expert_indices`` int32 ``[M,k]`` receives ``slot * M + token``.
     """
+    if token_expert_indices is None and _lib.host.topk_softmax(topk_weights, topk_indices, gating_output, Is_renormalize):
+        return
     _lib.require_cuda(topk_weights, topk_indices, token_expert_indices, gating_output)
     if gating_output.dim() != 2:
         raise RuntimeError("gating_output must be [num_tokens, num_experts]")
