@@ -848,14 +848,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       // ============================ MMA issuer (warp 1) ================================
       // A step of this role is a chain of dependent instructions and barrier round trips, which takes longer than the
       // tensor core needs for the step's MMAs.  So: lanes 0 and 1 each own one of the step's two barriers (operands ready,
-      // partial buffer free) and look at it in the same instruction; everything the MMAs take (ring positions, descriptors) is computed from values all lanes share,
-      // which keeps it in uniform registers (-11 % on the per-channel layer at 20 rows per expert against operands shuffled
-      // from the polling lanes).  The look at the next step's barriers comes behind this step's MMAs: the warp stands still until a look has its
-      // answer (some 100 cycles), and what a partial buffer waits for, from its hand-back to the MMAs and on to the promotion, is part of
-      // the loop that bounds wide chunks (4096 tokens 2970 -> 2936 us, Qwen3 2048 Zipf 815 -> 808, dense 4096 x 4096 x 7168 196 -> 193, per channel
-      // 2999 2246 -> 2228, 64 tokens in a graph 1433 -> 1429).  One thread for barriers and MMAs without votes is no faster than
-      // with the look in front, predicated MMAs without a branch are 3 % slower.  Per-channel mode accumulates an item's steps into one buffer: lane 1 waits for the
-      // accumulator once per item.
+      // partial buffer free) and look at it in the same instruction; everything the MMAs take (ring positions,
+      // descriptors) is computed from values all lanes share, which keeps it in uniform registers (-11 % on the per-channel layer at 20
+      // rows per expert against operands shuffled from the polling lanes).  Per-channel mode accumulates an item's steps into one buffer:
+      // lane 1 waits for the accumulator once per item.
+      // The look at the next step's barriers comes behind this step's MMAs: the warp stands still until a look has its answer (some 100
+      // cycles), and what a partial buffer waits for, from its hand-back to the MMAs and on to the promotion, is part of the loop that bounds
+      // wide chunks (in front and behind, us: 4096 tokens 2970, 2936; Qwen3 2048 Zipf 815, 808; dense 4096 x 4096 x 7168 196, 193; per channel 2999
+      // 2246, 2228; 128 tokens in a graph 1656, 1652; 48 1289, 1286).  With the narrow caps the weights are what is waited for, and the look
+      // stands in front: 32 tokens in a graph 1077, behind 1085; 16 x 4096 x 7168 16.7, 17.1; per channel with 64-row chunks (Qwen3 300, composed)
+      // 427, 432.  One thread for barriers and MMAs without votes is no faster than with the look in front, predicated MMAs without a
+      // branch are 3 % slower.
       uint32_t it = 0;
       // ring positions of the step's operands and partial buffer
       uint32_t sw = 0, sa = 0, sb = 0;
@@ -869,6 +872,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       const uint32_t my_base = smem_u32(lane == 0 ? &sm.ready[0] : (lane == 1 ? &sm.consumed[0] : &sm.peer_consumed[0]));
       const uint32_t my_off = lane == 0 ? 0u : 0u - (uint32_t)NBUF;
       uint32_t acc_par = 1;              // per-channel mode: phase of the accumulator ring
+      constexpr bool LOOK_BEHIND = A_ROWS > (MODE == GEMM_CHANNEL ? 64 : 32);
       bool ok = true, seen = lane >= WAITERS;
       for (ItemCursor<MODE, FORM, PAIR> items(p, num_chunks); ok && items.take(ch, nt);) {
         if (ch.expert < 0) continue;
@@ -889,6 +893,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           }
           tc_fence_after();
           const bool last = u == steps - 1;
+          auto look = [&] {
+            const uint32_t nx = it + 1u + my_off;
+            if (MODE == GEMM_CHANNEL) seen = lane > 1 || (lane == 1 && !last) || (lane == 0 && mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u));
+            else seen = lane >= WAITERS || mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u);
+          };
+          if (!LOOK_BEHIND) look();
           // descriptor start addresses are in 16-byte units
           const uint32_t adesc = desc_w0 + sw * (uint32_t)(W_TILE_BYTES >> 4);
           const uint32_t bdesc = desc_a0 + sa * (uint32_t)(CF::A_TILE_BYTES >> 4);
@@ -901,9 +911,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             umma_commit_addr<PAIR>(done0 + 8u * (it & (uint32_t)(ND - 1)));
             if (MODE == GEMM_CHANNEL && last) umma_commit_addr<PAIR>(smem_u32(&sm.tmem_full[sb]));
           }
-          const uint32_t nx = it + 1u + my_off;
-          if (MODE == GEMM_CHANNEL) seen = lane > 1 || (lane == 1 && !last) || (lane == 0 && mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u));
-          else seen = lane >= WAITERS || mbar_test_addr(my_base + 8u * (nx & (uint32_t)(ND - 1)), (nx >> 4) & 1u);
+          if (LOOK_BEHIND) look();
           __syncwarp();
           sw = sw + 1 == (uint32_t)NW ? 0u : sw + 1;
           sa = sa + 1 == (uint32_t)NA ? 0u : sa + 1;
