@@ -139,6 +139,7 @@ struct GemmArgs {
   const float *a_scale;     // [rows_a, K/128]
   int64_t rows_a;
   int max_chunk_rows;       // upper bound of Chunk::rows (0 = 128); selects the shared-memory staging depth
+  int64_t max_chunks;       // with a chunk table: chunks that it can have at most (0 = not known)
   int64_t expected_rows;    // rows an expert can be expected to have, capped at a chunk's (0 = not known); decides on pairs of CTAs
   const int8_t *B;          // [E, n_rows_per_expert, K] int8
   const float *b_scale;     // [E, n_rows_per_expert/128, K/128]

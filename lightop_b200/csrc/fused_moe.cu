@@ -90,6 +90,9 @@ inline int table_chunk_rows(int64_t rows, int chunk_max) {
   return 256;
 }
 
+// Chunks that a table of that size can have: one an expert with rows, and one more for every full chunk.
+inline int64_t most_chunks(int64_t rows, int experts, int chunk_rows) { return (rows < experts ? rows : experts) + rows / chunk_rows; }
+
 // Whether the quantiser of the block-scaled layer reads a token's positions before its row, so that rows of tokens without a local
 // expert are not read.  It then starts behind the alignment instead of beside it, which costs about 1 us: worth it where a fifth of
 // the tokens or more can be expected to have no local expert (ids spread evenly over the experts) and their rows are 8 MB or more.
@@ -222,7 +225,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   prof_mark(2, st);
   GemmArgs g1{};
   g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap;
-  g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(numel, align_E);
+  g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(numel, align_E); g1.max_chunks = most_chunks(numel, align_E, chunk_max);
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = numel;
@@ -239,7 +242,7 @@ extern "C" int lo_fused_moe_block_int8(const void *x, const int8_t *w1, const in
   prof_mark(3, st);
   GemmArgs g2{};
   g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap;
-  g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows; g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
+  g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows; g2.max_chunks = g1.max_chunks; g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
   g2.n_rows_per_expert = H; g2.K = I; g2.n_tiles = (int)(H / 128);
   g2.sorted_ids = L.sorted_ids; g2.numel_valid = numel;
   g2.chunks = L.chunks; g2.num_chunks = L.header + 1;
@@ -527,7 +530,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   prof_mark(2, st);
   GemmArgs g1{};
   g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap;
-  g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(numel, align_E);
+  g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(numel, align_E); g1.max_chunks = most_chunks(numel, align_E, chunk_max);
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(2 * I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = numel; g1.out_by_position = 1;
@@ -544,7 +547,7 @@ extern "C" int lo_fused_moe_channel_int8(const void *x, int x_dtype, const int8_
   // 4. down GEMM, routed weight in the epilogue -> cache3[token, slot, :]
   prof_mark(3, st);
   GemmArgs g2{};
-  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows;
+  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows; g2.max_chunks = g1.max_chunks;
   g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
   g2.n_rows_per_expert = H; g2.K = I; g2.n_tiles = (int)(H / 128);
   g2.sorted_ids = L.sorted_ids; g2.numel_valid = numel;
@@ -596,7 +599,7 @@ int expert_rows_impl(const int8_t *xq, const float *xs, int64_t x_stride, const 
   rc = launch_permute_rows(xq, xs, T, H, L.sorted_ids, L.sorted_cap, L.header, T, 1, L.xq, L.xs, st, 0, x_stride);
   if (rc != LO_OK) return rc;
   GemmArgs g1{};
-  g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap; g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(T, E_local);
+  g1.A = L.xq; g1.a_scale = L.xs; g1.rows_a = L.sorted_cap; g1.max_chunk_rows = chunk_max; g1.expected_rows = ceil_div(T, E_local); g1.max_chunks = most_chunks(T, E_local, chunk_max);
   g1.B = w1; g1.b_scale = w1_scale; g1.E = E_local;
   g1.n_rows_per_expert = 2 * I; g1.K = H; g1.n_tiles = (int)(I / 128);
   g1.sorted_ids = L.sorted_ids; g1.numel_valid = T;
@@ -608,7 +611,7 @@ int expert_rows_impl(const int8_t *xq, const float *xs, int64_t x_stride, const 
   rc = launch_grouped_gemm(GEMM_GATE_UP, g1, st);
   if (rc != LO_OK) return rc;
   GemmArgs g2{};
-  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows;
+  g2.A = L.act_q; g2.a_scale = L.act_s; g2.rows_a = L.sorted_cap; g2.max_chunk_rows = g1.max_chunk_rows; g2.expected_rows = g1.expected_rows; g2.max_chunks = g1.max_chunks;
   g2.B = w2; g2.b_scale = w2_scale; g2.E = E_local;
   g2.n_rows_per_expert = H; g2.K = I; g2.n_tiles = (int)(H / 128);
   g2.sorted_ids = L.sorted_ids; g2.numel_valid = T;

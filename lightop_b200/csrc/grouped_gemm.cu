@@ -1475,8 +1475,15 @@ int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   p.vec_store = (p.n_store & 7) == 0 && (a.row_dst != nullptr || (reinterpret_cast<uintptr_t>(a.C) & 15) == 0) ? 1 : 0;
   p.fixed_chunks = a.fixed_chunks; p.chunk_rows = a.max_chunk_rows; p.masked_m = a.masked_m; p.max_m = a.max_m; p.dense_rows = a.rows_a;
   p.n_split = a.partial != nullptr ? (int)ceil_div(p.KB, a.split_steps) : 1; p.split_steps = a.split_steps; p.partial = a.partial;
-  const int grid = sm_count();
+  int grid = sm_count();
   if (grid <= 0) return fail(LO_ERR_CUDA, "no CUDA device");
+  // No more CTAs than there can be items: each takes its SM's shared memory and the start of the next kernel waits for all of them.  One CTA a SM and
+  // so, in us: layer of 32 tokens of the tiny shape in a graph 18.4, 16.4; DeepSeek-V3 one token 71.2, 70.4; dense 40 x 7168 x 2048 10.7, 8.8, 100 x 2304 x
+  // 1280 10.1, 9.2.  A split K extent, which comes out near one item a SM, keeps one CTA a SM (6 x 576 x 7168 11.5, 12.1; why is not known).
+  if (FORM != SPLIT) {
+    const int64_t items = (a.chunks == nullptr ? (int64_t)a.fixed_chunks : (a.max_chunks > 0 ? a.max_chunks : grid)) * a.n_tiles;
+    if (items < grid) grid = (int)items;
+  }
   LO_CUDA_OK(launch_dependent_clusters(PAIR ? 2 : 1, grouped_gemm_kernel<MODE, A_ROWS, FORM, PAIR>, dim3(PAIR ? grid & ~1 : grid),
                                        dim3(CF::NUM_THREADS), smem_bytes, stream, wmap, amaps, p));
   return LO_OK;
