@@ -479,15 +479,6 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   return r;
 }
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-// a / b from the approximate reciprocal, corrected by the remainder once: within a unit in the last place or better of the
-// quotient, whose next use is a rounding to bf16.  Here as with div_by() (common.h) the reciprocal has to be a normal number, which it
-// is for every division of the epilogues: their denominators are in [1, 1e38] or a group scale of at least 1e-10 / 127.
-__device__ __forceinline__ float div_fast(float a, float b) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  const float q = __fmul_rn(a, y);
-  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-}
 struct KParams {
   const float *a_scale;     // [positions, KB]
   const float *b_scale;
@@ -1353,10 +1344,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                   float a[2];
 #pragma unroll
                   for (int e = 0; e < 2; ++e) {
+                    // SiLU as in silu_of_bf16(), but for denominators beyond 2^126, whose reciprocal is flushed (the quotient would be below 1e-36),
+                    // and for an infinite sum, which leaves a NaN in its quantisation group
                     const float gte = __uint_as_float(e ? g2[h][j] & 0xffff0000u : g2[h][j] << 16);
-                    // 1 + exp(-gate) capped below the fp32 maximum: the quotient is then zero instead of an invalid
-                    // operation in the correction (the exact quotient would be -0 or a number below 1e-36)
-                    a[e] = div_fast(gte, fminf(1.0f + expf(-gte), 1e38f));
+                    a[e] = __fmaf_rn(gte, rcp_approx(silu_denominator(gte)), gte * 0.0f);
                   }
                   // bf16(silu) * bf16(up), rounded once: the packed bf16 product
                   const uint32_t sl = pack_bf16(a[0], a[1]);

@@ -385,37 +385,26 @@ __global__ void __launch_bounds__(TOKEN_QUANT_THREADS) token_quant_kernel(const 
 // ---------------------------------------------------------------------------
 // SiLU(gate) * up followed by per-token INT8 quantisation, one CTA per row of a bf16 [rows, 2*d]
 // matrix (gate columns first).  Semantics of the reference's fused kernel
-// (csrc/kernels/gated_activation/fuse_silu_mul_quant.cu:90-131) with exact fp32 expf / division in
-// the SiLU: act = bf16(bf16(silu(gate)) * up); scale = max|act| / 127; q = rint(act * (127 / max)),
+// (csrc/kernels/gated_activation/fuse_silu_mul_quant.cu:90-131), the SiLU rounded as with fp32 expf and division
+// (silu_of_bf16()): act = bf16(bf16(silu(gate)) * up); scale = max|act| / 127; q = rint(act * (127 / max)),
 // saturated; a row of zeros gets scale 0 and q 0.  Rows whose entry in row_ids is a padding
 // sentinel (< 0 or >= numel_valid) are skipped.
-// A row's loads are on their way before its id is looked up: with the library's division and the loads behind the look-ups a row's
-// chain of latencies bound it: 24 000 rows of 2048 channels 139 us, now 99 (the bytes take 38; what bounds it now are the
-// instructions, an exponential and an exact quotient per element).  Threads a row, in us with 128 and 256:
-//   1 x 2048: 2.4, 2.1    148 x 4096: 3.2, 2.7    296 x 1408: 2.6, 2.4    444 x 1408: 2.7, 3.1    2368 x 2048: 8.4, 10.0
-//   64 x 8192: 7.6, 3.5    4000 x 8192: 79, 45    16 x 18432: 15.0, 9.9    2000 x 18432: 94, 93
+// A row's loads are on their way before its id is looked up.  24 000 rows of 2048 channels take 49 us (the bytes 38); with the library's
+// exponential and a refined quotient, 25 instructions an element more, 70; with the library's division and the loads behind the look-ups 139.
+// 4000 x 8192 45.6 -> 29.9, 2368 x 2048 9.4 -> 7.0.  Threads a row, in us with 128 and 256:
+//   1 x 2048: 1.9, 1.7    148 x 4096: 2.2, 2.2    296 x 1408: 2.1, 2.1    444 x 1408: 2.2, 2.7    2368 x 2048: 7.0, 8.6    24000 x 2048: 49, 69
+//   64 x 8192: 5.1, 2.7    4000 x 8192: 49, 30    16 x 18432: 9.4, 7.0    2000 x 18432: 63, 56
 // 256 up to two rows a SM, where a row's chain is all there is, and for rows of more than 4096 channels, half of which would not
 // stay in the registers of 128; 128 else, where the blocks fill the SMs and fewer warps wait at a row's barrier.
 // ---------------------------------------------------------------------------
 
-// g / (1 + exp(-g)), after its rounding to bf16 the same as with the library's division: the refined reciprocal is taken of the denominator times 2^-32, which keeps the
-// reciprocal normal up to the largest finite denominator.  What that form does not give has a denominator of 2 (next to zero, where
-// the quotient may be a subnormal), of 1 (large gates and infinity) or of infinity (g * 0: a signed zero or, for -inf, NaN).
-// The tests compare every bf16 gate with the library's division.
-__device__ __forceinline__ float silu_exact(float g) {
-  const float den = 1.0f + expf(-g);
-  const float b = den * 0x1p-32f;
-  const float q = div_by(g, b, rcp_refined(b)) * 0x1p-32f;
-  const float r = den == 2.0f ? g * 0.5f : (den == 1.0f ? g : q);
-  return den == INFINITY ? g * 0.0f : r;
-}
 // Eight activations, as bf16, of eight gates and up values; amax takes their largest magnitude.
 __device__ __forceinline__ uint4 act8(const uint4 &g, const uint4 &u, float &amax) {
   const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
   uint32_t out[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const __nv_bfloat162 sl = __floats2bfloat162_rn(silu_exact(__uint_as_float(gw[i] << 16)), silu_exact(__uint_as_float(gw[i] & 0xffff0000u)));
+    const __nv_bfloat162 sl = __floats2bfloat162_rn(silu_of_bf16(__uint_as_float(gw[i] << 16)), silu_of_bf16(__uint_as_float(gw[i] & 0xffff0000u)));
     const float2 f = __bfloat1622float2(sl);
     const __nv_bfloat162 a = __floats2bfloat162_rn(f.x * __uint_as_float(uw[i] << 16), f.y * __uint_as_float(uw[i] & 0xffff0000u));
     out[i] = *reinterpret_cast<const uint32_t *>(&a);
