@@ -12,8 +12,9 @@ namespace {
 // lane + 32*i), k rounds of warp arg-max with erase.  Selection is done on the
 // logits (softmax is monotonic); ties go to the lower expert id.  A round is two warp reductions
 // in one instruction each, of keys that order like the logits and of the ids that have the
-// largest key (five shuffle steps of value and id were three times the instructions, which
-// bound the kernel: 8192 rows of 256 experts).
+// largest key.  Bound by instructions: a lane's largest key comes from a tree of which a round walks one path, and the probabilities are formed
+// once, behind the rounds (8192 rows of 256 experts 1018 -> 740 instructions a row, 13.8 -> 12.3 us; 4096 10.0 -> 8.6, 777 rows of 512 8.2 -> 7.4; in a
+// graph 8192 x 256 9.8 -> 8.0, 1 x 256 2.7 -> 2.5).
 // ---------------------------------------------------------------------------
 
 template <typename T> __device__ __forceinline__ float to_float(T v);
@@ -22,6 +23,37 @@ template <> __device__ __forceinline__ float to_float<__half>(__half v) { return
 template <> __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 template <typename IdT> __device__ __forceinline__ void store_id(IdT *p, int v) { *p = (IdT)v; }
+
+// The largest of a lane's VPL keys and its index (the lower one of equals) as a tree in registers: node n has the children 2n and 2n + 1, the
+// keys are the nodes VPL + i.
+template <int VPL> struct LaneBest {
+  uint32_t key[2 * VPL];
+  int index[VPL];      // of the inner nodes
+  __device__ __forceinline__ int at(int n) const { return VPL == 1 ? 0 : index[n]; }
+  template <int NODE, int FIRST, int N> __device__ __forceinline__ void combine() {
+    const bool right = key[2 * NODE + 1] > key[2 * NODE];
+    const int l = N == 2 ? FIRST : index[(2 * NODE) % VPL], r = N == 2 ? FIRST + 1 : index[(2 * NODE + 1) % VPL];
+    key[NODE] = right ? key[2 * NODE + 1] : key[2 * NODE];
+    index[NODE] = right ? r : l;
+  }
+  template <int NODE, int FIRST, int N> __device__ __forceinline__ void build() {
+    if constexpr (N > 1) {
+      build<2 * NODE, FIRST, N / 2>();
+      build<2 * NODE + 1, FIRST + N / 2, N / 2>();
+      combine<NODE, FIRST, N>();
+    }
+  }
+  // key i becomes min(key i, limit); i is the same in all lanes, so that a path of the tree is walked and not all of it
+  template <int NODE, int FIRST, int N> __device__ __forceinline__ void erase(int i, uint32_t limit) {
+    if constexpr (N == 1) {
+      key[NODE] = min(key[NODE], limit);
+    } else {
+      if (i < FIRST + N / 2) erase<2 * NODE, FIRST, N / 2>(i, limit);
+      else erase<2 * NODE + 1, FIRST + N / 2, N / 2>(i, limit);
+      combine<NODE, FIRST, N>();
+    }
+  }
+};
 
 template <typename T, typename IdT, int VPL>
 __global__ void __launch_bounds__(256) topk_softmax_kernel(const T *__restrict__ gating, int64_t M, int E, int k,
@@ -51,34 +83,37 @@ __global__ void __launch_bounds__(256) topk_softmax_kernel(const T *__restrict__
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) denom += __shfl_xor_sync(0xffffffffu, denom, off);
 
-  float my_w = 0.f;   // lane j keeps the j-th selected probability
+  uint32_t my_key = 0u;   // lane j keeps the j-th selected logit and its expert
   int my_id = 0;
-  float sel_sum = 0.f;
-  uint32_t key[VPL];
+  float w = 0.f, sel_sum = 0.f;
+  // (one key a lane: a round is latency, under which its probability costs nothing: layer of 32 tokens of the tiny shape in a graph 16.4 us, behind
+  // the rounds 16.8)
+  constexpr bool FEW = VPL == 1;
+  LaneBest<VPL> best;
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) key[i] = order_key(v[i]);
+  for (int i = 0; i < VPL; ++i) best.key[VPL + i] = order_key(v[i]);
+  best.template build<1, 0, VPL>();
   const uint32_t erased = order_key(-INFINITY);
   for (int r = 0; r < k; ++r) {
-    uint32_t best = key[0];
-    int best_i = 0;
-#pragma unroll
-    for (int i = 1; i < VPL; ++i) {
-      if (key[i] > best) { best = key[i]; best_i = i; }   // strict: keeps the lower id on ties
+    const uint32_t top = __reduce_max_sync(0xffffffffu, best.key[1]);
+    const int best_e = (int)__reduce_min_sync(0xffffffffu, best.key[1] == top ? (uint32_t)(lane + 32 * best.at(1)) : 0xffffffffu);
+    if (lane == r) { my_key = top; my_id = best_e; }
+    if (FEW) {
+      const float p = expf(key_value(top) - mx) / denom;
+      sel_sum += p;
+      if (lane == r) w = p;
     }
-    const uint32_t top = __reduce_max_sync(0xffffffffu, best);
-    const int best_e = (int)__reduce_min_sync(0xffffffffu, best == top ? (uint32_t)(lane + 32 * best_i) : 0xffffffffu);
-    const float p = expf(key_value(top) - mx) / denom;
-    sel_sum += p;
-    if (lane == r) { my_w = p; my_id = best_e; }
     // erase the winner in its owner lane
-    if ((best_e & 31) == lane) {
-#pragma unroll
-      for (int i = 0; i < VPL; ++i)
-        if (i == best_e >> 5) key[i] = erased;
-    }
+    best.template erase<1, 0, VPL>(best_e >> 5, (best_e & 31) == lane ? erased : 0xffffffffu);
   }
+  if (!FEW) {
+    // the probabilities, each in its lane; their sum in the order of selection
+    w = expf(key_value(my_key) - mx) / denom;
+    if (renorm)
+      for (int r = 0; r < k; ++r) sel_sum += __shfl_sync(0xffffffffu, w, r);
+  }
+  if (renorm) w = w / sel_sum;
   if (lane < k) {
-    const float w = renorm ? my_w / sel_sum : my_w;
     weights[row * k + lane] = w;
     store_id<IdT>(ids + row * k + lane, my_id);
     if (src_rows) src_rows[row * k + lane] = (int32_t)(lane * M + row);
