@@ -104,3 +104,25 @@ def test_masked_layout_by_hint(max_m):
     assert all(torch.equal(outs[0], d) for d in outs[1:])
     for e in range(E):
         assert bool((outs[0][e, int(rows[e]):] == -5.0).all()) and not bool((outs[0][e, :int(rows[e])] == -5.0).all(1).any())
+
+
+def test_pairs_in_a_graph():
+    # captured with the kernels around them and replayed on other inputs at the same addresses
+    import lightop_b200 as lo
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x = torch.randn(1000, 7168, generator=g, device=DEV).to(torch.bfloat16)
+    w, w_s = _int8(g, 34 * 128, 7168), torch.rand(34, 56, generator=g, device=DEV) * 9e-3 + 1e-3
+    run = lambda: lo.gemm_ops.apply_w8a8_block_int8_linear(x, w, [128, 128], w_s)  # noqa: E731
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        run()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = run()
+    for _ in range(3):
+        x.copy_(torch.randn(1000, 7168, generator=g, device=DEV).to(torch.bfloat16))
+        graph.replay()
+        assert torch.equal(y, run())
+    lo.check_device_status()
