@@ -681,6 +681,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             }
           }
         }
+        if constexpr (MODE == GEMM_CHANNEL) {
+          // The commits of an item's steps arrive at done[] each for itself, in no promised order with the one that the epilogue waits for.
+          // The last ones are waited for here, so that none arrives at the memory of a CTA that has left (the block-scaled modes wait for the
+          // commit of every step anyway).
+          for (uint32_t u = it < (uint32_t)NW ? 0u : it - NW; ok && u < it; ++u) ok = mbar_wait(sm, &sm.done[u % ND], (u / ND) & 1u, p.status, 12, LO_SLEEP_PRODUCER);
+        }
       }
     } else if (warp == 3) {
       // ============ activation producer: the chunk's token rows of every K block.  Token rows are read from an

@@ -91,3 +91,14 @@ def test_the_linear_of_a_few_rows_has_the_ctas_its_rules_count_with():
     for before, _, ctas in forms:
         assert ctas == "ROW_CTAS" or "(int)grid.x <= sm_count()" in before
     assert "ctas = (int64_t)ROW_CTAS * sm_count()" in text and "N > outs * ctas" in text and "N > (int64_t)ROW_OUTS_MAX * ROW_CTAS * sm_count()" in text
+
+
+def test_every_commit_has_arrived_before_a_cta_leaves():
+    # per channel nobody but the weight producer waits for the commits of the steps, and it waits NW steps late: behind its loop it waits for the
+    # last NW, in each CTA of a pair (the closing barrier of a cluster orders threads, not arrivals still on their way)
+    st = _statements("grouped_gemm.cu")
+    loop = next(i for i, s in enumerate(st) if s.startswith("tma_load_2d(sm.w[s]"))
+    end = next(i for i in range(loop, len(st)) if "warp == 3" in st[i])
+    tail = " ; ".join(st[loop:end])
+    assert "if constexpr (MODE == GEMM_CHANNEL)" in tail
+    assert "u = it < (uint32_t)NW ? 0u : it - NW" in tail and "ok = mbar_wait(sm, &sm.done[u % ND], (u / ND) & 1u," in tail
