@@ -28,15 +28,29 @@ def _nvcc() -> str:
     return "nvcc"
 
 
+def _dependencies(out: str) -> list:
+    """The sources of an output (the object files that a build leaves beside them are none: they are newer than an output that was linked first)."""
+    headers = [os.path.join(HERE, "..", "include", "lightop_b200.h")]
+    if out == HOST:
+        return [os.path.join(CSRC, "host.cpp"), *headers]
+    return [*(os.path.join(CSRC, f) for f in SOURCES), *(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")), *headers]
+
+
+def outdated() -> list:
+    """The outputs, of LIB and HOST, that are missing or older than one of their sources."""
+    def old(out):
+        if not os.path.exists(out):
+            return True
+        t = os.path.getmtime(out)
+        return any(os.path.getmtime(d) > t for d in _dependencies(out))
+    return [out for out in (LIB, HOST) if old(out)]
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(HOST):
-        return True
-    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST))
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "lightop_b200.h")]
-    return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
+    return bool(outdated())
 
 
-def _host_command() -> list:
+def _host_command(out: str) -> list:
     # (found without importing torch: a first import of it takes a while)
     torch_dir = list(importlib.util.find_spec("torch").submodule_search_locations)[0]
     cuda_dir = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
@@ -44,31 +58,44 @@ def _host_command() -> list:
                os.path.join(cuda_dir, "include"), sysconfig.get_path("include")]
     lib = os.path.join(torch_dir, "lib")
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", *[f"-I{d}" for d in include], os.path.join(CSRC, "host.cpp"),
-            "-o", HOST, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{lib}"]
+            "-o", out, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{lib}"]
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB
-    objs = []
-    procs = [("host.cpp", subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True))]
-    for src in SOURCES:
-        obj = os.path.join(CSRC, src.replace(".cu", ".o"))
-        cmd = [_nvcc(), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
-        procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-        objs.append(obj)
-    for src, pr in procs:
-        out, _ = pr.communicate()
-        if pr.returncode != 0:
+def _compile(commands: list, verbose: bool = False) -> None:
+    """Runs (source, command) pairs side by side."""
+    procs = [(src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)) for src, cmd in commands]
+    results = [(src, pr.communicate()[0], pr.returncode) for src, pr in procs]
+    for src, out, rc in results:
+        if rc != 0:
             raise RuntimeError(f"the compiler failed on {src}:\n{out}")
         if verbose and out:
             print(out)
-    link = [_nvcc(), "-shared", "-o", LIB, *objs, "-cudart", "static"]
-    res = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"link failed:\n{res.stdout}")
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    todo = [LIB, HOST] if force else outdated()
+    # An output is written under another name and renamed when it is complete: a process that has the old file mapped keeps it, and a build that
+    # fails leaves it.
+    part = {out: f"{out[:-len('.so')]}.{os.getpid()}.so" for out in todo}
+    try:
+        commands, objs = [], []
+        if HOST in todo:
+            commands.append(("host.cpp", _host_command(part[HOST])))
+        for src in SOURCES if LIB in todo else []:
+            obj = os.path.join(CSRC, src.replace(".cu", ".o"))
+            commands.append((src, [_nvcc(), *(["-Xptxas=-v"] if verbose else []), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]))
+            objs.append(obj)
+        _compile(commands, verbose)
+        if LIB in todo:
+            res = subprocess.run([_nvcc(), "-shared", "-o", part[LIB], *objs, "-cudart", "static"], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+            if res.returncode != 0:
+                raise RuntimeError(f"link failed:\n{res.stdout}")
+        for out in todo:
+            os.replace(part[out], out)
+    finally:
+        for path in part.values():
+            if os.path.exists(path):
+                os.unlink(path)
     return LIB
 
 

@@ -1,0 +1,66 @@
+"""The build step: what counts as out of date.  Works on files of its own in place of the sources and outputs; no compiler runs."""
+import importlib.util
+import os
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture
+def tree(tmp_path, monkeypatch):
+    """build.py on a small tree: two CUDA sources, a header, the host module's source, the public header; everything built at time 1000, objects
+    left behind later than the outputs (the compilers run at the same time)."""
+    spec = importlib.util.spec_from_file_location("_lo_build_under_test", os.path.join(ROOT, "lightop_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    pkg = tmp_path / "pkg"
+    (pkg / "csrc").mkdir(parents=True)
+    (tmp_path / "include").mkdir()
+    files = {"a.cu": pkg / "csrc" / "a.cu", "b.cu": pkg / "csrc" / "b.cu", "common.h": pkg / "csrc" / "common.h", "host.cpp": pkg / "csrc" / "host.cpp",
+             "lightop_b200.h": tmp_path / "include" / "lightop_b200.h", "a.o": pkg / "csrc" / "a.o", "lib": pkg / "lib.so", "host": pkg / "_host.so"}
+    for name, path in files.items():
+        path.write_text("")
+        t = {"lib": 1001, "host": 1000, "a.o": 2000}.get(name, 900)
+        os.utime(path, (t, t))
+    for name, value in dict(HERE=str(pkg), CSRC=str(pkg / "csrc"), LIB=str(files["lib"]), HOST=str(files["host"]), SOURCES=["a.cu", "b.cu"]).items():
+        monkeypatch.setattr(build, name, value)
+    return build, files
+
+
+def test_a_finished_build_is_up_to_date(tree):
+    build, _ = tree
+    assert not build.needs_build()
+
+
+@pytest.mark.parametrize("name,lib,host", [("b.cu", True, False), ("common.h", True, False), ("host.cpp", False, True), ("lightop_b200.h", True, True),
+                                           ("a.o", False, False)])
+def test_each_output_has_its_own_sources(tree, name, lib, host):
+    build, files = tree
+    os.utime(files[name], (3000, 3000))
+    assert build.outdated() == [p for p, old in ((build.LIB, lib), (build.HOST, host)) if old]
+    assert build.needs_build() == (lib or host)
+
+
+@pytest.mark.parametrize("name", ["lib", "host"])
+def test_a_missing_output_is_built(tree, name):
+    build, files = tree
+    files[name].unlink()
+    assert build.outdated() == [str(files[name])]
+
+
+def test_an_output_that_fails_to_build_leaves_the_old_one(tree, monkeypatch):
+    build, files = tree
+    files["host"].write_text("old")
+    os.utime(files["host"], (1000, 1000))
+    os.utime(files["host.cpp"], (3000, 3000))
+
+    def command(out):
+        return ["sh", "-c", f"echo half > {out}; exit 1"]
+    monkeypatch.setattr(build, "_host_command", command)
+    with pytest.raises(RuntimeError, match="host.cpp"):
+        build.build()
+    assert files["host"].read_text() == "old" and sorted(os.listdir(build.HERE)) == ["_host.so", "csrc", "lib.so"]
+    monkeypatch.setattr(build, "_host_command", lambda out: ["sh", "-c", f"echo new > {out}"])
+    build.build()
+    assert files["host"].read_text() == "new\n" and not build.needs_build()
