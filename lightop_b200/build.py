@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import importlib.util
 import os
+import runpy
 import subprocess
 import sys
 import sysconfig
@@ -36,11 +37,30 @@ def _dependencies(out: str) -> list:
     return [*(os.path.join(CSRC, f) for f in SOURCES), *(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")), *headers]
 
 
+def _torch_dir() -> str:
+    # (found without importing torch: a first import of it takes a while)
+    return list(importlib.util.find_spec("torch").submodule_search_locations)[0]
+
+
+def built_for() -> str:
+    """What the host module is compiled against besides its sources; it carries this text, and one with another text is out of date."""
+    torch_version = runpy.run_path(os.path.join(_torch_dir(), "version.py"))["__version__"]
+    return f"torch {torch_version}, Python {sysconfig.get_config_var('SOABI')}"
+
+
+def _host_marker() -> bytes:
+    return f"[built for {built_for()}]".encode()
+
+
 def outdated() -> list:
-    """The outputs, of LIB and HOST, that are missing or older than one of their sources."""
+    """The outputs, of LIB and HOST, that are missing, older than one of their sources or (HOST) built for another torch or Python."""
     def old(out):
         if not os.path.exists(out):
             return True
+        if out == HOST:
+            with open(out, "rb") as f:
+                if _host_marker() not in f.read():
+                    return True
         t = os.path.getmtime(out)
         return any(os.path.getmtime(d) > t for d in _dependencies(out))
     return [out for out in (LIB, HOST) if old(out)]
@@ -51,13 +71,12 @@ def needs_build() -> bool:
 
 
 def _host_command(out: str) -> list:
-    # (found without importing torch: a first import of it takes a while)
-    torch_dir = list(importlib.util.find_spec("torch").submodule_search_locations)[0]
+    torch_dir = _torch_dir()
     cuda_dir = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
     include = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
                os.path.join(cuda_dir, "include"), sysconfig.get_path("include")]
     lib = os.path.join(torch_dir, "lib")
-    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", *[f"-I{d}" for d in include], os.path.join(CSRC, "host.cpp"),
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f'-DLIGHTOP_BUILT_FOR="{_host_marker().decode()}"', *[f"-I{d}" for d in include], os.path.join(CSRC, "host.cpp"),
             "-o", out, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{lib}"]
 
 

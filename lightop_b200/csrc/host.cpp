@@ -260,4 +260,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Host side of the calls th
 
 }  // namespace
 
-extern "C" PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+extern "C" PyMODINIT_FUNC PyInit__host(void) {
+  PyObject *m = PyModule_Create(&module);
+  // the torch and the Python that this was compiled against: the build looks for the text in the file, the package compares it with what it runs on
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", LIGHTOP_BUILT_FOR) != 0) Py_CLEAR(m);
+  return m;
+}

@@ -25,6 +25,9 @@ def tree(tmp_path, monkeypatch):
         os.utime(path, (t, t))
     for name, value in dict(HERE=str(pkg), CSRC=str(pkg / "csrc"), LIB=str(files["lib"]), HOST=str(files["host"]), SOURCES=["a.cu", "b.cu"]).items():
         monkeypatch.setattr(build, name, value)
+    monkeypatch.setattr(build, "built_for", lambda: "torch 1, Python x")
+    files["host"].write_bytes(b"..[built for torch 1, Python x]..")
+    os.utime(files["host"], (1000, 1000))
     return build, files
 
 
@@ -51,8 +54,7 @@ def test_a_missing_output_is_built(tree, name):
 
 def test_an_output_that_fails_to_build_leaves_the_old_one(tree, monkeypatch):
     build, files = tree
-    files["host"].write_text("old")
-    os.utime(files["host"], (1000, 1000))
+    old = files["host"].read_text()
     os.utime(files["host.cpp"], (3000, 3000))
 
     def command(out):
@@ -60,7 +62,20 @@ def test_an_output_that_fails_to_build_leaves_the_old_one(tree, monkeypatch):
     monkeypatch.setattr(build, "_host_command", command)
     with pytest.raises(RuntimeError, match="host.cpp"):
         build.build()
-    assert files["host"].read_text() == "old" and sorted(os.listdir(build.HERE)) == ["_host.so", "csrc", "lib.so"]
-    monkeypatch.setattr(build, "_host_command", lambda out: ["sh", "-c", f"echo new > {out}"])
+    assert files["host"].read_text() == old and sorted(os.listdir(build.HERE)) == ["_host.so", "csrc", "lib.so"]
+    monkeypatch.setattr(build, "_host_command", lambda out: ["sh", "-c", f"echo '[built for torch 1, Python x] new' > {out}"])
     build.build()
-    assert files["host"].read_text() == "new\n" and not build.needs_build()
+    assert files["host"].read_text().endswith("new\n") and not build.needs_build()
+
+
+@pytest.mark.parametrize("other", ["torch 2, Python x", "torch 1, Python y"])
+def test_a_host_module_for_another_torch_or_python_is_built_again(tree, monkeypatch, other):
+    build, _ = tree
+    monkeypatch.setattr(build, "built_for", lambda: other)
+    assert build.outdated() == [build.HOST]
+
+
+def test_the_host_module_says_what_it_was_built_for():
+    import torch
+    from lightop_b200 import _lib, build
+    assert torch.__version__ in build.built_for() and _lib.host.built_for == f"[built for {build.built_for()}]"
