@@ -1,19 +1,47 @@
 """ctypes binding of ``liblightop_b200.so`` (the C ABI declared in include/lightop_b200.h).
 
-There is no fallback: if the library is missing or a call fails, an exception is raised.
+There is no fallback: if the library is missing or a call fails, an exception is raised.  (``host``, the native host side of small calls, is
+an addition to this layer: what it does not take, this layer does.)
 """
 from __future__ import annotations
 
 import ctypes
 import os
+import sysconfig
+import warnings
 from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_void_p
 
 import torch
 
-try:
-    from . import _host as host      # csrc/host.cpp
-except ImportError as e:
-    raise ImportError("lightop_b200/_host.so is missing or unusable: build it with `python lightop_b200/build.py` (there is no fallback)") from e
+
+class _NoHost:
+    """In the place of the native host step where it cannot be used: it takes no call, so that the general path has them all."""
+
+    @staticmethod
+    def _nothing(*args):
+        return None
+
+    bind = topk_softmax = fused_experts = linear = _nothing
+
+
+def _import_host():
+    """csrc/host.cpp as it was built for this torch and Python, or a stand-in.  The kernels and their results are the same without it, small calls take
+    up to 20 us more on the host; a torch without CUDA has no use for it."""
+    if torch.version.cuda is None:
+        return _NoHost()
+    here = f"[built for torch {torch.__version__}, Python {sysconfig.get_config_var('SOABI')}]"
+    try:
+        from . import _host
+        if _host.built_for == here:
+            return _host
+        why = f"it is {_host.built_for[1:-1]}, this is {here[len('[built for '):-1]}"
+    except ImportError as e:
+        why = str(e)
+    warnings.warn(f"lightop_b200/_host.so is not used, small calls take longer on the host: {why}; `python lightop_b200/build.py` builds it", RuntimeWarning)
+    return _NoHost()
+
+
+host = _import_host()
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # LIGHTOP_B200_LIB overrides the location of the shared library (e.g. an instrumented build)

@@ -1,8 +1,8 @@
 """Build step of the C-ABI library: nvcc for sm_100a only, in-tree output.
 
 ``python lightop_b200/build.py`` (run by path: importing the package needs the built library) compiles ``csrc/*.cu`` into
-``lightop_b200/liblightop_b200.so`` and ``csrc/host.cpp`` (the host side of small calls, against the installed torch) into
-``lightop_b200/_host.so``.  nvcc cross-compiles without a GPU.
+``lightop_b200/liblightop_b200.so`` and, where a torch with CUDA is installed, ``csrc/host.cpp`` (the host side of small calls, against that
+torch) into ``lightop_b200/_host.so``.  nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -38,8 +38,15 @@ def _dependencies(out: str) -> list:
 
 
 def _torch_dir() -> str:
-    # (found without importing torch: a first import of it takes a while)
-    return list(importlib.util.find_spec("torch").submodule_search_locations)[0]
+    """Where the installed torch is, "" if there is none (found without importing it: a first import takes a while)."""
+    spec = importlib.util.find_spec("torch")
+    return list(spec.submodule_search_locations)[0] if spec is not None and spec.submodule_search_locations else ""
+
+
+def host_possible() -> bool:
+    """Whether there is a torch with CUDA to compile the host module against.  The C-ABI library needs none, and the package goes without the module."""
+    torch_dir = _torch_dir()
+    return bool(torch_dir) and os.path.exists(os.path.join(torch_dir, "lib", "libc10_cuda.so"))
 
 
 def built_for() -> str:
@@ -63,7 +70,11 @@ def outdated() -> list:
                     return True
         t = os.path.getmtime(out)
         return any(os.path.getmtime(d) > t for d in _dependencies(out))
-    return [out for out in (LIB, HOST) if old(out)]
+    return [out for out in _outputs() if old(out)]
+
+
+def _outputs() -> list:
+    return [LIB, HOST] if host_possible() else [LIB]
 
 
 def needs_build() -> bool:
@@ -92,25 +103,22 @@ def _compile(commands: list, verbose: bool = False) -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    todo = [LIB, HOST] if force else outdated()
+    todo = _outputs() if force else outdated()
     # An output is written under another name and renamed when it is complete: a process that has the old file mapped keeps it, and a build that
     # fails leaves it.
     part = {out: f"{out[:-len('.so')]}.{os.getpid()}.so" for out in todo}
     try:
-        commands, objs = [], []
-        if HOST in todo:
-            commands.append(("host.cpp", _host_command(part[HOST])))
-        for src in SOURCES if LIB in todo else []:
-            obj = os.path.join(CSRC, src.replace(".cu", ".o"))
-            commands.append((src, [_nvcc(), *(["-Xptxas=-v"] if verbose else []), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]))
-            objs.append(obj)
-        _compile(commands, verbose)
         if LIB in todo:
+            objs = [os.path.join(CSRC, src.replace(".cu", ".o")) for src in SOURCES]
+            _compile([(src, [_nvcc(), *(["-Xptxas=-v"] if verbose else []), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj])
+                      for src, obj in zip(SOURCES, objs)], verbose)
             res = subprocess.run([_nvcc(), "-shared", "-o", part[LIB], *objs, "-cudart", "static"], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
             if res.returncode != 0:
                 raise RuntimeError(f"link failed:\n{res.stdout}")
-        for out in todo:
-            os.replace(part[out], out)
+            os.replace(part[LIB], LIB)
+        if HOST in todo:      # last: where it does not compile, the library is there and the package works without it
+            _compile([("host.cpp", _host_command(part[HOST]))], verbose)
+            os.replace(part[HOST], HOST)
     finally:
         for path in part.values():
             if os.path.exists(path):

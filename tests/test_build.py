@@ -1,6 +1,8 @@
 """The build step: what counts as out of date.  Works on files of its own in place of the sources and outputs; no compiler runs."""
 import importlib.util
 import os
+import subprocess
+import sys
 
 import pytest
 
@@ -26,6 +28,8 @@ def tree(tmp_path, monkeypatch):
     for name, value in dict(HERE=str(pkg), CSRC=str(pkg / "csrc"), LIB=str(files["lib"]), HOST=str(files["host"]), SOURCES=["a.cu", "b.cu"]).items():
         monkeypatch.setattr(build, name, value)
     monkeypatch.setattr(build, "built_for", lambda: "torch 1, Python x")
+    build.really_possible = build.host_possible
+    monkeypatch.setattr(build, "host_possible", lambda: True)
     files["host"].write_bytes(b"..[built for torch 1, Python x]..")
     os.utime(files["host"], (1000, 1000))
     return build, files
@@ -79,3 +83,49 @@ def test_the_host_module_says_what_it_was_built_for():
     import torch
     from lightop_b200 import _lib, build
     assert torch.__version__ in build.built_for() and _lib.host.built_for == f"[built for {build.built_for()}]"
+
+
+@pytest.mark.parametrize("found", [False, True])
+def test_the_library_needs_no_torch(tree, monkeypatch, tmp_path, found):
+    # none installed, or one without CUDA
+    build, files = tree
+    spec = importlib.util.spec_from_file_location("torch", str(tmp_path / "__init__.py"), submodule_search_locations=[str(tmp_path)]) if found else None
+    monkeypatch.setattr(importlib.util, "find_spec", lambda name: spec)
+    monkeypatch.setattr(build, "host_possible", build.really_possible)
+    files["host"].unlink()
+    assert build.outdated() == []
+    os.utime(files["a.cu"], (3000, 3000))
+    assert build.outdated() == [build.LIB]
+
+
+_IMPORT = """
+import sys, types, warnings
+import torch
+case = sys.argv[1]
+if case == "missing":
+    sys.modules["lightop_b200._host"] = None          # (its import raises ImportError)
+elif case == "other":
+    sys.modules["lightop_b200._host"] = types.SimpleNamespace(built_for="[built for torch 1.0, Python x]")
+elif case == "cpu":
+    sys.modules["lightop_b200._host"] = None
+    torch.version.cuda = None
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter("always")
+    import lightop_b200 as lo
+seen = [str(w.message) for w in seen if "_host.so" in str(w.message)]
+assert len(seen) == (0 if case == "cpu" else 1) and all("build.py" in s for s in seen), seen
+from lightop_b200 import _lib
+assert _lib.load().lo_version() == 1
+assert _lib.host.topk_softmax(1, 2, 3, 4) is None and _lib.host.fused_experts() is None and _lib.host.linear() is None
+try:
+    lo.moe.topk_softmax(torch.zeros(2, 2), torch.zeros(2, 2, dtype=torch.int32), None, torch.zeros(2, 8), True)
+except RuntimeError as e:
+    assert "CUDA" in str(e)
+else:
+    raise SystemExit("a CPU tensor was taken")
+"""
+
+
+@pytest.mark.parametrize("case", ["missing", "other", "cpu"])
+def test_the_package_works_without_the_host_module(case):
+    subprocess.run([sys.executable, "-c", _IMPORT, case], cwd=ROOT, check=True, timeout=300)
