@@ -244,9 +244,10 @@ __device__ __forceinline__ float rcp_approx(float b) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
   return y;
 }
-// g / (1 + exp(-g)) of a bf16 gate for a rounding to bf16.  Each of the two approximations is within two units in the last place of fp32, 2^-14 of
-// the distance of two bf16 numbers: after the rounding the result is that of the library's exponential and division for every bf16 gate
-// (the tests compare all of them).  The reciprocal is taken of a quarter of the denominator: a normal number up to the largest finite one.
+// g / (1 + exp(-g)) of a bf16 gate for a rounding to bf16.  Less exact than the library's exponential and division: the argument of the power of two is
+// rounded, which puts up to |g| x 2^-24 (2^-18 at g = -84) on top of the 2^-22 of the instruction; the reciprocal adds 2^-23.  A unit of bf16 is
+// 2^-8, so that only a gate whose quotient lies that close to a tie could round the other way.  None does: that rests on the tests, which take all
+// finite gates one at a time, not on the bound.  The reciprocal is taken of a quarter of the denominator: a normal number up to the largest finite one.
 __device__ __forceinline__ float silu_of_bf16(float g) { return g * (rcp_approx(silu_denominator(g) * 0.25f) * 0.25f); }
 
 // Expert of (token, slot) number i, through the map where map_mode is 1; -1 where there is none.
