@@ -53,6 +53,8 @@ const char *lo_last_error(void);
 int lo_sm_count(void);
 /* Kernels this library has launched since it was loaded (all threads, all devices). */
 long long lo_launch_count(void);
+/* Grouped GEMMs among them that ran on pairs of CTAs (which form a call takes shows nowhere else: the results have the same bits). */
+long long lo_pair_launch_count(void);
 
 /*
  * Softmax over experts + top-k selection (+ optional renormalisation).

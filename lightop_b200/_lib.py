@@ -64,6 +64,7 @@ PROTOTYPES = {
     "lo_last_error": (c_char_p, []),
     "lo_sm_count": (c_int, []),
     "lo_launch_count": (ctypes.c_longlong, []),
+    "lo_pair_launch_count": (ctypes.c_longlong, []),
     "lo_topk_softmax": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                                 c_void_p, c_void_p]),
     "lo_moe_align_block_size": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_int, c_void_p,

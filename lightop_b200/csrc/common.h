@@ -47,6 +47,8 @@ inline int fail(int code, const char *fmt, ...) {
 
 // Kernels launched by this library since it was loaded (lo_launch_count): every launch site counts itself.
 extern std::atomic<long long> g_launch_count;
+// Grouped GEMMs among them that ran on pairs of CTAs (lo_pair_launch_count).
+extern std::atomic<long long> g_pair_launch_count;
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }

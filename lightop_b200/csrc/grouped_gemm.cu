@@ -1483,6 +1483,7 @@ int launch_mode(const GemmArgs &a, cudaStream_t stream) {
   }
   LO_CUDA_OK(launch_dependent_clusters(PAIR ? 2 : 1, grouped_gemm_kernel<MODE, A_ROWS, FORM, PAIR>, dim3(PAIR ? grid & ~1 : grid),
                                        dim3(CF::NUM_THREADS), smem_bytes, stream, wmap, amaps, p));
+  if (PAIR) g_pair_launch_count.fetch_add(1, std::memory_order_relaxed);
   return LO_OK;
 }
 
