@@ -32,9 +32,10 @@ def _import_host():
     here = f"[built for torch {torch.__version__}, Python {sysconfig.get_config_var('SOABI')}]"
     try:
         from . import _host
-        if _host.built_for == here:
+        built_for = getattr(_host, "built_for", "[built for a torch that it does not name]")
+        if built_for == here:
             return _host
-        why = f"it is {_host.built_for[1:-1]}, this is {here[len('[built for '):-1]}"
+        why = f"it is {built_for[1:-1]}, this is {here[len('[built for '):-1]}"
     except ImportError as e:
         why = str(e)
     warnings.warn(f"lightop_b200/_host.so is not used, small calls take longer on the host: {why}; `python lightop_b200/build.py` builds it", RuntimeWarning)

@@ -106,6 +106,8 @@ if case == "missing":
     sys.modules["lightop_b200._host"] = None          # (its import raises ImportError)
 elif case == "other":
     sys.modules["lightop_b200._host"] = types.SimpleNamespace(built_for="[built for torch 1.0, Python x]")
+elif case == "older":
+    sys.modules["lightop_b200._host"] = types.SimpleNamespace()      # from before it said so
 elif case == "cpu":
     sys.modules["lightop_b200._host"] = None
     torch.version.cuda = None
@@ -126,6 +128,6 @@ else:
 """
 
 
-@pytest.mark.parametrize("case", ["missing", "other", "cpu"])
+@pytest.mark.parametrize("case", ["missing", "other", "older", "cpu"])
 def test_the_package_works_without_the_host_module(case):
     subprocess.run([sys.executable, "-c", _IMPORT, case], cwd=ROOT, check=True, timeout=300)
