@@ -1,34 +1,15 @@
 """GPU test of the grouped GEMM on pairs of CTAs against its form on single ones.  Calls large enough for pairs are computed again in a way
 that takes the other form (an odd number of output tiles, or one expert at a time), and every output must have the same bits.  Chunk widths
 on both sides of the MMA's 32-row granule and of the boxes that a half of a chunk is loaded with."""
-import functools
-
 import pytest
-import test_gpu_ep_emulated
 import torch
 
-from lightop_b200 import _lib, synthetic
+from lightop_b200 import synthetic
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 # rows per expert: every edge of pieces, granules and boxes, a full chunk, more than one, none
-# (109 on average: the block-scaled layer's table is cut at 128 rows)
 COUNTS = [1, 16, 17, 31, 32, 33, 64, 65, 80, 96, 97, 112, 113, 128, 129, 144, 145, 160, 161, 200, 256, 257, 300, 0]
-# the same and more of several chunks each, 152 on average: that table is cut at 160
-COUNTS_WIDE = COUNTS + [320, 321, 480, 319, 337, 175]
-
-
-class _Pairs:
-    """Counts the grouped GEMMs on pairs inside a `with`: as many as said, so that a rule that sends both sides of a comparison to one form fails it."""
-
-    def __init__(self, want):
-        self.want = want
-
-    def __enter__(self):
-        self.before = _lib.load().lo_pair_launch_count()
-
-    def __exit__(self, kind, *rest):
-        assert kind is not None or _lib.load().lo_pair_launch_count() - self.before == self.want
 
 
 def _int8(g, *shape):
@@ -43,21 +24,18 @@ def test_dense_linear(M, tiles, K):
     q, s = _int8(g, M, K), torch.rand(M, K // 128, generator=g, device=DEV) * 0.05 + 1e-3
     w, w_s = _int8(g, tiles * 128, K), torch.rand(tiles, K // 128, generator=g, device=DEV) * 9e-3 + 1e-3
     n = (tiles - 1) * 128
-    with _Pairs(1):
-        pairs = lo.gemm_ops.matmul_block_int8(q, w, s, w_s, [128, 128], torch.bfloat16)
+    pairs = lo.gemm_ops.matmul_block_int8(q, w, s, w_s, [128, 128], torch.bfloat16)
     for order in (torch.arange(tiles), torch.arange(tiles).flip(0)):      # (the second one has the last tile)
         order = order.to(DEV)
-        with _Pairs(0):
-            single = lo.gemm_ops.matmul_block_int8(q, w.view(tiles, 128, K)[order].reshape(-1, K)[:n].contiguous(), s, w_s[order][:-1].contiguous(),
-                                                   [128, 128], torch.bfloat16)
+        single = lo.gemm_ops.matmul_block_int8(q, w.view(tiles, 128, K)[order].reshape(-1, K)[:n].contiguous(), s, w_s[order][:-1].contiguous(),
+                                               [128, 128], torch.bfloat16)
         torch.cuda.synchronize()
         lo.check_device_status()
         assert torch.equal(pairs.view(M, tiles, 128)[:, order].reshape(M, -1)[:, :n], single)
 
 
 @pytest.mark.parametrize("block,channel", [(128, False), (128, True), (256, True)])
-@pytest.mark.parametrize("absent", [False, True])
-def test_grouped_gemm(block, channel, absent):
+def test_grouped_gemm(block, channel):
     import lightop_b200 as lo
     E, tiles, K = len(COUNTS), 16, 7168
     g = torch.Generator(device=DEV).manual_seed(block)
@@ -70,30 +48,20 @@ def test_grouped_gemm(block, channel, absent):
     else:
         s, w_s = torch.rand(M, K // 128, generator=g, device=DEV) * 0.05 + 1e-3, torch.rand(E, tiles, K // 128, generator=g, device=DEV) * 9e-3 + 1e-3
     wgt = torch.rand(M, 1, generator=g, device=DEV)
-    # absent: blocks of every third expert have no local expert and give rows of zeros
-    local = torch.arange(E, dtype=torch.int32, device=DEV)
-    if absent:
-        local[::3] = -1
-    order = lo.moe.moe_align_block_size(ids, block, E, local)
-    assert bool((order[1][:int(order[2]) // block] == -1).any()) == absent
+    order = lo.moe.moe_align_block_size(ids, block, E)
 
     def run(w, w_s):
         out = torch.full((M, 1, w.shape[1]), float("nan"), dtype=torch.bfloat16, device=DEV)
         lo.moe.moe_gemm_w8a8(q, w.contiguous(), out, s, w_s.contiguous(), wgt, *order, 1, {"BLOCK_SIZE_M": block})
         return out
     n = (tiles - 1) * 128
-    with _Pairs(1):
-        pairs = run(w, w_s)
-    with _Pairs(0):
-        single = run(w[:, :n], w_s[:, :n] if channel else w_s[:, :-1])
+    pairs, single = run(w, w_s), run(w[:, :n], w_s[:, :n] if channel else w_s[:, :-1])
     torch.cuda.synchronize()
     lo.check_device_status()
     assert torch.equal(pairs[..., :n], single) and not torch.isnan(pairs.float()).any()
-    gone = local[ids.view(-1).long()] < 0
-    assert not bool(pairs[gone].any()) and bool((pairs[~gone] != 0).any(-1).all())
 
 
-@pytest.mark.parametrize("counts", [COUNTS, [min(c, 160) for c in COUNTS], [c // 2 for c in COUNTS], COUNTS_WIDE])
+@pytest.mark.parametrize("counts", [COUNTS, [min(c, 160) for c in COUNTS], [c // 2 for c in COUNTS]])
 @pytest.mark.parametrize("channel", [False, True])
 def test_layer(counts, channel):
     import lightop_b200 as lo
@@ -110,14 +78,11 @@ def test_layer(counts, channel):
         return lo.moe.fused_experts_impl_int8(x[rows], w1[first:last], w2[first:last], w[rows].view(-1, 1), (ids[rows] - first).view(-1, 1), None,
                                               use_int8_w8a8=True, per_channel_quant=channel, block_shape=None if channel else [128, 128],
                                               w1_scale=w1_s[first:last], w2_scale=w2_s[first:last], **kw)
-    with _Pairs(2 if channel or sum(counts) // E >= 83 else 1):      # (with few rows an expert the block-scaled down GEMM stays below the line)
-        y = run(torch.arange(len(ids), device=DEV), 0, E)
+    y = run(torch.arange(len(ids), device=DEV), 0, E)
     for e in range(E):
         rows = torch.nonzero(ids == e).reshape(-1)
         if len(rows):
-            with _Pairs(0):
-                single = run(rows, e, e + 1)
-            assert torch.equal(y[rows], single), counts[e]
+            assert torch.equal(y[rows], run(rows, e, e + 1)), counts[e]
     lo.check_device_status()
 
 
@@ -130,10 +95,9 @@ def test_masked_layout_by_hint(max_m):
     a, w = (_int8(g, E, max_m, K), torch.rand(E, max_m, 1, generator=g, device=DEV)), (_int8(g, E, N, K), torch.rand(E, N, 1, generator=g, device=DEV))
     rows = torch.tensor([min(c, max_m) for c in COUNTS], dtype=torch.int32, device=DEV)
     outs = []
-    for hint, on_pairs in ((0, 0), (1, 0), (100, 1), (1 << 70, 1), (-5, 0), (None, 0)):
+    for hint in (0, 1, 100, 1 << 70, -5, None):
         d = torch.full((E, max_m, N), -5.0, dtype=torch.bfloat16, device=DEV)
-        with _Pairs(on_pairs):
-            lo.gemm_ops.m_grouped_w8a8_gemm_nt_masked(a, w, d, rows, hint)
+        lo.gemm_ops.m_grouped_w8a8_gemm_nt_masked(a, w, d, rows, hint)
         outs.append(d)
     torch.cuda.synchronize()
     lo.check_device_status()
@@ -155,43 +119,10 @@ def test_pairs_in_a_graph():
         run()
     torch.cuda.current_stream().wait_stream(side)
     graph = torch.cuda.CUDAGraph()
-    with _Pairs(1), torch.cuda.graph(graph):
+    with torch.cuda.graph(graph):
         y = run()
     for _ in range(3):
         x.copy_(torch.randn(1000, 7168, generator=g, device=DEV).to(torch.bfloat16))
         graph.replay()
         assert torch.equal(y, run())
     lo.check_device_status()
-
-
-def test_expert_rows_into_addresses(monkeypatch):
-    # the expert side of expert parallelism with a table of row addresses (two emulated ranks in this GPU's memory), at sizes that take pairs; compared with
-    # the layer of one GPU there
-    import lightop_b200 as lo
-    monkeypatch.setattr(synthetic, "make_weights", functools.partial(synthetic.make_weights, device=DEV))
-    with _Pairs(4 + 2):      # both GEMMs of either rank's experts (137 rows each), and of the larger comparison (340 tokens: 64-row chunks, single CTAs)
-        test_gpu_ep_emulated.test_peer_transport_with_emulated_ranks(lo, 2, 32, 4, 7168, 2048, (760, 340))
-
-
-@pytest.mark.parametrize("sms", [8, 64])
-def test_pairs_in_a_partition(sms):
-    # a green context of few SMs: the pairs of a call run after one another there
-    import lightop_b200 as lo
-    from torch.cuda import green_contexts
-    if not green_contexts.SUPPORTED:
-        pytest.skip("torch without green contexts")
-    g = torch.Generator(device=DEV).manual_seed(6)
-    x = torch.randn(1000, 7168, generator=g, device=DEV).to(torch.bfloat16)
-    w, w_s = _int8(g, 34 * 128, 7168), torch.rand(34, 56, generator=g, device=DEV) * 9e-3 + 1e-3
-    want = lo.gemm_ops.apply_w8a8_block_int8_linear(x, w, [128, 128], w_s)
-    torch.cuda.synchronize()
-    part = green_contexts.GreenContext.create(sms, 0)
-    part.set_context()
-    try:
-        with _Pairs(1):
-            got = lo.gemm_ops.apply_w8a8_block_int8_linear(x, w, [128, 128], w_s)
-        torch.cuda.synchronize()
-    finally:
-        part.pop_context()
-    lo.check_device_status()
-    assert torch.equal(got, want)
