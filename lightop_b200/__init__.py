@@ -19,6 +19,14 @@ _lib.load()
 _status_words = {}
 
 
+def _has_memory(t: torch.Tensor) -> bool:
+    """False for what a tracer or a transform (fake tensors, torch.func) hands out in place of memory: of no use to the calls after it."""
+    try:
+        return type(t) is torch.Tensor and t.data_ptr() != 0
+    except RuntimeError:
+        return False
+
+
 def device_status_word(device) -> torch.Tensor:
     """Per-device int32 word that kernels set when one of their bounded waits ran out."""
     idx = device.index if isinstance(device, torch.device) else torch.device(device).index
@@ -27,7 +35,8 @@ def device_status_word(device) -> torch.Tensor:
     w = _status_words.get(idx)
     if w is None:
         w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status_words[idx] = w
+        if _has_memory(w):
+            _status_words[idx] = w
     return w
 
 
