@@ -68,7 +68,9 @@ FusedLayout carve_fused(void *ws, int64_t M, int num_experts_for_align, int topk
 //   176 .. 232            : 128-row chunks: nearly every expert has two chunks with either cap, and the narrower ones have the deeper rings.
 //                           128 / 160 rows, even routing: Qwen3 168 rows 1028 / 1003, 176 1052 / 1066, 184 1067 / 1106, 216 1190 / 1233, 232 1234 /
 //                           1265, 240 1253 / 1255; 7168 tokens of a shard with 32 experts (224) 719 / 743, 5376 (168) 610 / 612, 8192 (256) 828 / 789;
-//                           Zipf 176 1012 / 1023, 224 1238 / 1197
+//                           Zipf 176 1012 / 1023, 224 1238 / 1197.  On single CTAs (odd tile counts, small layers) the same: 32 experts of 1024 x 384
+//                           176 rows 55.4 / 59.6, 200 56.2 / 57.8, 232 59.5 / 61.2, Zipf 200 59.2 / 63.6; 64 of 4224 x 1408 184 500 / 532, 200 533 / 568, 232
+//                           575 / 583, Zipf 216 606 / 596; 16 of 7296 x 1920 200 320 / 329, 232 342 / 344, Zipf 200 331 / 315, 232 348 / 366
 //   otherwise >= 120      : 160-row chunks: with 128 rows per expert half of the experts have a few rows more than 128, and a
 //                           second chunk means a second pass over the expert's weights (256 rows: 1374 / 1313, Zipf 1368 / 1322).
 constexpr int CHUNK_ROWS = 128;
